@@ -20,7 +20,7 @@ Metric: sample-timesteps/s = samples x steps / seconds, whole job.
   t, passed to the step kernel as a launch argument, 8 bytes) then ``Solve(t, dt)``,
   then ``Norms(out=pinned)`` -- the FP64 per-sample norms and the non-finite
   watchdog read back into pinned host memory, which synchronises every step.  The
-  solver runs with ``norms_every = 1``: the persistent fan kernel accumulates the norms
+  solver runs with ``norms_every = 1``: the patch kernel accumulates the norms
   while it writes the new state, so they cost no second pass over the state
   (``--separate-norms``: the separate pass instead).
 * ``adjoint`` (default line): forward + adjoint gradient evaluations of the
@@ -277,7 +277,7 @@ def gpu_main(args, case, rank, world, local, dev):
     from cvfes_b200 import _lib
     variant = _lib.get_step_tuning(prec)["staged"]
     kernel = {0: "k_step", 1: "k_step_staged", 2: "k_step_gather", 3: "k_step_fan",
-              4: "k_step_pipe", 5: "k_step_burst", 6: "k_step_fanp", 7: "k_step_tile",
+              4: "k_step_pipe", 5: "k_step_burst", 6: "k_step_patch", 7: "k_step_tile",
               8: "k_step_fan (two ahead)"}.get(variant, str(variant))
     K, W = args.steps, args.warmup
     pres = torch.from_numpy(case.pressures(W + K)).to(dev)

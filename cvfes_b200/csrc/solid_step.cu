@@ -341,249 +341,6 @@ __global__ void __launch_bounds__(256, MINB) k_step_fan(StepArgs<T> A) {
     step_epilogue<T, V>(A, a, S, col, row, ua, acc, f);
 }
 
-// ------------------------------------------------------------ persistent fan step
-// The fan kernel as a persistent grid: each block walks work items (node block, sample
-// chunk; chunk fastest) with a stride of the grid, and stages the slot records and
-// stiffness rows of its NEXT item by TMA into the other of two shared-memory stages
-// while the warps multiply the current one, so the per-item staging latency is off the
-// critical path.  Stage s of the block's i-th item completes its mbarrier's phase
-// (i / 2) % 2; a block barrier at the end of every item frees the stage for reuse.
-template <typename T>
-__device__ __forceinline__ void fanp_issue(const StepArgs<T>& A, long long w, uint32_t bar,
-                                           int4* srec, T* sslab) {
-    const long long nb = w / A.nch;
-    const long long a0 = nb * A.npb;
-    const long long a1 = (a0 + A.npb < A.n_nodes) ? a0 + A.npb : A.n_nodes;
-    const int kb = __ldg(A.node_ptr + a0), ke = __ldg(A.node_ptr + a1);
-    const int nsl = ke - kb;
-    if (nsl > A.cap_slots || nsl <= 0) {
-        if (nsl > A.cap_slots && A.status) atomicOr(A.status, 2);
-        mbar_arrive_expect_tx(bar, 0);
-        return;
-    }
-    const uint32_t b_rec = (uint32_t)nsl * 16u;
-    const uint32_t b_slab = (uint32_t)nsl * (uint32_t)(kSlabStride * sizeof(T));
-    mbar_arrive_expect_tx(bar, b_rec + b_slab);
-    bulk_g2s(smem_u32(srec), A.rec + kb, b_rec, bar);
-    bulk_g2s(smem_u32(sslab), A.slab + (size_t)kb * kSlabStride, b_slab, bar);
-}
-
-// With A.norm_part (fused norms, shared-memory mode) the grid is a multiple of nch, so
-// block b always has sample chunk b % nch; its per-lane FP64 sums follow the two stages
-// in shared memory.  Without norms this is the plain persistent step.
-template <typename T, int V, bool DIFF, int MINB>
-__global__ void __launch_bounds__(256, MINB) k_step_fanp(StepArgs<T> A, long long n_items) {
-    extern __shared__ __align__(16) unsigned char smem[];
-    const int warp = threadIdx.x >> 5;
-    const int lane = threadIdx.x & 31;
-    const size_t stage_bytes = (size_t)A.cap_slots * (16 + kSlabStride * sizeof(T));
-    // stage q: barrier at smem + 8q, records then stiffness rows at smem + 16 + q * stage_bytes
-    const uint32_t bar0 = smem_u32(smem);
-    int4* const srec0 = reinterpret_cast<int4*>(smem + 16);
-    T* const sslab0 = reinterpret_cast<T*>(smem + 16 + (size_t)A.cap_slots * 16);
-    constexpr int kAcc = 4 * V * 32;  // doubles of one warp's norm accumulators
-    double* const nbase = reinterpret_cast<double*>(smem + 16 + 2 * stage_bytes);
-    double* const nacc = A.norm_part ? nbase + warp * kAcc + lane : nullptr;
-    if (nacc) {
-#pragma unroll
-        for (int q = 0; q < 4 * V; ++q) nacc[q * 32] = 0.0;
-    }
-    if (threadIdx.x == 0) {
-        mbar_init(bar0, 1);
-        mbar_init(bar0 + 8, 1);
-    }
-    __syncthreads();
-    long long w = blockIdx.x;
-    if (threadIdx.x == 0 && w < n_items) fanp_issue<T>(A, w, bar0, srec0, sslab0);
-    const size_t S = (size_t)A.S;
-    const T p = step_pressure<T>(A);
-    for (int it = 0; w < n_items; w += gridDim.x, ++it) {
-        const int sg = it & 1;
-        const long long wn = w + gridDim.x;
-        if (threadIdx.x == 0 && wn < n_items)
-            fanp_issue<T>(A, wn, bar0 + 8 * (sg ^ 1), stage_rec(srec0, stage_bytes, sg ^ 1), stage_slab(sslab0, stage_bytes, sg ^ 1));
-        const long long nb = w / A.nch;
-        const int chunk = (int)(w - nb * A.nch);
-        const long long a0 = nb * A.npb;
-        const long long a1 = (a0 + A.npb < A.n_nodes) ? a0 + A.npb : A.n_nodes;
-        const long long a = a0 + warp;
-        const bool active = warp < A.npb && a < a1;
-        const size_t col = ((size_t)chunk * 32 + lane) * V;
-        const size_t row = (size_t)a * 3 * S + col;
-        const bool clamped = a < A.n_clamped;
-        Vec<T, V> ua[3];
-        T f[3];
-        if (active && !clamped) {
-#pragma unroll
-            for (int d = 0; d < 3; ++d) {
-                ua[d] = ldg<T, V>(A.u + row + d * S);
-                prefetch_l2(A.up + row + d * S);
-            }
-            prefetch_l2(A.invm + (size_t)a * S + col);
-            node_load<T>(A, a, p, f);
-        }
-        // No L2 prefetch ahead here: the prefetching warp's dependent slot-record loads
-        // hold its whole block at the item barrier (measured 2.466 -> 3.579 ms/step on the
-        // 256x1024 tube with it; node rows alone 3.06 ms).
-        if (!mbar_wait_bounded(bar0 + 8 * sg, (uint32_t)((it >> 1) & 1), kMaxPolls)) {
-            if (lane == 0 && A.status) atomicOr(A.status, 1);
-            return;
-        }
-        if (active) {
-            if (clamped) {
-                clamp_store<T, V>(A, S, row, nacc, a, col);
-            } else {
-                const int kb = __ldg(A.node_ptr + a0);
-                const int k0 = __ldg(A.node_ptr + a) - kb, k1 = __ldg(A.node_ptr + a + 1) - kb;
-                Vec<T, V> acc[3];
-                ku_row_fan<T, V, DIFF>(stage_rec(srec0, stage_bytes, sg),
-                                       stage_slab(sslab0, stage_bytes, sg), k0, k1, A.u, A.coef,
-                                       S, col, ua, acc);
-                step_epilogue<T, V>(A, a, S, col, row, ua, acc, f, nacc);
-            }
-        }
-        __syncthreads();
-    }
-    if (A.norm_part) {  // this block's sums over its nodes, warps added in order
-        const int chunk = (int)(blockIdx.x % A.nch);
-        const long long prow = blockIdx.x / A.nch;
-        for (int t = threadIdx.x; t < kAcc; t += blockDim.x) {
-            const int q = t / (32 * V), c = t - q * 32 * V;  // c: sample of the chunk
-            const int ln = c / V, i = c - ln * V;
-            double sum = 0.0;
-            for (int w = 0; w < A.npb; ++w) sum += nbase[w * kAcc + (q * V + i) * 32 + ln];
-            A.norm_part[((size_t)prow * S + (size_t)chunk * 32 * V + c) * 4 + q] = sum;
-        }
-    }
-}
-
-// The persistent step with the norms fused in (tensor-memory mode, the default): the
-// grid is a multiple of nch, so block b always has sample chunk b % nch; each lane adds
-// its nodes' terms to FP64 sums in tensor memory (norms_add), and at its end the block
-// writes one row of partial sums, its warps added in order.  A kernel of its own: the
-// plain step without any tensor-memory instruction is 6% faster (2.30 against 2.44
-// ms/step on the 256x1024 tube, and 7.2 against 8.1 ms for 500 steps of the 64x128
-// tube).  Every wait is bounded: a wait that gives up sets status bit 0, the block stops
-// after the item (all warps leave the loop together), waits with a bound for the copies
-// it issued, frees its tensor memory and returns.
-template <typename T, int V, bool DIFF, int MINB>
-__global__ void __launch_bounds__(256, MINB) k_step_fanp_tm(StepArgs<T> A, long long n_items) {
-    extern __shared__ __align__(16) unsigned char smem[];
-    __shared__ uint32_t tmem_slot;
-    __shared__ int stop;
-    const int warp = threadIdx.x >> 5;
-    const int lane = threadIdx.x & 31;
-    const size_t stage_bytes = (size_t)A.cap_slots * (16 + kSlabStride * sizeof(T));
-    // stage q: barrier at smem + 8q, records then stiffness rows at smem + 16 + q * stage_bytes
-    const uint32_t bar0 = smem_u32(smem);
-    int4* const srec0 = reinterpret_cast<int4*>(smem + 16);
-    T* const sslab0 = reinterpret_cast<T*>(smem + 16 + (size_t)A.cap_slots * 16);
-    const uint32_t tcols = blockDim.x > 128 ? 64u : 32u;
-    if (warp == 0) {
-        tmem_alloc(&tmem_slot, tcols);
-        tmem_relinquish();
-    }
-    if (threadIdx.x == 0) {
-        mbar_init(bar0, 1);
-        mbar_init(bar0 + 8, 1);
-        stop = 0;
-    }
-    tmem_fence_before_sync();
-    __syncthreads();
-    tmem_fence_after_sync();
-    // this lane's TMEM row: the warp's lane quarter and, above 4 warps, the second 32 columns
-    const uint32_t tm =
-        tmem_slot + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)(warp >> 2) * 32u;
-    norms_zero<V>(tm);
-    long long w = blockIdx.x;
-    if (threadIdx.x == 0 && w < n_items) fanp_issue<T>(A, w, bar0, srec0, sslab0);
-    const size_t S = (size_t)A.S;
-    const T p = step_pressure<T>(A);
-    int stop_it = 0;  // the item at which a wait gave up
-    for (int it = 0; w < n_items; w += gridDim.x, ++it) {
-        const int sg = it & 1;
-        const long long wn = w + gridDim.x;
-        if (threadIdx.x == 0 && wn < n_items)
-            fanp_issue<T>(A, wn, bar0 + 8 * (sg ^ 1), stage_rec(srec0, stage_bytes, sg ^ 1), stage_slab(sslab0, stage_bytes, sg ^ 1));
-        const long long nb = w / A.nch;
-        const int chunk = (int)(w - nb * A.nch);
-        const long long a0 = nb * A.npb;
-        const long long a1 = (a0 + A.npb < A.n_nodes) ? a0 + A.npb : A.n_nodes;
-        const long long a = a0 + warp;
-        const bool active = warp < A.npb && a < a1;
-        const size_t col = ((size_t)chunk * 32 + lane) * V;
-        const size_t row = (size_t)a * 3 * S + col;
-        const bool clamped = a < A.n_clamped;
-        Vec<T, V> ua[3];
-        T f[3];
-        if (active && !clamped) {
-#pragma unroll
-            for (int d = 0; d < 3; ++d) {
-                ua[d] = ldg<T, V>(A.u + row + d * S);
-                prefetch_l2(A.up + row + d * S);
-            }
-            prefetch_l2(A.invm + (size_t)a * S + col);
-            node_load<T>(A, a, p, f);
-        }
-        // No L2 prefetch ahead here: the prefetching warp's dependent slot-record loads
-        // hold its whole block at the item barrier (measured 2.466 -> 3.579 ms/step on the
-        // 256x1024 tube with it; node rows alone 3.06 ms).
-        // warp-uniform, so that the tensor-memory accesses of the epilogue stay converged;
-        // a wait that gives up stops the whole block after this item
-        const bool ready = __all_sync(
-            0xffffffffu, mbar_wait_bounded(bar0 + 8 * sg, (uint32_t)((it >> 1) & 1), kMaxPolls));
-        if (!ready && lane == 0) {
-            if (A.status) atomicOr(A.status, 1);
-            stop = 1;
-        }
-        if (ready && active) {
-            if (clamped) {
-                clamp_store_tm<T, V>(A, S, row, tm, a, col);
-            } else {
-                const int kb = __ldg(A.node_ptr + a0);
-                const int k0 = __ldg(A.node_ptr + a) - kb, k1 = __ldg(A.node_ptr + a + 1) - kb;
-                Vec<T, V> acc[3];
-                ku_row_fan<T, V, DIFF>(stage_rec(srec0, stage_bytes, sg),
-                                       stage_slab(sslab0, stage_bytes, sg), k0, k1, A.u, A.coef,
-                                       S, col, ua, acc);
-                step_epilogue_tm<T, V>(A, a, S, col, row, ua, acc, f, tm);
-            }
-        }
-        __syncthreads();
-        if (*(volatile int*)&stop) {
-            stop_it = it;
-            break;
-        }
-    }
-    if (*(volatile int*)&stop && threadIdx.x == 0) {
-        // the copies still in flight into this block's stages: the timed-out one and the
-        // one issued for the next item
-        const int sg = stop_it & 1;
-        mbar_wait_bounded(bar0 + 8 * sg, (uint32_t)((stop_it >> 1) & 1), kMaxPolls);
-        if (w + gridDim.x < n_items)
-            mbar_wait_bounded(bar0 + 8 * (sg ^ 1), (uint32_t)(((stop_it + 1) >> 1) & 1),
-                              kMaxPolls);
-    }
-    // this block's sums over its nodes, warps added in order, in the (idle) stage memory
-    double* const scr = reinterpret_cast<double*>(smem + 16);
-    for (int wv = 0; wv < A.npb; ++wv) {
-        if (warp == wv) norms_fold<V>(tm, scr + lane, wv == 0);
-        __syncthreads();
-    }
-    const int chunk = (int)(blockIdx.x % A.nch);
-    const long long prow = blockIdx.x / A.nch;
-    for (int t = threadIdx.x; t < 4 * V * 32; t += blockDim.x) {
-        const int q = t / (32 * V), c = t - q * 32 * V;  // c: sample of the chunk
-        const int ln = c / V, i = c - ln * V;
-        A.norm_part[((size_t)prow * S + (size_t)chunk * 32 * V + c) * 4 + q] =
-            scr[(q * V + i) * 32 + ln];
-    }
-    tmem_fence_before_sync();
-    __syncthreads();
-    tmem_fence_after_sync();
-    if (warp == 0) tmem_dealloc(tmem_slot, tcols);
-}
-
 // ------------------------------------------------------------ burst-gather step
 // As k_step_fan (TMA-staged slot rows, a warp per node and sample chunk), but every
 // neighbour row of the node and every element coefficient row is requested at once,
@@ -1184,13 +941,10 @@ struct StepTuning {
     int staged;
     int minb;  // minimum resident blocks per SM asked of the compiler (register cap)
 };
-// Defaults from sweeps on the 256x1024 tube with 512 samples (B200), ms/step:
-// FP32 (velocity-state form): persistent fan 2.441 (4 nodes per block), 2.445 (2), 2.562
-// (3), fan 2.606 (2), 2.598 (4), fan with loads two elements ahead 2.637; FP64: fan 5.750,
-// persistent fan 6.088 (2 nodes per block), two ahead 5.981; on another box with the
-// final kernels, FP64 persistent fan with 4 nodes per block 5.421 against the fan's 5.821
-// (1 sample per thread at 3 blocks' registers: 6.47 to 8.07).  2 blocks per SM worth of
-// registers.
+// Defaults: variant 6 (solid_patch.cu, solid_group.cu).  256x512 tube, us a step: FP32
+// (velocity form, 256 samples) patch 385 against the fan's 600; FP64 (64 samples) 228
+// against 360.  Sweep of the others on the 256x1024 tube, 512 samples, ms a step: FP32 fan
+// 2.606 (2 nodes a block), 2.598 (4), loads two elements ahead 2.637; FP64 5.750, 5.981.
 static StepTuning g_tune32 = {4, 4, 6, 2};
 static StepTuning g_tune64 = {2, 4, 6, 2};
 // L2 prefetch of the fan kernels: distance in nodes (-1: the mesh's bandwidth + 128;
@@ -1295,7 +1049,7 @@ int fanp_blocks_per_sm(const void* kernel, int threads, size_t smem, int* per_sm
         size_t smem;
         int per_sm;
     };
-    static Entry cache[32];
+    static Entry cache[64];
     static int n_cache = 0;
     static std::mutex mu;
     int dev = 0;
@@ -1307,18 +1061,24 @@ int fanp_blocks_per_sm(const void* kernel, int threads, size_t smem, int* per_sm
             *per_sm = cache[i].per_sm;
             return CVFES_OK;
         }
-    if (smem > 48 * 1024) {
-        cudaError_t e =
-            cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        if (e != cudaSuccess)
-            return fail(CVFES_ERR_CUDA, "k_step_fanp smem attribute: %s", cudaGetErrorString(e));
-    }
     // From the kernel's registers and shared memory against the SM's budgets.  Not the
     // occupancy calculator: it reports one block per SM for a kernel that contains a
     // tensor-memory allocation, whose blocks here give up their allocation permit at
     // their start and hold 32 or 64 of the SM's 512 columns only when the norms are fused.
     cudaFuncAttributes fa;
     CVFES_CUDA_TRY(cudaFuncGetAttributes(&fa, kernel));
+    if (smem > 48 * 1024) {
+        // allow all that a block may have, not this launch's bytes: a later entry with fewer
+        // would take the allowance back from the ones already cached
+        int optin = 0;
+        CVFES_CUDA_TRY(
+            cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
+        cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                             optin - (int)fa.sharedSizeBytes);
+        if (e != cudaSuccess)
+            return fail(CVFES_ERR_CUDA, "persistent kernel smem attribute: %s",
+                        cudaGetErrorString(e));
+    }
     int regs_sm = 0, smem_sm = 0, reserved = 0, thr_sm = 0, blk_sm = 0;
     CVFES_CUDA_TRY(cudaDeviceGetAttribute(&regs_sm, cudaDevAttrMaxRegistersPerMultiprocessor, dev));
     CVFES_CUDA_TRY(
@@ -1336,67 +1096,15 @@ int fanp_blocks_per_sm(const void* kernel, int threads, size_t smem, int* per_sm
     const int by_smem = (int)((size_t)smem_sm / per_block);
     const int by_thr = thr_sm / (32 * warps);
     const int n = std::min(std::min(by_regs, by_smem), std::min(by_thr, blk_sm));
-    if (n <= 0) return fail(CVFES_ERR_CUDA, "k_step_fanp: no resident block fits");
-    if (n_cache < 32) cache[n_cache++] = Entry{kernel, dev, threads, smem, n};
+    if (n <= 0) return fail(CVFES_ERR_CUDA, "persistent kernel: no resident block fits");
+    if (n_cache < 64) cache[n_cache++] = Entry{kernel, dev, threads, smem, n};
     *per_sm = n;
     return CVFES_OK;
 }
 
-// Where the fused norms keep their sums: 0 tensor memory (k_step_fanp_tm), 1 shared memory
-// (k_step_fanp).  Both give bitwise the same norms.
+// Where the fused norms keep their sums: 0 tensor memory, 1 shared memory (two instances of
+// the patch kernel).  Both give bitwise the same norms.
 static std::atomic<int> g_norms_mode{0};
-
-// The persistent fan kernel on as many blocks as are resident (at most one per work
-// item).  With fused norms the grid is rounded down to a multiple of the sample chunks
-// and capped at max_rows chunks' worth, and *rows gets the partial rows written.
-template <typename K, typename T>
-int launch_fanp_k(K kernel, long long n_items, int threads, size_t smem, cudaStream_t st,
-                  const StepArgs<T>& A, long long max_rows, long long* rows) {
-    int per_sm = 0;
-    const int rc = fanp_blocks_per_sm(reinterpret_cast<const void*>(kernel), threads, smem,
-                                      &per_sm);
-    if (rc) return rc;
-    // fused norms in tensor memory: each block holds 32 columns (64 above 4 warps), and
-    // a block waits in its allocation until the SM's 512 columns have room
-    if (A.norm_part && g_norms_mode.load() == 0) {
-        const int cap = threads > 128 ? 8 : 16;
-        if (per_sm > cap) per_sm = cap;
-    }
-    long long blocks = (long long)per_sm * sm_count();
-    if (blocks > n_items) blocks = n_items;
-    if (A.norm_part) {
-        if (blocks > max_rows * A.nch) blocks = max_rows * A.nch;
-        blocks -= blocks % A.nch;
-        if (blocks < A.nch) blocks = A.nch;
-        if (rows) *rows = blocks / A.nch;
-    }
-    kernel<<<(unsigned)blocks, threads, smem, st>>>(A, n_items);
-    CVFES_LAUNCH_CHECK("k_step_fanp");
-    return CVFES_OK;
-}
-
-template <typename T, int V, bool DIFF>
-int launch_fanp(int minb, long long n_items, int threads, size_t smem, cudaStream_t st,
-                const StepArgs<T>& A, long long max_rows = 0, long long* rows = nullptr) {
-#define CVFES_FANP_K(K, MB) launch_fanp_k(K<T, V, DIFF, MB>, n_items, threads, smem, st, A, max_rows, rows)
-#define CVFES_FANP(K)                                   \
-    switch (minb) {                                     \
-        case 4: return CVFES_FANP_K(K, 4);              \
-        case 3: return CVFES_FANP_K(K, 3);              \
-        case 2: return CVFES_FANP_K(K, 2);              \
-        default: return CVFES_FANP_K(K, 1);             \
-    }
-    if (A.norm_part && g_norms_mode.load() == 0) {
-        // the block's sums are added up in the (idle) stage memory at its end
-        const size_t scratch = 16 + (size_t)4 * V * 32 * sizeof(double);
-        if (smem < scratch) smem = scratch;
-        CVFES_FANP(k_step_fanp_tm)
-    }
-    if (A.norm_part) smem += (size_t)A.npb * 4 * V * 32 * sizeof(double);
-    CVFES_FANP(k_step_fanp)
-#undef CVFES_FANP
-#undef CVFES_FANP_K
-}
 
 template <typename T, int V, bool DIFF, int MAXD>
 int launch_burst(int minb, dim3 g1, int threads, size_t smem, cudaStream_t st,
@@ -1412,11 +1120,6 @@ int launch_burst(int minb, dim3 g1, int threads, size_t smem, cudaStream_t st,
 template <typename T, int V, bool DIFF>
 int launch_staged_v(int variant, int minb, dim3 grid, int threads, size_t smem, cudaStream_t st,
                     const StepArgs<T>& A, long long max_degree = 0) {
-    if (variant == 6) {
-        const long long n_items = (long long)grid.x * grid.y;
-        const size_t smem2 = 16 + 2 * (smem - 16);
-        return launch_fanp<T, V, DIFF>(minb, n_items, threads, smem2, st, A);
-    }
     if (variant == 5 && max_degree > 0 && max_degree <= 8) {
         const dim3 g1((unsigned)((long long)grid.x * grid.y));
         if (max_degree <= 6) return launch_burst<T, V, DIFF, 6>(minb, g1, threads, smem, st, A);
@@ -1456,14 +1159,16 @@ int launch_staged_v(int variant, int minb, dim3 grid, int threads, size_t smem, 
 }
 
 // norm_work (optional): fuse the per-sample norms of the new state into the step (the
-// persistent fan kernel); *norm_rows gets the partial rows written to norm_work, or 0
-// when the shape has no fused kernel (the caller then runs the separate norms pass).
+// patch kernel); *norm_rows gets the partial rows written to norm_work, or 0 when the
+// shape has no fused kernel (the caller then runs the separate norms pass).
+// after_step: the launch before this one on the stream is a step of the same mesh, so
+// this one may start under its tail (programmatic dependent launch).
 template <typename T>
 int launch_step(const cvfes_solid_mesh* m, const T* coef, const T* invm, const T* u,
                 const T* up, T* un, const double* p_sched, const long long* clock, long long j,
                 double pressure, const T* trac, double dt, double damp, cudaStream_t st,
                 double* norm_work = nullptr, long long* norm_rows = nullptr,
-                long long max_rows = 0) {
+                long long max_rows = 0, bool after_step = false) {
     if (norm_rows) *norm_rows = 0;
     int rc = check_mesh(m, "cvfes_solid_step");
     if (rc) return rc;
@@ -1530,6 +1235,18 @@ int launch_step(const cvfes_solid_mesh* m, const T* coef, const T* invm, const T
     int V = pick_vec<T>(ptrs, 5, A.S);
     while (V > tune.vec) V /= 2;
     constexpr bool DIFF = std::is_same<T, float>::value;
+    const bool fused = norm_work && max_rows > 0 && !A.probe_polls;
+    if (tune.staged == 6 || fused) {
+        if (fused) A.norm_part = norm_work;
+        const int prc = launch_step_patch<T>(m, A, V, after_step, st, g_norms_mode.load(),
+                                             max_rows, norm_rows);
+        if (prc <= 0) return prc;
+        A.norm_part = nullptr;
+        if (tune.staged == 6) {
+            tune.staged = 3;
+            tune.minb = 2;
+        }
+    }
     // The warp-per-node kernels need S/V to be a multiple of 32: narrow the sample
     // vector to make it so (S = 64 with 4 per thread -> 2 per thread), else they fall
     // back to the row-gather kernel at the original width.
@@ -1578,22 +1295,6 @@ int launch_step(const cvfes_solid_mesh* m, const T* coef, const T* invm, const T
         A.pf_parts = prefetch_parts(A.pf_parts, A.nch);
         const dim3 grid((unsigned)((m->n_nodes + A.npb - 1) / A.npb), (unsigned)(A.S / V / 32));
         const int threads = 32 * A.npb;
-        if (norm_work && max_rows > 0 && !A.probe_polls) {  // fused norms: persistent fan
-            A.norm_part = norm_work;
-            const long long n_items = (long long)grid.x * grid.y;
-            const size_t smem2 = 16 + 2 * (smem - 16);
-            const int minb = tune.staged == 6 ? tune.minb : 2;
-            if (V == 4) {
-                if constexpr (sizeof(T) == 4)
-                    return launch_fanp<T, 4, DIFF>(minb, n_items, threads, smem2, st, A, max_rows,
-                                                   norm_rows);
-            } else if (V == 2) {
-                return launch_fanp<T, 2, DIFF>(minb, n_items, threads, smem2, st, A, max_rows,
-                                               norm_rows);
-            }
-            return launch_fanp<T, 1, DIFF>(minb, n_items, threads, smem2, st, A, max_rows,
-                                           norm_rows);
-        }
         if (V == 4) {
             if constexpr (sizeof(T) == 4)
                 rc = launch_staged_v<T, 4, DIFF>(tune.staged, tune.minb, grid, threads, smem, st,
@@ -1668,7 +1369,7 @@ int launch_advance(const cvfes_solid_mesh* m, const T* coef, const T* invm, T* b
     const bool vel = m && m->state_form == 1;
     for (long long j = 0; j < n_steps; ++j) {
         int rc = launch_step<T>(m, coef, invm, buf[cur], buf[prev], buf[nxt], p_sched, clock, j,
-                                0.0, nullptr, dt, damp, st);
+                                0.0, nullptr, dt, damp, st, nullptr, nullptr, 0, j > 0);
         if (rc) return rc;
         if (vel) {  // the increment stays in place; the displacement buffers swap
             const int t = cur;

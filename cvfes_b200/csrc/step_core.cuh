@@ -55,11 +55,11 @@ struct StepArgs {
     // polls: the wait gives up with nothing in flight, the kernel records bit 0 in
     // `status` and returns without writing the step.
     int probe_polls = 0;
-    // Fused per-sample norms (persistent fan kernel only; null: off).  Each block keeps
-    // one sample chunk for its whole life and accumulates, per lane and sample, the FP64
-    // sums of u_{n+1}^2, du^2, m du^2 and the non-finite count of u_{n+1} over all its
-    // nodes in shared memory; at its end it writes them to row blockIdx.x / nch of
-    // norm_part [rows][S][4], which k_norms_final then sums in row order.
+    // Fused per-sample norms (patch kernel only; null: off).  Each block keeps one sample
+    // chunk for its whole life and accumulates, per lane and sample, the FP64 sums of
+    // u_{n+1}^2, du^2, m du^2 and the non-finite count of u_{n+1} over all its nodes; at
+    // its end it writes them to row blockIdx.x / nch of norm_part [rows][S][4], which
+    // k_norms_final then sums in row order.
     double* norm_part = nullptr;
     // Damping per dof (the OpenCL class's calc_u): eta = dt damp / m per row, w = dt^2 / m.
     // Off: mass-proportional damping, one eta for all rows.  Set: A.eta holds dt damp.
@@ -103,8 +103,8 @@ __device__ __forceinline__ void tmem_alloc(uint32_t* slot, uint32_t cols) {  // 
                  ::"r"((uint32_t)__cvta_generic_to_shared(slot)), "r"(cols) : "memory");
 }
 // The block allocates no more tensor memory.  A kernel that contains an allocation gets
-// further blocks on an SM only after its resident blocks have said so (measured on the
-// persistent fan kernel: one block per SM otherwise), so every block says it, whether it
+// further blocks on an SM only after its resident blocks have said so (measured: one block
+// per SM otherwise), so every block says it, whether it
 // allocated or not.
 __device__ __forceinline__ void tmem_relinquish() {  // warp-wide
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
@@ -515,54 +515,22 @@ __device__ __forceinline__ void step_update(const StepArgs<T>& A, size_t S, size
 }
 
 // Dirichlet row: u_{n+1} = clamp; in the velocity-state form also v_{n+1} = clamp - u_n.
-// With nacc (fused norms) the row's contributions are added there.
 template <typename T, int V>
-__device__ __forceinline__ void clamp_store(const StepArgs<T>& A, size_t S, size_t row,
-                                            double* nacc = nullptr, long long a = 0,
-                                            size_t col = 0) {
+__device__ __forceinline__ void clamp_store(const StepArgs<T>& A, size_t S, size_t row) {
     const Vec<T, V> cl = vfill<T, V>(A.clamp);
-    T su[V], sv[V];
-    int nf[V];
-#pragma unroll
-    for (int i = 0; i < V; ++i) {
-        su[i] = sv[i] = T(0);
-        nf[i] = 0;
-    }
 #pragma unroll
     for (int d = 0; d < 3; ++d) {
-        if (A.vel || nacc) {
-            const Vec<T, V> dv = vsub(cl, ldg<T, V>(A.u + row + d * S));
-            if (A.vel) stcs<T, V>(A.vel + row + d * S, dv);
-            if (nacc) {
-#pragma unroll
-                for (int i = 0; i < V; ++i) {
-                    su[i] = fma(cl.v[i], cl.v[i], su[i]);
-                    sv[i] = fma(dv.v[i], dv.v[i], sv[i]);
-                    nf[i] += isfinite(cl.v[i]) ? 0 : 1;
-                }
-            }
-        }
+        if (A.vel) stcs<T, V>(A.vel + row + d * S, vsub(cl, ldg<T, V>(A.u + row + d * S)));
         stcs<T, V>(A.un + row + d * S, cl);
     }
-    if (nacc) norms_add_smem<T, V>(nacc, ldcs<T, V>(A.invm + (size_t)a * S + col), su, sv, nf);
 }
 
 // As step_update, reading the row's u_{n-1} (or v_n) and inverse mass here.
-// With nacc (fused norms) the row's contributions to the per-sample sums of u_{n+1}^2,
-// du^2 (v_{n+1}^2, or u_{n+1} - u_n) and m du^2 are added there (node terms as norms_add).
 template <typename T, int V>
 __device__ __forceinline__ void step_epilogue(const StepArgs<T>& A, long long a, size_t S,
                                               size_t col, size_t row, const Vec<T, V> (&ua)[3],
-                                              const Vec<T, V> (&acc)[3], const T (&f)[3],
-                                              double* nacc = nullptr) {
+                                              const Vec<T, V> (&acc)[3], const T (&f)[3]) {
     const Vec<T, V> im = ldcs<T, V>(A.invm + (size_t)a * S + col);
-    T su[V], sv[V];
-    int nf[V];
-#pragma unroll
-    for (int i = 0; i < V; ++i) {
-        su[i] = sv[i] = T(0);
-        nf[i] = 0;
-    }
     if (A.vel) {
         // velocity-state form: v_{n+1} = v_n (1 - eta) + w (p f - K u_n), u_{n+1} = u_n + v_{n+1};
         // a row without mass (u_{n+1} = 0) keeps v_{n+1} = -u_n, the exact increment.
@@ -578,16 +546,10 @@ __device__ __forceinline__ void step_epilogue(const StepArgs<T>& A, long long a,
                 const bool live = im.v[i] != T(0);
                 o.v[i] = live ? ua[d].v[i] + v : T(0);
                 vn.v[i] = live ? v : -ua[d].v[i];
-                if (nacc) {
-                    su[i] = fma(o.v[i], o.v[i], su[i]);
-                    sv[i] = fma(vn.v[i], vn.v[i], sv[i]);
-                    nf[i] += isfinite(o.v[i]) ? 0 : 1;
-                }
             }
             stcs<T, V>(A.un + row + d * S, o);
             stcs<T, V>(A.vel + row + d * S, vn);
         }
-        if (nacc) norms_add_smem<T, V>(nacc, im, su, sv, nf);
         return;
     }
 #pragma unroll
@@ -601,107 +563,9 @@ __device__ __forceinline__ void step_epilogue(const StepArgs<T>& A, long long a,
             const T w = A.w0 * im.v[i];
             const T v = fma(w, load - acc[d].v[i], fma(-row_eta(A, im.v[i]), dv, dv));
             o.v[i] = (im.v[i] != T(0)) ? ua[d].v[i] + v : T(0);
-            if (nacc) {
-                const T du = o.v[i] - ua[d].v[i];
-                su[i] = fma(o.v[i], o.v[i], su[i]);
-                sv[i] = fma(du, du, sv[i]);
-                nf[i] += isfinite(o.v[i]) ? 0 : 1;
-            }
         }
         stcs<T, V>(A.un + row + d * S, o);
     }
-    if (nacc) norms_add_smem<T, V>(nacc, im, su, sv, nf);
-}
-
-// clamp_store and step_epilogue with the norms' sums in tensor memory at tm (norms_add),
-// for the persistent step with the norms fused in.  Copies, not one template over both
-// sinks: with one template the plain persistent step compiled to a schedule 3.5% slower
-// (2.376 against 2.295 ms/step on the 256x1024 tube, same box), although its norm code
-// never runs.
-template <typename T, int V>
-__device__ __forceinline__ void clamp_store_tm(const StepArgs<T>& A, size_t S, size_t row,
-                                               uint32_t tm, long long a, size_t col) {
-    const Vec<T, V> cl = vfill<T, V>(A.clamp);
-    T su[V], sv[V];
-    int nf[V];
-#pragma unroll
-    for (int i = 0; i < V; ++i) {
-        su[i] = sv[i] = T(0);
-        nf[i] = 0;
-    }
-#pragma unroll
-    for (int d = 0; d < 3; ++d) {
-        const Vec<T, V> dv = vsub(cl, ldg<T, V>(A.u + row + d * S));
-        if (A.vel) stcs<T, V>(A.vel + row + d * S, dv);
-#pragma unroll
-        for (int i = 0; i < V; ++i) {
-            su[i] = fma(cl.v[i], cl.v[i], su[i]);
-            sv[i] = fma(dv.v[i], dv.v[i], sv[i]);
-            nf[i] += isfinite(cl.v[i]) ? 0 : 1;
-        }
-        stcs<T, V>(A.un + row + d * S, cl);
-    }
-    norms_add<T, V>(tm, ldcs<T, V>(A.invm + (size_t)a * S + col), su, sv, nf);
-}
-
-// As step_update, reading the row's u_{n-1} (or v_n) and inverse mass here.
-template <typename T, int V>
-__device__ __forceinline__ void step_epilogue_tm(const StepArgs<T>& A, long long a, size_t S,
-                                                 size_t col, size_t row, const Vec<T, V> (&ua)[3],
-                                                 const Vec<T, V> (&acc)[3], const T (&f)[3],
-                                                 uint32_t tm) {
-    const Vec<T, V> im = ldcs<T, V>(A.invm + (size_t)a * S + col);
-    T su[V], sv[V];
-    int nf[V];
-#pragma unroll
-    for (int i = 0; i < V; ++i) {
-        su[i] = sv[i] = T(0);
-        nf[i] = 0;
-    }
-    if (A.vel) {
-        // velocity-state form: v_{n+1} = v_n (1 - eta) + w (p f - K u_n), u_{n+1} = u_n + v_{n+1};
-        // a row without mass (u_{n+1} = 0) keeps v_{n+1} = -u_n, the exact increment.
-#pragma unroll
-        for (int d = 0; d < 3; ++d) {
-            const Vec<T, V> vo = ldcs<T, V>(A.up + row + d * S);
-            const T load = f[d];
-            Vec<T, V> o, vn;
-#pragma unroll
-            for (int i = 0; i < V; ++i) {
-                const T w = A.w0 * im.v[i];
-                const T v = fma(w, load - acc[d].v[i], fma(-row_eta(A, im.v[i]), vo.v[i], vo.v[i]));
-                const bool live = im.v[i] != T(0);
-                o.v[i] = live ? ua[d].v[i] + v : T(0);
-                vn.v[i] = live ? v : -ua[d].v[i];
-                su[i] = fma(o.v[i], o.v[i], su[i]);
-                sv[i] = fma(vn.v[i], vn.v[i], sv[i]);
-                nf[i] += isfinite(o.v[i]) ? 0 : 1;
-            }
-            stcs<T, V>(A.un + row + d * S, o);
-            stcs<T, V>(A.vel + row + d * S, vn);
-        }
-        norms_add<T, V>(tm, im, su, sv, nf);
-        return;
-    }
-#pragma unroll
-    for (int d = 0; d < 3; ++d) {
-        const Vec<T, V> up = ldcs<T, V>(A.up + row + d * S);
-        const T load = f[d];
-        Vec<T, V> o;
-#pragma unroll
-        for (int i = 0; i < V; ++i) {
-            const T dv = ua[d].v[i] - up.v[i];
-            const T w = A.w0 * im.v[i];
-            const T v = fma(w, load - acc[d].v[i], fma(-row_eta(A, im.v[i]), dv, dv));
-            o.v[i] = (im.v[i] != T(0)) ? ua[d].v[i] + v : T(0);
-            const T du = o.v[i] - ua[d].v[i];
-            su[i] = fma(o.v[i], o.v[i], su[i]);
-            sv[i] = fma(du, du, sv[i]);
-            nf[i] += isfinite(o.v[i]) ? 0 : 1;
-        }
-        stcs<T, V>(A.un + row + d * S, o);
-    }
-    norms_add<T, V>(tm, im, su, sv, nf);
 }
 
 // ------------------------------------------------------------ fan-rotation row
@@ -878,10 +742,75 @@ __device__ __forceinline__ void prefetch_l1(const void* p) {
     asm volatile("prefetch.global.L1 [%0];" ::"l"(p));
 }
 
+// Row i of an array with this row length in bytes (one 32 x 32 -> 64 bit multiply-add).
+template <typename T>
+__device__ __forceinline__ const T* row_at(const T* base, int i, uint32_t stride_bytes) {
+    return reinterpret_cast<const T*>(reinterpret_cast<const char*>(base) +
+                                      (uint64_t)(uint32_t)i * stride_bytes);
+}
+template <typename T>
+__device__ __forceinline__ T* row_at(T* base, int i, uint32_t stride_bytes) {
+    return reinterpret_cast<T*>(reinterpret_cast<char*>(base) +
+                                (uint64_t)(uint32_t)i * stride_bytes);
+}
+
+// 16-byte words of one slot's stiffness row that the patch and group kernels stage.  FP32:
+// words 2..6 (the difference form does not read the self block, values 0..8); FP64: all 14.
+// kBytes: with the slot's record.
+template <typename T>
+struct SlotStage {
+    static constexpr int kFirst = sizeof(T) == 4 ? 2 : 0;
+    static constexpr int kWords = sizeof(T) == 4 ? 5 : 14;
+    static constexpr int kSlotBytes = 16 * kWords;
+    static constexpr size_t kBytes = 16 + kSlotBytes;
+};
+
+// Programmatic dependent launch: a kernel launched with after_step may start while the step
+// before it is still running; until grid_dependency_wait returns (that step has ended and
+// its writes are visible) it may read only what no step writes.  release lets the launch
+// after this one start; both do nothing in a kernel launched without the attribute.
+__device__ __forceinline__ void grid_dependency_wait() {
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+__device__ __forceinline__ void grid_dependency_release() {
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+template <typename... P, typename... Q>
+int launch_step_kernel(void (*kernel)(P...), long long blocks, int threads, size_t smem,
+                       bool after_step, cudaStream_t st, const char* name, const Q&... args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)blocks);
+    cfg.blockDim = dim3((unsigned)threads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = after_step ? 1 : 0;
+    const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, args...);
+    if (e != cudaSuccess) return fail(CVFES_ERR_CUDA, "%s: %s", name, cudaGetErrorString(e));
+    return CVFES_OK;
+}
+
 // Resident blocks per SM of a persistent kernel (solid_step.cu; cached per kernel,
 // device, block size and shared memory) and the device's SM count.
 int fanp_blocks_per_sm(const void* kernel, int threads, size_t smem, int* per_sm);
 int device_sm_count();
+
+// Patch-ordered persistent step (solid_patch.cu): returns 1 without launching when the mesh
+// has no max_degree or its slots do not fit the stages.  With A.norm_part set the norms
+// are fused in (norms_mode 0: sums in tensor memory, 1: in shared memory), at most max_rows
+// rows of partials, *rows written.  after_step: may start under the previous step's tail.
+template <typename T>
+int launch_step_patch(const cvfes_solid_mesh* m, StepArgs<T> A, int vec_max, bool after_step,
+                      cudaStream_t st, int norms_mode, long long max_rows, long long* rows);
+
+// Group step (solid_group.cu) for few samples: returns 1 without launching when there are
+// more, or a node has more slots than it holds.
+template <typename T>
+int launch_step_group(const cvfes_solid_mesh* m, StepArgs<T> A, int vec_max, bool after_step,
+                      cudaStream_t st);
 
 // TMA-tiled step (solid_tile.cu): returns 1 without launching when the mesh has no
 // tiling or the shape does not fit the tiled kernel.

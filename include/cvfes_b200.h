@@ -85,8 +85,8 @@ typedef struct cvfes_solid_mesh {
                                      calc_ddu, physicsSolverSDampGPUs.cl:398-429) */
 } cvfes_solid_mesh;
 
-/* Step-kernel tuning (the autotuner sets these; defaults: variant 6 with 4 nodes per
- * block, vec 4 for FP32 and 2 for FP64; minb 2).
+/* Step-kernel tuning (the autotuner sets these; defaults: variant 6, vec 4 for FP32 and
+ * 2 for FP64).
  *   precision 32 | 64;  vec: samples per thread (FP32 1|2|4, FP64 1|2);
  *   npb: nodes per block when a warp owns one node (1..8, one warp each);
  *   staged: 0 = slot records, stiffness rows and gathers read through L1;
@@ -102,8 +102,12 @@ typedef struct cvfes_solid_mesh {
  *           5 = as 1, with the node's whole gather (every neighbour row and
  *               coefficient row) requested before the first product (meshes of
  *               node degree <= 8; otherwise as 3);
- *           6 = as 3, persistent, the next work item's slot rows staged while the
- *               current one is multiplied (two shared-memory stages);
+ *           6 = persistent patch kernel: free-running warps, a 4 x 4 patch of nodes per
+ *               block, the next node's slots staged and its rows prefetched into L2 while
+ *               the current one is multiplied; with few samples (at most 32 FP32, 20
+ *               FP64) the group kernel, several nodes to a warp and the whole gather in
+ *               flight at once.  Any S; npb and minb have no effect (as 3 when a node has
+ *               more slots than the stages hold, or max_degree is unknown);
  *           7 = TMA-tiled: a block owns a strip of tile_p nodes and one sample chunk
  *               (64 FP32 / 32 FP64 samples); 2D TMA tensor copies stage the strip's
  *               node windows (all neighbour rows) and element windows (coefficient
@@ -149,8 +153,7 @@ int cvfes_get_step_prefetch(int32_t precision, int32_t* distance, int32_t* parts
 int cvfes_set_wait_probe(int32_t polls);
 
 /* Where a step with the norms fused in (cvfes_solid_step_norms_*) keeps each lane's sums:
- * 0 (default) tensor memory, in a kernel of its own; 1 shared memory, in the plain
- * persistent kernel (16 KB more per block at 4 nodes per block and 4 samples per
+ * 0 (default) tensor memory; 1 shared memory (64 KB per block at 4 samples per
  * thread, taken from the L1 of the neighbour-row gathers).  Both give bitwise the
  * same norms.                                                                       */
 int cvfes_set_norms_memory(int32_t mode);
@@ -295,10 +298,10 @@ int cvfes_solid_step_f32(const cvfes_solid_mesh* mesh, const float* coef, const 
 /* One step as cvfes_solid_step_* and, in the same pass, the FP64 per-sample norms of the
  * new state (out f64 [S][4] as cvfes_solid_norms_*: sum u_next^2, sum du^2, sum m du^2,
  * non-finite count, du = u_next - u, or the new increment in the velocity-state form).
- * The persistent fan kernel accumulates each lane's sums in tensor memory (32 or 64
- * columns per block, freed at its end) while it writes the state, so the state is not
- * read a second time; shapes without it (S / vec not a multiple of 32, no max_degree)
- * run the step and the separate norms pass.
+ * The patch kernel accumulates each lane's sums in tensor memory (128 columns per block,
+ * freed at its end) while it writes the state, so the state is not read a second time;
+ * shapes without it (few samples, no max_degree) run the step and the separate norms
+ * pass.
  * work: cvfes_norms_work_size(N, S) doubles.  check_finite: as cvfes_solid_norms_*.
  * out_host (NULL, or S*4 doubles of pinned host memory): when given, the call also copies
  * out to out_host, reads and clears mesh->status (CVFES_ERR_TIMEOUT if a bounded wait
