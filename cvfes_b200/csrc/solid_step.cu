@@ -1236,6 +1236,10 @@ int launch_step(const cvfes_solid_mesh* m, const T* coef, const T* invm, const T
     while (V > tune.vec) V /= 2;
     constexpr bool DIFF = std::is_same<T, float>::value;
     const bool fused = norm_work && max_rows > 0 && !A.probe_polls;
+    if (tune.staged == 6) {  // few samples: the group kernel (and the separate norms pass)
+        const int grc = launch_step_group<T>(m, A, V, after_step, st);
+        if (grc <= 0) return grc;
+    }
     if (tune.staged == 6 || fused) {
         if (fused) A.norm_part = norm_work;
         const int prc = launch_step_patch<T>(m, A, V, after_step, st, g_norms_mode.load(),
