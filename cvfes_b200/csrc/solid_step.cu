@@ -839,41 +839,78 @@ inline long long norm_chunks(long long n_nodes) {
     return std::max(1LL, std::min(1024LL, c));
 }
 
+// One row of partial sums per node chunk.  A block's threads are tpn sample vectors times
+// groups of nodes: group g of a chunk takes every (groups)-th node, and the groups' sums
+// are added in order, so few samples still fill the block (one thread a sample left 120 of
+// 128 threads idle at 8 samples: 37 us for an 8,192-node wall, 4 us now) and many
+// samples load 16 bytes a thread.
 // VEL: `up` holds the increment v = u_n - u_{n-1} (velocity-state form), else u_{n-1}.
-template <typename T, bool VEL>
-__global__ void k_norms_partial(long long n_nodes, int S, long long npc, const T* __restrict__ u,
-                                const T* __restrict__ up, const T* __restrict__ invm,
-                                double* __restrict__ work) {
+template <typename T, int V, bool VEL>
+__global__ void __launch_bounds__(kNormThreads)
+    k_norms_partial(long long n_nodes, int S, long long npc, int tpn, const T* __restrict__ u,
+                    const T* __restrict__ up, const T* __restrict__ invm,
+                    double* __restrict__ work) {
+    __shared__ double part[4 * V][kNormThreads];
     const long long chunk = blockIdx.x;
-    const int s = blockIdx.y * kNormThreads + threadIdx.x;
-    if (s >= S) return;
+    const int groups = kNormThreads / tpn;
+    const int g = threadIdx.x / tpn, l = threadIdx.x - g * tpn;
+    const int vec = blockIdx.y * tpn + l;
+    const bool on = g < groups && vec * V < S;
     const long long a0 = chunk * npc, a1 = (a0 + npc < n_nodes) ? a0 + npc : n_nodes;
-    double su = 0.0, sv = 0.0, sm = 0.0;
-    long long nf = 0;
-    for (long long a = a0; a < a1; ++a) {
-        // the node terms in the state's type, in the fused step's order (norms_add)
-        const T im = invm[(size_t)a * S + s];
-        T su_a = T(0), dv2 = T(0);
+    double su[V], sv[V], sm[V];
+    int nf[V];
 #pragma unroll
-        for (int d = 0; d < 3; ++d) {
-            const size_t o = ((size_t)a * 3 + d) * S + s;
-            const T x = u[o], y = up[o];
-            if (!isfinite(x)) ++nf;
-            su_a = fma(x, x, su_a);
-            const T dv = VEL ? y : x - y;
-            dv2 = fma(dv, dv, dv2);
-        }
-        su += (double)su_a;
-        sv += (double)dv2;
-        sm += (double)(norm_mass(im) * dv2);
+    for (int i = 0; i < V; ++i) {
+        su[i] = sv[i] = sm[i] = 0.0;
+        nf[i] = 0;
     }
-    double* w = work + ((size_t)chunk * S + s) * 4;
-    w[0] = su;
-    w[1] = sv;
-    w[2] = sm;
-    w[3] = (double)nf;
+    if (on) {
+        const size_t col = (size_t)vec * V;
+#pragma unroll 2
+        for (long long a = a0 + g; a < a1; a += groups) {
+            // the node terms in the state's type, in the fused step's order (norms_add)
+            const Vec<T, V> im = ldcs<T, V>(invm + (size_t)a * S + col);
+            Vec<T, V> x[3], y[3];
+#pragma unroll
+            for (int d = 0; d < 3; ++d) {
+                x[d] = ldg<T, V>(u + ((size_t)a * 3 + d) * S + col);
+                y[d] = ldcs<T, V>(up + ((size_t)a * 3 + d) * S + col);
+            }
+#pragma unroll
+            for (int i = 0; i < V; ++i) {
+                T su_a = T(0), dv2 = T(0);
+#pragma unroll
+                for (int d = 0; d < 3; ++d) {
+                    if (!isfinite(x[d].v[i])) ++nf[i];
+                    su_a = fma(x[d].v[i], x[d].v[i], su_a);
+                    const T dv = VEL ? y[d].v[i] : x[d].v[i] - y[d].v[i];
+                    dv2 = fma(dv, dv, dv2);
+                }
+                su[i] += (double)su_a;
+                sv[i] += (double)dv2;
+                sm[i] += (double)(norm_mass(im.v[i]) * dv2);
+            }
+        }
+    }
+#pragma unroll
+    for (int i = 0; i < V; ++i) {
+        part[4 * i][threadIdx.x] = su[i];
+        part[4 * i + 1][threadIdx.x] = sv[i];
+        part[4 * i + 2][threadIdx.x] = sm[i];
+        part[4 * i + 3][threadIdx.x] = (double)nf[i];
+    }
+    __syncthreads();
+    for (int t = threadIdx.x; t < 4 * V * tpn; t += kNormThreads) {
+        const int q = t % (4 * V), ln = t / (4 * V);  // q = 4 * sample of the vector + quantity
+        const int s = (blockIdx.y * tpn + ln) * V + q / 4;
+        if (s >= S) continue;
+        double sum = part[q][ln];
+        for (int k = 1; k < groups; ++k) sum += part[q][k * tpn + ln];
+        work[((size_t)chunk * S + s) * 4 + (q & 3)] = sum;
+    }
 }
 
+// total_nonfinite (may be null): the sum of the non-finite counts is added there.
 // Sums of the partial rows per (sample, quantity): a block owns kFinalPairs consecutive
 // (sample, quantity) pairs (coalesced across its lanes) and kFinalGroups row groups;
 // group g adds rows g, g + kFinalGroups, ... into four accumulators, and the groups'
@@ -906,7 +943,7 @@ __global__ void __launch_bounds__(kFinalPairs * kFinalGroups)
 #pragma unroll
     for (int k = 0; k < kFinalGroups; ++k) acc += part[k][lp];
     out[t] = acc;
-    if ((t & 3) == 3 && acc != 0.0) atomicAdd(total_nonfinite, acc);
+    if ((t & 3) == 3 && acc != 0.0 && total_nonfinite) atomicAdd(total_nonfinite, acc);
 }
 inline unsigned final_grid(long long S) { return grid_1d(4 * S, kFinalPairs); }
 
@@ -1413,32 +1450,59 @@ int launch_init(const cvfes_solid_mesh* m, const T* coef, const T* invm, const T
 }
 
 template <typename T>
+int launch_norms_partial(long long n_nodes, long long S, long long nch, long long npc, const T* u,
+                         const T* up, const T* invm, double* work, bool vel, cudaStream_t st) {
+    const void* ptrs[3] = {u, up, invm};
+    const int V = pick_vec<T>(ptrs, 3, (int)S);
+    const int sv = (int)S / V, tpn = std::min(sv, kNormThreads);
+    const dim3 grid((unsigned)nch, (unsigned)((sv + tpn - 1) / tpn));
+#define CVFES_NORMS(VV)                                                                        \
+    if (vel)                                                                                   \
+        k_norms_partial<T, VV, true><<<grid, kNormThreads, 0, st>>>(n_nodes, (int)S, npc, tpn, \
+                                                                    u, up, invm, work);        \
+    else                                                                                       \
+        k_norms_partial<T, VV, false><<<grid, kNormThreads, 0, st>>>(n_nodes, (int)S, npc,     \
+                                                                     tpn, u, up, invm, work);
+    if (V == 4) {
+        if constexpr (sizeof(T) == 4) {
+            CVFES_NORMS(4)
+        }
+    } else if (V == 2) {
+        CVFES_NORMS(2)
+    } else {
+        CVFES_NORMS(1)
+    }
+#undef CVFES_NORMS
+    CVFES_LAUNCH_CHECK("k_norms_partial");
+    return CVFES_OK;
+}
+
+// CVFES_ERR_NONFINITE when the counter on the device is not zero (synchronises).
+static int read_nonfinite(const double* total, cudaStream_t st) {
+    double h = 0.0;
+    CVFES_CUDA_TRY(cudaMemcpyAsync(&h, total, sizeof(double), cudaMemcpyDeviceToHost, st));
+    CVFES_CUDA_TRY(cudaStreamSynchronize(st));
+    if (h != 0.0) return fail(CVFES_ERR_NONFINITE, "watchdog: %.0f non-finite state values", h);
+    return CVFES_OK;
+}
+
+// count: keep the non-finite total behind the partial rows (check_finite reads it).
+template <typename T>
 int launch_norms(long long n_nodes, long long S, const T* u, const T* up, const T* invm,
-                 double* work, double* out, int check_finite, cudaStream_t st, bool vel = false) {
+                 double* work, double* out, int check_finite, cudaStream_t st, bool vel = false,
+                 bool count = true) {
     if (n_nodes <= 0 || S <= 0 || S > INT32_MAX || !u || !up || !invm || !work || !out)
         return fail(CVFES_ERR_ARG, "cvfes_solid_norms: bad argument");
     const long long nch = norm_chunks(n_nodes);
     const long long npc = (n_nodes + nch - 1) / nch;
-    double* total = work + (size_t)nch * S * 4;
-    CVFES_CUDA_TRY(cudaMemsetAsync(total, 0, sizeof(double), st));
-    dim3 grid((unsigned)nch, (unsigned)((S + kNormThreads - 1) / kNormThreads));
-    if (vel)
-        k_norms_partial<T, true><<<grid, kNormThreads, 0, st>>>(n_nodes, (int)S, npc, u, up, invm,
-                                                                work);
-    else
-        k_norms_partial<T, false><<<grid, kNormThreads, 0, st>>>(n_nodes, (int)S, npc, u, up, invm,
-                                                                 work);
-    CVFES_LAUNCH_CHECK("k_norms_partial");
-    k_norms_final<<<final_grid(S), kFinalPairs * kFinalGroups, 0, st>>>(nch, (int)S, work, out, total);
+    double* total = count ? work + (size_t)nch * S * 4 : nullptr;
+    if (total) CVFES_CUDA_TRY(cudaMemsetAsync(total, 0, sizeof(double), st));
+    int rc = launch_norms_partial<T>(n_nodes, S, nch, npc, u, up, invm, work, vel, st);
+    if (rc) return rc;
+    k_norms_final<<<final_grid(S), kFinalPairs * kFinalGroups, 0, st>>>(nch, (int)S, work, out,
+                                                                        total);
     CVFES_LAUNCH_CHECK("k_norms_final");
-    if (check_finite) {
-        double h = 0.0;
-        CVFES_CUDA_TRY(cudaMemcpyAsync(&h, total, sizeof(double), cudaMemcpyDeviceToHost, st));
-        CVFES_CUDA_TRY(cudaStreamSynchronize(st));
-        if (h != 0.0)
-            return fail(CVFES_ERR_NONFINITE, "watchdog: %.0f non-finite state values", h);
-    }
-    return CVFES_OK;
+    return check_finite ? read_nonfinite(total, st) : CVFES_OK;
 }
 
 }  // namespace cvfes
@@ -1475,7 +1539,7 @@ extern "C" int cvfes_solid_step_f32(const cvfes_solid_mesh* mesh, const float* c
                               damp, (cudaStream_t)stream);
 }
 
-// One step and the FP64 norms of the new state: fused into the persistent fan kernel
+// One step and the FP64 norms of the new state: fused into the patch kernel
 // where the shape allows, else the step followed by the separate norms pass.
 template <typename T>
 int launch_step_norms(const cvfes_solid_mesh* m, const T* coef, const T* invm, const T* u,
@@ -1493,37 +1557,39 @@ int launch_step_norms(const cvfes_solid_mesh* m, const T* coef, const T* invm, c
                         work, &rows, max_rows);
     if (rc) return rc;
     const bool vel = m->state_form == 1;
-    double* total = nullptr;
     if (rows == 0) {  // no fused kernel for this shape: the separate pass over the new state
         rc = launch_norms<T>(N, S, un, vel ? up : u, invm, work, out, out_host ? 0 : check_finite,
-                             st, vel);
-        if (rc) return rc;
-        total = work + (size_t)norm_chunks(N) * S * 4;
+                             st, vel, out_host == nullptr);
+        if (rc || !out_host) return rc;
     } else {
-        total = work + (size_t)rows * S * 4;
-        CVFES_CUDA_TRY(cudaMemsetAsync(total, 0, sizeof(double), st));
+        double* total = out_host ? nullptr : work + (size_t)rows * S * 4;
+        if (total) CVFES_CUDA_TRY(cudaMemsetAsync(total, 0, sizeof(double), st));
         k_norms_final<<<final_grid(S), kFinalPairs * kFinalGroups, 0, st>>>(rows, (int)S, work,
                                                                             out, total);
         CVFES_LAUNCH_CHECK("k_norms_final");
+        if (!out_host) return check_finite ? read_nonfinite(total, st) : CVFES_OK;
     }
-    if (!out_host && !check_finite) return CVFES_OK;
-    // one synchronisation for everything the host reads: the norms (out_host), the
-    // non-finite total and the status word of the bounded waits (read and cleared)
-    double h = 0.0;
+    // What the host reads: the norms, then the status word of the bounded waits.  The status
+    // goes to pageable memory, so its copy returns only once it (and with it everything
+    // before it on the stream) has arrived: no further synchronisation, and the word is
+    // cleared only when it was set.  The non-finite total is the sum of the counts.
+    CVFES_CUDA_TRY(cudaMemcpyAsync(out_host, out, (size_t)S * 4 * sizeof(double),
+                                   cudaMemcpyDeviceToHost, st));
     int32_t stat = 0;
-    if (out_host)
-        CVFES_CUDA_TRY(cudaMemcpyAsync(out_host, out, (size_t)S * 4 * sizeof(double),
-                                       cudaMemcpyDeviceToHost, st));
-    CVFES_CUDA_TRY(cudaMemcpyAsync(&h, total, sizeof(double), cudaMemcpyDeviceToHost, st));
-    if (out_host && m->status) {
+    if (m->status)
         CVFES_CUDA_TRY(cudaMemcpyAsync(&stat, m->status, sizeof(stat), cudaMemcpyDeviceToHost, st));
-        CVFES_CUDA_TRY(cudaMemsetAsync(m->status, 0, sizeof(int32_t), st));
+    if (!m->status || stat) {
+        if (stat) CVFES_CUDA_TRY(cudaMemsetAsync(m->status, 0, sizeof(int32_t), st));
+        CVFES_CUDA_TRY(cudaStreamSynchronize(st));
     }
-    CVFES_CUDA_TRY(cudaStreamSynchronize(st));
     if (stat & 1) return fail(CVFES_ERR_TIMEOUT, "a bounded device wait gave up (status %d)", stat);
     if (stat) return fail(CVFES_ERR_ARG, "device status %d: slot stage overflow", stat);
-    if (check_finite && h != 0.0)
-        return fail(CVFES_ERR_NONFINITE, "watchdog: %.0f non-finite state values", h);
+    if (check_finite) {
+        double h = 0.0;
+        for (long long q = 0; q < S; ++q) h += out_host[4 * q + 3];
+        if (h != 0.0)
+            return fail(CVFES_ERR_NONFINITE, "watchdog: %.0f non-finite state values", h);
+    }
     return CVFES_OK;
 }
 
@@ -1837,18 +1903,9 @@ extern "C" int cvfes_solid_norms_noalloc_f32(int64_t n_nodes, int64_t n_samples,
     cudaStream_t st = (cudaStream_t)stream;
     double* total = work + (size_t)nch * S * 4;  // the non-finite counter starts at zero
     CVFES_CUDA_TRY(cudaMemsetAsync(total, 0, sizeof(double), st));
-    dim3 grid((unsigned)nch, (unsigned)((S + kNormThreads - 1) / kNormThreads));
-    k_norms_partial<float, false><<<grid, kNormThreads, 0, st>>>(n_nodes, (int)S, npc, u, u_prev,
-                                                                 invm, work);
-    CVFES_LAUNCH_CHECK("k_norms_partial (fixed scratch)");
+    rc = launch_norms_partial<float>(n_nodes, S, nch, npc, u, u_prev, invm, work, false, st);
+    if (rc) return rc;
     k_norms_final<<<final_grid(S), kFinalPairs * kFinalGroups, 0, st>>>(nch, (int)S, work, out, total);
     CVFES_LAUNCH_CHECK("k_norms_final (fixed scratch)");
-    if (check_finite) {
-        double h = 0.0;
-        CVFES_CUDA_TRY(cudaMemcpyAsync(&h, total, sizeof(double), cudaMemcpyDeviceToHost, st));
-        CVFES_CUDA_TRY(cudaStreamSynchronize(st));
-        if (h != 0.0)
-            return fail(CVFES_ERR_NONFINITE, "watchdog: %.0f non-finite state values", h);
-    }
-    return CVFES_OK;
+    return check_finite ? read_nonfinite(total, st) : CVFES_OK;
 }
