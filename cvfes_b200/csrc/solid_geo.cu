@@ -9,15 +9,21 @@
 // Nothing per sample is stored: the row of node a is formed matrix-free from the
 // slot's reference edge vectors X_b - X_a (exact, precomputed) plus the neighbour
 // displacement differences, so the FP32 form never subtracts large coordinates.
-// Per slot and sample: the local frame (x along edge 1->2, y the Gram-Schmidt of
-// edge 2->0, z = x cross y; unit vectors by rsqrt), the in-plane coordinates, the
-// area, the 3x3 local blocks
-// of B^T D B (membrane + transverse shear, D / (1 - nu^2)) of row a against its two
-// neighbours applied to the neighbours' displacement differences in the local frame,
-// and the result rotated back; rigid translations are in the null space, so the row
-// only needs u_b - u_a.  The update of the state is the linear form's.
+// The membrane block of an isotropic sheet does not depend on the local frame, so no frame
+// is formed.  With q1, q2 the deformed edges from a to its neighbours, e = q2 - q1, n the
+// unit normal of nn = q1 x q2 and h1 = q2 x n, h2 = n x q1 (2 A times the gradients of the
+// neighbours' shape functions; a's is -(h1 + h2)), the row applied to the displacement
+// differences d1, d2 is
+//   -K d = c / (4 A (1 - nu^2)) [ h1 (pe1 (h1.d1 + h2.d1) + nu s) + h2 (pe1 (h1.d2 + h2.d2) + nu s)
+//                                 + w + (k - 1) (n.w) n ],
+//   s = h1.d1 + h2.d2,  w = pe1 ((q2.e) d1 - (q1.e) d2),  pe1 = (1 - nu) / 2,  k = 5/6,
+// (-K d: a's own gradient has the minus sign), and the follower load is nn / 6: 93 operations and one rsqrt a slot
+// where the frame form took about 170 with two rsqrt and a division.  Rigid translations
+// are in the null space, so the row only needs u_b - u_a.  The update of the state is the
+// linear form's.
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <type_traits>
 
 #include "common.cuh"
@@ -51,100 +57,124 @@ __global__ void k_slot_geometry(long long n_slots, const double* __restrict__ no
     }
 }
 
-template <typename T>
-struct GeoConst {
-    T pe0;  // nu
-    T pe1;  // (1 - nu) / 2
-    T pe2;  // k (1 - nu) / 2
-    T pe3;  // 1 - nu^2
-    T inv4pe3;  // 1 / (4 (1 - nu^2))
-};
+// Element-wise products and sums of V samples with the roundings written out (FP32 pairs as
+// one packed instruction), so that every width rounds alike.
+template <typename T, int V, typename F2, typename F1>
+__device__ __forceinline__ Vec<T, V> vmap(const F2& f2, const F1& f1) {
+    Vec<T, V> r;
+    if constexpr (std::is_same<T, float>::value && V % 2 == 0) {
+#pragma unroll
+        for (int i = 0; i < V; i += 2) {
+            const float2 q = f2(i);
+            r.v[i] = q.x;
+            r.v[i + 1] = q.y;
+        }
+    } else {
+#pragma unroll
+        for (int i = 0; i < V; ++i) r.v[i] = f1(i);
+    }
+    return r;
+}
+template <int V>
+__device__ __forceinline__ float2 pair(const Vec<float, V>& a, int i) {
+    return make_float2(a.v[i], a.v[i + 1]);
+}
+template <int V>
+__device__ __forceinline__ float2 pair(const Vec<double, V>&, int) {
+    return make_float2(0.f, 0.f);
+}
+__device__ __forceinline__ float mul_rn(float a, float b) { return __fmul_rn(a, b); }
+__device__ __forceinline__ double mul_rn(double a, double b) { return __dmul_rn(a, b); }
+__device__ __forceinline__ float add_rn(float a, float b) { return __fadd_rn(a, b); }
+__device__ __forceinline__ double add_rn(double a, double b) { return __dadd_rn(a, b); }
 
-template <typename T>
-__device__ __forceinline__ T sel3(int i, T x0, T x1, T x2) {
-    return i == 0 ? x0 : (i == 1 ? x1 : x2);
+template <typename T, int V>
+__device__ __forceinline__ Vec<T, V> vmul(const Vec<T, V>& a, const Vec<T, V>& b) {
+    return vmap<T, V>([&](int i) { return __fmul2_rn(pair(a, i), pair(b, i)); },
+                      [&](int i) { return mul_rn(a.v[i], b.v[i]); });
+}
+template <typename T, int V>
+__device__ __forceinline__ Vec<T, V> vadd(const Vec<T, V>& a, const Vec<T, V>& b) {
+    return vmap<T, V>([&](int i) { return __fadd2_rn(pair(a, i), pair(b, i)); },
+                      [&](int i) { return add_rn(a.v[i], b.v[i]); });
+}
+template <typename T, int V>
+__device__ __forceinline__ Vec<T, V> vfma3(const Vec<T, V>& a, const Vec<T, V>& b,
+                                           const Vec<T, V>& c) {
+    return vmap<T, V>([&](int i) { return __ffma2_rn(pair(a, i), pair(b, i), pair(c, i)); },
+                      [&](int i) { return fma(a.v[i], b.v[i], c.v[i]); });
+}
+template <typename T, int V>
+__device__ __forceinline__ Vec<T, V> vdot(const Vec<T, V> (&a)[3], const Vec<T, V> (&b)[3]) {
+    return vfma3(a[2], b[2], vfma3(a[1], b[1], vmul(a[0], b[0])));
+}
+// a x b, with na = -a beside a
+template <typename T, int V>
+__device__ __forceinline__ void vcross(Vec<T, V> (&r)[3], const Vec<T, V> (&a)[3],
+                                       const Vec<T, V> (&na)[3], const Vec<T, V> (&b)[3]) {
+    r[0] = vfma3(na[2], b[1], vmul(a[1], b[2]));
+    r[1] = vfma3(na[0], b[2], vmul(a[2], b[0]));
+    r[2] = vfma3(na[1], b[0], vmul(a[0], b[1]));
 }
 
-// Row of node a (local index la) of c_e K_e(x + u_g) applied to the displacement
-// differences (d1, d2) of its neighbours b1 = local (la+1)%3, b2 = local (la+2)%3,
-// for one sample; q1, q2 are the deformed edge vectors from a.  Adds the row to acc
-// and (A/3) n to load.
 template <typename T>
-__device__ __forceinline__ void geo_row(int la, const T (&q1)[3], const T (&q2)[3],
-                                        const T (&d1)[3], const T (&d2)[3], T c,
-                                        const GeoConst<T>& K, T (&acc)[3], T (&load)[3]) {
-    // positions of the element's nodes 0, 1, 2 relative to a
-    const int l1 = la == 2 ? 0 : la + 1;  // local index of b1
-    T P[3][3];
+struct GeoConst {
+    T nu;
+    T pe1;    // (1 - nu) / 2
+    T shear;  // k - 1, k = 5/6 the shear factor
+    T half;   // 1 / (2 (1 - nu^2))
+};
+
+// A neighbour of a: displacement difference and deformed edge from a.
+template <typename T, int V>
+struct GeoEdge {
+    Vec<T, V> d[3], q[3];
+};
+
+// Adds -(row of a) of c_e K_e(x + u_g) applied to (A.d, B.d) to acc and nn to load (the
+// pressure load is nn / 6).
+template <typename T, int V>
+__device__ __forceinline__ void geo_row(const GeoEdge<T, V>& A, const GeoEdge<T, V>& B,
+                                        const Vec<T, V>& c, const GeoConst<T>& K,
+                                        Vec<T, V> (&acc)[3], Vec<T, V> (&load)[3]) {
+    Vec<T, V> e[3], ne[3], nn[3], n[3], m[3], h1[3], h2[3], w[3];
 #pragma unroll
-    for (int d = 0; d < 3; ++d) {
-        const T z = T(0);
-        // node k is a (la), b1 (l1) or b2 (the remaining one)
-        P[0][d] = la == 0 ? z : (l1 == 0 ? q1[d] : q2[d]);
-        P[1][d] = la == 1 ? z : (l1 == 1 ? q1[d] : q2[d]);
-        P[2][d] = la == 2 ? z : (l1 == 2 ? q1[d] : q2[d]);
+    for (int i = 0; i < 3; ++i) {
+        e[i] = vsub(B.q[i], A.q[i]);
+        ne[i] = vsub(A.q[i], B.q[i]);
     }
-    // frame: x along P2 - P1, y Gram-Schmidt of P0 - P2, z = x cross y
-    T ex[3], ey[3], ez[3];
+    // nn = q1 x q2 = q1 x e = -(e x q1)
+    vcross(nn, ne, e, A.q);
+    const Vec<T, V> det = vdot(nn, nn);
+    Vec<T, V> rs, nrs;
 #pragma unroll
-    for (int d = 0; d < 3; ++d) ex[d] = P[2][d] - P[1][d];
-    T inv = rsqrt(ex[0] * ex[0] + ex[1] * ex[1] + ex[2] * ex[2]);
-#pragma unroll
-    for (int d = 0; d < 3; ++d) ex[d] *= inv;
-#pragma unroll
-    for (int d = 0; d < 3; ++d) ey[d] = P[0][d] - P[2][d];
-    const T pr = ex[0] * ey[0] + ex[1] * ey[1] + ex[2] * ey[2];
-#pragma unroll
-    for (int d = 0; d < 3; ++d) ey[d] -= pr * ex[d];
-    inv = rsqrt(ey[0] * ey[0] + ey[1] * ey[1] + ey[2] * ey[2]);
-#pragma unroll
-    for (int d = 0; d < 3; ++d) ey[d] *= inv;
-    ez[0] = ex[1] * ey[2] - ex[2] * ey[1];
-    ez[1] = ex[2] * ey[0] - ex[0] * ey[2];
-    ez[2] = ex[0] * ey[1] - ex[1] * ey[0];
-    // in-plane coordinates, area and the strain-displacement coefficients
-    T lx[3], ly[3];
-#pragma unroll
-    for (int k = 0; k < 3; ++k) {
-        lx[k] = P[k][0] * ex[0] + P[k][1] * ex[1] + P[k][2] * ex[2];
-        ly[k] = P[k][0] * ey[0] + P[k][1] * ey[1] + P[k][2] * ey[2];
+    for (int i = 0; i < V; ++i) {
+        rs.v[i] = rsqrt(det.v[i]);
+        nrs.v[i] = -rs.v[i];
     }
-    const T area = T(0.5) * ((lx[1] * ly[2] - lx[2] * ly[1]) - (lx[0] * ly[2] - lx[2] * ly[0]) +
-                             (lx[0] * ly[1] - lx[1] * ly[0]));
-    const T b0 = ly[1] - ly[2], b1 = ly[2] - ly[0], b2 = ly[0] - ly[1];
-    const T c0 = lx[2] - lx[1], c1 = lx[0] - lx[2], c2 = lx[1] - lx[0];
-    const int l2 = 3 - la - l1;
-    const T bi = sel3(la, b0, b1, b2), ci = sel3(la, c0, c1, c2);
-    const T bj1 = sel3(l1, b0, b1, b2), cj1 = sel3(l1, c0, c1, c2);
-    const T bj2 = sel3(l2, b0, b1, b2), cj2 = sel3(l2, c0, c1, c2);
-    // neighbour differences in the local frame
-    T w1[3], w2[3];
-    w1[0] = ex[0] * d1[0] + ex[1] * d1[1] + ex[2] * d1[2];
-    w1[1] = ey[0] * d1[0] + ey[1] * d1[1] + ey[2] * d1[2];
-    w1[2] = ez[0] * d1[0] + ez[1] * d1[1] + ez[2] * d1[2];
-    w2[0] = ex[0] * d2[0] + ex[1] * d2[1] + ex[2] * d2[2];
-    w2[1] = ey[0] * d2[0] + ey[1] * d2[1] + ey[2] * d2[2];
-    w2[2] = ez[0] * d2[0] + ez[1] * d2[1] + ez[2] * d2[2];
-    // local blocks (i = a, j = b1 / b2) applied: 2x2 membrane part + transverse shear
-    T r[3];
-    {
-        const T bb = bi * bj1, bc = bi * cj1, cb = ci * bj1, cc = ci * cj1;
-        r[0] = (bb + cc * K.pe1) * w1[0] + (bc * K.pe0 + cb * K.pe1) * w1[1];
-        r[1] = (cb * K.pe0 + bc * K.pe1) * w1[0] + (cc + bb * K.pe1) * w1[1];
-        r[2] = (bb + cc) * K.pe2 * w1[2];
-    }
-    {
-        const T bb = bi * bj2, bc = bi * cj2, cb = ci * bj2, cc = ci * cj2;
-        r[0] += (bb + cc * K.pe1) * w2[0] + (bc * K.pe0 + cb * K.pe1) * w2[1];
-        r[1] += (cb * K.pe0 + bc * K.pe1) * w2[0] + (cc + bb * K.pe1) * w2[1];
-        r[2] += (bb + cc) * K.pe2 * w2[2];
-    }
-    const T scale = c * K.inv4pe3 / area;
-    const T a3 = area * T(1.0 / 3.0);
 #pragma unroll
-    for (int d = 0; d < 3; ++d) {
-        acc[d] += scale * (r[0] * ex[d] + r[1] * ey[d] + r[2] * ez[d]);
-        load[d] += a3 * ez[d];
+    for (int i = 0; i < 3; ++i) {
+        load[i] = vadd(load[i], nn[i]);
+        n[i] = vmul(nn[i], rs);
+        m[i] = vmul(nn[i], nrs);
+    }
+    vcross(h1, m, n, B.q);  // q2 x n = (-n) x q2
+    vcross(h2, n, m, A.q);  // n x q1
+    const Vec<T, V> pe1 = vfill<T, V>(K.pe1);
+    const Vec<T, V> w1 = vmul(vdot(B.q, e), pe1), w2 = vmul(vdot(A.q, ne), pe1);
+    const Vec<T, V> a11 = vdot(h1, A.d), a21 = vdot(h2, A.d);
+    const Vec<T, V> a12 = vdot(h1, B.d), a22 = vdot(h2, B.d);
+    const Vec<T, V> ns = vmul(vadd(a11, a22), vfill<T, V>(K.nu));
+    const Vec<T, V> b1 = vfma3(vadd(a11, a21), pe1, ns);
+    const Vec<T, V> b2 = vfma3(vadd(a12, a22), pe1, ns);
+#pragma unroll
+    for (int i = 0; i < 3; ++i) w[i] = vfma3(w2, B.d[i], vmul(w1, A.d[i]));
+    const Vec<T, V> sm = vmul(vdot(n, w), vfill<T, V>(K.shear));
+    const Vec<T, V> scale = vmul(vmul(c, vfill<T, V>(K.half)), rs);
+#pragma unroll
+    for (int i = 0; i < 3; ++i) {
+        const Vec<T, V> f = vfma3(h1[i], b1, vfma3(h2[i], b2, vfma3(n[i], sm, w[i])));
+        acc[i] = vfma3(scale, f, acc[i]);
     }
 }
 
@@ -155,125 +185,129 @@ struct GeoArgs {
     GeoConst<T> K;
 };
 
-// Everything one slot needs: neighbour differences of u_n (and of u_g when it is a
-// different state), the coefficient row, the reference edge vectors, a's local index.
-template <typename T, int V, bool SAME>
-struct GeoSlot {
-    Vec<T, V> x1[3], x2[3];
-    Vec<T, V> g1[SAME ? 1 : 3], g2[SAME ? 1 : 3];
-    Vec<T, V> c;
-    T e1[3], e2[3];
-    int la;
-};
-
-template <typename T, int V, bool SAME>
-__device__ __forceinline__ void geo_slot_load(GeoSlot<T, V, SAME>& g, const StepArgs<T>& A,
-                                              const GeoArgs<T>& G, int k, size_t S, size_t col,
-                                              const Vec<T, V> (&ua)[3], const Vec<T, V> (&ga)[3]) {
-    const int4 r = __ldg(A.rec + k);
-    g.la = (r.w >> 8) & 3;
-    const size_t o1 = (size_t)r.y * 3 * S + col, o2 = (size_t)r.z * 3 * S + col;
-#pragma unroll
-    for (int d = 0; d < 3; ++d) {
-        g.x1[d] = vsub(ldg<T, V>(A.u + o1 + d * S), ua[d]);
-        g.x2[d] = vsub(ldg<T, V>(A.u + o2 + d * S), ua[d]);
-        if constexpr (!SAME) {
-            g.g1[d] = vsub(ldg<T, V>(G.ug + o1 + d * S), ga[d]);
-            g.g2[d] = vsub(ldg<T, V>(G.ug + o2 + d * S), ga[d]);
-        }
-    }
-    g.c = ldg<T, V>(A.coef + (size_t)r.x * S + col);
-#pragma unroll
-    for (int d = 0; d < 3; ++d) {
-        g.e1[d] = __ldg(G.geo + (size_t)kGeoStride * k + d);
-        g.e2[d] = __ldg(G.geo + (size_t)kGeoStride * k + 3 + d);
-    }
-}
-
-// One step, rows through L1: per slot the neighbour rows of u_n (and of u_g when it
-// is a different state), the coefficient row and the slot's edge vectors.
+// One step: a thread walks its node's fan with the next element's neighbour rows and
+// coefficient in flight.  Consecutive elements of a fan share an edge, so one neighbour is
+// gathered per element (two were, and their rows were 6 of the 7 gathered).  What bounds it
+// is the arithmetic: 93 packed or FP64 operations a slot against one row.
+// SAME: the geometry is the current state (ug == u).
 template <typename T, int V, bool SAME>
 __global__ void __launch_bounds__(256) k_step_geo(StepArgs<T> A, GeoArgs<T> G) {
-    long long a;
-    int vec;
-    if (!map_row(A.tpn, A.npb, A.n_nodes, A.S / V, a, vec)) return;
-    const size_t S = (size_t)A.S;
-    const size_t col = (size_t)vec * V;
-    const size_t row = (size_t)a * 3 * S + col;
+    const int t = threadIdx.x / A.tpn;
+    const long long a = (long long)blockIdx.x * A.npb + t;
+    const int vec = blockIdx.y * A.tpn + (threadIdx.x - t * A.tpn);
+    const bool active = t < A.npb && a < A.n_nodes && vec * V < A.S;
+    int k = 0, k1 = 0;
+    if (active) {
+        k = __ldg(A.node_ptr + a);
+        k1 = __ldg(A.node_ptr + a + 1);
+    }
+    grid_dependency_release();
+    grid_dependency_wait();
+    if (!active) return;
+    const size_t S = (size_t)A.S, col = (size_t)vec * V;
+    const uint32_t rowb = (uint32_t)A.S * sizeof(T), nodeb = 3 * rowb;
     if (a < A.n_clamped) {
         const Vec<T, V> cl = vfill<T, V>(A.clamp);
 #pragma unroll
-        for (int d = 0; d < 3; ++d) stcs<T, V>(A.un + row + d * S, cl);
+        for (int d = 0; d < 3; ++d) stcs<T, V>(row_at(A.un + col, (int)a, nodeb) + d * S, cl);
         return;
     }
-    Vec<T, V> ua[3], ga[3];
+    const T* const u = A.u + col;
+    const T* const ug = G.ug + col;
+    Vec<T, V> ua[3], ga[SAME ? 1 : 3], acc[3], load[3];
+    auto rows = [&](Vec<T, V> (&x)[3], const T* q) {
 #pragma unroll
-    for (int d = 0; d < 3; ++d) {
-        ua[d] = ldg<T, V>(A.u + row + d * S);
-        if constexpr (!SAME) ga[d] = ldg<T, V>(G.ug + row + d * S);
-    }
-    const T p = step_pressure<T>(A);
-    T acc[V][3], load[V][3];
+        for (int d = 0; d < 3; ++d) x[d] = ldg<T, V>(q + d * S);
+    };
+    rows(ua, row_at(u, (int)a, nodeb));
+    if constexpr (!SAME) rows(ga, row_at(ug, (int)a, nodeb));
 #pragma unroll
-    for (int i = 0; i < V; ++i)
+    for (int d = 0; d < 3; ++d) acc[d] = load[d] = vzero<T, V>();
+    // raw rows of a neighbour, and the reference edge to it (first or second of slot k)
+    Vec<T, V> x[3], g[SAME ? 1 : 3], c, cn;
+    T E[3];
+    auto request = [&](int slot, int b, int second) {
+        rows(x, row_at(u, b, nodeb));
+        if constexpr (!SAME) rows(g, row_at(ug, b, nodeb));
 #pragma unroll
-        for (int d = 0; d < 3; ++d) acc[i][d] = load[i][d] = T(0);
-    const int k0 = __ldg(A.node_ptr + a), k1 = __ldg(A.node_ptr + a + 1);
-    // The rows, coefficient and edge vectors of slot k+1 are requested before slot k is
-    // formed (one slot of lookahead; the per-slot geometry hides their latency).
-    GeoSlot<T, V, SAME> nx;
-    if (k0 < k1) geo_slot_load<T, V, SAME>(nx, A, G, k0, S, col, ua, ga);
-    for (int k = k0; k < k1; ++k) {
-        const GeoSlot<T, V, SAME> cu = nx;
-        if (k + 1 < k1) geo_slot_load<T, V, SAME>(nx, A, G, k + 1, S, col, ua, ga);
+        for (int d = 0; d < 3; ++d) E[d] = __ldg(G.geo + (size_t)kGeoStride * slot + 3 * second + d);
+    };
+    auto edge = [&](GeoEdge<T, V>& o) {
 #pragma unroll
-        for (int i = 0; i < V; ++i) {
-            T q1[3], q2[3], d1[3], d2[3];
-#pragma unroll
-            for (int d = 0; d < 3; ++d) {
-                const T g1 = SAME ? cu.x1[d].v[i] : cu.g1[d].v[i];
-                const T g2 = SAME ? cu.x2[d].v[i] : cu.g2[d].v[i];
-                q1[d] = cu.e1[d] + g1;
-                q2[d] = cu.e2[d] + g2;
-                d1[d] = cu.x1[d].v[i];
-                d2[d] = cu.x2[d].v[i];
+        for (int d = 0; d < 3; ++d) {
+            o.d[d] = vsub(x[d], ua[d]);
+            if constexpr (SAME)
+                o.q[d] = vadd(o.d[d], vfill<T, V>(E[d]));
+            else
+                o.q[d] = vadd(vsub(g[d], ga[d]), vfill<T, V>(E[d]));
+        }
+    };
+    if (k < k1) {
+        GeoEdge<T, V> P, Q;
+        int4 r = __ldg(A.rec + k);
+        request(k, r.y, 0);
+        edge(P);
+        request(k, r.z, 1);
+        cn = ldg<T, V>(row_at(A.coef + col, r.x, rowb));
+        auto phase = [&](GeoEdge<T, V>& first, GeoEdge<T, V>& second) {
+            edge(second);
+            c = cn;
+            const bool more = k + 1 < k1;
+            if (more) {
+                r = __ldg(A.rec + k + 1);
+                request(k + 1, r.z, 1);
+                cn = ldg<T, V>(row_at(A.coef + col, r.x, rowb));
             }
-            geo_row<T>(cu.la, q1, q2, d1, d2, cu.c.v[i], G.K, acc[i], load[i]);
+            geo_row<T, V>(first, second, c, G.K, acc, load);
+            if (more && !(r.w & 1)) {  // fan break: the next first neighbour is a new one
+                request(k + 1, r.y, 0);
+                edge(second);
+                request(k + 1, r.z, 1);
+            }
+            ++k;
+        };
+        while (true) {
+            phase(P, Q);
+            if (k >= k1) break;
+            phase(Q, P);
+            if (k >= k1) break;
         }
     }
-    const Vec<T, V> im = ldcs<T, V>(A.invm + (size_t)a * S + col);
+    const T p = step_pressure<T>(A) * T(1.0 / 6.0);
+    const Vec<T, V> im = ldcs<T, V>(row_at(A.invm + col, (int)a, rowb));
+    const T* const up = row_at(A.up + col, (int)a, nodeb);
+    T* const un = row_at(A.un + col, (int)a, nodeb);
 #pragma unroll
     for (int d = 0; d < 3; ++d) {
-        const Vec<T, V> up = ldcs<T, V>(A.up + row + d * S);
+        const Vec<T, V> vo = ldcs<T, V>(up + d * S);
         // nodal traction (calc_u_appTrac, physicsSolverSDampGPUs.cl:436-446), one per node
-        const T tr = A.trac ? __ldg(A.trac + 4 * a + d) : T(0);
+        const T tr = A.trac ? __ldg(A.trac + 4 * (size_t)a + d) : T(0);
         Vec<T, V> o;
 #pragma unroll
         for (int i = 0; i < V; ++i) {
-            const T dv = ua[d].v[i] - up.v[i];
-            const T w = A.w0 * im.v[i];
-            T f = p * load[i][d];
-            if (A.trac) f += tr;
-            const T v = fma(w, f - acc[i][d], fma(-row_eta(A, im.v[i]), dv, dv));
-            o.v[i] = (im.v[i] != T(0)) ? ua[d].v[i] + v : T(0);
+            const T dv = ua[d].v[i] - vo.v[i];
+            const T w = mul_rn(A.w0, im.v[i]);
+            T f = mul_rn(p, load[d].v[i]);
+            if (A.trac) f = add_rn(f, tr);
+            const T v = fma(w, add_rn(f, acc[d].v[i]), fma(-row_eta(A, im.v[i]), dv, dv));
+            o.v[i] = (im.v[i] != T(0)) ? add_rn(ua[d].v[i], v) : T(0);
         }
-        stcs<T, V>(A.un + row + d * S, o);
+        stcs<T, V>(un + d * S, o);
     }
 }
 
 struct GeoTuning {
-    int vec;    // samples per thread (upper bound)
+    int vec;    // samples per thread (upper bound; 4 runs as 2, one packed pair)
     int block;  // threads per block (64, 128 or 256)
 };
-// Defaults from sweeps on the 256x1024 tube, 512 samples (B200).
-static GeoTuning g_geo32 = {4, 128};
+static GeoTuning g_geo32 = {2, 128};
 static GeoTuning g_geo64 = {1, 128};
 
 template <typename T>
 int launch_step_geo(const cvfes_solid_mesh* m, const T* coef, const T* invm, const T* geo,
                     const T* u, const T* up, T* un, const T* ug, const double* p_sched,
                     const long long* clock, long long j, double pressure, const T* trac,
-                    double nu, double dt, double damp, cudaStream_t st) {
+                    double nu, double dt, double damp, cudaStream_t st, bool after_step = false) {
     if (!m || m->n_nodes <= 0 || m->n_samples <= 0 || m->n_samples > INT32_MAX || !m->node_ptr ||
         !m->slot_rec || m->n_clamped < 0 || m->n_clamped > m->n_nodes)
         return fail(CVFES_ERR_ARG, "cvfes_solid_step_geo: incomplete mesh descriptor");
@@ -311,41 +345,30 @@ int launch_step_geo(const cvfes_solid_mesh* m, const T* coef, const T* invm, con
     GeoArgs<T> G;
     G.geo = geo;
     G.ug = ug ? ug : u;
-    const double shear_k = 5.0 / 6.0;
-    G.K.pe0 = (T)nu;
+    G.K.nu = (T)nu;
     G.K.pe1 = (T)(0.5 * (1.0 - nu));
-    G.K.pe2 = (T)(0.5 * shear_k * (1.0 - nu));
-    G.K.pe3 = (T)(1.0 - nu * nu);
-    G.K.inv4pe3 = (T)(0.25 / (1.0 - nu * nu));
+    G.K.shear = (T)(5.0 / 6.0 - 1.0);
+    G.K.half = (T)(0.5 / (1.0 - nu * nu));
     const bool same = G.ug == u;
     const void* ptrs[6] = {coef, invm, u, up, un, G.ug};
     const GeoTuning& tu = sizeof(T) == 4 ? g_geo32 : g_geo64;
-    int V = (int)(16 / sizeof(T));
-    while (V > tu.vec) V /= 2;
+    int V = std::min(2, tu.vec);
     for (; V > 1; V /= 2) {
         bool ok = A.S % V == 0;
         for (int i = 0; i < 6; ++i)
             if (reinterpret_cast<uintptr_t>(ptrs[i]) % (V * sizeof(T))) ok = false;
         if (ok) break;
     }
-    const int block = tu.block;
-    const RowGrid rg = row_grid(m->n_nodes, A.S / V, block);
-    A.tpn = rg.tpn;
-    A.npb = rg.npb;
-    if (V == 4) {
-        if constexpr (sizeof(T) == 4) {
-            if (same) k_step_geo<T, 4, true><<<rg.grid, block, 0, st>>>(A, G);
-            else k_step_geo<T, 4, false><<<rg.grid, block, 0, st>>>(A, G);
-        }
-    } else if (V == 2) {
-        if (same) k_step_geo<T, 2, true><<<rg.grid, block, 0, st>>>(A, G);
-        else k_step_geo<T, 2, false><<<rg.grid, block, 0, st>>>(A, G);
-    } else {
-        if (same) k_step_geo<T, 1, true><<<rg.grid, block, 0, st>>>(A, G);
-        else k_step_geo<T, 1, false><<<rg.grid, block, 0, st>>>(A, G);
-    }
-    CVFES_LAUNCH_CHECK("k_step_geo");
-    return CVFES_OK;
+    if (m->n_samples >= (1 << 27) || m->n_nodes >= INT32_MAX)
+        return fail(CVFES_ERR_ARG, "cvfes_solid_step_geo: too many samples or nodes");
+    // lanes of a node: its sample vectors in equal parts of at most 32
+    const int sv = A.S / V, parts = (sv + 31) / 32;
+    A.tpn = (sv + parts - 1) / parts;
+    A.npb = tu.block / A.tpn;
+    const dim3 grid((unsigned)((m->n_nodes + A.npb - 1) / A.npb), (unsigned)parts);
+    auto kernel = V == 2 ? (same ? k_step_geo<T, 2, true> : k_step_geo<T, 2, false>)
+                         : (same ? k_step_geo<T, 1, true> : k_step_geo<T, 1, false>);
+    return launch_step_kernel(kernel, grid, tu.block, 0, after_step, st, "k_step_geo", A, G);
 }
 
 __global__ void k_geo_clock_add(long long* clock, long long n) { clock[0] += n; }
@@ -367,11 +390,13 @@ int launch_advance_geo(const cvfes_solid_mesh* m, const T* coef, const T* invm, 
     long long c = *counter;
     bool live = geo_live != 0;  // geometry is the current state (interval 1 after an update)
     for (long long j = 0; j < n_steps; ++j) {
+        bool after_step = j > 0;  // the launch before this one is the previous step
         if (c >= interval) {
             if (interval == 1) {
                 live = true;
             } else {
                 CVFES_CUDA_TRY(cudaMemcpyAsync(ugeo, buf[cur], bytes, cudaMemcpyDeviceToDevice, st));
+                after_step = false;
             }
             c = 1;
         } else {
@@ -379,7 +404,7 @@ int launch_advance_geo(const cvfes_solid_mesh* m, const T* coef, const T* invm, 
         }
         const T* ug = live ? buf[cur] : ugeo;
         int rc = launch_step_geo<T>(m, coef, invm, geo, buf[cur], buf[prev], buf[nxt], ug, p_sched,
-                                    clock, j, 0.0, nullptr, nu, dt, damp, st);
+                                    clock, j, 0.0, nullptr, nu, dt, damp, st, after_step);
         if (rc) return rc;
         const int old_prev = prev;
         prev = cur;

@@ -159,7 +159,7 @@ static int launch_group_k(const StepArgs<T>& A, bool after_step, cudaStream_t st
         fanp_blocks_per_sm(reinterpret_cast<const void*>(kernel), kGroupThreads, smem, &per_sm);
     if (rc) return rc;
     const long long blocks = (A.n_nodes + A.npb - 1) / A.npb;
-    return launch_step_kernel(kernel, blocks, kGroupThreads, smem, after_step, st, "k_step_group",
+    return launch_step_kernel(kernel, dim3((unsigned)blocks), kGroupThreads, smem, after_step, st, "k_step_group",
                               A);
 }
 

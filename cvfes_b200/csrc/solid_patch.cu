@@ -479,7 +479,7 @@ static int launch_patch_k(const StepArgs<T>& A, const PatchMap& M, int max_degre
         per_chunk = std::min(per_chunk, max_rows);
         if (rows) *rows = per_chunk;
     }
-    return launch_step_kernel(kernel, per_chunk * A.nch, 32 * kPatchWarps, smem, after_step, st,
+    return launch_step_kernel(kernel, dim3((unsigned)(per_chunk * A.nch)), 32 * kPatchWarps, smem, after_step, st,
                               "k_step_patch", A, M, max_degree);
 }
 

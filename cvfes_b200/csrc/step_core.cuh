@@ -776,10 +776,10 @@ __device__ __forceinline__ void grid_dependency_release() {
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
 template <typename... P, typename... Q>
-int launch_step_kernel(void (*kernel)(P...), long long blocks, int threads, size_t smem,
+int launch_step_kernel(void (*kernel)(P...), dim3 grid, int threads, size_t smem,
                        bool after_step, cudaStream_t st, const char* name, const Q&... args) {
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)blocks);
+    cfg.gridDim = grid;
     cfg.blockDim = dim3((unsigned)threads);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = st;
