@@ -27,6 +27,7 @@
 #include <type_traits>
 
 #include "common.cuh"
+#include "patch_walk.cuh"
 #include "step_core.cuh"
 
 namespace cvfes {
@@ -185,6 +186,35 @@ struct GeoArgs {
     GeoConst<T> K;
 };
 
+// Update of one node row from its -K u (acc) and load sums; p6 = pressure / 6.
+template <typename T, int V>
+__device__ __forceinline__ void geo_update(const StepArgs<T>& A, int a, size_t col, T p6,
+                                           const Vec<T, V> (&ua)[3], const Vec<T, V> (&acc)[3],
+                                           const Vec<T, V> (&load)[3], bool on) {
+    const size_t S = (size_t)A.S;
+    const uint32_t rowb = (uint32_t)A.S * sizeof(T), nodeb = 3 * rowb;
+    const Vec<T, V> im = ldcs<T, V>(row_at(A.invm + col, a, rowb));
+    const T* const up = row_at(A.up + col, a, nodeb);
+    T* const un = row_at(A.un + col, a, nodeb);
+#pragma unroll
+    for (int d = 0; d < 3; ++d) {
+        const Vec<T, V> vo = ldcs<T, V>(up + d * S);
+        // nodal traction (calc_u_appTrac, physicsSolverSDampGPUs.cl:436-446), one per node
+        const T tr = A.trac ? __ldg(A.trac + 4 * (size_t)a + d) : T(0);
+        Vec<T, V> o;
+#pragma unroll
+        for (int i = 0; i < V; ++i) {
+            const T dv = ua[d].v[i] - vo.v[i];
+            const T w = mul_rn(A.w0, im.v[i]);
+            T f = mul_rn(p6, load[d].v[i]);
+            if (A.trac) f = add_rn(f, tr);
+            const T v = fma(w, add_rn(f, acc[d].v[i]), fma(-row_eta(A, im.v[i]), dv, dv));
+            o.v[i] = (im.v[i] != T(0)) ? add_rn(ua[d].v[i], v) : T(0);
+        }
+        if (on) stcs<T, V>(un + d * S, o);
+    }
+}
+
 // One step: a thread walks its node's fan with the next element's neighbour rows and
 // coefficient in flight.  Consecutive elements of a fan share an edge, so one neighbour is
 // gathered per element (two were, and their rows were 6 of the 7 gathered).  What bounds it
@@ -273,27 +303,160 @@ __global__ void __launch_bounds__(256) k_step_geo(StepArgs<T> A, GeoArgs<T> G) {
             if (k >= k1) break;
         }
     }
-    const T p = step_pressure<T>(A) * T(1.0 / 6.0);
-    const Vec<T, V> im = ldcs<T, V>(row_at(A.invm + col, (int)a, rowb));
-    const T* const up = row_at(A.up + col, (int)a, nodeb);
-    T* const un = row_at(A.un + col, (int)a, nodeb);
-#pragma unroll
-    for (int d = 0; d < 3; ++d) {
-        const Vec<T, V> vo = ldcs<T, V>(up + d * S);
-        // nodal traction (calc_u_appTrac, physicsSolverSDampGPUs.cl:436-446), one per node
-        const T tr = A.trac ? __ldg(A.trac + 4 * (size_t)a + d) : T(0);
-        Vec<T, V> o;
-#pragma unroll
-        for (int i = 0; i < V; ++i) {
-            const T dv = ua[d].v[i] - vo.v[i];
-            const T w = mul_rn(A.w0, im.v[i]);
-            T f = mul_rn(p, load[d].v[i]);
-            if (A.trac) f = add_rn(f, tr);
-            const T v = fma(w, add_rn(f, acc[d].v[i]), fma(-row_eta(A, im.v[i]), dv, dv));
-            o.v[i] = (im.v[i] != T(0)) ? add_rn(ua[d].v[i], v) : T(0);
+    geo_update<T, V>(A, (int)a, col, step_pressure<T>(A) * T(1.0 / 6.0), ua, acc, load, true);
+}
+
+// The same step with free-running warps on patches of nodes (patch_walk.cuh): 32 * V samples
+// of one node at a time, the next node's slots staged in shared memory and its rows
+// prefetched into L2 under the current one.  As in the linear step the plain kernel's time
+// went into DRAM misses of first-touched rows: 128 x 400 wall, 128 samples, FP32 306 -> 193 us
+// a step; 64 samples, FP64 329 -> 232 us.
+// Warps of a block (one block an SM): what the registers allow.  FP32 pairs, 128 x 400 wall,
+// 128 samples, us a step at 16 / 20 / 24 warps: current geometry 221 / 204 / 193, stored
+// geometry - / 236 / 248 (200 bytes spilled).
+template <typename T, bool SAME>
+struct GeoWarps {
+    static constexpr int kWarps = sizeof(T) == 4 ? (SAME ? 24 : 20) : 16;
+};
+template <typename T, int V, bool SAME>
+__global__ void __launch_bounds__(32 * GeoWarps<T, SAME>::kWarps, 1)
+    k_step_geo_patch(StepArgs<T> A, GeoArgs<T> G, PatchMap M, int max_degree) {
+    extern __shared__ __align__(16) unsigned char smem[];
+    constexpr int W = GeoWarps<T, SAME>::kWarps;
+    constexpr int kWords = kGeoStride * (int)sizeof(T) / 16;
+    const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
+    const uint32_t b_rec = 16u * max_degree, b_stage = b_rec + 16u * kWords * max_degree;
+    unsigned char* const wb = smem + warp * (2 * b_stage);
+    const uint32_t rowb = (uint32_t)A.S * sizeof(T), nodeb = 3 * rowb;
+    const int chunk = blockIdx.x % A.nch;
+    const int vec = chunk * 32 + lane, last = A.S / V - 1;
+    const bool on = vec <= last;
+    const size_t S = (size_t)A.S, col = (size_t)(on ? vec : last) * V;
+    const int bpc = gridDim.x / A.nch;
+    PatchWalk walk(M, warp, blockIdx.x / A.nch, bpc, A.n_clamped, (int)A.n_nodes, W);
+    auto stage = [&](int b, int k0, int n, int sg) {
+        if (b >= 0) {
+            const uint32_t d = smem_u32(wb + sg * b_stage);
+            const char* r = reinterpret_cast<const char*>(A.rec + k0);
+            const char* g = reinterpret_cast<const char*>(G.geo + (size_t)k0 * kGeoStride);
+            for (int q = lane; q < n; q += 32) cp_async<16>(d + 16 * q, r + 16 * q);
+            for (int q = lane; q < kWords * n; q += 32) cp_async<16>(d + b_rec + 16 * q, g + 16 * q);
         }
-        stcs<T, V>(un + d * S, o);
+        cp_async_commit();
+    };
+    bool more = walk.more(M);
+    int a = walk.node(M), n, an, k0, nn;
+    node_slots(A.node_ptr, a, k0, n);
+    stage(a, k0, n, 0);
+    walk.advance(M);
+    an = walk.node(M);
+    node_slots(A.node_ptr, an, k0, nn);
+    const RowLines<T, V> ln(lane, chunk, rowb);
+    const char* const obase =
+        reinterpret_cast<const char*>(ln.row < 3   ? A.u + (size_t)ln.row * S
+                                      : ln.row < 6 ? A.up + (size_t)(ln.row - 3) * S
+                                                   : A.invm) + ln.off;
+    const uint32_t ostride = ln.row < 6 ? nodeb : rowb;
+    const char* const cbase = reinterpret_cast<const char*>(A.coef) + ln.off;
+    const T* const u = A.u + col;
+    const T* const ug = G.ug + col;
+    grid_dependency_release();
+    grid_dependency_wait();
+    const T p = step_pressure<T>(A) * T(1.0 / 6.0);
+    for (int b = blockIdx.x / A.nch * W + warp; b < A.n_clamped; b += bpc * W) {
+        const Vec<T, V> cl = vfill<T, V>(A.clamp);
+#pragma unroll
+        for (int d = 0; d < 3; ++d)
+            if (on) stcs<T, V>(row_at(A.un + col, b, nodeb) + d * S, cl);
     }
+    for (int sg = 0; more; sg ^= 1) {
+        Vec<T, V> ua[3], ga[SAME ? 1 : 3];
+        auto rows = [&](Vec<T, V> (&x)[3], const T* q) {
+#pragma unroll
+            for (int d = 0; d < 3; ++d) x[d] = ldg<T, V>(q + d * S);
+        };
+        if (a >= 0) {
+            rows(ua, row_at(u, a, nodeb));
+            if constexpr (!SAME) rows(ga, row_at(ug, a, nodeb));
+        }
+        cp_async_wait_all();
+        __syncwarp();
+        const unsigned char* const st = wb + sg * b_stage;
+        const int4* const srec = reinterpret_cast<const int4*>(st);
+        const T* const sgeo = reinterpret_cast<const T*>(st + b_rec);
+        stage(an, k0, nn, sg ^ 1);
+        if (an >= 0 && ln.row < 7 && ln.on) prefetch_l2(obase + (uint64_t)(uint32_t)an * ostride);
+        const int nn_cur = nn;
+        more = walk.more(M);
+        walk.advance(M);
+        const int ax = walk.node(M);
+        node_slots(A.node_ptr, ax, k0, nn);
+        if (a >= 0) {
+            Vec<T, V> acc[3], load[3], x[3], g[SAME ? 1 : 3], c, cn;
+            T E[3];
+#pragma unroll
+            for (int d = 0; d < 3; ++d) acc[d] = load[d] = vzero<T, V>();
+            auto request = [&](int slot, int b, int second) {
+                rows(x, row_at(u, b, nodeb));
+                if constexpr (!SAME) rows(g, row_at(ug, b, nodeb));
+#pragma unroll
+                for (int d = 0; d < 3; ++d) E[d] = sgeo[kGeoStride * slot + 3 * second + d];
+            };
+            auto edge = [&](GeoEdge<T, V>& o) {
+#pragma unroll
+                for (int d = 0; d < 3; ++d) {
+                    o.d[d] = vsub(x[d], ua[d]);
+                    if constexpr (SAME)
+                        o.q[d] = vadd(o.d[d], vfill<T, V>(E[d]));
+                    else
+                        o.q[d] = vadd(vsub(g[d], ga[d]), vfill<T, V>(E[d]));
+                }
+            };
+            if (n > 0) {
+                GeoEdge<T, V> P, Q;
+                int k = 0;
+                request(0, srec[0].y, 0);
+                edge(P);
+                request(0, srec[0].z, 1);
+                cn = ldg<T, V>(row_at(A.coef + col, srec[0].x, rowb));
+                auto phase = [&](GeoEdge<T, V>& one, GeoEdge<T, V>& two) {
+                    edge(two);
+                    c = cn;
+                    const bool next = k + 1 < n;
+                    int4 r = make_int4(0, 0, 0, 1);
+                    if (next) {
+                        r = srec[k + 1];
+                        request(k + 1, r.z, 1);
+                        cn = ldg<T, V>(row_at(A.coef + col, r.x, rowb));
+                    }
+                    geo_row<T, V>(one, two, c, G.K, acc, load);
+                    if (next && !(r.w & 1)) {  // fan break: the next first neighbour is new
+                        request(k + 1, r.y, 0);
+                        edge(two);
+                        request(k + 1, r.z, 1);
+                    }
+                    ++k;
+                };
+                while (true) {
+                    phase(P, Q);
+                    if (k >= n) break;
+                    phase(Q, P);
+                    if (k >= n) break;
+                }
+            }
+            cp_async_wait_all();
+            __syncwarp();
+            if (an >= 0 && ln.on && ln.row < nn_cur)
+                prefetch_l2(cbase + (uint64_t)(uint32_t)reinterpret_cast<const int4*>(
+                                        wb + (sg ^ 1) * b_stage)[ln.row].x * rowb);
+            geo_update<T, V>(A, a, col, p, ua, acc, load, on);
+        }
+        __syncwarp();
+        a = an;
+        n = nn_cur;
+        an = ax;
+    }
+    cp_async_wait_all();
 }
 
 struct GeoTuning {
@@ -361,6 +524,33 @@ int launch_step_geo(const cvfes_solid_mesh* m, const T* coef, const T* invm, con
     }
     if (m->n_samples >= (1 << 27) || m->n_nodes >= INT32_MAX)
         return fail(CVFES_ERR_ARG, "cvfes_solid_step_geo: too many samples or nodes");
+    const int W = same ? GeoWarps<T, true>::kWarps : GeoWarps<T, false>::kWarps;
+    const size_t stages = (size_t)W * 2 * (16 + kGeoStride * sizeof(T)) * m->max_degree;
+    // The patch kernel where the samples fill its warps: at least 3/4 of the lanes, or 9/10
+    // when the step's rows (100 MB) fit L2 and there are few DRAM misses to hide.  us a
+    // step, plain / patch: 128 x 400 wall, FP32 128 samples 306 / 204, 100 samples (78%
+    // filled) 264 / 211, 40 samples (62%) 94 / 109; FP64 64 samples 329 / 232, 50 samples
+    // (78%) 285 / 240; 96 x 200 wall (92 MB), FP64 50 samples 88 / 94, 64 samples 109 / 94.
+    A.nch = (A.S / V + 31) / 32;
+    const double lanes = (double)(A.S / V) / (32.0 * A.nch);
+    const bool in_l2 = 12.0 * m->n_nodes * A.S * sizeof(T) < 100e6;
+    if ((sizeof(T) == 4 || V == 1) && lanes >= (in_l2 ? 0.9 : 0.75) && m->max_degree > 0 &&
+        m->max_degree < 1024 && stages <= 96 * 1024) {
+        const PatchMap M = patch_map(m->n_nodes - A.n_clamped, m->bandwidth, W);
+        constexpr int V2 = sizeof(T) == 4 ? 2 : 1;  // (FP64 pairs would spill)
+        auto kp = V == 2 ? (same ? k_step_geo_patch<T, V2, true> : k_step_geo_patch<T, V2, false>)
+                         : (same ? k_step_geo_patch<T, 1, true> : k_step_geo_patch<T, 1, false>);
+        int per_sm = 0;
+        const int rc = fanp_blocks_per_sm(reinterpret_cast<const void*>(kp), 32 * W, stages, &per_sm);
+        if (rc) return rc;
+        const long long places =
+            std::max<long long>((long long)M.n_strips * M.tps, (A.n_clamped + W - 1) / W);
+        const long long per_chunk = std::max(
+            1LL, std::min((long long)per_sm * device_sm_count() / A.nch, places));
+        return launch_step_kernel(kp, dim3((unsigned)(per_chunk * A.nch)), 32 * W, stages,
+                                  after_step, st, "k_step_geo_patch", A, G, M,
+                                  (int)m->max_degree);
+    }
     // lanes of a node: its sample vectors in equal parts of at most 32
     const int sv = A.S / V, parts = (sv + 31) / 32;
     A.tpn = (sv + parts - 1) / parts;

@@ -35,17 +35,10 @@
 #include <type_traits>
 
 #include "common.cuh"
+#include "patch_walk.cuh"
 #include "step_core.cuh"
 
 namespace cvfes {
-
-constexpr int kPatchWarps = 16;
-
-// Node order: patches of L x (16 / L) nodes over rows of R nodes after the clamped prefix,
-// patch after patch along a strip of 16 / L rows.
-struct PatchMap {
-    int R, L, tps, n_strips;
-};
 
 // One node row's update (increment form) and store; su, sv, nf: its norm terms.
 template <typename T, int V, bool VEL, bool NORMS>
@@ -139,25 +132,8 @@ __global__ void __launch_bounds__(32 * kPatchWarps, 1)
     const T* const cf = A.coef + col;
     const int n_nodes = (int)A.n_nodes, first = A.n_clamped;
 
-    // ---- this warp's nodes: place (wj, wi) of every patch the block takes
-    const int J = W / M.L, wj = warp / M.L, wi = warp - wj * M.L;
-    const int bpc = gridDim.x / A.nch;
-    const int dstrip = bpc / M.tps, dtile = bpc - dstrip * M.tps;
-    int tile = blockIdx.x / A.nch, strip = tile / M.tps;
-    tile -= strip * M.tps;
-    auto node = [&]() {  // -1: no node at this place (mesh row or mesh ends)
-        const int c = tile * M.L + wi;
-        const int b = first + (strip * J + wj) * M.R + c;
-        return strip < M.n_strips && c < M.R && b < n_nodes ? b : -1;
-    };
-    auto advance = [&]() {
-        strip += dstrip;
-        tile += dtile;
-        if (tile >= M.tps) {
-            tile -= M.tps;
-            ++strip;
-        }
-    };
+    const int bpc = gridDim.x / A.nch;  // blocks of a chunk
+    PatchWalk walk(M, warp, blockIdx.x / A.nch, bpc, first, n_nodes);
     // ---- slot staging: lane l copies word l % kWords of slot l / kWords (FP32), or every
     // 32nd word (FP64); records by the first lanes
     const int qs = lane / P::kWords, qw = lane - qs * P::kWords;
@@ -179,32 +155,22 @@ __global__ void __launch_bounds__(32 * kPatchWarps, 1)
         }
         cp_async_commit();
     };
-    auto slots = [&](int b, int& k0, int& n) {
-        k0 = n = 0;
-        if (b >= 0) {
-            k0 = __ldg(A.node_ptr + b);
-            n = __ldg(A.node_ptr + b + 1) - k0;
-        }
-    };
-    bool more = strip < M.n_strips;
-    int a = node(), n, an, k0, nn;
-    slots(a, k0, n);
+    bool more = walk.more(M);
+    int a = walk.node(M), n, an, k0, nn;
+    node_slots(A.node_ptr, a, k0, n);
     stage(a, k0, n, 0);
-    advance();
-    an = node();
-    slots(an, k0, nn);
+    walk.advance(M);
+    an = walk.node(M);
+    node_slots(A.node_ptr, an, k0, nn);
 
-    // ---- line prefetch: lane l takes line l % kLines of row l / kLines of this chunk
-    constexpr int kRow = 32 * V * (int)sizeof(T), kLines = kRow / 128;
-    const int pr = lane / kLines;
-    const size_t poff = (size_t)chunk * kRow + (lane % kLines) * 128;
-    const bool pon = poff < rowb;
+    // ---- line prefetch: u, u_{n-1} and inverse mass rows of a node; coefficient rows
+    const RowLines<T, V> ln(lane, chunk, rowb);
     const char* const obase =
-        reinterpret_cast<const char*>(pr < 3   ? A.u + (size_t)pr * A.S
-                                      : pr < 6 ? A.up + (size_t)(pr - 3) * A.S
-                                               : A.invm) + poff;
-    const uint32_t ostride = pr < 6 ? nodeb : rowb;
-    const char* const cbase = reinterpret_cast<const char*>(A.coef) + poff;
+        reinterpret_cast<const char*>(ln.row < 3   ? A.u + (size_t)ln.row * A.S
+                                      : ln.row < 6 ? A.up + (size_t)(ln.row - 3) * A.S
+                                                   : A.invm) + ln.off;
+    const uint32_t ostride = ln.row < 6 ? nodeb : rowb;
+    const char* const cbase = reinterpret_cast<const char*>(A.coef) + ln.off;
 
     grid_dependency_release();
     grid_dependency_wait();
@@ -283,20 +249,20 @@ __global__ void __launch_bounds__(32 * kPatchWarps, 1)
         const T* const K = reinterpret_cast<const T*>(st + b_rec) - 16 / (int)sizeof(T) * P::kFirst;
         constexpr int kStep = P::kSlotBytes / (int)sizeof(T);
         stage(an, k0, nn, sg ^ 1);
-        if (an >= 0 && pr < 7 && pon) prefetch_l2(obase + (uint64_t)(uint32_t)an * ostride);
+        if (an >= 0 && ln.row < 7 && ln.on) prefetch_l2(obase + (uint64_t)(uint32_t)an * ostride);
         const int nn_cur = nn;
-        more = strip < M.n_strips;
-        advance();
-        const int ax = node();
-        slots(ax, k0, nn);
-        // coefficient rows of the next node's elements (the first 32 / kLines of them: a loop
+        more = walk.more(M);
+        walk.advance(M);
+        const int ax = walk.node(M);
+        node_slots(A.node_ptr, ax, k0, nn);
+        // coefficient rows of the next node's elements (the first kRows of them: a loop
         // over more cost the spill-free allocation, 385 -> 400 us and FP64 228 -> 270 us)
         auto prefetch_coef = [&]() {
             cp_async_wait_all();
             __syncwarp();
             const int4* nr = reinterpret_cast<const int4*>(wb + (sg ^ 1) * b_stage);
-            if (an >= 0 && pon && pr < nn_cur)
-                prefetch_l2(cbase + (uint64_t)(uint32_t)nr[pr].x * rowb);
+            if (an >= 0 && ln.on && ln.row < nn_cur)
+                prefetch_l2(cbase + (uint64_t)(uint32_t)nr[ln.row].x * rowb);
         };
         if (a >= 0) {
             auto rows = [&](Vec<T, V> (&x)[3], int b) {
@@ -411,13 +377,13 @@ __global__ void __launch_bounds__(32 * kPatchWarps, 1)
         const long long prow = blockIdx.x / A.nch;
         for (int t = threadIdx.x; t < kAcc; t += blockDim.x) {
             const int q = t / (32 * V), c = t - q * 32 * V;  // c: sample of the chunk
-            const int ln = c / V, i = c - ln * V;
+            const int lane_c = c / V, i = c - lane_c * V;
             double sum = 0.0;
             if constexpr (NORMS == 1) {
-                sum = scr[(q * V + i) * 32 + ln];
+                sum = scr[(q * V + i) * 32 + lane_c];
             } else {
                 for (int w = 0; w < W; ++w) {
-                    const double x = nbase[w * kAcc + (q * V + i) * 32 + ln];
+                    const double x = nbase[w * kAcc + (q * V + i) * 32 + lane_c];
                     sum = w == 0 ? x : sum + x;
                 }
             }
@@ -431,30 +397,6 @@ __global__ void __launch_bounds__(32 * kPatchWarps, 1)
             if (warp == 0) tmem_dealloc(tmem_slot, 32 * (W / 4));
         }
     }
-}
-
-// Patch shape for a mesh of this bandwidth: rows of bandwidth - 1 nodes (the distance to
-// the next mesh row in a row-by-row numbering).  A strip that the mesh does not fill, or a
-// run that a row does not fill, idles warps, so 4 x 4 is taken while at most an eighth of
-// the places are empty, else 8 x 2, else runs of 16 (any numbering; what locality is left
-// is that of consecutive nodes).
-static PatchMap patch_map(long long n_free, long long bandwidth) {
-    PatchMap m;
-    const long long R = bandwidth - 1;
-    for (int L = 4; L <= 8; L *= 2) {
-        const int J = kPatchWarps / L;
-        if (R < L || R > n_free / J) continue;
-        m.R = (int)R;
-        m.L = L;
-        m.tps = (int)((R + L - 1) / L);
-        m.n_strips = (int)((n_free + J * R - 1) / (J * R));
-        if ((long long)m.n_strips * m.tps * kPatchWarps * 8 <= n_free * 9) return m;
-    }
-    m.R = (int)std::max(n_free, 1LL);
-    m.L = kPatchWarps;
-    m.tps = (int)((m.R + kPatchWarps - 1) / kPatchWarps);
-    m.n_strips = n_free > 0 ? 1 : 0;
-    return m;
 }
 
 template <typename T, int V, bool VEL, int NORMS>

@@ -107,3 +107,34 @@ def test_step_norms_against_sums_of_the_state(lib, cuda, precision, kind, sample
     assert np.all(got[:, 3] == 0) and np.all(want > 0)
     np.testing.assert_allclose(got[:, :3], want, rtol=tol, atol=0)
     np.testing.assert_allclose(got, s.__class__.Norms(s), rtol=0, atol=0)
+
+
+def run_geo(mesh, precision, interval, vec, steps=5):
+    saved = [_lib.C.c_int32(), _lib.C.c_int32()]
+    _lib.call("cvfes_get_geo_tuning", precision, _lib.C.byref(saved[0]), _lib.C.byref(saved[1]))
+    try:
+        _lib.call("cvfes_set_geo_tuning", precision, vec, 128)
+        cfg = Cfg(1e-8, mesh.nSmp, precision, "auto")
+        cfg.update_interval = interval
+        s = GPUSolidSolver(LocalComm(), mesh, cfg)
+        s.Advance(1e4 * (1.0 + np.arange(steps)))
+        return s.bufs[s.cur].clone()
+    finally:
+        _lib.call("cvfes_set_geo_tuning", precision, saved[0].value, saved[1].value)
+
+
+@pytest.mark.parametrize("precision", [32, 64])
+@pytest.mark.parametrize("interval", [1, 2])
+@pytest.mark.parametrize("kind,samples", [("tube", 30), ("tube", 64), ("tube", 96), ("short", 64),
+                                          ("shuffled", 64), ("irregular", 62), ("irregular", 130)])
+def test_geometric_step_alone_or_in_an_ensemble(lib, cuda, precision, interval, kind, samples):
+    """Samples never interact and every width and kernel rounds alike: the first three
+    samples of an ensemble (patch kernel where its lanes are filled) and the same three
+    alone (plain kernel, one a thread) have the same bits."""
+    mesh = wall(kind, samples)
+    few = SolidMesh(mesh.nodes, mesh.elementNodeIds, mesh.boundary, 3, density=1.0, v=0.49,
+                    damp=100.0, elmE=mesh.elmE[:, :3], elmThick=mesh.elmThick[:, :3],
+                    iniU=mesh.iniU, iniDu=mesh.iniDu)
+    got = run_geo(mesh, precision, interval, 2 if precision == 32 else 1)
+    want = run_geo(few, precision, interval, 1)
+    assert torch.isfinite(got).all() and torch.equal(got[:, :3], want)
