@@ -28,9 +28,11 @@
 // Every element and node accumulator is written by one thread: no atomics.
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <type_traits>
 
 #include "common.cuh"
+#include "patch_walk.cuh"
 #include "step_core.cuh"
 
 namespace cvfes {
@@ -110,13 +112,23 @@ __global__ void k_obs(int n_obs, int S, const int32_t* __restrict__ obs_nodes,
     if (!record) jpart_k[(size_t)blockIdx.x * S + s] = acc;
 }
 
-// J[s] = sum over observation steps and node blocks, in a fixed order.
-__global__ void k_obs_reduce(long long n_parts, int S, const double* __restrict__ jpart,
-                             double* __restrict__ J) {
-    const int s = blockIdx.x * blockDim.x + threadIdx.x;
-    if (s >= S) return;
+// J[s] = sum over observation steps and node blocks, in a fixed order: group g of a block adds
+// parts g, g + kReduceGroups, ..., the groups' sums are added in order (one thread a sample
+// summing all parts took 40 us for 320 parts, one dependent addition after another).
+constexpr int kReduceSamples = 32, kReduceGroups = 16;
+__global__ void __launch_bounds__(kReduceSamples * kReduceGroups)
+    k_obs_reduce(long long n_parts, int S, const double* __restrict__ jpart,
+                 double* __restrict__ J) {
+    __shared__ double part[kReduceGroups][kReduceSamples];
+    const int l = threadIdx.x % kReduceSamples, g = threadIdx.x / kReduceSamples;
+    const int s = blockIdx.x * kReduceSamples + l;
     double acc = 0.0;
-    for (long long k = 0; k < n_parts; ++k) acc += jpart[(size_t)k * S + s];
+    if (s < S)
+        for (long long k = g; k < n_parts; k += kReduceGroups) acc += jpart[(size_t)k * S + s];
+    part[g][l] = acc;
+    __syncthreads();
+    if (g != 0 || s >= S) return;
+    for (int q = 1; q < kReduceGroups; ++q) acc += part[q][l];
     J[s] = acc;
 }
 
@@ -223,15 +235,16 @@ __device__ __forceinline__ void load27(const T* K, T (&kk)[27]) {
     }
 }
 
-// Gamma_e += dchi^T Khat_e du for the element owned by this slot: (u1, u2) and (x1, x2) are
+// dchi^T Khat_e du for the element owned by this slot: (u1, u2) and (x1, x2) are
 // the first and second neighbour rows of u_n and chi_{n+1}, already differences
 // u_b - u_a in the DIFF form, raw rows otherwise.
 template <typename T, int V, bool DIFF, bool SMEM_OWN = false>
-__device__ __forceinline__ void owner_grad(const RevArgs<T>& A, int e, const T* own, size_t S,
-                                           size_t col,
-                                           const Vec<T, V> (&u1)[3], const Vec<T, V> (&u2)[3],
-                                           const Vec<T, V> (&x1)[3], const Vec<T, V> (&x2)[3],
-                                           const Vec<T, V> (&ua)[3], const Vec<T, V> (&ca)[3]) {
+__device__ __forceinline__ Vec<T, V> owner_form(const T* own, const Vec<T, V> (&u1)[3],
+                                                const Vec<T, V> (&u2)[3],
+                                                const Vec<T, V> (&x1)[3],
+                                                const Vec<T, V> (&x2)[3],
+                                                const Vec<T, V> (&ua)[3],
+                                                const Vec<T, V> (&ca)[3]) {
     Vec<T, V> du1[3], du2[3], dy1[3], dy2[3];
 #pragma unroll
     for (int d = 0; d < 3; ++d) {
@@ -268,11 +281,80 @@ __device__ __forceinline__ void owner_grad(const RevArgs<T>& A, int e, const T* 
         vfma(g, dy1[i], z1);
         vfma(g, dy2[i], z2);
     }
+    return g;
+}
+
+// Gamma_e += that form.
+template <typename T, int V, bool DIFF, bool SMEM_OWN = false>
+__device__ __forceinline__ void owner_grad(const RevArgs<T>& A, int e, const T* own, size_t S,
+                                           size_t col,
+                                           const Vec<T, V> (&u1)[3], const Vec<T, V> (&u2)[3],
+                                           const Vec<T, V> (&x1)[3], const Vec<T, V> (&x2)[3],
+                                           const Vec<T, V> (&ua)[3], const Vec<T, V> (&ca)[3]) {
+    const Vec<T, V> g = owner_form<T, V, DIFF, SMEM_OWN>(own, u1, u2, x1, x2, ua, ca);
     T* gp = A.gam + (size_t)e * S + col;
     Vec<T, V> gv = ld<T, V>(gp);
 #pragma unroll
     for (int q = 0; q < V; ++q) gv.v[q] += g.v[q];
     st<T, V>(gp, gv);
+}
+
+// The rows that a free node's update reads besides its own u_n and chi_{n+1}.
+template <typename T, int V>
+struct RevRows {
+    Vec<T, V> u1[3], x2[3], im, gm;
+    T f[3];
+};
+template <typename T, int V, bool GM>
+__device__ __forceinline__ void rev_rows(const RevArgs<T>& A, int a, size_t col,
+                                         RevRows<T, V>& R) {
+    const size_t S = (size_t)A.S;
+    const uint32_t rowb = (uint32_t)A.S * sizeof(T), nodeb = 3 * rowb;
+    const T* qu = row_at(A.uo + col, a, nodeb);
+    const T* qx = row_at(A.xo + col, a, nodeb);
+#pragma unroll
+    for (int d = 0; d < 3; ++d) {
+        R.u1[d] = ld<T, V>(qu + d * S);
+        R.x2[d] = ld<T, V>(qx + d * S);
+        R.f[d] = __ldg(A.fhat + 4 * (size_t)a + d);
+    }
+    R.im = ldg<T, V>(row_at(A.invm + col, a, rowb));
+    if constexpr (GM) R.gm = ld<T, V>(row_at(A.gm + col, a, rowb));
+}
+// A free node's update from those rows.
+template <typename T, int V, bool GM>
+__device__ __forceinline__ void rev_update(const RevArgs<T>& A, int a, size_t col,
+                                           const Vec<T, V> (&ua)[3], const Vec<T, V> (&ca)[3],
+                                           const Vec<T, V> (&accU)[3],
+                                           const Vec<T, V> (&accC)[3], RevRows<T, V>& R, bool on) {
+    const size_t S = (size_t)A.S;
+    const uint32_t rowb = (uint32_t)A.S * sizeof(T), nodeb = 3 * rowb;
+    T* uo = row_at(A.uo + col, a, nodeb);
+    T* xo = row_at(A.xo + col, a, nodeb);
+    const T p = (T)A.p[0];
+    Vec<T, V> gacc = vzero<T, V>();
+#pragma unroll
+    for (int d = 0; d < 3; ++d) {
+        Vec<T, V> um, xn;
+#pragma unroll
+        for (int i = 0; i < V; ++i) {
+            const bool live = R.im.v[i] != T(0);
+            const T w = A.w0 * R.im.v[i];
+            const T r = fma(p, R.f[d], -accU[d].v[i]);
+            const T dv = ((R.u1[d].v[i] - ua[d].v[i]) - w * r) * A.inv1meta;
+            um.v[i] = live ? ua[d].v[i] - dv : T(0);
+            const T dx = ca[d].v[i] - R.x2[d].v[i];
+            xn.v[i] = live ? ca[d].v[i] + fma(-A.eta, dx, dx) - w * accC[d].v[i] : T(0);
+            if constexpr (GM) gacc.v[i] = fma(ca[d].v[i], r, gacc.v[i]);
+        }
+        if (on) st<T, V>(uo + d * S, um);
+        if (on) st<T, V>(xo + d * S, xn);
+    }
+    if constexpr (GM) {
+#pragma unroll
+        for (int q = 0; q < V; ++q) R.gm.v[q] += gacc.v[q];
+        if (on) st<T, V>(row_at(A.gm + col, a, rowb), R.gm);
+    }
 }
 
 // Node update of one reverse step: u_{n-1} (backward step), chi_n, and G += chi_{n+1} . r_n.
@@ -281,46 +363,19 @@ __device__ __forceinline__ void rev_epilogue(const RevArgs<T>& A, long long a, s
                                              size_t col, size_t row, const Vec<T, V> (&ua)[3],
                                              const Vec<T, V> (&ca)[3],
                                              const Vec<T, V> (&accU)[3],
-                                             const Vec<T, V> (&accC)[3]) {
+                                             const Vec<T, V> (&accC)[3], bool on = true) {
     if (a < A.n_clamped) {
         const Vec<T, V> cl = vfill<T, V>(A.clamp), z = vzero<T, V>();
 #pragma unroll
         for (int d = 0; d < 3; ++d) {
-            st<T, V>(A.uo + row + d * S, cl);
-            st<T, V>(A.xo + row + d * S, z);
+            if (on) st<T, V>(A.uo + row + d * S, cl);
+            if (on) st<T, V>(A.xo + row + d * S, z);
         }
         return;
     }
-    const T p = (T)A.p[0];
-    const Vec<T, V> im = ldg<T, V>(A.invm + (size_t)a * S + col);
-    Vec<T, V> gacc = vzero<T, V>();
-#pragma unroll
-    for (int d = 0; d < 3; ++d) {
-        const T f = p * __ldg(A.fhat + 4 * a + d);
-        const Vec<T, V> u1 = ld<T, V>(A.uo + row + d * S);
-        const Vec<T, V> x2o = ld<T, V>(A.xo + row + d * S);
-        Vec<T, V> um, xn;
-#pragma unroll
-        for (int i = 0; i < V; ++i) {
-            const bool live = im.v[i] != T(0);
-            const T w = A.w0 * im.v[i];
-            const T r = f - accU[d].v[i];
-            const T dv = ((u1.v[i] - ua[d].v[i]) - w * r) * A.inv1meta;
-            um.v[i] = live ? ua[d].v[i] - dv : T(0);
-            const T dx = ca[d].v[i] - x2o.v[i];
-            xn.v[i] = live ? ca[d].v[i] + fma(-A.eta, dx, dx) - w * accC[d].v[i] : T(0);
-            if constexpr (GM) gacc.v[i] = fma(ca[d].v[i], r, gacc.v[i]);
-        }
-        st<T, V>(A.uo + row + d * S, um);
-        st<T, V>(A.xo + row + d * S, xn);
-    }
-    if constexpr (GM) {
-        T* gp = A.gm + (size_t)a * S + col;
-        Vec<T, V> gv = ld<T, V>(gp);
-#pragma unroll
-        for (int q = 0; q < V; ++q) gv.v[q] += gacc.v[q];
-        st<T, V>(gp, gv);
-    }
+    RevRows<T, V> R;
+    rev_rows<T, V, GM>(A, (int)a, col, R);
+    rev_update<T, V, GM>(A, (int)a, col, ua, ca, accU, accC, R, on);
 }
 
 // One reverse step for (node a, V samples): reconstruct u_{n-1}, advance chi, accumulate
@@ -609,128 +664,221 @@ __global__ void __launch_bounds__(256, MINB) k_reverse_fan(RevArgs<T> A) {
     rev_epilogue<T, V, GM>(A, a, S, col, row, ua, ca, accU, accC);
 }
 
-// ------------------------------------------------------------ persistent reverse step
-// k_reverse_fan as a persistent grid: each block walks work items (node block, sample
-// chunk; chunk fastest) with a stride of the grid and stages the slot records,
-// stiffness rows and owner blocks of its NEXT item by TMA into the other of two
-// shared-memory stages while its warps run the current one.  Stage s of the block's
-// i-th item completes its mbarrier's phase (i / 2) % 2; a block barrier at the end of
-// every item frees the stage for reuse.  Same products in the same order: same bits.
-template <typename T>
-__device__ __forceinline__ void revp_issue(const RevArgs<T>& A, long long w, uint32_t bar,
-                                           int4* srec, T* sslab, T* sown) {
-    const long long nb = w / A.nch;
-    const long long a0 = nb * A.npb;
-    const long long a1 = (a0 + A.npb < A.n_nodes) ? a0 + A.npb : A.n_nodes;
-    const int kb = __ldg(A.node_ptr + a0), ke = __ldg(A.node_ptr + a1);
-    const int nsl = ke - kb;
-    if (nsl > A.cap_slots || nsl <= 0) {
-        if (nsl > A.cap_slots && A.status) atomicOr(A.status, 2);
-        mbar_arrive_expect_tx(bar, 0);
-        return;
-    }
-    const uint32_t b_rec = (uint32_t)nsl * 16u;
-    const uint32_t b_slab = (uint32_t)nsl * (uint32_t)(kSlabStride * sizeof(T));
-    mbar_arrive_expect_tx(bar, b_rec + 2 * b_slab);
-    bulk_g2s(smem_u32(srec), A.rec + kb, b_rec, bar);
-    bulk_g2s(smem_u32(sslab), A.slab + (size_t)kb * kSlabStride, b_slab, bar);
-    bulk_g2s(smem_u32(sown), A.own + (size_t)kb * kOwnStride, b_slab, bar);
-}
-
-template <typename T, int V, bool DIFF, bool GM, int MINB>
-__global__ void __launch_bounds__(256, MINB) k_reverse_fanp(RevArgs<T> A, long long n_items) {
+// ------------------------------------------------------------ patch reverse step
+// The reverse step with free-running warps on patches of nodes, as the forward patch kernel
+// (solid_patch.cu): 32 * V samples of one node at a time, the next node's slots (records,
+// stiffness rows, owner blocks) staged in shared memory and its rows prefetched into L2
+// under the current node.  Clamped nodes are walked like the others: they own elements.
+// It waits on the gathers of two states a neighbour, so the closed fan of six is unrolled
+// (one element ahead; the update's rows in the place of element 7) and an owned element's
+// Gamma row is requested before its products.  us a step, fan or persistent fan / this:
+// 128 x 400 wall, FP32 64 samples 155 / 116, 128 samples with G 315 / 235; 128 x 320 wall, FP64
+// 64 samples with G 267 / 213; 64 x 128 wall, 64 samples FP32 22.4 / 21.3, FP64 54.7 / 46.4.
+template <typename T, int V, bool GM>
+__global__ void __launch_bounds__(32 * kPatchWarps, 1)
+    k_reverse_patch(RevArgs<T> A, PatchMap M, int max_degree) {
     extern __shared__ __align__(16) unsigned char smem[];
-    const int warp = threadIdx.x >> 5;
-    const int lane = threadIdx.x & 31;
-    const size_t cap = (size_t)A.cap_slots;
-    const size_t stage_bytes = cap * (16 + 2 * kSlabStride * sizeof(T));
-    // stage q: records, stiffness rows, owner blocks at smem + 16 + q * stage_bytes
-    const uint32_t bar0 = smem_u32(smem);
-    auto srec_of = [&](int q) {
-        return reinterpret_cast<int4*>(smem + 16 + q * stage_bytes);
+    constexpr bool DIFF = std::is_same<T, float>::value;
+    using P = SlotStage<T>;
+    constexpr int kOwnWords = kOwnStride * (int)sizeof(T) / 16;
+    const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
+    const uint32_t b_rec = 16u * max_degree, b_slab = P::kSlotBytes * max_degree;
+    const uint32_t b_stage = b_rec + b_slab + 16u * kOwnWords * max_degree;
+    unsigned char* const wb = smem + warp * (2 * b_stage);
+    const uint32_t rowb = (uint32_t)A.S * sizeof(T), nodeb = 3 * rowb;
+    const int chunk = blockIdx.x % A.nch;
+    const int vec = chunk * 32 + lane, last = A.S / V - 1;
+    const bool on = vec <= last;
+    const size_t S = (size_t)A.S, col = (size_t)(on ? vec : last) * V;
+    PatchWalk walk(M, warp, blockIdx.x / A.nch, gridDim.x / A.nch, 0, (int)A.n_nodes);
+    auto stage = [&](int b, int k0, int n, int sg) {
+        if (b >= 0) {
+            const uint32_t d = smem_u32(wb + sg * b_stage);
+            const char* r = reinterpret_cast<const char*>(A.rec + k0);
+            const char* s = reinterpret_cast<const char*>(A.slab + (size_t)k0 * kSlabStride);
+            const char* o = reinterpret_cast<const char*>(A.own + (size_t)k0 * kOwnStride);
+            for (int q = lane; q < n; q += 32) cp_async<16>(d + 16 * q, r + 16 * q);
+            for (int q = lane; q < P::kWords * n; q += 32) {
+                const int sl = q / P::kWords, w = q - sl * P::kWords;
+                cp_async<16>(d + b_rec + 16 * q,
+                             s + sl * (kSlabStride * (int)sizeof(T)) + (P::kFirst + w) * 16);
+            }
+            for (int q = lane; q < kOwnWords * n; q += 32)
+                cp_async<16>(d + b_rec + b_slab + 16 * q, o + 16 * q);
+        }
+        cp_async_commit();
     };
-    auto sslab_of = [&](int q) {
-        return reinterpret_cast<T*>(smem + 16 + q * stage_bytes + cap * 16);
+    bool more = walk.more(M);
+    int a = walk.node(M), n, an, k0, nn;
+    node_slots(A.node_ptr, a, k0, n);
+    stage(a, k0, n, 0);
+    walk.advance(M);
+    an = walk.node(M);
+    node_slots(A.node_ptr, an, k0, nn);
+    // line prefetch: rows 0..2 u_n, 3..5 chi_{n+1}, 6..8 u_{n+1}, 9..11 chi_{n+2}, 12 inverse
+    // mass, 13 G; then coefficient rows and, by the owner, Gamma rows
+    const RowLines<T, V> ln(lane, chunk, rowb);
+    auto prefetch_node = [&](int b) {
+        if (b < 0 || !ln.on) return;
+#pragma unroll
+        for (int r0 = 0; r0 < (GM ? 14 : 13); r0 += RowLines<T, V>::kRows) {
+            const int r = r0 + ln.row;
+            const T* q = r < 3    ? A.u + r * S
+                         : r < 6  ? A.x + (r - 3) * S
+                         : r < 9  ? A.uo + (r - 6) * S
+                         : r < 12 ? A.xo + (r - 9) * S
+                         : r < 13 ? A.invm
+                                  : A.gm;
+            if (r < (GM ? 14 : 13))
+                prefetch_l2(reinterpret_cast<const char*>(q) + ln.off +
+                            (uint64_t)(uint32_t)b * (r < 12 ? nodeb : rowb));
+        }
     };
-    auto sown_of = [&](int q) { return sslab_of(q) + cap * kSlabStride; };
-    if (threadIdx.x == 0) {
-        mbar_init(bar0, 1);
-        mbar_init(bar0 + 8, 1);
-    }
-    __syncthreads();
-    long long w = blockIdx.x;
-    if (threadIdx.x == 0 && w < n_items) revp_issue<T>(A, w, bar0, srec_of(0), sslab_of(0), sown_of(0));
-    const size_t S = (size_t)A.S;
-    for (int it = 0; w < n_items; w += gridDim.x, ++it) {
-        const int sg = it & 1;
-        const long long wn = w + gridDim.x;
-        if (threadIdx.x == 0 && wn < n_items)
-            revp_issue<T>(A, wn, bar0 + 8 * (sg ^ 1), srec_of(sg ^ 1), sslab_of(sg ^ 1),
-                          sown_of(sg ^ 1));
-        const long long nb = w / A.nch;
-        const int chunk = (int)(w - nb * A.nch);
-        const long long a0 = nb * A.npb;
-        const long long a1 = (a0 + A.npb < A.n_nodes) ? a0 + A.npb : A.n_nodes;
-        const long long a = a0 + warp;
-        const bool active = warp < A.npb && a < a1;
-        const size_t col = ((size_t)chunk * 32 + lane) * V;
-        const size_t row = (size_t)a * 3 * S + col;
+    grid_dependency_release();
+    grid_dependency_wait();
+    const T* const u = A.u + col;
+    const T* const x = A.x + col;
+    const T* const cf = A.coef + col;
+    T* const gam = A.gam + col;
+    for (int sg = 0; more; sg ^= 1) {
         Vec<T, V> ua[3], ca[3];
-        if (active) {
+        auto rows = [&](Vec<T, V> (&p)[3], Vec<T, V> (&q)[3], int b) {
+            const uint64_t o = (uint64_t)(uint32_t)b * nodeb;
+            const T* pu = reinterpret_cast<const T*>(reinterpret_cast<const char*>(u) + o);
+            const T* px = reinterpret_cast<const T*>(reinterpret_cast<const char*>(x) + o);
 #pragma unroll
             for (int d = 0; d < 3; ++d) {
-                ua[d] = ldg<T, V>(A.u + row + d * S);
-                ca[d] = ldg<T, V>(A.x + row + d * S);
-                prefetch_l2(A.uo + row + d * S);
-                prefetch_l2(A.xo + row + d * S);
+                p[d] = ldg<T, V>(pu + d * S);
+                q[d] = ldg<T, V>(px + d * S);
             }
-            prefetch_l2(A.invm + (size_t)a * S + col);
-        }
-        if (A.pf_dist > 0 && chunk == 0 && nb % A.pf_group == 0 && warp == A.npb - 1)
-            rev_prefetch<T, GM>(A, a0 + A.pf_dist, A.npb * A.pf_group, lane);
-        if (!mbar_wait_bounded(bar0 + 8 * sg, (uint32_t)((it >> 1) & 1), kMaxPolls)) {
-            if (lane == 0 && A.status) atomicOr(A.status, 1);
-            return;
-        }
-        if (active) {
-            const int4* srec = srec_of(sg);
-            const T* sslab = sslab_of(sg);
-            const T* sown = sown_of(sg);
-            const int kb = __ldg(A.node_ptr + a0);
+        };
+        if (a >= 0) rows(ua, ca, a);
+        cp_async_wait_all();
+        __syncwarp();
+        const unsigned char* const st = wb + sg * b_stage;
+        const int4* const srec = reinterpret_cast<const int4*>(st);
+        const T* const K = reinterpret_cast<const T*>(st + b_rec) - 16 / (int)sizeof(T) * P::kFirst;
+        const T* const own = reinterpret_cast<const T*>(st + b_rec + b_slab);
+        constexpr int kStep = P::kSlotBytes / (int)sizeof(T);
+        stage(an, k0, nn, sg ^ 1);
+        prefetch_node(an);
+        const int nn_cur = nn;
+        more = walk.more(M);
+        walk.advance(M);
+        const int ax = walk.node(M);
+        node_slots(A.node_ptr, ax, k0, nn);
+        auto prefetch_elems = [&]() {  // coefficient rows and owned Gamma rows of the next node
+            cp_async_wait_all();
+            __syncwarp();
+            const int4* nr = reinterpret_cast<const int4*>(wb + (sg ^ 1) * b_stage);
+            constexpr int kHalf = RowLines<T, V>::kRows / 2;
+            const int q = ln.row % kHalf;
+            if (an >= 0 && ln.on && q < nn_cur) {
+                const bool gamma = ln.row >= kHalf;
+                const int4 r = nr[q];
+                if (!gamma || ((r.w >> 8) & 3) == 0)
+                    prefetch_l2(reinterpret_cast<const char*>(gamma ? A.gam : A.coef) + ln.off +
+                                (uint64_t)(uint32_t)r.x * rowb);
+            }
+        };
+        if (a >= 0) {
             Vec<T, V> accU[3], accC[3];
 #pragma unroll
-            for (int d = 0; d < 3; ++d) {
-                accU[d] = vzero<T, V>();
-                accC[d] = vzero<T, V>();
-            }
-            const int k0 = __ldg(A.node_ptr + a) - kb, k1 = __ldg(A.node_ptr + a + 1) - kb;
-            if (k0 < k1) {
+            for (int d = 0; d < 3; ++d) accU[d] = accC[d] = vzero<T, V>();
+            auto element = [&](int k, const int4& r, const Vec<T, V>& c, const Vec<T, V> (&u1)[3],
+                               const Vec<T, V> (&u2)[3], const Vec<T, V> (&x1)[3],
+                               const Vec<T, V> (&x2)[3]) {
+                const bool owner = ((r.w >> 8) & 3) == 0;
+                Vec<T, V> gv = vzero<T, V>();
+                T* const gp = row_at(gam, r.x, rowb);
+                if (owner) gv = ld<T, V>(gp);  // requested before the products
+                slot_fma2<T, V, DIFF>(K + kStep * k, c, u1, u2, x1, x2, ua, ca, accU, accC);
+                if (owner) {
+                    const Vec<T, V> g = owner_form<T, V, DIFF, true>(own + kOwnStride * k, u1, u2,
+                                                                     x1, x2, ua, ca);
+#pragma unroll
+                    for (int q = 0; q < V; ++q) gv.v[q] += g.v[q];
+                    if (on) cvfes::st<T, V>(gp, gv);
+                }
+            };
+            RevRows<T, V> R;
+            const int flag = lane < n ? srec[lane].w : 1;
+            const bool six = n == 6 && __all_sync(0xffffffffu, (flag & 1) || lane == 0);
+            if (six) {  // closed fan: unrolled, the update's rows in the place of element 6
+                Vec<T, V> U[8][3], X[8][3], C[7];
+                rows(U[0], X[0], srec[0].y);
+                rows(U[1], X[1], srec[0].z);
+                C[0] = ldg<T, V>(row_at(cf, srec[0].x, rowb));
+                diff3<T, V, DIFF>(U[0], ua);
+                diff3<T, V, DIFF>(X[0], ca);
+#pragma unroll
+                for (int k = 0; k < 6; ++k) {
+                    if (k < 5) {
+                        const int4 rn = srec[k + 1];
+                        rows(U[k + 2], X[k + 2], rn.z);
+                        C[k + 1] = ldg<T, V>(row_at(cf, rn.x, rowb));
+                    } else {
+                        if (a >= A.n_clamped) rev_rows<T, V, GM>(A, a, col, R);
+                    }
+                    if (k == 2) prefetch_elems();
+                    if constexpr (DIFF) __syncwarp();
+                    diff3<T, V, DIFF>(U[k + 1], ua);
+                    diff3<T, V, DIFF>(X[k + 1], ca);
+                    element(k, srec[k], C[k], U[k], U[k + 1], X[k], X[k + 1]);
+                    if constexpr (DIFF) __syncwarp();
+                }
+            } else if (n > 0) {
                 Vec<T, V> U0[3], U1[3], U2[3], X0[3], X1[3], X2[3], c0, c1, c2;
-                const int4 r0 = srec[k0];
-                load3<T, V>(U0, A.u, r0.y, S, col);
-                load3<T, V>(X0, A.x, r0.y, S, col);
-                load3<T, V>(U1, A.u, r0.z, S, col);
-                load3<T, V>(X1, A.x, r0.z, S, col);
-                c1 = ldg<T, V>(A.coef + (size_t)r0.x * S + col);
+                int4 r = srec[0];
+                rows(U0, X0, r.y);
+                rows(U1, X1, r.z);
+                c1 = ldg<T, V>(row_at(cf, r.x, rowb));
                 diff3<T, V, DIFF>(U0, ua);
                 diff3<T, V, DIFF>(X0, ca);
-                int k = k0;
+                int k = 0;
+                auto phase = [&](Vec<T, V> (&pu)[3], Vec<T, V> (&px)[3], Vec<T, V> (&cu)[3],
+                                 Vec<T, V> (&cx)[3], const Vec<T, V>& c, Vec<T, V> (&nu)[3],
+                                 Vec<T, V> (&nx)[3], Vec<T, V>& cn) {
+                    const bool next = k + 1 < n;
+                    int4 rn = make_int4(0, 0, 0, 1);
+                    if (next) {
+                        rn = srec[k + 1];
+                        rows(nu, nx, rn.z);
+                        cn = ldg<T, V>(row_at(cf, rn.x, rowb));
+                    }
+                    diff3<T, V, DIFF>(cu, ua);
+                    diff3<T, V, DIFF>(cx, ca);
+                    element(k, r, c, pu, cu, px, cx);
+                    if (next && !(rn.w & 1)) {  // fan break: the next first neighbour is new
+                        rows(cu, cx, rn.y);
+                        diff3<T, V, DIFF>(cu, ua);
+                        diff3<T, V, DIFF>(cx, ca);
+                    }
+                    r = rn;
+                    ++k;
+                };
                 while (true) {
-                    rev_phase<T, V, DIFF>(k, k1, srec, sslab, sown, A, S, col, ua, ca, accU, accC,
-                                          U0, X0, U1, X1, c1, U2, X2, c2);
-                    if (k >= k1) break;
-                    rev_phase<T, V, DIFF>(k, k1, srec, sslab, sown, A, S, col, ua, ca, accU, accC,
-                                          U1, X1, U2, X2, c2, U0, X0, c0);
-                    if (k >= k1) break;
-                    rev_phase<T, V, DIFF>(k, k1, srec, sslab, sown, A, S, col, ua, ca, accU, accC,
-                                          U2, X2, U0, X0, c0, U1, X1, c1);
-                    if (k >= k1) break;
+                    phase(U0, X0, U1, X1, c1, U2, X2, c2);
+                    if (k >= n) break;
+                    phase(U1, X1, U2, X2, c2, U0, X0, c0);
+                    if (k >= n) break;
+                    phase(U2, X2, U0, X0, c0, U1, X1, c1);
+                    if (k >= n) break;
                 }
             }
-            rev_epilogue<T, V, GM>(A, a, S, col, row, ua, ca, accU, accC);
+            if (!six) prefetch_elems();
+            if (six && a >= A.n_clamped)
+                rev_update<T, V, GM>(A, a, col, ua, ca, accU, accC, R, on);
+            else
+                rev_epilogue<T, V, GM>(A, a, S, col, (size_t)a * 3 * S + col, ua, ca, accU, accC,
+                                       on);
         }
-        __syncthreads();
+        __syncwarp();
+        a = an;
+        n = nn_cur;
+        an = ax;
     }
+    cp_async_wait_all();
 }
 
 // dJ/dlogE = -c Gamma; dJ/dlogh = -c Gamma - h sum_a alpha_{e,a} G_a / m_a.
@@ -768,14 +916,12 @@ struct RevTuning {
     int vec;      // samples per thread (upper bound)
     int npb;      // nodes (warps) per block of the fan kernel
     int variant;  // 0: L1-gather kernel; 1: fan-rotation kernel with staged slots;
-                  // 2: as 1, persistent, the next item's slots staged under the current
+                  // 2: persistent patch kernel (npb and minb have no effect)
     int minb;     // resident blocks per SM asked of the compiler (fan kernel)
 };
-// Defaults from sweeps on B200: FP32 on the 256x1024 tube with 128 samples and the
-// stenosed 512x2048 tube (reverse 6.25 s per 1000 steps; the persistent variant 7.89 s);
-// FP64 on the 64x128 tube with 64 samples (reverse pass of 500 steps: vec 1 with 4 nodes
-// per block 29.6 ms, vec 2 with 2 nodes 30.6 ms, persistent 30.2 ms).
-static RevTuning g_rev32 = {2, 2, 1, 2};
+// Defaults: the patch kernel, which takes 2 FP32 samples or 1 FP64 sample a thread (figures
+// at the kernel).
+static RevTuning g_rev32 = {2, 2, 2, 2};
 static RevTuning g_rev64 = {1, 4, 2, 2};
 template <typename T>
 RevTuning& rev_tuning() {
@@ -809,47 +955,32 @@ int launch_rev_fan_m(int minb, unsigned grid, int threads, size_t smem, cudaStre
     }
 }
 
-// The persistent reverse kernel on as many blocks as are resident (at most one per item).
-template <typename Kern, typename T>
-int launch_rev_fanp(Kern kernel, long long n_items, int threads, size_t smem, cudaStream_t st,
-                    const RevArgs<T>& A) {
+// The patch kernel (variant 2); returns 1 without launching when a node's slots do not fit.
+template <typename T, int V>
+int launch_rev_patch(const cvfes_solid_mesh* m, RevArgs<T> A, bool after_step, cudaStream_t st) {
+    const size_t slot = SlotStage<T>::kBytes + kOwnStride * sizeof(T);
+    if (m->max_degree <= 0 || m->max_degree >= 1024 || A.S >= (1 << 27) ||
+        m->n_nodes >= INT32_MAX / 2)
+        return 1;
+    const size_t smem = (size_t)kPatchWarps * 2 * slot * m->max_degree;
+    if (smem > 160 * 1024) return 1;
+    A.nch = (A.S / V + 31) / 32;
+    const PatchMap M = patch_map(m->n_nodes, m->bandwidth);
+    auto kernel = A.gm ? k_reverse_patch<T, V, true> : k_reverse_patch<T, V, false>;
     int per_sm = 0;
-    const int rc =
-        fanp_blocks_per_sm(reinterpret_cast<const void*>(kernel), threads, smem, &per_sm);
+    const int rc = fanp_blocks_per_sm(reinterpret_cast<const void*>(kernel), 32 * kPatchWarps,
+                                      smem, &per_sm);
     if (rc) return rc;
-    long long blocks = (long long)per_sm * device_sm_count();
-    if (blocks > n_items) blocks = n_items;
-    kernel<<<(unsigned)blocks, threads, smem, st>>>(A, n_items);
-    CVFES_LAUNCH_CHECK("k_reverse_fanp");
-    return CVFES_OK;
-}
-
-template <typename T, int V, bool DIFF, bool GM>
-int launch_rev_fanp_m(int minb, long long n_items, int threads, size_t smem, cudaStream_t st,
-                      const RevArgs<T>& A) {
-    switch (minb) {
-        case 3:
-            return launch_rev_fanp(k_reverse_fanp<T, V, DIFF, GM, 3>, n_items, threads, smem, st,
-                                   A);
-        case 2:
-            return launch_rev_fanp(k_reverse_fanp<T, V, DIFF, GM, 2>, n_items, threads, smem, st,
-                                   A);
-        default:
-            return launch_rev_fanp(k_reverse_fanp<T, V, DIFF, GM, 1>, n_items, threads, smem, st,
-                                   A);
-    }
+    const long long places = std::max(1LL, (long long)M.n_strips * M.tps);
+    const long long per_chunk =
+        std::max(1LL, std::min((long long)per_sm * device_sm_count() / A.nch, places));
+    return launch_step_kernel(kernel, dim3((unsigned)(per_chunk * A.nch)), 32 * kPatchWarps, smem,
+                              after_step, st, "k_reverse_patch", A, M, (int)m->max_degree);
 }
 
 template <typename T, int V, bool DIFF>
 int launch_rev_v(const RevTuning& tu, bool fan, bool gmv, unsigned fan_grid, size_t smem,
                  const RowGrid& rg, cudaStream_t st, const RevArgs<T>& A) {
-    if (fan && tu.variant == 2) {
-        const int threads = 32 * tu.npb;
-        const size_t smem2 = 16 + 2 * (smem - 16);
-        return gmv ? launch_rev_fanp_m<T, V, DIFF, true>(tu.minb, fan_grid, threads, smem2, st, A)
-                   : launch_rev_fanp_m<T, V, DIFF, false>(tu.minb, fan_grid, threads, smem2, st,
-                                                          A);
-    }
     if (fan) {
         const int threads = 32 * tu.npb;
         return gmv ? launch_rev_fan_m<T, V, DIFF, true>(tu.minb, fan_grid, threads, smem, st, A)
@@ -863,7 +994,7 @@ int launch_rev_v(const RevTuning& tu, bool fan, bool gmv, unsigned fan_grid, siz
 
 template <typename T>
 int launch_reverse_step(const cvfes_adjoint_desc* d, const T* u, T* uo, const T* x, T* xo,
-                        long long n, cudaStream_t st) {
+                        long long n, bool after_step, cudaStream_t st) {
     const cvfes_solid_mesh* m = &d->mesh;
     RevArgs<T> A;
     A.node_ptr = m->node_ptr;
@@ -902,6 +1033,16 @@ int launch_reverse_step(const cvfes_adjoint_desc* d, const T* u, T* uo, const T*
         for (int i = 0; i < 8; ++i)
             if (ptrs[i] && reinterpret_cast<uintptr_t>(ptrs[i]) % (V * sizeof(T))) ok = false;
         if (ok) break;
+    }
+    // below 20 samples most lanes of a patch warp would idle: the row-gather kernel (128 x 400
+    // wall, FP32, us a step: 16 samples 69 against about 92, 24 samples 104 / 92)
+    if (tu.variant == 2 && A.S >= 20) {
+        int prc = 1;
+        if constexpr (sizeof(T) == 4) {
+            if (V >= 2 && (A.S + 31) / 32 > (A.S / 2 + 31) / 32) prc = launch_rev_patch<T, 2>(m, A, after_step, st);
+        }
+        if (prc == 1) prc = launch_rev_patch<T, 1>(m, A, after_step, st);
+        if (prc <= 0) return prc;
     }
     const RowGrid rg = row_grid(m->n_nodes, A.S / V, 256);
     A.tpn = rg.tpn;
@@ -954,6 +1095,8 @@ int check_adjoint(const cvfes_adjoint_desc* d, const char* who) {
     return CVFES_OK;
 }
 
+__global__ void k_set_clock(long long* clock, long long n) { clock[0] = n; }
+
 template <typename T>
 int adjoint_forward(const cvfes_adjoint_desc* d, int* out_cur, int* out_prev, cudaStream_t st) {
     int rc = check_adjoint(d, "cvfes_adjoint_forward");
@@ -968,7 +1111,6 @@ int adjoint_forward(const cvfes_adjoint_desc* d, int* out_cur, int* out_prev, cu
     T* ck = static_cast<T*>(d->ckpt);
     T* obs = static_cast<T*>(d->obs);
     for (int q = 0; q < 3; ++q) CVFES_CUDA_TRY(cudaMemsetAsync(buf[q], 0, sbytes, st));
-    CVFES_CUDA_TRY(cudaMemsetAsync(d->clock, 0, sizeof(int64_t), st));
     CVFES_CUDA_TRY(cudaMemsetAsync(d->J, 0, S * sizeof(double), st));
     const int nchunk = (d->n_obs + kObsChunk - 1) / kObsChunk;
     int cur = 0, prev = 1, nxt = 2;
@@ -985,12 +1127,12 @@ int adjoint_forward(const cvfes_adjoint_desc* d, int* out_cur, int* out_prev, cu
         if constexpr (sizeof(T) == 8)
             rc = cvfes_solid_advance_f64(m, static_cast<const double*>(d->coef),
                                          static_cast<const double*>(d->invm), buf[cur], buf[prev],
-                                         buf[nxt], d->p_sched, d->clock, next - n, d->dt, d->damp,
+                                         buf[nxt], d->p_sched + n, nullptr, next - n, d->dt, d->damp,
                                          &ci, &pi, st);
         else
             rc = cvfes_solid_advance_f32(m, static_cast<const float*>(d->coef),
                                          static_cast<const float*>(d->invm), buf[cur], buf[prev],
-                                         buf[nxt], d->p_sched, d->clock, next - n, d->dt, d->damp,
+                                         buf[nxt], d->p_sched + n, nullptr, next - n, d->dt, d->damp,
                                          &ci, &pi, st);
         if (rc) return rc;
         cur = order[ci];
@@ -1012,10 +1154,12 @@ int adjoint_forward(const cvfes_adjoint_desc* d, int* out_cur, int* out_prev, cu
             CVFES_LAUNCH_CHECK("k_obs");
         }
     }
+    k_set_clock<<<1, 1, 0, st>>>(reinterpret_cast<long long*>(d->clock), T_);
+    CVFES_LAUNCH_CHECK("k_set_clock");
     const long long n_obs_steps = T_ / K;
     if (!d->record && d->n_obs > 0 && n_obs_steps > 0) {
-        k_obs_reduce<<<(unsigned)((S + 127) / 128), 128, 0, st>>>(n_obs_steps * nchunk, (int)S,
-                                                                 d->jpart, d->J);
+        k_obs_reduce<<<grid_1d(S, kReduceSamples), kReduceSamples * kReduceGroups, 0, st>>>(
+            n_obs_steps * nchunk, (int)S, d->jpart, d->J);
         CVFES_LAUNCH_CHECK("k_obs_reduce");
     }
     if (out_cur) *out_cur = cur;
@@ -1060,15 +1204,18 @@ int adjoint_reverse(const cvfes_adjoint_desc* d, int cur, int prev, cudaStream_t
         rc = adjoint_force<T>(d, uB, xA, T_ / K - 1, st);
         if (rc) return rc;
     }
+    bool after_step = false;  // the launch before is a reverse step: this one may overlap it
     for (long long n = T_ - 1; n >= 0; --n) {
         if (n % C == 0) {
+            after_step = false;
             const T* slot = ck + (size_t)(n / C) * 2 * state;
             CVFES_CUDA_TRY(cudaMemcpyAsync(uA, slot, sbytes, cudaMemcpyDeviceToDevice, st));
             CVFES_CUDA_TRY(
                 cudaMemcpyAsync(uB, slot + state, sbytes, cudaMemcpyDeviceToDevice, st));
         }
-        rc = launch_reverse_step<T>(d, uA, uB, xA, xB, n, st);
+        rc = launch_reverse_step<T>(d, uA, uB, xA, xB, n, after_step, st);
         if (rc) return rc;
+        after_step = true;
         T* t = uA;
         uA = uB;
         uB = t;
@@ -1079,6 +1226,7 @@ int adjoint_reverse(const cvfes_adjoint_desc* d, int cur, int prev, cudaStream_t
         if (n > 0 && n % K == 0) {
             rc = adjoint_force<T>(d, uB, xA, n / K - 1, st);
             if (rc) return rc;
+            after_step = after_step && d->n_obs <= 0;
         }
     }
     return CVFES_OK;
