@@ -507,9 +507,11 @@ def measure_batched(args, prec, rank, world, local, dev, steps, warm, meshes_cas
         "steps": steps, "warmup": warm, "finite": finite, "state_form": batch.state_form,
         "value": world * S_total * steps / (ms_max * 1e-3), "unit": UNIT,
         "ms_per_step": ms_max / steps,
-        "kernel": "fan" if batch.variant == 1 else "row gather", "vec": tuned.get("vec"),
+        "kernel": "single-mesh" if batch.by_mesh else
+        "fan" if batch.variant == 1 else "row gather", "vec": tuned.get("vec"),
         "grid": tuned.get("grid"), "launch_groups": n_groups,
-        "gpu_launches": n_groups * (steps + steps // batch.graph_chunk + 1),
+        "gpu_launches": (len(meshes) if batch.by_mesh else n_groups) *
+        (steps + steps // batch.graph_chunk + 1),
         "roofline": {"bound": "hbm", "achieved": achieved, "peak": peaks["hbm_gbs"],
                      "unit": "GB/s", "frac": achieved / peaks["hbm_gbs"],
                      "peak_source": peak_kind, "bytes_per_step": bstep},

@@ -9,7 +9,7 @@ slot rows staged by TMA, fan-rotation gathers) and the row-gather kernel
 (``variant`` 0).  A mesh advanced in a batch is bitwise identical to the same mesh
 advanced alone by the single-mesh kernels.
 
-Meshes are packed in groups of one work-item shape (nodes per fan item, which the
+In the table, meshes are packed in groups of one work-item shape (nodes per fan item, which the
 sample count sets), one table and one launch per group and step.  The fan kernel's
 shared-memory stage is sized for the largest item of its launch, and shared memory
 comes out of the same on-chip storage as L1: in one launch over the whole uneven
@@ -50,6 +50,14 @@ def fan_item_nodes(S: int, vec: int) -> int:
     return 32 // min(32, sv)
 
 
+def _roles(state_form, rot):
+    """Buffers of (u_n, u_{n-1} or the increment, free) at phase rot (steps taken mod 6)."""
+    if state_form == "velocity":
+        return (2, 1, 0) if rot & 1 else (0, 1, 2)
+    cur = (3 - rot % 3) % 3
+    return cur, (cur + 1) % 3, (cur + 2) % 3
+
+
 class _Group:
     """Meshes of one fan-item shape: their table, counts, clock and graphs."""
 
@@ -59,6 +67,12 @@ class _Group:
         self.clock = torch.zeros(1, dtype=torch.int64, device=device)
         self.table = torch.empty(n_bytes, dtype=torch.uint8, device=device)
         self.graphs = {}
+
+
+# Node-samples below which a mesh's step does not fill the chip (its launches run beside
+# other small meshes').  SMALLNOTE
+SMALL_MESH = 400_000
+SMALL_STREAMS = 4
 
 
 class BatchedSolidSolver:
@@ -98,6 +112,8 @@ class BatchedSolidSolver:
         # then share the SMs and L2 for their whole length, not only at their tails.
         self.concurrent = concurrent
         self._group_streams: List[torch.cuda.Stream] = []
+        self._mesh_clocks = torch.zeros(len(meshes), dtype=torch.int64, device=self.device)
+        self._mesh_graphs: List[dict] = [dict() for _ in meshes]
         self.totals = (_lib.C.c_int64 * 3)()
         self.graph_chunk = graph_chunk
         self.rot = 0
@@ -184,6 +200,11 @@ class BatchedSolidSolver:
             self._pack()
         with torch.cuda.device(self.device):
             self._p[:n].copy_(torch.from_numpy(p), non_blocking=False)
+            if self.by_mesh:
+                self._advance_by_mesh(n, use_graph)
+                self.steps += n
+                self.sync_roles()
+                return self
             for g in self.groups:
                 g.clock.zero_()
             done = 0
@@ -208,6 +229,72 @@ class BatchedSolidSolver:
         self.sync_roles()
         return self
 
+    @property
+    def by_mesh(self) -> bool:
+        """Whether the meshes take the single-mesh kernels one after another."""
+        return (self.variant == 1 and self.grid == 0 and self.grouped and not self.concurrent)
+
+    def _advance_by_mesh(self, n, use_graph):
+        """n steps of every mesh: the small meshes side by side, then the others in turn."""
+        main = torch.cuda.current_stream(self.device)
+        self._mesh_clocks.zero_()
+        small = [i for i, s in enumerate(self.solvers)
+                 if s.lclNNodes * s.nSmp < SMALL_MESH]
+        if len(small) > 1:
+            while len(self._group_streams) < min(SMALL_STREAMS, len(small)):
+                self._group_streams.append(torch.cuda.Stream(device=self.device))
+            streams = self._group_streams[:min(SMALL_STREAMS, len(small))]
+            start = torch.cuda.Event()
+            start.record(main)
+            for st in streams:
+                st.wait_event(start)
+            try:
+                for j, i in enumerate(small):
+                    self._advance_mesh(i, n, use_graph, streams[j % len(streams)].cuda_stream)
+            finally:  # the caller's stream waits for whatever was launched
+                for st in streams:
+                    end = torch.cuda.Event()
+                    end.record(st)
+                    main.wait_event(end)
+        else:
+            small = []
+        for i in range(len(self.solvers)):
+            if i not in small:
+                self._advance_mesh(i, n, use_graph, main.cuda_stream)
+        self.rot = (self.rot + n) % 6
+
+    def _advance_mesh(self, i, n, use_graph, stream):
+        """n steps of mesh i on one stream: plain steps until the rotation is back at 0,
+        graph chunks, the remainder."""
+        s, rot, done, chunk = self.solvers[i], self.rot, 0, self.graph_chunk
+        clock = self._mesh_clocks[i:i + 1]
+
+        def plain(k):
+            b = [s.bufs[q] for q in _roles(s.state_form, rot)]
+            call("cvfes_solid_advance_f32" if self.precision == 32 else "cvfes_solid_advance_f64",
+                 _lib.C.byref(s._desc), ptr(s.plan.coef(self.precision)),
+                 ptr(s.plan.invm(self.precision)), ptr(b[0]), ptr(b[1]), ptr(b[2]), ptr(self._p),
+                 ptr(clock), k, self.dts[i], float(s.damp), None, None, stream)
+
+        if use_graph and n >= chunk + 5:
+            lead = (6 - rot) % 6
+            if lead:
+                plain(lead)
+                rot, done = 0, lead
+            h = self._mesh_graphs[i].get(chunk)
+            if h is None:
+                out = _lib.C.c_void_p()
+                call("cvfes_graph_capture_advance", _lib.C.byref(s._desc), self.precision,
+                     ptr(s.plan.coef(self.precision)), ptr(s.plan.invm(self.precision)),
+                     ptr(s.bufs[0]), ptr(s.bufs[1]), ptr(s.bufs[2]), ptr(self._p), ptr(clock),
+                     chunk, self.dts[i], float(s.damp), stream, _lib.C.byref(out))
+                h = self._mesh_graphs[i][chunk] = out.value
+            for _ in range((n - done) // chunk):
+                call("cvfes_graph_launch", h, stream)
+            done += (n - done) // chunk * chunk
+        if n - done:
+            plain(n - done)
+
     def _launch_concurrent(self, graphs, n_chunks):
         """n_chunks replays of each group's graph on the group's own stream, after the
         caller's stream's work so far, and the caller's stream waits for all of them."""
@@ -228,12 +315,7 @@ class BatchedSolidSolver:
         """Set each mesh solver's buffer roles from the batch's rotation phase
         (``rot`` = steps taken mod 6; the rule of ``cvfes_batch_step``)."""
         for s in self.solvers:
-            if s.state_form == "velocity":
-                s.cur, s.prev = (2 if self.rot & 1 else 0), 1
-                s.nxt = 2 - s.cur
-            else:
-                cur = (3 - self.rot % 3) % 3
-                s.cur, s.prev, s.nxt = cur, (cur + 1) % 3, (cur + 2) % 3
+            s.cur, s.prev, s.nxt = _roles(s.state_form, self.rot)
             s.step_count = self.steps
 
     def _graph(self, g: _Group, chunk):
@@ -250,10 +332,11 @@ class BatchedSolidSolver:
     def release_graphs(self):
         for st in getattr(self, "_group_streams", []):
             st.synchronize()  # no graph is destroyed while its replays may still run
-        for g in getattr(self, "groups", []):
-            for h in g.graphs.values():
+        for graphs in [g.graphs for g in getattr(self, "groups", [])] + \
+                getattr(self, "_mesh_graphs", []):
+            for h in graphs.values():
                 call("cvfes_graph_destroy", h)
-            g.graphs.clear()
+            graphs.clear()
 
     def __del__(self):
         try:
