@@ -70,8 +70,11 @@ class _Group:
 
 
 # Node-samples below which a mesh's step does not fill the chip (its launches run beside
-# other small meshes').  SMALLNOTE
-SMALL_MESH = 400_000
+# other small meshes').  24 tubes of 2,000 to 10,000 nodes with 16 or 32 samples, us a step:
+# 92 one after another, 60 side by side (two streams 67, eight 61), 84 as table launches;
+# ten tubes of 4,000 to 80,000 nodes with 16 to 256 samples: 350 either way, 492 as table
+# launches.
+SMALL_MESH = 200_000
 SMALL_STREAMS = 4
 
 
