@@ -6,7 +6,16 @@
 // [[xx, xy, xz], [xy, yy, yz], [xz, yz, 0]] rotated to the global frame (T^T s T),
 // and its xx, yy, xy, xz, yz entries.  B annihilates rigid translations, so the
 // displacement enters as differences from the element's node 0 (exact in FP32 for
-// small relative motion).  One thread per (element, sample), samples fastest.
+// small relative motion).
+//
+// On the undeformed wall the frame is the element's, not the sample's, so the five global
+// stresses are E times a 5 x 6 matrix of the element applied to (u_1 - u_0, u_2 - u_0): a
+// block forms the matrices of 32 elements (one lane each, FP64), then every thread applies
+// one to V samples, 30 products in place of some 150 operations.  What bounds it then is
+// the stores (5 of 7 values moved): a warp's results, contiguous in memory but 5 V values
+// apart in its lanes, pass through shared memory and leave as whole 16-byte lines.
+// 256 x 400 wall, 128 samples, FP32: 365 -> 171 us (0.89 GB, 5.2 TB/s).
+// On a deformed wall (ug) the frame is formed per (element, sample), one thread each.
 #include <cuda_runtime.h>
 
 #include "common.cuh"
@@ -108,12 +117,151 @@ __global__ void k_stress(long long n_elems, int S, const double* __restrict__ no
     o[4] = G[1][2];
 }
 
+constexpr int kStressElems = 32, kStressThreads = 128;
+
+template <typename T, int V>
+__global__ void __launch_bounds__(kStressThreads)
+    k_stress_undeformed(long long n_elems, int S, const double* __restrict__ nodes,
+                        const int32_t* __restrict__ elems, const double* __restrict__ young,
+                        const T* __restrict__ u, double nu, T* __restrict__ stress) {
+    __shared__ T mat[kStressElems][30];  // [stress][6 displacement differences]
+    __shared__ int nid[kStressElems][3];
+    __shared__ __align__(16) T out[kStressThreads / 32][32 * 5 * V];
+    const long long e0 = (long long)blockIdx.x * kStressElems;
+    const int ne = (int)min((long long)kStressElems, n_elems - e0);
+    if ((int)threadIdx.x < ne) {
+        const int l = threadIdx.x;
+        double P[3][3];
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+            nid[l][k] = elems[3 * (e0 + l) + k];
+#pragma unroll
+            for (int d = 0; d < 3; ++d) P[k][d] = nodes[3 * (size_t)nid[l][k] + d];
+        }
+        // frame: x along P2 - P1, y Gram-Schmidt of P0 - P2, z = x cross y
+        double R[3][3];
+#pragma unroll
+        for (int d = 0; d < 3; ++d) {
+            R[0][d] = P[2][d] - P[1][d];
+            R[1][d] = P[0][d] - P[2][d];
+        }
+        double inv = 1.0 / sqrt(R[0][0] * R[0][0] + R[0][1] * R[0][1] + R[0][2] * R[0][2]);
+#pragma unroll
+        for (int d = 0; d < 3; ++d) R[0][d] *= inv;
+        const double pr = R[0][0] * R[1][0] + R[0][1] * R[1][1] + R[0][2] * R[1][2];
+#pragma unroll
+        for (int d = 0; d < 3; ++d) R[1][d] -= pr * R[0][d];
+        inv = 1.0 / sqrt(R[1][0] * R[1][0] + R[1][1] * R[1][1] + R[1][2] * R[1][2]);
+#pragma unroll
+        for (int d = 0; d < 3; ++d) R[1][d] *= inv;
+        R[2][0] = R[0][1] * R[1][2] - R[0][2] * R[1][1];
+        R[2][1] = R[0][2] * R[1][0] - R[0][0] * R[1][2];
+        R[2][2] = R[0][0] * R[1][1] - R[0][1] * R[1][0];
+        double lx[3], ly[3];
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {  // relative to node 0
+            lx[k] = ly[k] = 0.0;
+#pragma unroll
+            for (int d = 0; d < 3; ++d) {
+                lx[k] += (P[k][d] - P[0][d]) * R[0][d];
+                ly[k] += (P[k][d] - P[0][d]) * R[1][d];
+            }
+        }
+        const double area2 = lx[1] * ly[2] - lx[2] * ly[1];
+        const double f = 1.0 / ((1.0 - nu * nu) * area2);
+        const double sh = 0.5 * (1.0 - nu), k56 = 5.0 / 6.0;
+        const double b[3] = {0.0, ly[2] - ly[0], ly[0] - ly[1]};
+        const double c[3] = {0.0, lx[0] - lx[2], lx[1] - lx[0]};
+        for (int k = 1; k < 3; ++k)
+            for (int d = 0; d < 3; ++d) {  // stresses of a unit displacement d of node k
+                const double xx = f * (b[k] * R[0][d] + nu * c[k] * R[1][d]);
+                const double yy = f * (nu * b[k] * R[0][d] + c[k] * R[1][d]);
+                const double xy = f * sh * (c[k] * R[0][d] + b[k] * R[1][d]);
+                const double xz = f * k56 * sh * b[k] * R[2][d];
+                const double yz = f * k56 * sh * c[k] * R[2][d];
+                auto global = [&](int i, int j) {  // entry (i, j) of R^T L R
+                    const double v0 = xx * R[0][j] + xy * R[1][j] + xz * R[2][j];
+                    const double v1 = xy * R[0][j] + yy * R[1][j] + yz * R[2][j];
+                    const double v2 = xz * R[0][j] + yz * R[1][j];
+                    return R[0][i] * v0 + R[1][i] * v1 + R[2][i] * v2;
+                };
+                const int q = 3 * (k - 1) + d;
+                mat[l][q] = (T)global(0, 0);
+                mat[l][6 + q] = (T)global(1, 1);
+                mat[l][12 + q] = (T)global(0, 1);
+                mat[l][18 + q] = (T)global(0, 2);
+                mat[l][24 + q] = (T)global(1, 2);
+            }
+    }
+    __syncthreads();
+    // (element, sample vector) pairs of the block in memory order
+    const int sv = S / V, total = ne * sv, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    T* const w = out[warp];
+    for (int base = warp * 32; base < total; base += kStressThreads) {
+        const int idx = base + lane, n = min(32, total - base);
+        if (lane < n) {
+            const int l = idx / sv;
+            const size_t col = (size_t)(idx - l * sv) * V;
+            Vec<T, V> r0[3], r1[3], r2[3], E;
+#pragma unroll
+            for (int d = 0; d < 3; ++d) {
+                r0[d] = ldg<T, V>(u + (3 * (size_t)nid[l][0] + d) * S + col);
+                r1[d] = ldg<T, V>(u + (3 * (size_t)nid[l][1] + d) * S + col);
+                r2[d] = ldg<T, V>(u + (3 * (size_t)nid[l][2] + d) * S + col);
+            }
+            const double* y = young + (size_t)(e0 + l) * S + col;
+#pragma unroll
+            for (int i = 0; i < V; ++i) E.v[i] = (T)__ldcs(y + i);
+#pragma unroll
+            for (int d = 0; d < 3; ++d) {
+                r1[d] = vsub(r1[d], r0[d]);
+                r2[d] = vsub(r2[d], r0[d]);
+            }
+#pragma unroll
+            for (int q = 0; q < 5; ++q) {
+                Vec<T, V> t = vzero<T, V>();
+#pragma unroll
+                for (int d = 0; d < 3; ++d) axpy(t, mat[l][6 * q + d], r1[d]);
+#pragma unroll
+                for (int d = 0; d < 3; ++d) axpy(t, mat[l][6 * q + 3 + d], r2[d]);
+#pragma unroll
+                for (int i = 0; i < V; ++i) w[(lane * V + i) * 5 + q] = E.v[i] * t.v[i];
+            }
+        }
+        __syncwarp();
+        T* o = stress + ((size_t)e0 * S + (size_t)base * V) * 5;
+        constexpr int kVec = 16 / (int)sizeof(T);
+        if constexpr (V == kVec) {
+            for (int i = lane; i < n * 5; i += 32)
+                stcs<T, kVec>(o + kVec * i, lds<T, kVec>(reinterpret_cast<unsigned char*>(w + kVec * i)));
+        } else {
+            for (int i = lane; i < n * 5 * V; i += 32) __stcs(o + i, w[i]);
+        }
+        __syncwarp();
+    }
+}
+
 template <typename T>
 int launch_stress(long long n_elems, long long S, const double* nodes, const int32_t* elems,
                   const double* young, const T* u, const T* ug, double nu, T* stress,
                   cudaStream_t st) {
     if (n_elems <= 0 || S <= 0 || S > INT32_MAX || !nodes || !elems || !young || !u || !stress)
         return fail(CVFES_ERR_ARG, "cvfes_solid_stress: bad argument");
+    if (!ug && S <= (1 << 24)) {
+        int V = (int)(16 / sizeof(T));
+        while (V > 1 && (S % V || reinterpret_cast<uintptr_t>(u) % (V * sizeof(T)) ||
+                         reinterpret_cast<uintptr_t>(stress) % 16))
+            V /= 2;
+        auto kernel = k_stress_undeformed<T, 1>;
+        if (V == 2) kernel = k_stress_undeformed<T, 2>;
+        if constexpr (sizeof(T) == 4) {
+            if (V == 4) kernel = k_stress_undeformed<T, 4>;
+        }
+        kernel<<<grid_1d(n_elems, kStressElems), kStressThreads, 0, st>>>(
+            n_elems, (int)S, nodes, elems, young, u, nu, stress);
+        CVFES_LAUNCH_CHECK("k_stress_undeformed");
+        return CVFES_OK;
+    }
     k_stress<T><<<grid_1d(n_elems * S, 256), 256, 0, st>>>(n_elems, (int)S, nodes, elems, young,
                                                            u, ug, (T)nu, stress);
     CVFES_LAUNCH_CHECK("k_stress");

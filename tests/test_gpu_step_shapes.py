@@ -138,3 +138,19 @@ def test_geometric_step_alone_or_in_an_ensemble(lib, cuda, precision, interval, 
     got = run_geo(mesh, precision, interval, 2 if precision == 32 else 1)
     want = run_geo(few, precision, interval, 1)
     assert torch.isfinite(got).all() and torch.equal(got[:, :3], want)
+
+
+@pytest.mark.parametrize("precision", [32, 64])
+@pytest.mark.parametrize("kind,samples", [("tube", 2), ("tube", 6), ("tube", 64), ("tube", 129),
+                                          ("irregular", 36)])
+def test_stress_alone_or_in_an_ensemble(lib, cuda, precision, kind, samples):
+    """The stresses of an ensemble's first sample are those of that sample alone (one sample a
+    thread, the ensemble up to four), bit for bit."""
+    mesh = wall(kind, samples)
+    one = SolidMesh(mesh.nodes, mesh.elementNodeIds, mesh.boundary, 1, density=1.0, v=0.49,
+                    damp=100.0, elmE=mesh.elmE[:, :1], elmThick=mesh.elmThick[:, :1],
+                    iniU=mesh.iniU, iniDu=mesh.iniDu)
+    got, want = [GPUSolidSolver(LocalComm(), m, Cfg(1e-8, m.nSmp, precision, "auto")).Stress()
+                 for m in (mesh, one)]
+    assert torch.isfinite(got).all() and want.abs().max() > 0
+    assert torch.equal(got[:, :1], want)
