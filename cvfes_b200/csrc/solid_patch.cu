@@ -111,13 +111,12 @@ __device__ __forceinline__ void patch_epilogue(const StepArgs<T>& A, T* un, T* v
 // NORMS: 0 none; 1 the per-sample norms of the new state, each lane's sums in tensor
 // memory; 2 the same in shared memory behind the stages.  The grid is a multiple of the
 // chunks, so a block keeps one chunk for its whole life and writes one row of partials.
-template <typename T, int V, bool VEL, int NORMS>
-__global__ void __launch_bounds__(32 * kPatchWarps, 1)
+template <typename T, int V, bool VEL, int NORMS, int W>
+__global__ void __launch_bounds__(32 * W, 1)
     k_step_patch(StepArgs<T> A, PatchMap M, int max_degree) {
     extern __shared__ __align__(16) unsigned char smem[];
     using P = SlotStage<T>;
     constexpr bool DIFF = std::is_same<T, float>::value;
-    constexpr int W = kPatchWarps;
     const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
     const uint32_t b_rec = 16u * max_degree, b_stage = b_rec + P::kSlotBytes * max_degree;
     unsigned char* const wb = smem + warp * (2 * b_stage);
@@ -133,7 +132,7 @@ __global__ void __launch_bounds__(32 * kPatchWarps, 1)
     const int n_nodes = (int)A.n_nodes, first = A.n_clamped;
 
     const int bpc = gridDim.x / A.nch;  // blocks of a chunk
-    PatchWalk walk(M, warp, blockIdx.x / A.nch, bpc, first, n_nodes);
+    PatchWalk walk(M, warp, blockIdx.x / A.nch, bpc, first, n_nodes, W);
     // ---- slot staging: lane l copies word l % kWords of slot l / kWords (FP32), or every
     // 32nd word (FP64); records by the first lanes
     const int qs = lane / P::kWords, qw = lane - qs * P::kWords;
@@ -399,29 +398,42 @@ __global__ void __launch_bounds__(32 * kPatchWarps, 1)
     }
 }
 
+// Warps of a block (one block an SM): what the registers allow.  us a step at 16 / 20 / 24
+// (28) warps: FP32 pairs, 256 x 512 wall, 64 samples 142 / 136 / 133, 64 x 128 wall 10.7 /
+// 10.7 / 12.2; FP32 singles, 128 x 400 wall, 33 samples 93 / - / 81 (74); FP64 singles, 37
+// samples 125 / 128 / 129.  With the norms 16: tensor memory holds the sums of 16 warps in
+// 128 columns.
+template <typename T, int V, int NORMS>
+struct PatchBlock {
+    static constexpr int kWarps =
+        NORMS || sizeof(T) == 8 || V == 4 ? 16 : (V == 2 ? 20 : 28);
+};
+
 template <typename T, int V, bool VEL, int NORMS>
-static int launch_patch_k(const StepArgs<T>& A, const PatchMap& M, int max_degree,
+static int launch_patch_k(const StepArgs<T>& A, const cvfes_solid_mesh* m, int max_degree,
                           long long max_rows, long long* rows, bool after_step,
                           cudaStream_t st) {
-    auto kernel = k_step_patch<T, V, VEL, NORMS>;
-    size_t smem = (size_t)kPatchWarps * 2 * max_degree * SlotStage<T>::kBytes;
+    constexpr int W = PatchBlock<T, V, NORMS>::kWarps;
+    const PatchMap M = patch_map(m->n_nodes - A.n_clamped, m->bandwidth, W);
+    auto kernel = k_step_patch<T, V, VEL, NORMS, W>;
+    size_t smem = (size_t)W * 2 * max_degree * SlotStage<T>::kBytes;
     const size_t sums = (size_t)4 * V * 32 * sizeof(double);
     if (NORMS == 1) smem = std::max(smem, sums);
-    if (NORMS == 2) smem += kPatchWarps * sums;
+    if (NORMS == 2) smem += W * sums;
     int per_sm = 0;
-    const int rc = fanp_blocks_per_sm(reinterpret_cast<const void*>(kernel), 32 * kPatchWarps,
+    const int rc = fanp_blocks_per_sm(reinterpret_cast<const void*>(kernel), 32 * W,
                                       smem, &per_sm);
     if (rc) return rc;
     // whole rounds of the chunks, so that a block keeps its chunk
     const long long places = std::max<long long>((long long)M.n_strips * M.tps,
-                                                 (A.n_clamped + kPatchWarps - 1) / kPatchWarps);
+                                                 (A.n_clamped + W - 1) / W);
     long long per_chunk = std::max(1LL, (long long)per_sm * device_sm_count() / A.nch);
     per_chunk = std::min(per_chunk, std::max(places, 1LL));
     if (NORMS) {
         per_chunk = std::min(per_chunk, max_rows);
         if (rows) *rows = per_chunk;
     }
-    return launch_step_kernel(kernel, dim3((unsigned)(per_chunk * A.nch)), 32 * kPatchWarps, smem, after_step, st,
+    return launch_step_kernel(kernel, dim3((unsigned)(per_chunk * A.nch)), 32 * W, smem, after_step, st,
                               "k_step_patch", A, M, max_degree);
 }
 
@@ -439,18 +451,17 @@ int launch_step_patch(const cvfes_solid_mesh* m, StepArgs<T> A, int vec_max, boo
                       cudaStream_t st, int norms_mode, long long max_rows, long long* rows) {
     const int md = (int)m->max_degree;
     if (m->max_degree <= 0 || A.S >= (1 << 27) || m->n_nodes >= INT32_MAX / 2 ||
-        (size_t)kPatchWarps * 2 * std::min<size_t>(m->max_degree, 1 << 16) *
-                SlotStage<T>::kBytes > 96 * 1024)
+        (size_t)28 * 2 * std::min<size_t>(m->max_degree, 1 << 16) *
+                SlotStage<T>::kBytes > 160 * 1024)
         return 1;
     const int V = patch_vec(A.S, vec_max);
     A.nch = (A.S / V + 31) / 32;
-    const PatchMap M = patch_map(m->n_nodes - A.n_clamped, m->bandwidth);
     const int norms = A.norm_part ? (norms_mode == 0 ? 1 : 2) : 0;
 #define CVFES_PATCH(VV, VEL)                                                                   \
     switch (norms) {                                                                           \
-        case 1: return launch_patch_k<T, VV, VEL, 1>(A, M, md, max_rows, rows, false, st);     \
-        case 2: return launch_patch_k<T, VV, VEL, 2>(A, M, md, max_rows, rows, false, st);     \
-        default: return launch_patch_k<T, VV, VEL, 0>(A, M, md, 0, nullptr, after_step, st);   \
+        case 1: return launch_patch_k<T, VV, VEL, 1>(A, m, md, max_rows, rows, false, st);     \
+        case 2: return launch_patch_k<T, VV, VEL, 2>(A, m, md, max_rows, rows, false, st);     \
+        default: return launch_patch_k<T, VV, VEL, 0>(A, m, md, 0, nullptr, after_step, st);   \
     }
     if (V == 4) {
         if constexpr (sizeof(T) == 4) {
