@@ -237,8 +237,8 @@ __device__ __forceinline__ void load27(const T* K, T (&kk)[27]) {
 
 // dchi^T Khat_e du for the element owned by this slot: (u1, u2) and (x1, x2) are
 // the first and second neighbour rows of u_n and chi_{n+1}, already differences
-// u_b - u_a in the DIFF form, raw rows otherwise.
-template <typename T, int V, bool DIFF, bool SMEM_OWN = false>
+// u_b - u_a.
+template <typename T, int V, bool SMEM_OWN = false>
 __device__ __forceinline__ Vec<T, V> owner_form(const T* own, const Vec<T, V> (&u1)[3],
                                                 const Vec<T, V> (&u2)[3],
                                                 const Vec<T, V> (&x1)[3],
@@ -248,17 +248,10 @@ __device__ __forceinline__ Vec<T, V> owner_form(const T* own, const Vec<T, V> (&
     Vec<T, V> du1[3], du2[3], dy1[3], dy2[3];
 #pragma unroll
     for (int d = 0; d < 3; ++d) {
-        if constexpr (DIFF) {
-            du1[d] = u1[d];
-            du2[d] = u2[d];
-            dy1[d] = x1[d];
-            dy2[d] = x2[d];
-        } else {
-            du1[d] = vsub(u1[d], ua[d]);
-            du2[d] = vsub(u2[d], ua[d]);
-            dy1[d] = vsub(x1[d], ca[d]);
-            dy2[d] = vsub(x2[d], ca[d]);
-        }
+        du1[d] = u1[d];
+        du2[d] = u2[d];
+        dy1[d] = x1[d];
+        dy2[d] = x2[d];
     }
     // own points into global memory (gather kernel) or shared memory (fan kernel, SMEM_OWN):
     // plain generic loads, not the global-only read-only path.  From shared memory they
@@ -285,13 +278,13 @@ __device__ __forceinline__ Vec<T, V> owner_form(const T* own, const Vec<T, V> (&
 }
 
 // Gamma_e += that form.
-template <typename T, int V, bool DIFF, bool SMEM_OWN = false>
+template <typename T, int V, bool SMEM_OWN = false>
 __device__ __forceinline__ void owner_grad(const RevArgs<T>& A, int e, const T* own, size_t S,
                                            size_t col,
                                            const Vec<T, V> (&u1)[3], const Vec<T, V> (&u2)[3],
                                            const Vec<T, V> (&x1)[3], const Vec<T, V> (&x2)[3],
                                            const Vec<T, V> (&ua)[3], const Vec<T, V> (&ca)[3]) {
-    const Vec<T, V> g = owner_form<T, V, DIFF, SMEM_OWN>(own, u1, u2, x1, x2, ua, ca);
+    const Vec<T, V> g = owner_form<T, V, SMEM_OWN>(own, u1, u2, x1, x2, ua, ca);
     T* gp = A.gam + (size_t)e * S + col;
     Vec<T, V> gv = ld<T, V>(gp);
 #pragma unroll
@@ -381,7 +374,7 @@ __device__ __forceinline__ void rev_epilogue(const RevArgs<T>& A, long long a, s
 // One reverse step for (node a, V samples): reconstruct u_{n-1}, advance chi, accumulate
 // Gamma over the elements this node owns and G of this node.  Rows are gathered
 // through L1; a fan continuation reuses the previous slot's second neighbour.
-template <typename T, int V, bool DIFF, bool GM>
+template <typename T, int V, bool GM>
 __global__ void __launch_bounds__(256) k_reverse(RevArgs<T> A) {
     long long a;
     int vec;
@@ -419,10 +412,8 @@ __global__ void __launch_bounds__(256) k_reverse(RevArgs<T> A) {
             for (int d = 0; d < 3; ++d) {
                 x1[d] = ldg<T, V>(A.u + o1 + d * S);
                 y1[d] = ldg<T, V>(A.x + o1 + d * S);
-                if constexpr (DIFF) {
-                    x1[d] = vsub(x1[d], ua[d]);
-                    y1[d] = vsub(y1[d], ca[d]);
-                }
+                x1[d] = vsub(x1[d], ua[d]);
+                y1[d] = vsub(y1[d], ca[d]);
             }
         }
         const size_t o2 = (size_t)r.z * 3 * S + col;
@@ -430,10 +421,8 @@ __global__ void __launch_bounds__(256) k_reverse(RevArgs<T> A) {
         for (int d = 0; d < 3; ++d) {
             x2[d] = ldg<T, V>(A.u + o2 + d * S);
             y2[d] = ldg<T, V>(A.x + o2 + d * S);
-            if constexpr (DIFF) {
-                x2[d] = vsub(x2[d], ua[d]);
-                y2[d] = vsub(y2[d], ca[d]);
-            }
+            x2[d] = vsub(x2[d], ua[d]);
+            y2[d] = vsub(y2[d], ca[d]);
         }
         const Vec<T, V> c = ldg<T, V>(A.coef + (size_t)r.x * S + col);
         T kk[27];
@@ -441,13 +430,6 @@ __global__ void __launch_bounds__(256) k_reverse(RevArgs<T> A) {
 #pragma unroll
         for (int i = 0; i < 3; ++i) {
             Vec<T, V> tu = vzero<T, V>(), tc = vzero<T, V>();
-            if constexpr (!DIFF) {
-#pragma unroll
-                for (int jj = 0; jj < 3; ++jj) {
-                    axpy(tu, kk[3 * i + jj], ua[jj]);
-                    axpy(tc, kk[3 * i + jj], ca[jj]);
-                }
-            }
 #pragma unroll
             for (int jj = 0; jj < 3; ++jj) {
                 axpy(tu, kk[9 + 3 * i + jj], x1[jj]);
@@ -462,7 +444,7 @@ __global__ void __launch_bounds__(256) k_reverse(RevArgs<T> A) {
             vfma(accC[i], c, tc);
         }
         if (((r.w >> 8) & 3) == 0)
-            owner_grad<T, V, DIFF>(A, r.x, A.own + (size_t)kOwnStride * k, S, col, x1, x2, y1, y2,
+            owner_grad<T, V>(A, r.x, A.own + (size_t)kOwnStride * k, S, col, x1, x2, y1, y2,
                                    ua, ca);
 #pragma unroll
         for (int d = 0; d < 3; ++d) {
@@ -485,16 +467,14 @@ __device__ __forceinline__ void load3(Vec<T, V> (&x)[3], const T* __restrict__ b
 #pragma unroll
     for (int d = 0; d < 3; ++d) x[d] = ldg<T, V>(p + d * S);
 }
-template <typename T, int V, bool DIFF>
+template <typename T, int V>
 __device__ __forceinline__ void diff3(Vec<T, V> (&x)[3], const Vec<T, V> (&ref)[3]) {
-    if constexpr (DIFF) {
 #pragma unroll
-        for (int d = 0; d < 3; ++d) x[d] = vsub(x[d], ref[d]);
-    }
+    for (int d = 0; d < 3; ++d) x[d] = vsub(x[d], ref[d]);
 }
 
 // Both row products of one slot from one read of its stiffness rows (shared memory).
-template <typename T, int V, bool DIFF>
+template <typename T, int V>
 __device__ __forceinline__ void slot_fma2(const T* K, const Vec<T, V>& c,
                                           const Vec<T, V> (&u1)[3], const Vec<T, V> (&u2)[3],
                                           const Vec<T, V> (&x1)[3], const Vec<T, V> (&x2)[3],
@@ -503,7 +483,7 @@ __device__ __forceinline__ void slot_fma2(const T* K, const Vec<T, V>& c,
     T kk[28];
     if constexpr (sizeof(T) == 4) {
 #pragma unroll
-        for (int q = (DIFF ? 2 : 0); q < 7; ++q) {
+        for (int q = 2; q < 7; ++q) {
             const float4 t = reinterpret_cast<const float4*>(K)[q];
             kk[4 * q] = t.x;
             kk[4 * q + 1] = t.y;
@@ -512,7 +492,7 @@ __device__ __forceinline__ void slot_fma2(const T* K, const Vec<T, V>& c,
         }
     } else {
 #pragma unroll
-        for (int q = (DIFF ? 4 : 0); q < 14; ++q) {
+        for (int q = 4; q < 14; ++q) {
             const double2 t = reinterpret_cast<const double2*>(K)[q];
             kk[2 * q] = t.x;
             kk[2 * q + 1] = t.y;
@@ -521,13 +501,6 @@ __device__ __forceinline__ void slot_fma2(const T* K, const Vec<T, V>& c,
 #pragma unroll
     for (int i = 0; i < 3; ++i) {
         Vec<T, V> tu = vzero<T, V>(), tc = vzero<T, V>();
-        if constexpr (!DIFF) {
-#pragma unroll
-            for (int jj = 0; jj < 3; ++jj) {
-                axpy(tu, kk[3 * i + jj], ua[jj]);
-                axpy(tc, kk[3 * i + jj], ca[jj]);
-            }
-        }
 #pragma unroll
         for (int jj = 0; jj < 3; ++jj) {
             axpy(tu, kk[9 + 3 * i + jj], u1[jj]);
@@ -543,7 +516,7 @@ __device__ __forceinline__ void slot_fma2(const T* K, const Vec<T, V>& c,
     }
 }
 
-template <typename T, int V, bool DIFF>
+template <typename T, int V>
 __device__ __forceinline__ void rev_phase(int& k, int k1, const int4* srec, const T* sslab,
                                           const T* sown, const RevArgs<T>& A, size_t S, size_t col,
                                           const Vec<T, V> (&ua)[3], const Vec<T, V> (&ca)[3],
@@ -560,24 +533,24 @@ __device__ __forceinline__ void rev_phase(int& k, int k1, const int4* srec, cons
         load3<T, V>(nx, A.x, rn.z, S, col);
         cnxt = ldg<T, V>(A.coef + (size_t)rn.x * S + col);
     }
-    diff3<T, V, DIFF>(cu, ua);
-    diff3<T, V, DIFF>(cx, ca);
+    diff3<T, V>(cu, ua);
+    diff3<T, V>(cx, ca);
     const int4 r = srec[k];
-    slot_fma2<T, V, DIFF>(sslab + (size_t)kSlabStride * k, ccur, pu, cu, px, cx, ua, ca, accU,
+    slot_fma2<T, V>(sslab + (size_t)kSlabStride * k, ccur, pu, cu, px, cx, ua, ca, accU,
                           accC);
     if (((r.w >> 8) & 3) == 0)
-        owner_grad<T, V, DIFF, true>(A, r.x, sown + (size_t)kOwnStride * k, S, col, pu, cu, px, cx, ua,
+        owner_grad<T, V, true>(A, r.x, sown + (size_t)kOwnStride * k, S, col, pu, cu, px, cx, ua,
                                ca);
     if (more && !(rn.w & 1)) {  // fan break: the next slot's first neighbour is new
         load3<T, V>(cu, A.u, rn.y, S, col);
         load3<T, V>(cx, A.x, rn.y, S, col);
-        diff3<T, V, DIFF>(cu, ua);
-        diff3<T, V, DIFF>(cx, ca);
+        diff3<T, V>(cu, ua);
+        diff3<T, V>(cx, ca);
     }
     ++k;
 }
 
-template <typename T, int V, bool DIFF, bool GM, int MINB>
+template <typename T, int V, bool GM, int MINB>
 __global__ void __launch_bounds__(256, MINB) k_reverse_fan(RevArgs<T> A) {
     extern __shared__ __align__(16) unsigned char smem[];
     const int warp = threadIdx.x >> 5;
@@ -646,17 +619,17 @@ __global__ void __launch_bounds__(256, MINB) k_reverse_fan(RevArgs<T> A) {
         load3<T, V>(U1, A.u, r0.z, S, col);
         load3<T, V>(X1, A.x, r0.z, S, col);
         c1 = ldg<T, V>(A.coef + (size_t)r0.x * S + col);
-        diff3<T, V, DIFF>(U0, ua);
-        diff3<T, V, DIFF>(X0, ca);
+        diff3<T, V>(U0, ua);
+        diff3<T, V>(X0, ca);
         int k = k0;
         while (true) {
-            rev_phase<T, V, DIFF>(k, k1, srec, sslab, sown, A, S, col, ua, ca, accU, accC, U0, X0, U1,
+            rev_phase<T, V>(k, k1, srec, sslab, sown, A, S, col, ua, ca, accU, accC, U0, X0, U1,
                                   X1, c1, U2, X2, c2);
             if (k >= k1) break;
-            rev_phase<T, V, DIFF>(k, k1, srec, sslab, sown, A, S, col, ua, ca, accU, accC, U1, X1, U2,
+            rev_phase<T, V>(k, k1, srec, sslab, sown, A, S, col, ua, ca, accU, accC, U1, X1, U2,
                                   X2, c2, U0, X0, c0);
             if (k >= k1) break;
-            rev_phase<T, V, DIFF>(k, k1, srec, sslab, sown, A, S, col, ua, ca, accU, accC, U2, X2, U0,
+            rev_phase<T, V>(k, k1, srec, sslab, sown, A, S, col, ua, ca, accU, accC, U2, X2, U0,
                                   X0, c0, U1, X1, c1);
             if (k >= k1) break;
         }
@@ -678,7 +651,6 @@ template <typename T, int V, bool GM>
 __global__ void __launch_bounds__(32 * kPatchWarps, 1)
     k_reverse_patch(RevArgs<T> A, PatchMap M, int max_degree) {
     extern __shared__ __align__(16) unsigned char smem[];
-    constexpr bool DIFF = std::is_same<T, float>::value;
     using P = SlotStage<T>;
     constexpr int kOwnWords = kOwnStride * (int)sizeof(T) / 16;
     const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
@@ -792,9 +764,9 @@ __global__ void __launch_bounds__(32 * kPatchWarps, 1)
                 Vec<T, V> gv = vzero<T, V>();
                 T* const gp = row_at(gam, r.x, rowb);
                 if (owner) gv = ld<T, V>(gp);  // requested before the products
-                slot_fma2<T, V, DIFF>(K + kStep * k, c, u1, u2, x1, x2, ua, ca, accU, accC);
+                slot_fma2<T, V>(K + kStep * k, c, u1, u2, x1, x2, ua, ca, accU, accC);
                 if (owner) {
-                    const Vec<T, V> g = owner_form<T, V, DIFF, true>(own + kOwnStride * k, u1, u2,
+                    const Vec<T, V> g = owner_form<T, V, true>(own + kOwnStride * k, u1, u2,
                                                                      x1, x2, ua, ca);
 #pragma unroll
                     for (int q = 0; q < V; ++q) gv.v[q] += g.v[q];
@@ -809,8 +781,8 @@ __global__ void __launch_bounds__(32 * kPatchWarps, 1)
                 rows(U[0], X[0], srec[0].y);
                 rows(U[1], X[1], srec[0].z);
                 C[0] = ldg<T, V>(row_at(cf, srec[0].x, rowb));
-                diff3<T, V, DIFF>(U[0], ua);
-                diff3<T, V, DIFF>(X[0], ca);
+                diff3<T, V>(U[0], ua);
+                diff3<T, V>(X[0], ca);
 #pragma unroll
                 for (int k = 0; k < 6; ++k) {
                     if (k < 5) {
@@ -821,11 +793,11 @@ __global__ void __launch_bounds__(32 * kPatchWarps, 1)
                         if (a >= A.n_clamped) rev_rows<T, V, GM>(A, a, col, R);
                     }
                     if (k == 2) prefetch_elems();
-                    if constexpr (DIFF) __syncwarp();
-                    diff3<T, V, DIFF>(U[k + 1], ua);
-                    diff3<T, V, DIFF>(X[k + 1], ca);
+                    if constexpr (sizeof(T) == 4) __syncwarp();
+                    diff3<T, V>(U[k + 1], ua);
+                    diff3<T, V>(X[k + 1], ca);
                     element(k, srec[k], C[k], U[k], U[k + 1], X[k], X[k + 1]);
-                    if constexpr (DIFF) __syncwarp();
+                    if constexpr (sizeof(T) == 4) __syncwarp();
                 }
             } else if (n > 0) {
                 Vec<T, V> U0[3], U1[3], U2[3], X0[3], X1[3], X2[3], c0, c1, c2;
@@ -833,8 +805,8 @@ __global__ void __launch_bounds__(32 * kPatchWarps, 1)
                 rows(U0, X0, r.y);
                 rows(U1, X1, r.z);
                 c1 = ldg<T, V>(row_at(cf, r.x, rowb));
-                diff3<T, V, DIFF>(U0, ua);
-                diff3<T, V, DIFF>(X0, ca);
+                diff3<T, V>(U0, ua);
+                diff3<T, V>(X0, ca);
                 int k = 0;
                 auto phase = [&](Vec<T, V> (&pu)[3], Vec<T, V> (&px)[3], Vec<T, V> (&cu)[3],
                                  Vec<T, V> (&cx)[3], const Vec<T, V>& c, Vec<T, V> (&nu)[3],
@@ -846,13 +818,13 @@ __global__ void __launch_bounds__(32 * kPatchWarps, 1)
                         rows(nu, nx, rn.z);
                         cn = ldg<T, V>(row_at(cf, rn.x, rowb));
                     }
-                    diff3<T, V, DIFF>(cu, ua);
-                    diff3<T, V, DIFF>(cx, ca);
+                    diff3<T, V>(cu, ua);
+                    diff3<T, V>(cx, ca);
                     element(k, r, c, pu, cu, px, cx);
                     if (next && !(rn.w & 1)) {  // fan break: the next first neighbour is new
                         rows(cu, cx, rn.y);
-                        diff3<T, V, DIFF>(cu, ua);
-                        diff3<T, V, DIFF>(cx, ca);
+                        diff3<T, V>(cu, ua);
+                        diff3<T, V>(cx, ca);
                     }
                     r = rn;
                     ++k;
@@ -944,14 +916,14 @@ int launch_rev_fan(Kern kernel, unsigned grid, int threads, size_t smem, cudaStr
     return CVFES_OK;
 }
 
-template <typename T, int V, bool DIFF, bool GM>
+template <typename T, int V, bool GM>
 int launch_rev_fan_m(int minb, unsigned grid, int threads, size_t smem, cudaStream_t st,
                      const RevArgs<T>& A) {
     switch (minb) {
-        case 4: return launch_rev_fan(k_reverse_fan<T, V, DIFF, GM, 4>, grid, threads, smem, st, A);
-        case 3: return launch_rev_fan(k_reverse_fan<T, V, DIFF, GM, 3>, grid, threads, smem, st, A);
-        case 2: return launch_rev_fan(k_reverse_fan<T, V, DIFF, GM, 2>, grid, threads, smem, st, A);
-        default: return launch_rev_fan(k_reverse_fan<T, V, DIFF, GM, 1>, grid, threads, smem, st, A);
+        case 4: return launch_rev_fan(k_reverse_fan<T, V, GM, 4>, grid, threads, smem, st, A);
+        case 3: return launch_rev_fan(k_reverse_fan<T, V, GM, 3>, grid, threads, smem, st, A);
+        case 2: return launch_rev_fan(k_reverse_fan<T, V, GM, 2>, grid, threads, smem, st, A);
+        default: return launch_rev_fan(k_reverse_fan<T, V, GM, 1>, grid, threads, smem, st, A);
     }
 }
 
@@ -959,8 +931,10 @@ int launch_rev_fan_m(int minb, unsigned grid, int threads, size_t smem, cudaStre
 template <typename T, int V>
 int launch_rev_patch(const cvfes_solid_mesh* m, RevArgs<T> A, bool after_step, cudaStream_t st) {
     const size_t slot = SlotStage<T>::kBytes + kOwnStride * sizeof(T);
+    // (the slots are staged in 16-byte words)
     if (m->max_degree <= 0 || m->max_degree >= 1024 || A.S >= (1 << 27) ||
-        m->n_nodes >= INT32_MAX / 2)
+        m->n_nodes >= INT32_MAX / 2 || reinterpret_cast<uintptr_t>(A.own) % 16 ||
+        reinterpret_cast<uintptr_t>(A.slab) % 16 || reinterpret_cast<uintptr_t>(A.rec) % 16)
         return 1;
     const size_t smem = (size_t)kPatchWarps * 2 * slot * m->max_degree;
     if (smem > 160 * 1024) return 1;
@@ -978,16 +952,16 @@ int launch_rev_patch(const cvfes_solid_mesh* m, RevArgs<T> A, bool after_step, c
                               after_step, st, "k_reverse_patch", A, M, (int)m->max_degree);
 }
 
-template <typename T, int V, bool DIFF>
+template <typename T, int V>
 int launch_rev_v(const RevTuning& tu, bool fan, bool gmv, unsigned fan_grid, size_t smem,
                  const RowGrid& rg, cudaStream_t st, const RevArgs<T>& A) {
     if (fan) {
         const int threads = 32 * tu.npb;
-        return gmv ? launch_rev_fan_m<T, V, DIFF, true>(tu.minb, fan_grid, threads, smem, st, A)
-                   : launch_rev_fan_m<T, V, DIFF, false>(tu.minb, fan_grid, threads, smem, st, A);
+        return gmv ? launch_rev_fan_m<T, V, true>(tu.minb, fan_grid, threads, smem, st, A)
+                   : launch_rev_fan_m<T, V, false>(tu.minb, fan_grid, threads, smem, st, A);
     }
-    if (gmv) k_reverse<T, V, DIFF, true><<<rg.grid, 256, 0, st>>>(A);
-    else k_reverse<T, V, DIFF, false><<<rg.grid, 256, 0, st>>>(A);
+    if (gmv) k_reverse<T, V, true><<<rg.grid, 256, 0, st>>>(A);
+    else k_reverse<T, V, false><<<rg.grid, 256, 0, st>>>(A);
     CVFES_LAUNCH_CHECK("k_reverse");
     return CVFES_OK;
 }
@@ -1063,15 +1037,14 @@ int launch_reverse_step(const cvfes_adjoint_desc* d, const T* u, T* uo, const T*
         A.cap_slots = (int)cap;
         fan_grid = (unsigned)(((m->n_nodes + A.npb - 1) / A.npb) * A.nch);
     }
-    constexpr bool DIFF = std::is_same<T, float>::value;
     const bool gmv = d->gmass != nullptr;
     if (V == 4) {
         if constexpr (sizeof(T) == 4)
-            return launch_rev_v<T, 4, DIFF>(tu, fan, gmv, fan_grid, smem, rg, st, A);
+            return launch_rev_v<T, 4>(tu, fan, gmv, fan_grid, smem, rg, st, A);
         return fail(CVFES_ERR_UNSUPPORTED, "k_reverse: vec 4 is FP32 only");
     }
-    if (V == 2) return launch_rev_v<T, 2, DIFF>(tu, fan, gmv, fan_grid, smem, rg, st, A);
-    return launch_rev_v<T, 1, DIFF>(tu, fan, gmv, fan_grid, smem, rg, st, A);
+    if (V == 2) return launch_rev_v<T, 2>(tu, fan, gmv, fan_grid, smem, rg, st, A);
+    return launch_rev_v<T, 1>(tu, fan, gmv, fan_grid, smem, rg, st, A);
 }
 
 int check_adjoint(const cvfes_adjoint_desc* d, const char* who) {

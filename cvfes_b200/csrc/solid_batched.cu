@@ -89,7 +89,7 @@ __device__ __forceinline__ int batch_mesh_of(const BatchMesh* __restrict__ tab, 
     return lo;
 }
 
-template <typename T, int V, bool DIFF>
+template <typename T, int V>
 __global__ void __launch_bounds__(256) k_step_batched(const BatchMesh* __restrict__ tab,
                                                      int n_meshes, long long total, int rot,
                                                      const long long* clock, long long j) {
@@ -143,7 +143,7 @@ __global__ void __launch_bounds__(256) k_step_batched(const BatchMesh* __restric
         T f[3];
         node_load<T>(A, a, step_pressure<T>(A), f);
         Vec<T, V> acc[3];
-        ku_row<T, V, DIFF>(A.node_ptr, A.rec, A.slab, A.coef, A.u, S, col, a, ua, acc);
+        ku_row<T, V>(A.node_ptr, A.rec, A.slab, A.coef, A.u, S, col, a, ua, acc);
         step_epilogue<T, V>(A, a, S, col, row, ua, acc, f);
     }
 }
@@ -176,7 +176,7 @@ __device__ __forceinline__ int batch_fan_issue(const BatchMesh* __restrict__ tab
     return m;
 }
 
-template <typename T, int V, bool DIFF, int MINB>
+template <typename T, int V, int MINB>
 __global__ void __launch_bounds__(32 * kBatchWarps, MINB)
     k_batch_fan(const BatchMesh* __restrict__ tab, int n_meshes, long long total, int cap,
                 int rot, const long long* clock, long long j) {
@@ -266,7 +266,7 @@ __global__ void __launch_bounds__(32 * kBatchWarps, MINB)
                 const int kb = __ldg(M.node_ptr + a0);
                 const int k0 = __ldg(M.node_ptr + a) - kb, k1 = __ldg(M.node_ptr + a + 1) - kb;
                 Vec<T, V> acc[3];
-                ku_row_fan<T, V, DIFF>(stage_rec(srec0, stage_bytes, sg),
+                ku_row_fan<T, V>(stage_rec(srec0, stage_bytes, sg),
                                        stage_slab(sslab0, stage_bytes, sg), k0, k1, A.u, A.coef,
                                        S, col, ua, acc);
                 step_epilogue<T, V>(A, a, S, col, row, ua, acc, f);
@@ -281,16 +281,15 @@ __global__ void k_batch_clock_add(long long* clock, long long n) { clock[0] += n
 template <typename T>
 int launch_batched(const BatchMesh* tab, int n_meshes, long long total, int vec, int rot,
                    const long long* clock, long long j, int grid, cudaStream_t st) {
-    constexpr bool DIFF = std::is_same<T, float>::value;
     if (total <= 0) return CVFES_OK;
     if (grid <= 0 || grid > total) grid = (int)(total < (1LL << 30) ? total : (1 << 30));
     if (vec == 4) {
         if constexpr (sizeof(T) == 4)
-            k_step_batched<T, 4, DIFF><<<grid, 256, 0, st>>>(tab, n_meshes, total, rot, clock, j);
+            k_step_batched<T, 4><<<grid, 256, 0, st>>>(tab, n_meshes, total, rot, clock, j);
     } else if (vec == 2) {
-        k_step_batched<T, 2, DIFF><<<grid, 256, 0, st>>>(tab, n_meshes, total, rot, clock, j);
+        k_step_batched<T, 2><<<grid, 256, 0, st>>>(tab, n_meshes, total, rot, clock, j);
     } else {
-        k_step_batched<T, 1, DIFF><<<grid, 256, 0, st>>>(tab, n_meshes, total, rot, clock, j);
+        k_step_batched<T, 1><<<grid, 256, 0, st>>>(tab, n_meshes, total, rot, clock, j);
     }
     CVFES_LAUNCH_CHECK("k_step_batched");
     return CVFES_OK;
@@ -330,7 +329,6 @@ int launch_batch_fan_k(K kernel, const BatchMesh* tab, int n_meshes, long long t
 template <typename T>
 int launch_batch_fan(const BatchMesh* tab, int n_meshes, long long total, int cap, int vec,
                      int rot, const long long* clock, long long j, int grid, cudaStream_t st) {
-    constexpr bool DIFF = std::is_same<T, float>::value;
     if (total <= 0) return CVFES_OK;
     const size_t smem = 16 + 2 * (size_t)cap * (16 + kSlabStride * sizeof(T));
     if (cap <= 0 || smem > 200 * 1024)
@@ -338,14 +336,14 @@ int launch_batch_fan(const BatchMesh* tab, int n_meshes, long long total, int ca
                     cap);
     if (vec == 4) {
         if constexpr (sizeof(T) == 4)
-            return launch_batch_fan_k(k_batch_fan<T, 4, DIFF, 8>, tab, n_meshes, total, cap, rot,
+            return launch_batch_fan_k(k_batch_fan<T, 4, 8>, tab, n_meshes, total, cap, rot,
                                       clock, j, grid, smem, st);
         return fail(CVFES_ERR_ARG, "cvfes_batch_step: vec 4 is FP32 only");
     }
     if (vec == 2)
-        return launch_batch_fan_k(k_batch_fan<T, 2, DIFF, 8>, tab, n_meshes, total, cap, rot, clock,
+        return launch_batch_fan_k(k_batch_fan<T, 2, 8>, tab, n_meshes, total, cap, rot, clock,
                                   j, grid, smem, st);
-    return launch_batch_fan_k(k_batch_fan<T, 1, DIFF, 8>, tab, n_meshes, total, cap, rot, clock, j,
+    return launch_batch_fan_k(k_batch_fan<T, 1, 8>, tab, n_meshes, total, cap, rot, clock, j,
                               grid, smem, st);
 }
 

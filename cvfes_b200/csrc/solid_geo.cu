@@ -535,7 +535,8 @@ int launch_step_geo(const cvfes_solid_mesh* m, const T* coef, const T* invm, con
     const double lanes = (double)(A.S / V) / (32.0 * A.nch);
     const bool in_l2 = 12.0 * m->n_nodes * A.S * sizeof(T) < 100e6;
     if ((sizeof(T) == 4 || V == 1) && lanes >= (in_l2 ? 0.9 : 0.75) && m->max_degree > 0 &&
-        m->max_degree < 1024 && stages <= 96 * 1024) {
+        m->max_degree < 1024 && stages <= 96 * 1024 &&
+        reinterpret_cast<uintptr_t>(geo) % 16 == 0) {  // (staged in 16-byte words)
         const PatchMap M = patch_map(m->n_nodes - A.n_clamped, m->bandwidth, W);
         constexpr int V2 = sizeof(T) == 4 ? 2 : 1;  // (FP64 pairs would spill)
         auto kp = V == 2 ? (same ? k_step_geo_patch<T, V2, true> : k_step_geo_patch<T, V2, false>)

@@ -35,7 +35,6 @@ template <typename T, int V, bool VEL, int MAXD>
 __global__ void __launch_bounds__(kGroupThreads, MAXD <= 6 ? 4 : 3)
     k_step_group(StepArgs<T> A) {
     extern __shared__ __align__(16) unsigned char smem[];
-    constexpr bool DIFF = std::is_same<T, float>::value;
     using P = SlotStage<T>;
     constexpr int kStep = P::kSlotBytes / (int)sizeof(T);
     const int a0 = blockIdx.x * A.npb, n_nodes = (int)A.n_nodes;
@@ -116,18 +115,18 @@ __global__ void __launch_bounds__(kGroupThreads, MAXD <= 6 ? 4 : 3)
                        (size_t)k0 * kStep;
 #pragma unroll
     for (int d = 0; d < 3; ++d) acc[d] = vzero<T, V>();
-    if (deg > 0) to_diff<T, V, DIFF>(R[0], ua);
+    if (deg > 0) to_diff<T, V>(R[0], ua);
 #pragma unroll
     for (int j = 0; j < MAXD; ++j) {
         if (j < deg) {
-            to_diff<T, V, DIFF>(R[j + 1], ua);
+            to_diff<T, V>(R[j + 1], ua);
             if (j > 0 && !(srec[k0 + j].w & 1)) {  // fan break: a first neighbour of its own
                 Vec<T, V> b[3];
                 rows(b, row_at(u, srec[k0 + j].y, nodeb));
-                to_diff<T, V, DIFF>(b, ua);
-                slot_fma<T, V, DIFF>(K + kStep * j, C[j], b, R[j + 1], ua, acc);
+                to_diff<T, V>(b, ua);
+                slot_fma<T, V>(K + kStep * j, C[j], b, R[j + 1], ua, acc);
             } else {
-                slot_fma<T, V, DIFF>(K + kStep * j, C[j], R[j], R[j + 1], ua, acc);
+                slot_fma<T, V>(K + kStep * j, C[j], R[j], R[j + 1], ua, acc);
             }
         }
     }

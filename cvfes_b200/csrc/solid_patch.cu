@@ -116,7 +116,6 @@ __global__ void __launch_bounds__(32 * W, 1)
     k_step_patch(StepArgs<T> A, PatchMap M, int max_degree) {
     extern __shared__ __align__(16) unsigned char smem[];
     using P = SlotStage<T>;
-    constexpr bool DIFF = std::is_same<T, float>::value;
     const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
     const uint32_t b_rec = 16u * max_degree, b_stage = b_rec + P::kSlotBytes * max_degree;
     unsigned char* const wb = smem + warp * (2 * b_stage);
@@ -289,8 +288,8 @@ __global__ void __launch_bounds__(32 * W, 1)
                 C[0] = ldg<T, V>(row_at(cf, r0.x, rowb));
                 rows(X[2], r1.z);
                 C[1] = ldg<T, V>(row_at(cf, r1.x, rowb));
-                if constexpr (DIFF) __syncwarp();
-                to_diff<T, V, DIFF>(X[0], ua);
+                if constexpr (sizeof(T) == 4) __syncwarp();
+                to_diff<T, V>(X[0], ua);
 #pragma unroll
                 for (int k = 0; k < 6; ++k) {
                     if (k < 4) {
@@ -302,10 +301,10 @@ __global__ void __launch_bounds__(32 * W, 1)
                     if (k == 2) prefetch_coef();
                     // FP32: the warp barriers keep the compiler from sinking the loads to
                     // their uses (400 against 425 us); FP64 is faster without (241 against 253)
-                    if constexpr (DIFF) __syncwarp();
-                    to_diff<T, V, DIFF>(X[k + 1], ua);
-                    slot_fma<T, V, DIFF>(K + kStep * k, C[k], X[k], X[k + 1], ua, acc);
-                    if constexpr (DIFF) __syncwarp();
+                    if constexpr (sizeof(T) == 4) __syncwarp();
+                    to_diff<T, V>(X[k + 1], ua);
+                    slot_fma<T, V>(K + kStep * k, C[k], X[k], X[k + 1], ua, acc);
+                    if constexpr (sizeof(T) == 4) __syncwarp();
                 }
             } else {
                 if (n > 0) {  // any fan: three buffers rotate, one element ahead
@@ -314,7 +313,7 @@ __global__ void __launch_bounds__(32 * W, 1)
                     rows(B0, r0.y);
                     rows(B1, r0.z);
                     c1 = ldg<T, V>(row_at(cf, r0.x, rowb));
-                    to_diff<T, V, DIFF>(B0, ua);
+                    to_diff<T, V>(B0, ua);
                     int k = 0;
                     auto phase = [&](Vec<T, V> (&prev)[3], Vec<T, V> (&cur)[3], const Vec<T, V>& c,
                                      Vec<T, V> (&nx)[3], Vec<T, V>& cn) {
@@ -325,11 +324,11 @@ __global__ void __launch_bounds__(32 * W, 1)
                             rows(nx, r.z);
                             cn = ldg<T, V>(row_at(cf, r.x, rowb));
                         }
-                        to_diff<T, V, DIFF>(cur, ua);
-                        slot_fma<T, V, DIFF>(K + kStep * k, c, prev, cur, ua, acc);
+                        to_diff<T, V>(cur, ua);
+                        slot_fma<T, V>(K + kStep * k, c, prev, cur, ua, acc);
                         if (next && !(r.w & 1)) {  // fan break: a first neighbour of its own
                             rows(cur, r.y);
-                            to_diff<T, V, DIFF>(cur, ua);
+                            to_diff<T, V>(cur, ua);
                         }
                         ++k;
                     };

@@ -18,10 +18,11 @@
 // with c = damp*m, rearranged so that the coefficients multiplying u_n carry no
 // rounding error (this matters for the FP32 state form).
 //
-// FP32 form (DIFF): each element row is applied to neighbour differences
-// (u_b - u_a); the self block is minus the sum of the two others, so rigid
-// translations are exactly in the null space and the FP32 cancellation error
-// scales with |u_b - u_a| instead of |u|.
+// Each element row is applied to neighbour differences (u_b - u_a); the self block is minus
+// the sum of the two others and is not read, so rigid translations are exactly in the null
+// space, the cancellation error scales with |u_b - u_a| instead of |u|, and a row takes 18
+// products instead of 27 (FP64: 256x512 tube, 64 samples 231 -> 210 us a step; reverse step
+// 215 -> 202 us on 128x320 nodes).
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -34,7 +35,7 @@
 
 namespace cvfes {
 
-template <typename T, int V, bool DIFF>
+template <typename T, int V>
 __global__ void __launch_bounds__(256) k_step(StepArgs<T> A) {
     long long a;
     int vec;
@@ -52,7 +53,7 @@ __global__ void __launch_bounds__(256) k_step(StepArgs<T> A) {
     T f[3];
     node_load<T>(A, a, step_pressure<T>(A), f);
     Vec<T, V> acc[3];
-    ku_row<T, V, DIFF>(A.node_ptr, A.rec, A.slab, A.coef, A.u, S, col, a, ua, acc);
+    ku_row<T, V>(A.node_ptr, A.rec, A.slab, A.coef, A.u, S, col, a, ua, acc);
     step_epilogue<T, V>(A, a, S, col, row, ua, acc, f);
 }
 
@@ -60,7 +61,7 @@ __global__ void __launch_bounds__(256) k_step(StepArgs<T> A) {
 // Row a of K_s u_s with the node's slot records and stiffness rows read from
 // shared memory; the gathers of element k+1 are issued before element k is
 // multiplied, so two elements' loads are in flight per warp.
-template <typename T, int V, bool DIFF>
+template <typename T, int V>
 __device__ __forceinline__ void ku_row_staged(const int4* srec, const T* sslab, int k0, int k1,
                                               const T* __restrict__ u, const T* __restrict__ coef,
                                               size_t S, size_t col, const Vec<T, V> (&ua)[3],
@@ -96,16 +97,12 @@ __device__ __forceinline__ void ku_row_staged(const int4* srec, const T* sslab, 
         Vec<T, V> d1[3], d2[3];
 #pragma unroll
         for (int d = 0; d < 3; ++d) {
-            d1[d] = DIFF ? vsub(x1[d], ua[d]) : x1[d];
-            d2[d] = DIFF ? vsub(x2[d], ua[d]) : x2[d];
+            d1[d] = vsub(x1[d], ua[d]);
+            d2[d] = vsub(x2[d], ua[d]);
         }
 #pragma unroll
         for (int i = 0; i < 3; ++i) {
             Vec<T, V> t = vzero<T, V>();
-            if constexpr (!DIFF) {
-#pragma unroll
-                for (int jj = 0; jj < 3; ++jj) axpy(t, K[3 * i + jj], ua[jj]);
-            }
 #pragma unroll
             for (int jj = 0; jj < 3; ++jj) axpy(t, K[9 + 3 * i + jj], d1[jj]);
 #pragma unroll
@@ -133,7 +130,7 @@ __device__ __forceinline__ void ku_row_staged(const int4* srec, const T* sslab, 
 // of one sample chunk (blockIdx.y).  Thread 0 stages the block's slot records and
 // stiffness rows with two TMA bulk copies while every warp loads its node's own
 // displacement and prefetches its epilogue rows into L2.
-template <typename T, int V, bool DIFF, int MINB>
+template <typename T, int V, int MINB>
 __global__ void __launch_bounds__(256, MINB) k_step_staged(StepArgs<T> A) {
     extern __shared__ __align__(16) unsigned char smem[];
     const int warp = threadIdx.x >> 5;
@@ -189,11 +186,11 @@ __global__ void __launch_bounds__(256, MINB) k_step_staged(StepArgs<T> A) {
     }
     Vec<T, V> acc[3];
     const int k0 = __ldg(A.node_ptr + a) - kb, k1 = __ldg(A.node_ptr + a + 1) - kb;
-    ku_row_staged<T, V, DIFF>(srec, sslab, k0, k1, A.u, A.coef, S, col, ua, acc);
+    ku_row_staged<T, V>(srec, sslab, k0, k1, A.u, A.coef, S, col, ua, acc);
     step_epilogue<T, V>(A, a, S, col, row, ua, acc, f);
 }
 
-template <typename T, int V, bool DIFF>
+template <typename T, int V>
 __global__ void __launch_bounds__(256)
     k_kmul(const int32_t* node_ptr, const int4* rec, const T* slab, const T* coef, const T* u,
            T* res, long long n_nodes, int S_, int accumulate, int tpn, int npb) {
@@ -206,7 +203,7 @@ __global__ void __launch_bounds__(256)
     Vec<T, V> ua[3], acc[3];
 #pragma unroll
     for (int d = 0; d < 3; ++d) ua[d] = ldg<T, V>(u + row + d * S);
-    ku_row<T, V, DIFF>(node_ptr, rec, slab, coef, u, S, col, a, ua, acc);
+    ku_row<T, V>(node_ptr, rec, slab, coef, u, S, col, a, ua, acc);
 #pragma unroll
     for (int d = 0; d < 3; ++d) {
         Vec<T, V> o = acc[d];
@@ -272,7 +269,7 @@ __global__ void k_clock_add(long long* clock, long long n) { clock[0] += n; }
 // With pf_dist > 0 the last warp of the first chunk of every pf_group-th node block
 // prefetches the rows of the pf_group node blocks pf_dist nodes ahead.
 // AHEAD = 2: each element's rows are requested two elements ahead (ku_row_fan2).
-template <typename T, int V, bool DIFF, int MINB, int AHEAD = 1>
+template <typename T, int V, int MINB, int AHEAD = 1>
 __global__ void __launch_bounds__(256, MINB) k_step_fan(StepArgs<T> A) {
     extern __shared__ __align__(16) unsigned char smem[];
     const int warp = threadIdx.x >> 5;
@@ -335,9 +332,9 @@ __global__ void __launch_bounds__(256, MINB) k_step_fan(StepArgs<T> A) {
     Vec<T, V> acc[3];
     const int k0 = __ldg(A.node_ptr + a) - kb, k1 = __ldg(A.node_ptr + a + 1) - kb;
     if constexpr (AHEAD == 2)
-        ku_row_fan2<T, V, DIFF>(srec, sslab, k0, k1, A.u, A.coef, S, col, ua, acc);
+        ku_row_fan2<T, V>(srec, sslab, k0, k1, A.u, A.coef, S, col, ua, acc);
     else
-        ku_row_fan<T, V, DIFF>(srec, sslab, k0, k1, A.u, A.coef, S, col, ua, acc);
+        ku_row_fan<T, V>(srec, sslab, k0, k1, A.u, A.coef, S, col, ua, acc);
     step_epilogue<T, V>(A, a, S, col, row, ua, acc, f);
 }
 
@@ -349,7 +346,7 @@ __global__ void __launch_bounds__(256, MINB) k_step_fan(StepArgs<T> A) {
 // over the fan kernel's one-element lookahead.  Neighbour row j+1 is the second
 // neighbour of slot j and the first of slot j+1 (fan order); a fan break past slot 0
 // loads its first neighbour when the slot is multiplied.
-template <typename T, int V, bool DIFF, int MAXD, int MINB>
+template <typename T, int V, int MAXD, int MINB>
 __global__ void __launch_bounds__(256, MINB) k_step_burst(StepArgs<T> A) {
     extern __shared__ __align__(16) unsigned char smem[];
     const int warp = threadIdx.x >> 5;
@@ -421,20 +418,20 @@ __global__ void __launch_bounds__(256, MINB) k_step_burst(StepArgs<T> A) {
     Vec<T, V> acc[3];
 #pragma unroll
     for (int d = 0; d < 3; ++d) acc[d] = vzero<T, V>();
-    if (deg > 0) to_diff<T, V, DIFF>(R[0], ua);
+    if (deg > 0) to_diff<T, V>(R[0], ua);
 #pragma unroll
     for (int j = 0; j < MAXD; ++j) {
         if (j < deg) {
-            to_diff<T, V, DIFF>(R[j + 1], ua);
+            to_diff<T, V>(R[j + 1], ua);
             const int4 r = srec[k0 + j];
             if (j > 0 && !(r.w & 1)) {  // fan break: a first neighbour of its own
                 Vec<T, V> b1[3];
                 load_rows<T, V>(b1, A.u, r.y, S, col);
-                to_diff<T, V, DIFF>(b1, ua);
-                slot_fma<T, V, DIFF>(sslab + (size_t)kSlabStride * (k0 + j), C[j], b1, R[j + 1],
+                to_diff<T, V>(b1, ua);
+                slot_fma<T, V>(sslab + (size_t)kSlabStride * (k0 + j), C[j], b1, R[j + 1],
                                      ua, acc);
             } else {
-                slot_fma<T, V, DIFF>(sslab + (size_t)kSlabStride * (k0 + j), C[j], R[j], R[j + 1],
+                slot_fma<T, V>(sslab + (size_t)kSlabStride * (k0 + j), C[j], R[j], R[j + 1],
                                      ua, acc);
             }
         }
@@ -477,7 +474,7 @@ __device__ __forceinline__ int4 shfl4(int4 v, int src) {
                      __shfl_sync(0xffffffffu, v.z, src), __shfl_sync(0xffffffffu, v.w, src));
 }
 
-template <typename T, int V, bool DIFF, int STAGES>
+template <typename T, int V, int STAGES>
 __global__ void __launch_bounds__(256, 1) k_step_pipe(PipeArgs<T> P) {
     extern __shared__ __align__(16) unsigned char smem[];
     const StepArgs<T>& A = P.s;
@@ -620,19 +617,19 @@ __global__ void __launch_bounds__(256, 1) k_step_pipe(PipeArgs<T> P) {
                 const unsigned char* x1p = open ? ln + 7 * RB : ln + (kPipeFixedRows + 4 * (deg - 1)) * RB;
 #pragma unroll
                 for (int d = 0; d < 3; ++d) d1[d] = lds<T, V>(x1p + d * RB);
-                to_diff<T, V, DIFF>(d1, ua);
+                to_diff<T, V>(d1, ua);
                 for (int k = 0; k < deg; ++k) {
                     const unsigned char* xp = ln + (kPipeFixedRows + 4 * k) * RB;
                     if (k > 0 && !(srec[k].w & 1)) {  // fan break: first neighbour from global
                         load_rows<T, V>(d1, A.u, srec[k].y, S, col);
-                        to_diff<T, V, DIFF>(d1, ua);
+                        to_diff<T, V>(d1, ua);
                     }
                     Vec<T, V> d2[3];
 #pragma unroll
                     for (int d = 0; d < 3; ++d) d2[d] = lds<T, V>(xp + d * RB);
-                    to_diff<T, V, DIFF>(d2, ua);
+                    to_diff<T, V>(d2, ua);
                     const Vec<T, V> c = lds<T, V>(xp + 3 * RB);
-                    slot_fma<T, V, DIFF>(sslab + (size_t)kSlabStride * k, c, d1, d2, ua, acc);
+                    slot_fma<T, V>(sslab + (size_t)kSlabStride * k, c, d1, d2, ua, acc);
 #pragma unroll
                     for (int d = 0; d < 3; ++d) d1[d] = d2[d];
                 }
@@ -673,7 +670,7 @@ __global__ void __launch_bounds__(256, 1) k_step_pipe(PipeArgs<T> P) {
 // rows of the per-warp buffer: 3 (first x1) + 4 per slot (x2 dofs, coef) + 4 (u_prev, invm)
 __host__ __device__ constexpr int gather_rows(int max_degree) { return 7 + 4 * max_degree; }
 
-template <typename T, int V, bool DIFF, int MINB>
+template <typename T, int V, int MINB>
 __global__ void __launch_bounds__(256, MINB) k_step_gather(StepArgs<T> A) {
     extern __shared__ __align__(16) unsigned char smem[];
     constexpr int LB = V * (int)sizeof(T);  // bytes of one lane's slice of a row
@@ -770,17 +767,15 @@ __global__ void __launch_bounds__(256, MINB) k_step_gather(StepArgs<T> A) {
 #pragma unroll
         for (int d = 0; d < 3; ++d) {
             d2[d] = lds<T, V>(x2p + d * RB);
-            if constexpr (DIFF) {
-                d1[d] = vsub(d1[d], ua[d]);
-                d2[d] = vsub(d2[d], ua[d]);
-            }
+            d1[d] = vsub(d1[d], ua[d]);
+            d2[d] = vsub(d2[d], ua[d]);
         }
         const Vec<T, V> c = lds<T, V>(x2p + 3 * RB);
         const T* K = sslab + (size_t)kSlabStride * k;
         T kk[28];
         if constexpr (sizeof(T) == 4) {
 #pragma unroll
-            for (int q = (DIFF ? 2 : 0); q < 7; ++q) {
+            for (int q = 2; q < 7; ++q) {
                 const float4 t = reinterpret_cast<const float4*>(K)[q];
                 kk[4 * q] = t.x;
                 kk[4 * q + 1] = t.y;
@@ -789,7 +784,7 @@ __global__ void __launch_bounds__(256, MINB) k_step_gather(StepArgs<T> A) {
             }
         } else {
 #pragma unroll
-            for (int q = (DIFF ? 4 : 0); q < 14; ++q) {
+            for (int q = 4; q < 14; ++q) {
                 const double2 t = reinterpret_cast<const double2*>(K)[q];
                 kk[2 * q] = t.x;
                 kk[2 * q + 1] = t.y;
@@ -798,10 +793,6 @@ __global__ void __launch_bounds__(256, MINB) k_step_gather(StepArgs<T> A) {
 #pragma unroll
         for (int i = 0; i < 3; ++i) {
             Vec<T, V> t = vzero<T, V>();
-            if constexpr (!DIFF) {
-#pragma unroll
-                for (int jj = 0; jj < 3; ++jj) axpy(t, kk[3 * i + jj], ua[jj]);
-            }
 #pragma unroll
             for (int jj = 0; jj < 3; ++jj) axpy(t, kk[9 + 3 * i + jj], d1[jj]);
 #pragma unroll
@@ -1032,7 +1023,7 @@ inline int sm_count() {
 }
 
 // Persistent pipelined step: `warps` warps per block, `stages` stages per warp.
-template <typename T, int V, bool DIFF, int STAGES>
+template <typename T, int V, int STAGES>
 int launch_pipe_s(const StepArgs<T>& A, long long max_deg, int warps, cudaStream_t st) {
     constexpr int RB = 32 * V * (int)sizeof(T);
     PipeArgs<T> P;
@@ -1045,7 +1036,7 @@ int launch_pipe_s(const StepArgs<T>& A, long long max_deg, int warps, cudaStream
     P.stage_bytes = (P.hdr_off + 64 + 127) / 128 * 128;
     const size_t smem = (size_t)warps * ((size_t)STAGES * P.stage_bytes + 64);
     if (smem > 227 * 1024) return CVFES_ERR_UNSUPPORTED;
-    auto kernel = k_step_pipe<T, V, DIFF, STAGES>;
+    auto kernel = k_step_pipe<T, V, STAGES>;
     if (smem > 48 * 1024) {
         cudaError_t e =
             cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
@@ -1065,12 +1056,12 @@ int launch_pipe_s(const StepArgs<T>& A, long long max_deg, int warps, cudaStream
     return CVFES_OK;
 }
 
-template <typename T, int V, bool DIFF>
+template <typename T, int V>
 int launch_pipe(const StepArgs<T>& A, long long max_deg, int warps, int stages, cudaStream_t st) {
     switch (stages) {
-        case 4: return launch_pipe_s<T, V, DIFF, 4>(A, max_deg, warps, st);
-        case 3: return launch_pipe_s<T, V, DIFF, 3>(A, max_deg, warps, st);
-        default: return launch_pipe_s<T, V, DIFF, 2>(A, max_deg, warps, st);
+        case 4: return launch_pipe_s<T, V, 4>(A, max_deg, warps, st);
+        case 3: return launch_pipe_s<T, V, 3>(A, max_deg, warps, st);
+        default: return launch_pipe_s<T, V, 2>(A, max_deg, warps, st);
     }
 }
 
@@ -1143,55 +1134,55 @@ int fanp_blocks_per_sm(const void* kernel, int threads, size_t smem, int* per_sm
 // the patch kernel).  Both give bitwise the same norms.
 static std::atomic<int> g_norms_mode{0};
 
-template <typename T, int V, bool DIFF, int MAXD>
+template <typename T, int V, int MAXD>
 int launch_burst(int minb, dim3 g1, int threads, size_t smem, cudaStream_t st,
                  const StepArgs<T>& A) {
     switch (minb) {
-        case 4: return launch_staged(k_step_burst<T, V, DIFF, MAXD, 4>, g1, threads, smem, st, A);
-        case 3: return launch_staged(k_step_burst<T, V, DIFF, MAXD, 3>, g1, threads, smem, st, A);
-        case 2: return launch_staged(k_step_burst<T, V, DIFF, MAXD, 2>, g1, threads, smem, st, A);
-        default: return launch_staged(k_step_burst<T, V, DIFF, MAXD, 1>, g1, threads, smem, st, A);
+        case 4: return launch_staged(k_step_burst<T, V, MAXD, 4>, g1, threads, smem, st, A);
+        case 3: return launch_staged(k_step_burst<T, V, MAXD, 3>, g1, threads, smem, st, A);
+        case 2: return launch_staged(k_step_burst<T, V, MAXD, 2>, g1, threads, smem, st, A);
+        default: return launch_staged(k_step_burst<T, V, MAXD, 1>, g1, threads, smem, st, A);
     }
 }
 
-template <typename T, int V, bool DIFF>
+template <typename T, int V>
 int launch_staged_v(int variant, int minb, dim3 grid, int threads, size_t smem, cudaStream_t st,
                     const StepArgs<T>& A, long long max_degree = 0) {
     if (variant == 5 && max_degree > 0 && max_degree <= 8) {
         const dim3 g1((unsigned)((long long)grid.x * grid.y));
-        if (max_degree <= 6) return launch_burst<T, V, DIFF, 6>(minb, g1, threads, smem, st, A);
-        return launch_burst<T, V, DIFF, 8>(minb, g1, threads, smem, st, A);
+        if (max_degree <= 6) return launch_burst<T, V, 6>(minb, g1, threads, smem, st, A);
+        return launch_burst<T, V, 8>(minb, g1, threads, smem, st, A);
     }
     if (variant == 8) {
         const dim3 g1((unsigned)((long long)grid.x * grid.y));
         switch (minb) {
-            case 3: return launch_staged(k_step_fan<T, V, DIFF, 3, 2>, g1, threads, smem, st, A);
-            case 2: return launch_staged(k_step_fan<T, V, DIFF, 2, 2>, g1, threads, smem, st, A);
-            default: return launch_staged(k_step_fan<T, V, DIFF, 1, 2>, g1, threads, smem, st, A);
+            case 3: return launch_staged(k_step_fan<T, V, 3, 2>, g1, threads, smem, st, A);
+            case 2: return launch_staged(k_step_fan<T, V, 2, 2>, g1, threads, smem, st, A);
+            default: return launch_staged(k_step_fan<T, V, 1, 2>, g1, threads, smem, st, A);
         }
     }
     if (variant == 3 || variant == 5) {
         const dim3 g1((unsigned)((long long)grid.x * grid.y));
         switch (minb) {
-            case 4: return launch_staged(k_step_fan<T, V, DIFF, 4>, g1, threads, smem, st, A);
-            case 3: return launch_staged(k_step_fan<T, V, DIFF, 3>, g1, threads, smem, st, A);
-            case 2: return launch_staged(k_step_fan<T, V, DIFF, 2>, g1, threads, smem, st, A);
-            default: return launch_staged(k_step_fan<T, V, DIFF, 1>, g1, threads, smem, st, A);
+            case 4: return launch_staged(k_step_fan<T, V, 4>, g1, threads, smem, st, A);
+            case 3: return launch_staged(k_step_fan<T, V, 3>, g1, threads, smem, st, A);
+            case 2: return launch_staged(k_step_fan<T, V, 2>, g1, threads, smem, st, A);
+            default: return launch_staged(k_step_fan<T, V, 1>, g1, threads, smem, st, A);
         }
     }
     if (variant == 2) {
         switch (minb) {
-            case 4: return launch_staged(k_step_gather<T, V, DIFF, 4>, grid, threads, smem, st, A);
-            case 3: return launch_staged(k_step_gather<T, V, DIFF, 3>, grid, threads, smem, st, A);
-            case 2: return launch_staged(k_step_gather<T, V, DIFF, 2>, grid, threads, smem, st, A);
-            default: return launch_staged(k_step_gather<T, V, DIFF, 1>, grid, threads, smem, st, A);
+            case 4: return launch_staged(k_step_gather<T, V, 4>, grid, threads, smem, st, A);
+            case 3: return launch_staged(k_step_gather<T, V, 3>, grid, threads, smem, st, A);
+            case 2: return launch_staged(k_step_gather<T, V, 2>, grid, threads, smem, st, A);
+            default: return launch_staged(k_step_gather<T, V, 1>, grid, threads, smem, st, A);
         }
     }
     switch (minb) {
-        case 4: return launch_staged(k_step_staged<T, V, DIFF, 4>, grid, threads, smem, st, A);
-        case 3: return launch_staged(k_step_staged<T, V, DIFF, 3>, grid, threads, smem, st, A);
-        case 2: return launch_staged(k_step_staged<T, V, DIFF, 2>, grid, threads, smem, st, A);
-        default: return launch_staged(k_step_staged<T, V, DIFF, 1>, grid, threads, smem, st, A);
+        case 4: return launch_staged(k_step_staged<T, V, 4>, grid, threads, smem, st, A);
+        case 3: return launch_staged(k_step_staged<T, V, 3>, grid, threads, smem, st, A);
+        case 2: return launch_staged(k_step_staged<T, V, 2>, grid, threads, smem, st, A);
+        default: return launch_staged(k_step_staged<T, V, 1>, grid, threads, smem, st, A);
     }
 }
 
@@ -1271,7 +1262,6 @@ int launch_step(const cvfes_solid_mesh* m, const T* coef, const T* invm, const T
     }
     int V = pick_vec<T>(ptrs, 5, A.S);
     while (V > tune.vec) V /= 2;
-    constexpr bool DIFF = std::is_same<T, float>::value;
     const bool fused = norm_work && max_rows > 0 && !A.probe_polls;
     if (tune.staged == 6) {  // few samples: the group kernel (and the separate norms pass)
         const int grc = launch_step_group<T>(m, A, V, after_step, st);
@@ -1314,11 +1304,11 @@ int launch_step(const cvfes_solid_mesh* m, const T* coef, const T* invm, const T
         int prc = CVFES_ERR_UNSUPPORTED;
         if (V == 4) {
             if constexpr (sizeof(T) == 4)
-                prc = launch_pipe<T, 4, DIFF>(A, m->max_degree, tune.npb, stages, st);
+                prc = launch_pipe<T, 4>(A, m->max_degree, tune.npb, stages, st);
         } else if (V == 2) {
-            prc = launch_pipe<T, 2, DIFF>(A, m->max_degree, tune.npb, stages, st);
+            prc = launch_pipe<T, 2>(A, m->max_degree, tune.npb, stages, st);
         } else {
-            prc = launch_pipe<T, 1, DIFF>(A, m->max_degree, tune.npb, stages, st);
+            prc = launch_pipe<T, 1>(A, m->max_degree, tune.npb, stages, st);
         }
         if (prc != CVFES_ERR_UNSUPPORTED) return prc;  // else fall through to a smaller kernel
     }
@@ -1338,13 +1328,13 @@ int launch_step(const cvfes_solid_mesh* m, const T* coef, const T* invm, const T
         const int threads = 32 * A.npb;
         if (V == 4) {
             if constexpr (sizeof(T) == 4)
-                rc = launch_staged_v<T, 4, DIFF>(tune.staged, tune.minb, grid, threads, smem, st,
+                rc = launch_staged_v<T, 4>(tune.staged, tune.minb, grid, threads, smem, st,
                                                  A, m->max_degree);
         } else if (V == 2) {
-            rc = launch_staged_v<T, 2, DIFF>(tune.staged, tune.minb, grid, threads, smem, st, A,
+            rc = launch_staged_v<T, 2>(tune.staged, tune.minb, grid, threads, smem, st, A,
                                              m->max_degree);
         } else {
-            rc = launch_staged_v<T, 1, DIFF>(tune.staged, tune.minb, grid, threads, smem, st, A,
+            rc = launch_staged_v<T, 1>(tune.staged, tune.minb, grid, threads, smem, st, A,
                                              m->max_degree);
         }
         return rc;
@@ -1359,11 +1349,11 @@ int launch_step(const cvfes_solid_mesh* m, const T* coef, const T* invm, const T
     A.tpn = rg.tpn;
     A.npb = rg.npb;
     if (V == 4) {
-        if constexpr (sizeof(T) == 4) k_step<T, 4, DIFF><<<rg.grid, block, 0, st>>>(A);
+        if constexpr (sizeof(T) == 4) k_step<T, 4><<<rg.grid, block, 0, st>>>(A);
     } else if (V == 2) {
-        k_step<T, 2, DIFF><<<rg.grid, block, 0, st>>>(A);
+        k_step<T, 2><<<rg.grid, block, 0, st>>>(A);
     } else {
-        k_step<T, 1, DIFF><<<rg.grid, block, 0, st>>>(A);
+        k_step<T, 1><<<rg.grid, block, 0, st>>>(A);
     }
     CVFES_LAUNCH_CHECK("k_step");
     return CVFES_OK;
@@ -1381,18 +1371,17 @@ int launch_kmul(const cvfes_solid_mesh* m, const T* coef, const T* u, T* res, in
     const int block = 256;
     const RowGrid rg = row_grid(m->n_nodes, S / V, block);
     const dim3 grid = rg.grid;
-    constexpr bool DIFF = std::is_same<T, float>::value;
     const int4* rec = reinterpret_cast<const int4*>(m->slot_rec);
     const T* slab = static_cast<const T*>(m->slot_k);
     if (V == 4) {
         if constexpr (sizeof(T) == 4)
-            k_kmul<T, 4, DIFF><<<grid, block, 0, st>>>(m->node_ptr, rec, slab, coef, u, res,
+            k_kmul<T, 4><<<grid, block, 0, st>>>(m->node_ptr, rec, slab, coef, u, res,
                                                        m->n_nodes, S, accumulate, rg.tpn, rg.npb);
     } else if (V == 2) {
-        k_kmul<T, 2, DIFF><<<grid, block, 0, st>>>(m->node_ptr, rec, slab, coef, u, res,
+        k_kmul<T, 2><<<grid, block, 0, st>>>(m->node_ptr, rec, slab, coef, u, res,
                                                    m->n_nodes, S, accumulate, rg.tpn, rg.npb);
     } else {
-        k_kmul<T, 1, DIFF><<<grid, block, 0, st>>>(m->node_ptr, rec, slab, coef, u, res,
+        k_kmul<T, 1><<<grid, block, 0, st>>>(m->node_ptr, rec, slab, coef, u, res,
                                                    m->n_nodes, S, accumulate, rg.tpn, rg.npb);
     }
     CVFES_LAUNCH_CHECK("k_kmul");

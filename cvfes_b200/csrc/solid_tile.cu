@@ -176,7 +176,6 @@ __global__ void __launch_bounds__(512, 1)
     k_step_tile(StepArgs<T> A, TileArgs TA, const __grid_constant__ CUtensorMap mu,
                 const __grid_constant__ CUtensorMap mc) {
     constexpr int C = 32 * V;
-    constexpr bool DIFF = std::is_same<T, float>::value;
     extern __shared__ __align__(128) unsigned char smem[];
     const int warp = threadIdx.x >> 5;
     const int lane = threadIdx.x & 31;
@@ -254,9 +253,9 @@ __global__ void __launch_bounds__(512, 1)
                     const Vec<T, V> c = r.x >= 0
                                             ? lds_row<T, V>(sc + (size_t)r.x * C + lv)
                                             : ldg<T, V>(A.coef + (size_t)(-1 - r.x) * S + col);
-                    to_diff<T, V, DIFF>(d1, ua);
-                    to_diff<T, V, DIFF>(d2, ua);
-                    slot_fma<T, V, DIFF>(sslab + (size_t)kSlabStride * k, c, d1, d2, ua, acc);
+                    to_diff<T, V>(d1, ua);
+                    to_diff<T, V>(d2, ua);
+                    slot_fma<T, V>(sslab + (size_t)kSlabStride * k, c, d1, d2, ua, acc);
                 }
                 step_update<T, V>(A, S, row, ua, acc, fc, upc, imc);
             }

@@ -400,7 +400,7 @@ inline RowGrid row_grid(long long n_nodes, int sv, int block) {
 }
 
 // Row a of K_s u_s for VEC samples starting at column col.
-template <typename T, int V, bool DIFF>
+template <typename T, int V>
 __device__ __forceinline__ void ku_row(const int32_t* __restrict__ node_ptr,
                                        const int4* __restrict__ rec, const T* __restrict__ slab,
                                        const T* __restrict__ coef, const T* __restrict__ u,
@@ -424,14 +424,14 @@ __device__ __forceinline__ void ku_row(const int32_t* __restrict__ node_ptr,
 #pragma unroll
             for (int d = 0; d < 3; ++d) {
                 x1[d] = ldg<T, V>(p1 + d * S);
-                if constexpr (DIFF) x1[d] = vsub(x1[d], ua[d]);
+                x1[d] = vsub(x1[d], ua[d]);
             }
         }
         const T* p2 = u + (size_t)r.z * 3 * S + col;
 #pragma unroll
         for (int d = 0; d < 3; ++d) {
             x2[d] = ldg<T, V>(p2 + d * S);
-            if constexpr (DIFF) x2[d] = vsub(x2[d], ua[d]);
+            x2[d] = vsub(x2[d], ua[d]);
         }
         const Vec<T, V> c = ldg<T, V>(coef + (size_t)r.x * S + col);
         const T* K = slab + (size_t)kSlabStride * k;
@@ -456,10 +456,6 @@ __device__ __forceinline__ void ku_row(const int32_t* __restrict__ node_ptr,
 #pragma unroll
         for (int i = 0; i < 3; ++i) {
             Vec<T, V> t = vzero<T, V>();
-            if constexpr (!DIFF) {
-#pragma unroll
-                for (int jj = 0; jj < 3; ++jj) axpy(t, kk[3 * i + jj], ua[jj]);
-            }
 #pragma unroll
             for (int jj = 0; jj < 3; ++jj) axpy(t, kk[9 + 3 * i + jj], x1[jj]);
 #pragma unroll
@@ -582,21 +578,19 @@ __device__ __forceinline__ void load_rows(Vec<T, V> (&x)[3], const T* __restrict
 #pragma unroll
     for (int d = 0; d < 3; ++d) x[d] = ldg<T, V>(p + d * S);
 }
-template <typename T, int V, bool DIFF>
+template <typename T, int V>
 __device__ __forceinline__ void to_diff(Vec<T, V> (&x)[3], const Vec<T, V> (&ua)[3]) {
-    if constexpr (DIFF) {
 #pragma unroll
-        for (int d = 0; d < 3; ++d) x[d] = vsub(x[d], ua[d]);
-    }
+    for (int d = 0; d < 3; ++d) x[d] = vsub(x[d], ua[d]);
 }
-template <typename T, int V, bool DIFF>
+template <typename T, int V>
 __device__ __forceinline__ void slot_fma(const T* K, const Vec<T, V>& c, const Vec<T, V> (&d1)[3],
                                          const Vec<T, V> (&d2)[3], const Vec<T, V> (&ua)[3],
                                          Vec<T, V> (&acc)[3]) {
     T kk[28];
     if constexpr (sizeof(T) == 4) {
 #pragma unroll
-        for (int q = (DIFF ? 2 : 0); q < 7; ++q) {
+        for (int q = 2; q < 7; ++q) {
             const float4 t = reinterpret_cast<const float4*>(K)[q];
             kk[4 * q] = t.x;
             kk[4 * q + 1] = t.y;
@@ -605,7 +599,7 @@ __device__ __forceinline__ void slot_fma(const T* K, const Vec<T, V>& c, const V
         }
     } else {
 #pragma unroll
-        for (int q = (DIFF ? 4 : 0); q < 14; ++q) {
+        for (int q = 4; q < 14; ++q) {
             const double2 t = reinterpret_cast<const double2*>(K)[q];
             kk[2 * q] = t.x;
             kk[2 * q + 1] = t.y;
@@ -614,10 +608,6 @@ __device__ __forceinline__ void slot_fma(const T* K, const Vec<T, V>& c, const V
 #pragma unroll
     for (int i = 0; i < 3; ++i) {
         Vec<T, V> t = vzero<T, V>();
-        if constexpr (!DIFF) {
-#pragma unroll
-            for (int jj = 0; jj < 3; ++jj) axpy(t, kk[3 * i + jj], ua[jj]);
-        }
 #pragma unroll
         for (int jj = 0; jj < 3; ++jj) axpy(t, kk[9 + 3 * i + jj], d1[jj]);
 #pragma unroll
@@ -628,7 +618,7 @@ __device__ __forceinline__ void slot_fma(const T* K, const Vec<T, V>& c, const V
 
 // One element of the fan: prev holds the first neighbour (difference), cur the
 // second one as loaded; the next element's row set is issued into nxt first.
-template <typename T, int V, bool DIFF>
+template <typename T, int V>
 __device__ __forceinline__ void fan_phase(int& k, int k1, const int4* srec, const T* sslab,
                                           const T* __restrict__ u, const T* __restrict__ coef,
                                           size_t S, size_t col, const Vec<T, V> (&ua)[3],
@@ -642,16 +632,16 @@ __device__ __forceinline__ void fan_phase(int& k, int k1, const int4* srec, cons
         load_rows<T, V>(nxt, u, rn.z, S, col);
         cnxt = ldg<T, V>(coef + (size_t)rn.x * S + col);
     }
-    to_diff<T, V, DIFF>(cur, ua);
-    slot_fma<T, V, DIFF>(sslab + (size_t)kSlabStride * k, ccur, prev, cur, ua, acc);
+    to_diff<T, V>(cur, ua);
+    slot_fma<T, V>(sslab + (size_t)kSlabStride * k, ccur, prev, cur, ua, acc);
     if (more && !(rn.w & 1)) {  // fan break: the next element's first neighbour is new
         load_rows<T, V>(cur, u, rn.y, S, col);
-        to_diff<T, V, DIFF>(cur, ua);
+        to_diff<T, V>(cur, ua);
     }
     ++k;
 }
 
-template <typename T, int V, bool DIFF>
+template <typename T, int V>
 __device__ __forceinline__ void ku_row_fan(const int4* srec, const T* sslab, int k0, int k1,
                                            const T* __restrict__ u, const T* __restrict__ coef,
                                            size_t S, size_t col, const Vec<T, V> (&ua)[3],
@@ -664,14 +654,14 @@ __device__ __forceinline__ void ku_row_fan(const int4* srec, const T* sslab, int
     load_rows<T, V>(B0, u, r0.y, S, col);
     load_rows<T, V>(B1, u, r0.z, S, col);
     c1 = ldg<T, V>(coef + (size_t)r0.x * S + col);
-    to_diff<T, V, DIFF>(B0, ua);
+    to_diff<T, V>(B0, ua);
     int k = k0;
     while (true) {
-        fan_phase<T, V, DIFF>(k, k1, srec, sslab, u, coef, S, col, ua, acc, B0, B1, c1, B2, c2);
+        fan_phase<T, V>(k, k1, srec, sslab, u, coef, S, col, ua, acc, B0, B1, c1, B2, c2);
         if (k >= k1) break;
-        fan_phase<T, V, DIFF>(k, k1, srec, sslab, u, coef, S, col, ua, acc, B1, B2, c2, B0, c0);
+        fan_phase<T, V>(k, k1, srec, sslab, u, coef, S, col, ua, acc, B1, B2, c2, B0, c0);
         if (k >= k1) break;
-        fan_phase<T, V, DIFF>(k, k1, srec, sslab, u, coef, S, col, ua, acc, B2, B0, c0, B1, c1);
+        fan_phase<T, V>(k, k1, srec, sslab, u, coef, S, col, ua, acc, B2, B0, c0, B1, c1);
         if (k >= k1) break;
     }
 }
@@ -681,7 +671,7 @@ __device__ __forceinline__ void ku_row_fan(const int4* srec, const T* sslab, int
 // two elements ahead: four register buffers rotate (first neighbour, second neighbour,
 // and the next two elements' rows in flight), the slot loop unrolled four times.  The
 // products and their order are those of ku_row_fan, so the bits are the same.
-template <typename T, int V, bool DIFF>
+template <typename T, int V>
 __device__ __forceinline__ void fan2_phase(int& k, int k1, const int4* srec, const T* sslab,
                                            const T* __restrict__ u, const T* __restrict__ coef,
                                            size_t S, size_t col, const Vec<T, V> (&ua)[3],
@@ -693,19 +683,19 @@ __device__ __forceinline__ void fan2_phase(int& k, int k1, const int4* srec, con
         load_rows<T, V>(n2, u, r2.z, S, col);
         c2 = ldg<T, V>(coef + (size_t)r2.x * S + col);
     }
-    to_diff<T, V, DIFF>(cur, ua);
-    slot_fma<T, V, DIFF>(sslab + (size_t)kSlabStride * k, ccur, prev, cur, ua, acc);
+    to_diff<T, V>(cur, ua);
+    slot_fma<T, V>(sslab + (size_t)kSlabStride * k, ccur, prev, cur, ua, acc);
     if (k + 1 < k1) {
         const int4 r1 = srec[k + 1];
         if (!(r1.w & 1)) {  // fan break: the next element's first neighbour is new
             load_rows<T, V>(cur, u, r1.y, S, col);
-            to_diff<T, V, DIFF>(cur, ua);
+            to_diff<T, V>(cur, ua);
         }
     }
     ++k;
 }
 
-template <typename T, int V, bool DIFF>
+template <typename T, int V>
 __device__ __forceinline__ void ku_row_fan2(const int4* srec, const T* sslab, int k0, int k1,
                                             const T* __restrict__ u, const T* __restrict__ coef,
                                             size_t S, size_t col, const Vec<T, V> (&ua)[3],
@@ -723,16 +713,16 @@ __device__ __forceinline__ void ku_row_fan2(const int4* srec, const T* sslab, in
         load_rows<T, V>(B2, u, r1.z, S, col);
         c1 = ldg<T, V>(coef + (size_t)r1.x * S + col);
     }
-    to_diff<T, V, DIFF>(B0, ua);
+    to_diff<T, V>(B0, ua);
     int k = k0;
     while (true) {
-        fan2_phase<T, V, DIFF>(k, k1, srec, sslab, u, coef, S, col, ua, acc, B0, B1, c0, B3, c2);
+        fan2_phase<T, V>(k, k1, srec, sslab, u, coef, S, col, ua, acc, B0, B1, c0, B3, c2);
         if (k >= k1) break;
-        fan2_phase<T, V, DIFF>(k, k1, srec, sslab, u, coef, S, col, ua, acc, B1, B2, c1, B0, c3);
+        fan2_phase<T, V>(k, k1, srec, sslab, u, coef, S, col, ua, acc, B1, B2, c1, B0, c3);
         if (k >= k1) break;
-        fan2_phase<T, V, DIFF>(k, k1, srec, sslab, u, coef, S, col, ua, acc, B2, B3, c2, B1, c0);
+        fan2_phase<T, V>(k, k1, srec, sslab, u, coef, S, col, ua, acc, B2, B3, c2, B1, c0);
         if (k >= k1) break;
-        fan2_phase<T, V, DIFF>(k, k1, srec, sslab, u, coef, S, col, ua, acc, B3, B0, c3, B2, c1);
+        fan2_phase<T, V>(k, k1, srec, sslab, u, coef, S, col, ua, acc, B3, B0, c3, B2, c1);
         if (k >= k1) break;
     }
 }
@@ -759,8 +749,8 @@ __device__ __forceinline__ T* row_at(T* base, int i, uint32_t stride_bytes) {
 // kBytes: with the slot's record.
 template <typename T>
 struct SlotStage {
-    static constexpr int kFirst = sizeof(T) == 4 ? 2 : 0;
-    static constexpr int kWords = sizeof(T) == 4 ? 5 : 14;
+    static constexpr int kFirst = sizeof(T) == 4 ? 2 : 4;
+    static constexpr int kWords = sizeof(T) == 4 ? 5 : 10;
     static constexpr int kSlotBytes = 16 * kWords;
     static constexpr size_t kBytes = 16 + kSlotBytes;
 };
