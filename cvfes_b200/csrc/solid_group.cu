@@ -10,14 +10,14 @@
 //     registers) is read before the kernel waits for the step before it (programmatic
 //     dependent launch), under that step's tail;
 //   * after the wait all rows of u and u_{n-1} that the node needs are requested at once.
-// A block holds 128 threads' nodes; their slots are contiguous, so staging is coalesced.
+// A block holds 64 threads' nodes; their slots are contiguous, so staging is coalesced.
 // The register cost of the burst (up to nine rows of three vectors) allows 1 FP64 or 2
 // FP32 samples a thread.  Bits as the other step kernels: the same products in the same
 // order.
 //
-// 64 x 128 wall, 8 samples: FP64 8.4 -> 4.6 us a step, FP32 6.1 -> 3.5 us (graph replays);
-// 128 x 400 wall, FP32: 8 samples 14.7 -> 11.4 us, 16 samples 21.5 -> 20.2 us, 3 samples
-// 16.5 -> 9.4 us; FP64, 8 samples 48 -> 30 us.
+// 64 x 128 wall, 8 samples: FP64 8.4 -> 4.1 us a step, FP32 6.1 -> 3.5 us (graph replays);
+// 128 x 400 wall, FP32: 8 samples 14.7 -> 11.1 us, 16 samples 21.5 -> 19.3 us, 3 samples
+// 16.5 -> 9.3 us; FP64, 8 samples 48 -> 30 us.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -28,11 +28,11 @@
 
 namespace cvfes {
 
-constexpr int kGroupThreads = 128;
+constexpr int kGroupThreads = 64;  // FP64 64 x 128 wall, 8 samples: 4.25 us at 128, 4.64 at 256
 constexpr int kGroupDegree = 8;  // slots of a node held in registers
 
 template <typename T, int V, bool VEL, int MAXD>
-__global__ void __launch_bounds__(kGroupThreads, MAXD <= 6 ? 4 : 3)
+__global__ void __launch_bounds__(kGroupThreads, MAXD <= 6 ? 8 : 6)
     k_step_group(StepArgs<T> A) {
     extern __shared__ __align__(16) unsigned char smem[];
     using P = SlotStage<T>;
@@ -164,8 +164,8 @@ static int launch_group_k(const StepArgs<T>& A, bool after_step, cudaStream_t st
 
 // Taken for at most 16 sample vectors a node (2 FP32 samples each from 8 samples on), or 20
 // single samples: there the patch kernel leaves half its lanes idle.  Either side of the
-// line, 128 x 400 wall, us a step, group / patch: FP32 16 samples 20.2 / 44.1, 32 samples
-// 45.3 / 50.2, 64 samples 87 / 58; FP64 16 samples 56.3 / 67.8, 25 samples 92.7 / 68.3.
+// line, 128 x 400 wall, us a step, group / patch: FP32 16 samples 19.3 / 44.1, 32 samples
+// 43.2 / 50.2, 64 samples 87 / 57; FP64 16 samples 55.3 / 67.8, 25 samples 92 / 63.
 // Below 8 FP32 samples one a thread is the faster (4 samples: 8.4 against 10.1 us).
 template <typename T>
 int launch_step_group(const cvfes_solid_mesh* m, StepArgs<T> A, int vec_max, bool after_step,
@@ -177,8 +177,8 @@ int launch_step_group(const cvfes_solid_mesh* m, StepArgs<T> A, int vec_max, boo
         return 1;
     A.tpn = sv;
     A.nch = 1;
-    // at most 72 KB of slots: three blocks share an SM (one or two samples only)
-    const int fit = (int)(72 * 1024 / ((size_t)m->max_degree * SlotStage<T>::kBytes));
+    // at most 36 KB of slots: six blocks share an SM (one or two samples only)
+    const int fit = (int)(36 * 1024 / ((size_t)m->max_degree * SlotStage<T>::kBytes));
     A.npb = std::min(kGroupThreads / A.tpn, fit);
     A.cap_slots = A.npb * (int)m->max_degree;
 #define CVFES_GROUP(VV)                                                                     \
