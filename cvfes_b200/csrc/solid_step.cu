@@ -842,6 +842,8 @@ __global__ void __launch_bounds__(kNormThreads)
                     const T* __restrict__ up, const T* __restrict__ invm,
                     double* __restrict__ work) {
     __shared__ double part[4 * V][kNormThreads];
+    grid_dependency_release();
+    grid_dependency_wait();
     const long long chunk = blockIdx.x;
     const int groups = kNormThreads / tpn;
     const int g = threadIdx.x / tpn, l = threadIdx.x - g * tpn;
@@ -901,16 +903,19 @@ __global__ void __launch_bounds__(kNormThreads)
     }
 }
 
+// out_host (may be null): pinned host memory that the device can write, a copy of out.
 // total_nonfinite (may be null): the sum of the non-finite counts is added there.
 // Sums of the partial rows per (sample, quantity): a block owns kFinalPairs consecutive
 // (sample, quantity) pairs (coalesced across its lanes) and kFinalGroups row groups;
 // group g adds rows g, g + kFinalGroups, ... into four accumulators, and the groups'
 // sums are added in group order, so the result depends only on the row count.
-constexpr int kFinalPairs = 32, kFinalGroups = 8;
+constexpr int kFinalPairs = 32, kFinalGroups = 32;
 __global__ void __launch_bounds__(kFinalPairs * kFinalGroups)
     k_norms_final(long long n_chunks, int S, const double* __restrict__ work,
-                  double* __restrict__ out, double* __restrict__ total_nonfinite) {
+                  double* __restrict__ out, double* __restrict__ out_host,
+                  double* __restrict__ total_nonfinite) {
     __shared__ double part[kFinalGroups][kFinalPairs];
+    grid_dependency_wait();
     const int lp = threadIdx.x % kFinalPairs, g = threadIdx.x / kFinalPairs;
     const long long t = (long long)blockIdx.x * kFinalPairs + lp;  // pair s * 4 + q
     const long long P = 4LL * S;
@@ -934,6 +939,7 @@ __global__ void __launch_bounds__(kFinalPairs * kFinalGroups)
 #pragma unroll
     for (int k = 0; k < kFinalGroups; ++k) acc += part[k][lp];
     out[t] = acc;
+    if (out_host) out_host[t] = acc;
     if ((t & 3) == 3 && acc != 0.0 && total_nonfinite) atomicAdd(total_nonfinite, acc);
 }
 inline unsigned final_grid(long long S) { return grid_1d(4 * S, kFinalPairs); }
@@ -1440,30 +1446,34 @@ int launch_init(const cvfes_solid_mesh* m, const T* coef, const T* invm, const T
 
 template <typename T>
 int launch_norms_partial(long long n_nodes, long long S, long long nch, long long npc, const T* u,
-                         const T* up, const T* invm, double* work, bool vel, cudaStream_t st) {
+                         const T* up, const T* invm, double* work, bool vel, bool after_step,
+                         cudaStream_t st) {
     const void* ptrs[3] = {u, up, invm};
     const int V = pick_vec<T>(ptrs, 3, (int)S);
     const int sv = (int)S / V, tpn = std::min(sv, kNormThreads);
     const dim3 grid((unsigned)nch, (unsigned)((sv + tpn - 1) / tpn));
-#define CVFES_NORMS(VV)                                                                        \
-    if (vel)                                                                                   \
-        k_norms_partial<T, VV, true><<<grid, kNormThreads, 0, st>>>(n_nodes, (int)S, npc, tpn, \
-                                                                    u, up, invm, work);        \
-    else                                                                                       \
-        k_norms_partial<T, VV, false><<<grid, kNormThreads, 0, st>>>(n_nodes, (int)S, npc,     \
-                                                                     tpn, u, up, invm, work);
-    if (V == 4) {
-        if constexpr (sizeof(T) == 4) {
+#define CVFES_NORMS(VV)                                                                       \
+    return launch_step_kernel(vel ? k_norms_partial<T, VV, true> : k_norms_partial<T, VV, false>, \
+                              grid, kNormThreads, 0, after_step, st, "k_norms_partial",       \
+                              n_nodes, (int)S, npc, tpn, u, up, invm, work);
+    if constexpr (sizeof(T) == 4) {
+        if (V == 4) {
             CVFES_NORMS(4)
         }
-    } else if (V == 2) {
-        CVFES_NORMS(2)
-    } else {
-        CVFES_NORMS(1)
     }
+    if (V == 2) {
+        CVFES_NORMS(2)
+    }
+    CVFES_NORMS(1)
 #undef CVFES_NORMS
-    CVFES_LAUNCH_CHECK("k_norms_partial");
-    return CVFES_OK;
+}
+
+// The sums over the partial rows.  after: the launch before it on the stream is the kernel
+// that wrote them, so it may start under that kernel's tail.
+static int launch_norms_final(long long rows, long long S, const double* work, double* out,
+                              double* out_host, double* total, bool after, cudaStream_t st) {
+    return launch_step_kernel(k_norms_final, dim3(final_grid(S)), kFinalPairs * kFinalGroups, 0,
+                              after, st, "k_norms_final", rows, (int)S, work, out, out_host, total);
 }
 
 // CVFES_ERR_NONFINITE when the counter on the device is not zero (synchronises).
@@ -1475,22 +1485,22 @@ static int read_nonfinite(const double* total, cudaStream_t st) {
     return CVFES_OK;
 }
 
-// count: keep the non-finite total behind the partial rows (check_finite reads it).
+// out_host: as k_norms_final's.  count: keep the non-finite total behind the partial rows
+// (check_finite reads it).  after_step: the launch before it on the stream is a step.
 template <typename T>
 int launch_norms(long long n_nodes, long long S, const T* u, const T* up, const T* invm,
                  double* work, double* out, int check_finite, cudaStream_t st, bool vel = false,
-                 bool count = true) {
+                 double* out_host = nullptr, bool count = true, bool after_step = false) {
     if (n_nodes <= 0 || S <= 0 || S > INT32_MAX || !u || !up || !invm || !work || !out)
         return fail(CVFES_ERR_ARG, "cvfes_solid_norms: bad argument");
     const long long nch = norm_chunks(n_nodes);
     const long long npc = (n_nodes + nch - 1) / nch;
     double* total = count ? work + (size_t)nch * S * 4 : nullptr;
     if (total) CVFES_CUDA_TRY(cudaMemsetAsync(total, 0, sizeof(double), st));
-    int rc = launch_norms_partial<T>(n_nodes, S, nch, npc, u, up, invm, work, vel, st);
+    int rc = launch_norms_partial<T>(n_nodes, S, nch, npc, u, up, invm, work, vel,
+                                     after_step && !total, st);
+    if (!rc) rc = launch_norms_final(nch, S, work, out, out_host, total, true, st);
     if (rc) return rc;
-    k_norms_final<<<final_grid(S), kFinalPairs * kFinalGroups, 0, st>>>(nch, (int)S, work, out,
-                                                                        total);
-    CVFES_LAUNCH_CHECK("k_norms_final");
     return check_finite ? read_nonfinite(total, st) : CVFES_OK;
 }
 
@@ -1546,24 +1556,34 @@ int launch_step_norms(const cvfes_solid_mesh* m, const T* coef, const T* invm, c
                         work, &rows, max_rows);
     if (rc) return rc;
     const bool vel = m->state_form == 1;
+    // pinned host memory that this device can write gets the norms from the kernel itself
+    double* direct = nullptr;
+    if (out_host) {
+        cudaPointerAttributes at{};
+        if (cudaPointerGetAttributes(&at, out_host) == cudaSuccess &&
+            at.type == cudaMemoryTypeHost)
+            direct = static_cast<double*>(at.devicePointer);
+        else
+            (void)cudaGetLastError();
+    }
     if (rows == 0) {  // no fused kernel for this shape: the separate pass over the new state
         rc = launch_norms<T>(N, S, un, vel ? up : u, invm, work, out, out_host ? 0 : check_finite,
-                             st, vel, out_host == nullptr);
+                             st, vel, direct, out_host == nullptr, true);
         if (rc || !out_host) return rc;
     } else {
         double* total = out_host ? nullptr : work + (size_t)rows * S * 4;
         if (total) CVFES_CUDA_TRY(cudaMemsetAsync(total, 0, sizeof(double), st));
-        k_norms_final<<<final_grid(S), kFinalPairs * kFinalGroups, 0, st>>>(rows, (int)S, work,
-                                                                            out, total);
-        CVFES_LAUNCH_CHECK("k_norms_final");
+        rc = launch_norms_final(rows, S, work, out, direct, total, total == nullptr, st);
+        if (rc) return rc;
         if (!out_host) return check_finite ? read_nonfinite(total, st) : CVFES_OK;
     }
     // What the host reads: the norms, then the status word of the bounded waits.  The status
     // goes to pageable memory, so its copy returns only once it (and with it everything
     // before it on the stream) has arrived: no further synchronisation, and the word is
     // cleared only when it was set.  The non-finite total is the sum of the counts.
-    CVFES_CUDA_TRY(cudaMemcpyAsync(out_host, out, (size_t)S * 4 * sizeof(double),
-                                   cudaMemcpyDeviceToHost, st));
+    if (!direct)
+        CVFES_CUDA_TRY(cudaMemcpyAsync(out_host, out, (size_t)S * 4 * sizeof(double),
+                                       cudaMemcpyDeviceToHost, st));
     int32_t stat = 0;
     if (m->status)
         CVFES_CUDA_TRY(cudaMemcpyAsync(&stat, m->status, sizeof(stat), cudaMemcpyDeviceToHost, st));
@@ -1892,9 +1912,8 @@ extern "C" int cvfes_solid_norms_noalloc_f32(int64_t n_nodes, int64_t n_samples,
     cudaStream_t st = (cudaStream_t)stream;
     double* total = work + (size_t)nch * S * 4;  // the non-finite counter starts at zero
     CVFES_CUDA_TRY(cudaMemsetAsync(total, 0, sizeof(double), st));
-    rc = launch_norms_partial<float>(n_nodes, S, nch, npc, u, u_prev, invm, work, false, st);
+    rc = launch_norms_partial<float>(n_nodes, S, nch, npc, u, u_prev, invm, work, false, false, st);
+    if (!rc) rc = launch_norms_final(nch, S, work, out, nullptr, total, true, st);
     if (rc) return rc;
-    k_norms_final<<<final_grid(S), kFinalPairs * kFinalGroups, 0, st>>>(nch, (int)S, work, out, total);
-    CVFES_LAUNCH_CHECK("k_norms_final (fixed scratch)");
     return check_finite ? read_nonfinite(total, st) : CVFES_OK;
 }
