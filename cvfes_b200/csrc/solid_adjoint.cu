@@ -647,8 +647,8 @@ __global__ void __launch_bounds__(256, MINB) k_reverse_fan(RevArgs<T> A) {
 // Gamma row is requested before its products.  us a step, fan or persistent fan / this:
 // 128 x 400 wall, FP32 64 samples 155 / 116, 128 samples with G 315 / 235; 128 x 320 wall, FP64
 // 64 samples with G 267 / 213; 64 x 128 wall, 64 samples FP32 22.4 / 21.3, FP64 54.7 / 46.4.
-template <typename T, int V, bool GM>
-__global__ void __launch_bounds__(32 * kPatchWarps, 1)
+template <typename T, int V, bool GM, int W>
+__global__ void __launch_bounds__(32 * W, 1)
     k_reverse_patch(RevArgs<T> A, PatchMap M, int max_degree) {
     extern __shared__ __align__(16) unsigned char smem[];
     using P = SlotStage<T>;
@@ -662,7 +662,7 @@ __global__ void __launch_bounds__(32 * kPatchWarps, 1)
     const int vec = chunk * 32 + lane, last = A.S / V - 1;
     const bool on = vec <= last;
     const size_t S = (size_t)A.S, col = (size_t)(on ? vec : last) * V;
-    PatchWalk walk(M, warp, blockIdx.x / A.nch, gridDim.x / A.nch, 0, (int)A.n_nodes);
+    PatchWalk walk(M, warp, blockIdx.x / A.nch, gridDim.x / A.nch, 0, (int)A.n_nodes, W);
     auto stage = [&](int b, int k0, int n, int sg) {
         if (b >= 0) {
             const uint32_t d = smem_u32(wb + sg * b_stage);
@@ -936,19 +936,21 @@ int launch_rev_patch(const cvfes_solid_mesh* m, RevArgs<T> A, bool after_step, c
         m->n_nodes >= INT32_MAX / 2 || reinterpret_cast<uintptr_t>(A.own) % 16 ||
         reinterpret_cast<uintptr_t>(A.slab) % 16 || reinterpret_cast<uintptr_t>(A.rec) % 16)
         return 1;
-    const size_t smem = (size_t)kPatchWarps * 2 * slot * m->max_degree;
+    // what the registers allow (single FP32 samples, 128 x 400 wall, 37 samples: 183 us a step
+    // at 16 warps, 157 at 24; the others are slower above 16)
+    constexpr int W = sizeof(T) == 4 && V == 1 ? 24 : 16;
+    const size_t smem = (size_t)W * 2 * slot * m->max_degree;
     if (smem > 160 * 1024) return 1;
     A.nch = (A.S / V + 31) / 32;
-    const PatchMap M = patch_map(m->n_nodes, m->bandwidth);
-    auto kernel = A.gm ? k_reverse_patch<T, V, true> : k_reverse_patch<T, V, false>;
+    const PatchMap M = patch_map(m->n_nodes, m->bandwidth, W);
+    auto kernel = A.gm ? k_reverse_patch<T, V, true, W> : k_reverse_patch<T, V, false, W>;
     int per_sm = 0;
-    const int rc = fanp_blocks_per_sm(reinterpret_cast<const void*>(kernel), 32 * kPatchWarps,
-                                      smem, &per_sm);
+    const int rc = fanp_blocks_per_sm(reinterpret_cast<const void*>(kernel), 32 * W, smem, &per_sm);
     if (rc) return rc;
     const long long places = std::max(1LL, (long long)M.n_strips * M.tps);
     const long long per_chunk =
         std::max(1LL, std::min((long long)per_sm * device_sm_count() / A.nch, places));
-    return launch_step_kernel(kernel, dim3((unsigned)(per_chunk * A.nch)), 32 * kPatchWarps, smem,
+    return launch_step_kernel(kernel, dim3((unsigned)(per_chunk * A.nch)), 32 * W, smem,
                               after_step, st, "k_reverse_patch", A, M, (int)m->max_degree);
 }
 

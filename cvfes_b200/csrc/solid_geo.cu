@@ -219,9 +219,10 @@ __device__ __forceinline__ void geo_update(const StepArgs<T>& A, int a, size_t c
 // coefficient in flight.  Consecutive elements of a fan share an edge, so one neighbour is
 // gathered per element (two were, and their rows were 6 of the 7 gathered).  What bounds it
 // is the arithmetic: 93 packed or FP64 operations a slot against one row.
-// SAME: the geometry is the current state (ug == u).
-template <typename T, int V, bool SAME>
-__global__ void __launch_bounds__(256) k_step_geo(StepArgs<T> A, GeoArgs<T> G) {
+// SAME: the geometry is the current state (ug == u).  MAXT, MINB: threads of a block and
+// blocks an SM that the registers must allow (0: no say).
+template <typename T, int V, bool SAME, int MAXT = 256, int MINB = 0>
+__global__ void __launch_bounds__(MAXT, MINB) k_step_geo(StepArgs<T> A, GeoArgs<T> G) {
     const int t = threadIdx.x / A.tpn;
     const long long a = (long long)blockIdx.x * A.npb + t;
     const int vec = blockIdx.y * A.tpn + (threadIdx.x - t * A.tpn);
@@ -559,6 +560,11 @@ int launch_step_geo(const cvfes_solid_mesh* m, const T* coef, const T* invm, con
     const dim3 grid((unsigned)((m->n_nodes + A.npb - 1) / A.npb), (unsigned)parts);
     auto kernel = V == 2 ? (same ? k_step_geo<T, 2, true> : k_step_geo<T, 2, false>)
                          : (same ? k_step_geo<T, 1, true> : k_step_geo<T, 1, false>);
+    // On the current geometry FP64 singles and FP32 pairs fit 96 registers, five blocks of 128
+    // threads an SM: 96 x 200 wall, FP64 50 samples 88 -> 74 us a step, 128 x 400 wall, FP32 40
+    // samples 93 -> 80 (stored geometry at 96 registers: 98 -> 106).
+    constexpr int VT = sizeof(T) == 4 ? 2 : 1;
+    if (same && V == VT && tu.block <= 128) kernel = k_step_geo<T, VT, true, 128, 5>;
     return launch_step_kernel(kernel, grid, tu.block, 0, after_step, st, "k_step_geo", A, G);
 }
 
