@@ -1098,7 +1098,7 @@ int fanp_blocks_per_sm(const void* kernel, int threads, size_t smem, int* per_sm
     // From the kernel's registers and shared memory against the SM's budgets.  Not the
     // occupancy calculator: it reports one block per SM for a kernel that contains a
     // tensor-memory allocation, whose blocks here give up their allocation permit at
-    // their start and hold 32 or 64 of the SM's 512 columns only when the norms are fused.
+    // their start and hold 128 of the SM's 512 columns only when the norms are fused.
     cudaFuncAttributes fa;
     CVFES_CUDA_TRY(cudaFuncGetAttributes(&fa, kernel));
     if (smem > 48 * 1024) {

@@ -461,8 +461,10 @@ int cvfes_batch_graph_capture(const void* table_dev, int32_t n_meshes, const int
  *       zero), added to the force of every sample as calc_u_appTrac does
  *       (physicsSolverSDampGPUs.cl:436-446) -- as cvfes_solid_step's trac.
  * nu: Poisson ratio of D (physicsSolver.py:184-188, shear factor 5/6).          */
-/* Geometric-step kernel choice per precision: samples per thread (1|2|4, FP64 1|2) and
- * threads per block (64|128|256); every choice gives bitwise the same results. */
+/* Geometric-step kernel choice per precision: samples per thread (1|2|4, FP64 1|2; 4 runs
+ * as 2) and threads per block of the plain kernel (64|128|256); where the samples fill its
+ * warps a persistent patch kernel runs instead (FP64: at 1 sample per thread).  Every
+ * choice gives bitwise the same results. */
 int cvfes_set_geo_tuning(int32_t precision, int32_t vec, int32_t block);
 int cvfes_get_geo_tuning(int32_t precision, int32_t* vec, int32_t* block);
 int cvfes_solid_slot_geometry_f64(int64_t n_elems, const double* nodes, const int32_t* elems,
