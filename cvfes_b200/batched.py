@@ -1,13 +1,15 @@
 """Many independent wall meshes advanced together on one GPU.
 
 Each mesh keeps its own ``GPUSolidSolver`` (plan, material, three state buffers,
-start-up state), so its sample count, time step and damping are its own.  The
-batch packs one descriptor per mesh into a device table and advances the meshes
-with persistent kernel launches (``cvfes_batch_step``), captured in CUDA graphs of
-``graph_chunk`` steps.  Two kernels: the fan kernel (``variant`` 1, the default:
-slot rows staged by TMA, fan-rotation gathers) and the row-gather kernel
-(``variant`` 0).  A mesh advanced in a batch is bitwise identical to the same mesh
-advanced alone by the single-mesh kernels.
+start-up state), so its sample count, time step and damping are its own.  By default
+every mesh takes the single-mesh kernels, ``graph_chunk`` steps at a time: its rows stay
+in L2 for the chunk where they fit, it gets the kernel of its own size, and small meshes
+run side by side.  With an explicit ``grid``, one launch for all (``grouped`` False),
+``concurrent`` or ``variant`` 0, the batch is advanced through a device table of one
+descriptor per mesh with persistent launches (``cvfes_batch_step``) in CUDA graphs of
+``graph_chunk`` steps: the fan kernel (``variant`` 1: slot rows staged by TMA,
+fan-rotation gathers) or the row-gather kernel (``variant`` 0).  Either way a mesh is
+bitwise identical to the same mesh advanced alone.
 
 In the table, meshes are packed in groups of one work-item shape (nodes per fan item, which the
 sample count sets), one table and one launch per group and step.  The fan kernel's
