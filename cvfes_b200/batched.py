@@ -2,9 +2,9 @@
 
 Each mesh keeps its own ``GPUSolidSolver`` (plan, material, three state buffers,
 start-up state), so its sample count, time step and damping are its own.  By default
-every mesh takes the single-mesh kernels, ``graph_chunk`` steps at a time: its rows stay
-in L2 for the chunk where they fit, it gets the kernel of its own size, and small meshes
-run side by side.  With an explicit ``grid``, one launch for all (``grouped`` False),
+every mesh takes the single-mesh kernels, all steps of a call before the next mesh's: its
+rows stay in L2 where they fit, it gets the kernel of its own size, and small meshes run
+side by side.  With an explicit ``grid``, one launch for all (``grouped`` False),
 ``concurrent`` or ``variant`` 0, the batch is advanced through a device table of one
 descriptor per mesh with persistent launches (``cvfes_batch_step``) in CUDA graphs of
 ``graph_chunk`` steps: the fan kernel (``variant`` 1: slot rows staged by TMA,
