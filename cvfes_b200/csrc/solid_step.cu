@@ -31,6 +31,7 @@
 #include <type_traits>
 
 #include "common.cuh"
+#include "norms_read.h"
 #include "step_core.cuh"
 
 namespace cvfes {
@@ -1538,6 +1539,23 @@ extern "C" int cvfes_solid_step_f32(const cvfes_solid_mesh* mesh, const float* c
                               damp, (cudaStream_t)stream);
 }
 
+// The stream's side of read_step_norms.
+struct StreamRead {
+    cudaStream_t st;
+    int copy(void* dst, const void* src, unsigned long long bytes) {
+        CVFES_CUDA_TRY(cudaMemcpyAsync(dst, src, (size_t)bytes, cudaMemcpyDeviceToHost, st));
+        return CVFES_OK;
+    }
+    int wait() {
+        CVFES_CUDA_TRY(cudaStreamSynchronize(st));
+        return CVFES_OK;
+    }
+    int clear(int32_t* p) {
+        CVFES_CUDA_TRY(cudaMemsetAsync(p, 0, sizeof(int32_t), st));
+        return CVFES_OK;
+    }
+};
+
 // One step and the FP64 norms of the new state: fused into the patch kernel
 // where the shape allows, else the step followed by the separate norms pass.
 template <typename T>
@@ -1577,28 +1595,16 @@ int launch_step_norms(const cvfes_solid_mesh* m, const T* coef, const T* invm, c
         if (rc) return rc;
         if (!out_host) return check_finite ? read_nonfinite(total, st) : CVFES_OK;
     }
-    // What the host reads: the norms, then the status word of the bounded waits.  The status
-    // goes to pageable memory, so its copy returns only once it (and with it everything
-    // before it on the stream) has arrived: no further synchronisation, and the word is
-    // cleared only when it was set.  The non-finite total is the sum of the counts.
-    if (!direct)
-        CVFES_CUDA_TRY(cudaMemcpyAsync(out_host, out, (size_t)S * 4 * sizeof(double),
-                                       cudaMemcpyDeviceToHost, st));
-    int32_t stat = 0;
-    if (m->status)
-        CVFES_CUDA_TRY(cudaMemcpyAsync(&stat, m->status, sizeof(stat), cudaMemcpyDeviceToHost, st));
-    if (!m->status || stat) {
-        if (stat) CVFES_CUDA_TRY(cudaMemsetAsync(m->status, 0, sizeof(int32_t), st));
-        CVFES_CUDA_TRY(cudaStreamSynchronize(st));
-    }
-    if (stat & 1) return fail(CVFES_ERR_TIMEOUT, "a bounded device wait gave up (status %d)", stat);
-    if (stat) return fail(CVFES_ERR_ARG, "device status %d: slot stage overflow", stat);
-    if (check_finite) {
-        double h = 0.0;
-        for (long long q = 0; q < S; ++q) h += out_host[4 * q + 3];
-        if (h != 0.0)
-            return fail(CVFES_ERR_NONFINITE, "watchdog: %.0f non-finite state values", h);
-    }
+    StreamRead api{st};
+    StepReadBack r;
+    rc = read_step_norms(api, out_host, direct ? nullptr : out, S, m->status, r);
+    if (rc) return rc;
+    if (r.status & 1)
+        return fail(CVFES_ERR_TIMEOUT, "a bounded device wait gave up (status %d)", r.status);
+    if (r.status)
+        return fail(CVFES_ERR_ARG, "device status %d: slot stage overflow", r.status);
+    if (check_finite && r.nonfinite != 0.0)
+        return fail(CVFES_ERR_NONFINITE, "watchdog: %.0f non-finite state values", r.nonfinite);
     return CVFES_OK;
 }
 
