@@ -50,6 +50,36 @@ __device__ __forceinline__ Vec<T, V> ldg(const T* p) {
     }
     return r;
 }
+// Rows that another kernel may write while this one is already resident (programmatic dependent
+// launch): ld.global, not the read-only path of ldg, which is defined only for data that stays
+// the same for the kernel's whole life.  volatile keeps it behind grid_dependency_wait (volatile
+// statements keep their order) without a clobber that would pin the loads around it.  CS: the
+// streaming form, for rows read once per launch.
+#define CVFES_LD_STATE(OP)                                                                    \
+    if constexpr (sizeof(T) == 4 && V == 4)                                                   \
+        asm volatile(OP ".v4.f32 {%0, %1, %2, %3}, [%4];"                                     \
+                     : "=f"(r.v[0]), "=f"(r.v[1]), "=f"(r.v[2]), "=f"(r.v[3])                 \
+                     : "l"(g));                                                               \
+    else if constexpr (sizeof(T) == 4 && V == 2)                                              \
+        asm volatile(OP ".v2.f32 {%0, %1}, [%2];" : "=f"(r.v[0]), "=f"(r.v[1]) : "l"(g));     \
+    else if constexpr (sizeof(T) == 4)                                                        \
+        asm volatile(OP ".f32 %0, [%1];" : "=f"(r.v[0]) : "l"(g));                            \
+    else if constexpr (V == 2)                                                                \
+        asm volatile(OP ".v2.f64 {%0, %1}, [%2];" : "=d"(r.v[0]), "=d"(r.v[1]) : "l"(g));     \
+    else                                                                                      \
+        asm volatile(OP ".f64 %0, [%1];" : "=d"(r.v[0]) : "l"(g));
+template <typename T, int V, bool CS = false>
+__device__ __forceinline__ Vec<T, V> ld_state(const T* p) {
+    Vec<T, V> r;
+    const size_t g = __cvta_generic_to_global(p);
+    if constexpr (CS) {
+        CVFES_LD_STATE("ld.global.cs")
+    } else {
+        CVFES_LD_STATE("ld.global")
+    }
+    return r;
+}
+#undef CVFES_LD_STATE
 // Asynchronous global -> shared copy of BYTES (4, 8 or 16) per thread (LSU path).
 template <int BYTES>
 __device__ __forceinline__ void cp_async(uint32_t dst, const void* src) {

@@ -198,7 +198,7 @@ __device__ __forceinline__ void geo_update(const StepArgs<T>& A, int a, size_t c
     T* const un = row_at(A.un + col, a, nodeb);
 #pragma unroll
     for (int d = 0; d < 3; ++d) {
-        const Vec<T, V> vo = ldcs<T, V>(up + d * S);
+        const Vec<T, V> vo = ld_state<T, V, true>(up + d * S);
         // nodal traction (calc_u_appTrac, physicsSolverSDampGPUs.cl:436-446), one per node
         const T tr = A.trac ? __ldg(A.trac + 4 * (size_t)a + d) : T(0);
         Vec<T, V> o;
@@ -248,7 +248,7 @@ __global__ void __launch_bounds__(MAXT, MINB) k_step_geo(StepArgs<T> A, GeoArgs<
     Vec<T, V> ua[3], ga[SAME ? 1 : 3], acc[3], load[3];
     auto rows = [&](Vec<T, V> (&x)[3], const T* q) {
 #pragma unroll
-        for (int d = 0; d < 3; ++d) x[d] = ldg<T, V>(q + d * S);
+        for (int d = 0; d < 3; ++d) x[d] = ld<T, V>(q + d * S);
     };
     rows(ua, row_at(u, (int)a, nodeb));
     if constexpr (!SAME) rows(ga, row_at(ug, (int)a, nodeb));
@@ -374,7 +374,7 @@ __global__ void __launch_bounds__(32 * GeoWarps<T, SAME>::kWarps, 1)
         Vec<T, V> ua[3], ga[SAME ? 1 : 3];
         auto rows = [&](Vec<T, V> (&x)[3], const T* q) {
 #pragma unroll
-            for (int d = 0; d < 3; ++d) x[d] = ldg<T, V>(q + d * S);
+            for (int d = 0; d < 3; ++d) x[d] = ld<T, V>(q + d * S);
         };
         if (a >= 0) {
             rows(ua, row_at(u, a, nodeb));

@@ -98,7 +98,7 @@ __global__ void __launch_bounds__(kGroupThreads, MAXD <= 6 ? 8 : 6)
     Vec<T, V> ua[3], vo[3], R[MAXD + 1][3], acc[3];
     auto rows = [&](Vec<T, V> (&x)[3], const T* q) {
 #pragma unroll
-        for (int d = 0; d < 3; ++d) x[d] = ldg<T, V>(q + d * S);
+        for (int d = 0; d < 3; ++d) x[d] = ld<T, V>(q + d * S);
     };
     rows(ua, row_at(u, a, nodeb));
     if (deg > 0) rows(R[0], row_at(u, srec[k0].y, nodeb));
@@ -108,7 +108,7 @@ __global__ void __launch_bounds__(kGroupThreads, MAXD <= 6 ? 8 : 6)
     {
         const T* q = row_at(A.up + col, a, nodeb);
 #pragma unroll
-        for (int d = 0; d < 3; ++d) vo[d] = ldcs<T, V>(q + d * S);
+        for (int d = 0; d < 3; ++d) vo[d] = ld_state<T, V, true>(q + d * S);
     }
     const T p = step_pressure<T>(A);
     const T* const K = reinterpret_cast<const T*>(sslab) - 16 / (int)sizeof(T) * P::kFirst +

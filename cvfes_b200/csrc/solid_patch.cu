@@ -215,7 +215,7 @@ __global__ void __launch_bounds__(32 * W, 1)
         for (int d = 0; d < 3; ++d) {
             if (VEL || NORMS) {
                 const Vec<T, V> dv =
-                    vsub(cl, ldg<T, V>(row_at(u0, b, nodeb) + d * (size_t)A.S));
+                    vsub(cl, ld_state<T, V>(row_at(u0, b, nodeb) + d * (size_t)A.S));
                 if (VEL && on) stcs<T, V>(row_at(A.vel + col, b, nodeb) + d * (size_t)A.S, dv);
                 if constexpr (NORMS != 0) {
 #pragma unroll
@@ -236,9 +236,9 @@ __global__ void __launch_bounds__(32 * W, 1)
     for (int sg = 0; more; sg ^= 1) {
         Vec<T, V> ua[3];
         if (a >= 0) {
-            ua[0] = ldg<T, V>(row_at(u0, a, nodeb));
-            ua[1] = ldg<T, V>(row_at(u1, a, nodeb));
-            ua[2] = ldg<T, V>(row_at(u2, a, nodeb));
+            ua[0] = ld_state<T, V>(row_at(u0, a, nodeb));
+            ua[1] = ld_state<T, V>(row_at(u1, a, nodeb));
+            ua[2] = ld_state<T, V>(row_at(u2, a, nodeb));
         }
         cp_async_wait_all();
         __syncwarp();
@@ -264,9 +264,9 @@ __global__ void __launch_bounds__(32 * W, 1)
         };
         if (a >= 0) {
             auto rows = [&](Vec<T, V> (&x)[3], int b) {
-                x[0] = ldg<T, V>(row_at(u0, b, nodeb));
-                x[1] = ldg<T, V>(row_at(u1, b, nodeb));
-                x[2] = ldg<T, V>(row_at(u2, b, nodeb));
+                x[0] = ld_state<T, V>(row_at(u0, b, nodeb));
+                x[1] = ld_state<T, V>(row_at(u1, b, nodeb));
+                x[2] = ld_state<T, V>(row_at(u2, b, nodeb));
             };
             Vec<T, V> acc[3], vo[3], im;
             T f[3];
@@ -277,7 +277,7 @@ __global__ void __launch_bounds__(32 * W, 1)
                 im = ldcs<T, V>(row_at(A.invm + col, a, rowb));
                 const T* q = row_at(A.up + col, a, nodeb);
 #pragma unroll
-                for (int d = 0; d < 3; ++d) vo[d] = ldcs<T, V>(q + d * (size_t)A.S);
+                for (int d = 0; d < 3; ++d) vo[d] = ld_state<T, V, true>(q + d * (size_t)A.S);
             };
             const int flag = lane < n ? srec[lane].w : 1;
             if (n == 6 && __all_sync(0xffffffffu, (flag & 1) || lane == 0)) {
@@ -288,7 +288,6 @@ __global__ void __launch_bounds__(32 * W, 1)
                 C[0] = ldg<T, V>(row_at(cf, r0.x, rowb));
                 rows(X[2], r1.z);
                 C[1] = ldg<T, V>(row_at(cf, r1.x, rowb));
-                if constexpr (sizeof(T) == 4) __syncwarp();
                 to_diff<T, V>(X[0], ua);
 #pragma unroll
                 for (int k = 0; k < 6; ++k) {
@@ -299,12 +298,8 @@ __global__ void __launch_bounds__(32 * W, 1)
                     }
                     if (k == 4) epilogue_rows();
                     if (k == 2) prefetch_coef();
-                    // FP32: the warp barriers keep the compiler from sinking the loads to
-                    // their uses (400 against 425 us); FP64 is faster without (241 against 253)
-                    if constexpr (sizeof(T) == 4) __syncwarp();
                     to_diff<T, V>(X[k + 1], ua);
                     slot_fma<T, V>(K + kStep * k, C[k], X[k], X[k + 1], ua, acc);
-                    if constexpr (sizeof(T) == 4) __syncwarp();
                 }
             } else {
                 if (n > 0) {  // any fan: three buffers rotate, one element ahead

@@ -839,9 +839,8 @@ inline long long norm_chunks(long long n_nodes) {
 // VEL: `up` holds the increment v = u_n - u_{n-1} (velocity-state form), else u_{n-1}.
 template <typename T, int V, bool VEL>
 __global__ void __launch_bounds__(kNormThreads)
-    k_norms_partial(long long n_nodes, int S, long long npc, int tpn, const T* __restrict__ u,
-                    const T* __restrict__ up, const T* __restrict__ invm,
-                    double* __restrict__ work) {
+    k_norms_partial(long long n_nodes, int S, long long npc, int tpn, const T* u, const T* up,
+                    const T* invm, double* work) {
     __shared__ double part[4 * V][kNormThreads];
     grid_dependency_release();
     grid_dependency_wait();
@@ -867,8 +866,8 @@ __global__ void __launch_bounds__(kNormThreads)
             Vec<T, V> x[3], y[3];
 #pragma unroll
             for (int d = 0; d < 3; ++d) {
-                x[d] = ldg<T, V>(u + ((size_t)a * 3 + d) * S + col);
-                y[d] = ldcs<T, V>(up + ((size_t)a * 3 + d) * S + col);
+                x[d] = ld_state<T, V>(u + ((size_t)a * 3 + d) * S + col);
+                y[d] = ld_state<T, V, true>(up + ((size_t)a * 3 + d) * S + col);
             }
 #pragma unroll
             for (int i = 0; i < V; ++i) {
@@ -912,9 +911,8 @@ __global__ void __launch_bounds__(kNormThreads)
 // sums are added in group order, so the result depends only on the row count.
 constexpr int kFinalPairs = 32, kFinalGroups = 32;
 __global__ void __launch_bounds__(kFinalPairs * kFinalGroups)
-    k_norms_final(long long n_chunks, int S, const double* __restrict__ work,
-                  double* __restrict__ out, double* __restrict__ out_host,
-                  double* __restrict__ total_nonfinite) {
+    k_norms_final(long long n_chunks, int S, const double* work, double* out, double* out_host,
+                  double* total_nonfinite) {
     __shared__ double part[kFinalGroups][kFinalPairs];
     grid_dependency_wait();
     const int lp = threadIdx.x % kFinalPairs, g = threadIdx.x / kFinalPairs;

@@ -516,7 +516,7 @@ __device__ __forceinline__ void clamp_store(const StepArgs<T>& A, size_t S, size
     const Vec<T, V> cl = vfill<T, V>(A.clamp);
 #pragma unroll
     for (int d = 0; d < 3; ++d) {
-        if (A.vel) stcs<T, V>(A.vel + row + d * S, vsub(cl, ldg<T, V>(A.u + row + d * S)));
+        if (A.vel) stcs<T, V>(A.vel + row + d * S, vsub(cl, ld_state<T, V>(A.u + row + d * S)));
         stcs<T, V>(A.un + row + d * S, cl);
     }
 }
@@ -759,6 +759,10 @@ struct SlotStage {
 // before it is still running; until grid_dependency_wait returns (that step has ended and
 // its writes are visible) it may read only what no step writes.  release lets the launch
 // after this one start; both do nothing in a kernel launched without the attribute.
+// State rows (u, u_{n-1} or the increment, chi, partial norms) change while such a kernel is
+// resident: they are read after the wait, by ld_state or plain loads, never through the
+// read-only path (__ldg, const __restrict__).  Slots, coefficients, masses and loads, which no
+// kernel in flight writes, are.
 __device__ __forceinline__ void grid_dependency_wait() {
     asm volatile("griddepcontrol.wait;" ::: "memory");
 }
