@@ -90,12 +90,32 @@ struct RowLines {
     }
 };
 
-__device__ __forceinline__ void node_slots(const int32_t* node_ptr, int b, int& k0, int& n) {
+// Slots of node b.  A node with more than the descriptor's max_degree, for which the stages
+// are sized, is left out (b = -1) and the warp's flag (shared memory) set: such nodes follow
+// after the loop, from global memory.
+__device__ __forceinline__ void node_slots(const int32_t* node_ptr, int max_degree, int* flag,
+                                           int& b, int& k0, int& n) {
     k0 = n = 0;
     if (b >= 0) {
         k0 = __ldg(node_ptr + b);
         n = __ldg(node_ptr + b + 1) - k0;
+        if (n > max_degree) {
+            *flag = 1;
+            b = -1;
+            n = 0;
+        }
     }
 }
+
+// The launch read again, opaque to the compiler: what follows from it (after a long loop) is
+// computed anew and holds no registers during the loop.
+struct LaunchAgain {
+    int block, blocks, thread;
+    __device__ __forceinline__ LaunchAgain() {
+        asm volatile("mov.u32 %0, %%ctaid.x;" : "=r"(block));
+        asm volatile("mov.u32 %0, %%nctaid.x;" : "=r"(blocks));
+        asm volatile("mov.u32 %0, %%tid.x;" : "=r"(thread));
+    }
+};
 
 }  // namespace cvfes

@@ -647,6 +647,48 @@ __global__ void __launch_bounds__(256, MINB) k_reverse_fan(RevArgs<T> A) {
 // Gamma row is requested before its products.  us a step, fan or persistent fan / this:
 // 128 x 400 wall, FP32 64 samples 155 / 116, 128 samples with G 315 / 235; 128 x 320 wall, FP64
 // 64 samples with G 267 / 213; 64 x 128 wall, 64 samples FP32 22.4 / 21.3, FP64 54.7 / 46.4.
+// Both row products and the Gamma update of a node that is not staged (more slots than the
+// descriptor's max_degree), all from global memory, as ku_row_unstaged.
+template <typename T, int V>
+__device__ __forceinline__ void rev_row_unstaged(const RevArgs<T>& A, int k0, int n, const T* u,
+                                                 const T* x, size_t col, uint32_t rowb, bool on,
+                                                 const Vec<T, V> (&ua)[3],
+                                                 const Vec<T, V> (&ca)[3], Vec<T, V> (&accU)[3],
+                                                 Vec<T, V> (&accC)[3]) {
+    const size_t S = rowb / sizeof(T);
+    Vec<T, V> u1[3], u2[3], x1[3], x2[3];
+    auto rows = [&](Vec<T, V> (&p)[3], Vec<T, V> (&q)[3], int b) {
+#pragma unroll
+        for (int d = 0; d < 3; ++d) {
+            p[d] = vsub(ld_state<T, V>(row_at(u, b, 3 * rowb) + d * S), ua[d]);
+            q[d] = vsub(ld_state<T, V>(row_at(x, b, 3 * rowb) + d * S), ca[d]);
+        }
+    };
+#pragma unroll 1
+    for (int k = k0; k < k0 + n; ++k) {
+        const int4 r = __ldg(A.rec + k);
+#pragma unroll
+        for (int d = 0; d < 3; ++d) {
+            u1[d] = u2[d];
+            x1[d] = x2[d];
+        }
+        if (k == k0 || !(r.w & 1)) rows(u1, x1, r.y);
+        rows(u2, x2, r.z);
+        slot_fma2<T, V>(A.slab + (size_t)kSlabStride * k,
+                        ldg<T, V>(row_at(A.coef + col, r.x, rowb)), u1, u2, x1, x2, ua, ca, accU,
+                        accC);
+        if (((r.w >> 8) & 3) == 0) {
+            T* const gp = row_at(A.gam + col, r.x, rowb);
+            Vec<T, V> gv = ld<T, V>(gp);
+            const Vec<T, V> g =
+                owner_form<T, V>(A.own + (size_t)kOwnStride * k, u1, u2, x1, x2, ua, ca);
+#pragma unroll
+            for (int i = 0; i < V; ++i) gv.v[i] += g.v[i];
+            if (on) st<T, V>(gp, gv);
+        }
+    }
+}
+
 template <typename T, int V, bool GM, int W>
 __global__ void __launch_bounds__(32 * W, 1)
     k_reverse_patch(RevArgs<T> A, PatchMap M, int max_degree) {
@@ -680,13 +722,16 @@ __global__ void __launch_bounds__(32 * W, 1)
         }
         cp_async_commit();
     };
+    __shared__ int unstaged[W];  // a node of the warp was not staged
+    if (lane == 0) unstaged[warp] = 0;
+    __syncwarp();
     bool more = walk.more(M);
     int a = walk.node(M), n, an, k0, nn;
-    node_slots(A.node_ptr, a, k0, n);
+    node_slots(A.node_ptr, max_degree, unstaged + warp, a, k0, n);
     stage(a, k0, n, 0);
     walk.advance(M);
     an = walk.node(M);
-    node_slots(A.node_ptr, an, k0, nn);
+    node_slots(A.node_ptr, max_degree, unstaged + warp, an, k0, nn);
     // line prefetch: rows 0..2 u_n, 3..5 chi_{n+1}, 6..8 u_{n+1}, 9..11 chi_{n+2}, 12 inverse
     // mass, 13 G; then coefficient rows and, by the owner, Gamma rows
     const RowLines<T, V> ln(lane, chunk, rowb);
@@ -737,8 +782,8 @@ __global__ void __launch_bounds__(32 * W, 1)
         const int nn_cur = nn;
         more = walk.more(M);
         walk.advance(M);
-        const int ax = walk.node(M);
-        node_slots(A.node_ptr, ax, k0, nn);
+        int ax = walk.node(M);
+        node_slots(A.node_ptr, max_degree, unstaged + warp, ax, k0, nn);
         auto prefetch_elems = [&]() {  // coefficient rows and owned Gamma rows of the next node
             cp_async_wait_all();
             __syncwarp();
@@ -852,6 +897,32 @@ __global__ void __launch_bounds__(32 * W, 1)
         an = ax;
     }
     cp_async_wait_all();
+    __syncwarp();
+    if (!unstaged[threadIdx.x >> 5]) return;
+    // the nodes that were not staged, after all others: they cost the loop no registers
+    const LaunchAgain L;
+    const int vec2 = L.block % A.nch * 32 + (L.thread & 31);
+    const bool on2 = vec2 * V < A.S;
+    const size_t col2 = (size_t)min(vec2, A.S / V - 1) * V;
+    const uint32_t rb = (uint32_t)A.S * sizeof(T);
+    PatchWalk again(M, L.thread >> 5, L.block / A.nch, L.blocks / A.nch, 0, (int)A.n_nodes, W);
+    for (; again.more(M); again.advance(M)) {
+        const int b = again.node(M);
+        if (b < 0) continue;
+        const int s0 = __ldg(A.node_ptr + b), ns = __ldg(A.node_ptr + b + 1) - s0;
+        if (ns <= max_degree) continue;
+        Vec<T, V> ua[3], ca[3], accU[3], accC[3];
+#pragma unroll
+        for (int d = 0; d < 3; ++d) {
+            ua[d] = ld_state<T, V>(row_at(A.u + col2, b, 3 * rb) + d * (size_t)A.S);
+            ca[d] = ld_state<T, V>(row_at(A.x + col2, b, 3 * rb) + d * (size_t)A.S);
+            accU[d] = accC[d] = vzero<T, V>();
+        }
+        rev_row_unstaged<T, V>(A, s0, ns, A.u + col2, A.x + col2, col2,
+                               rb, on2, ua, ca, accU, accC);
+        rev_epilogue<T, V, GM>(A, b, (size_t)A.S, col2, (size_t)b * 3 * A.S + col2, ua, ca, accU,
+                               accC, on2);
+    }
 }
 
 // dJ/dlogE = -c Gamma; dJ/dlogh = -c Gamma - h sum_a alpha_{e,a} G_a / m_a.

@@ -215,6 +215,42 @@ __device__ __forceinline__ void geo_update(const StepArgs<T>& A, int a, size_t c
     }
 }
 
+// One node (its first slot k0) with its slots from global memory.
+template <typename T, int V, bool SAME>
+__device__ __forceinline__ void geo_node_any(const StepArgs<T>& A, const GeoArgs<T>& G, int a,
+                                             int k0, size_t col, T p6, bool on) {
+    const size_t S = (size_t)A.S;
+    const uint32_t nodeb = 3 * (uint32_t)A.S * sizeof(T);
+    const int k1 = __ldg(A.node_ptr + a + 1);
+    Vec<T, V> ua[3], ga[3], acc[3], load[3];
+#pragma unroll
+    for (int d = 0; d < 3; ++d) {
+        ua[d] = ld<T, V>(row_at(A.u + col, a, nodeb) + d * S);
+        ga[d] = ld<T, V>(row_at(G.ug + col, a, nodeb) + d * S);
+        acc[d] = load[d] = vzero<T, V>();
+    }
+    GeoEdge<T, V> one, two;
+    auto edge = [&](GeoEdge<T, V>& o, int k, int b, int second) {
+#pragma unroll
+        for (int d = 0; d < 3; ++d) {
+            const Vec<T, V> e = vfill<T, V>(__ldg(G.geo + (size_t)kGeoStride * k + 3 * second + d));
+            o.d[d] = vsub(ld<T, V>(row_at(A.u + col, b, nodeb) + d * S), ua[d]);
+            if constexpr (SAME)
+                o.q[d] = vadd(o.d[d], e);
+            else
+                o.q[d] = vadd(vsub(ld<T, V>(row_at(G.ug + col, b, nodeb) + d * S), ga[d]), e);
+        }
+    };
+    for (int k = k0; k < k1; ++k) {
+        const int4 r = __ldg(A.rec + k);
+        one = two;
+        if (k == k0 || !(r.w & 1)) edge(one, k, r.y, 0);
+        edge(two, k, r.z, 1);
+        geo_row<T, V>(one, two, ldg<T, V>(A.coef + (size_t)r.x * S + col), G.K, acc, load);
+    }
+    geo_update<T, V>(A, a, col, p6, ua, acc, load, on);
+}
+
 // One step: a thread walks its node's fan with the next element's neighbour rows and
 // coefficient in flight.  Consecutive elements of a fan share an edge, so one neighbour is
 // gathered per element (two were, and their rows were 6 of the 7 gathered).  What bounds it
@@ -319,6 +355,28 @@ template <typename T, bool SAME>
 struct GeoWarps {
     static constexpr int kWarps = sizeof(T) == 4 ? (SAME ? 24 : 20) : 16;
 };
+// The nodes of this warp that the patch kernel could not stage (more slots than max_degree):
+// after all others, and everything found again from the launch, so that they cost its loop no
+// registers (10 steps of the 128 x 400 wall, FP32, 128 samples: 1.97 ms without them, 2.01 with,
+// 2.05 with a function call in or after the loop).
+template <typename T, int V, bool SAME, int W>
+__device__ __forceinline__ void geo_unstaged(const StepArgs<T>& A, const GeoArgs<T>& G,
+                                             const PatchMap& M, int max_degree) {
+    const LaunchAgain L;
+    const int vec = L.block % A.nch * 32 + (L.thread & 31), last = A.S / V - 1;
+    const size_t col = (size_t)min(vec, last) * V;
+    PatchWalk walk(M, L.thread >> 5, L.block / A.nch, L.blocks / A.nch, A.n_clamped,
+                   (int)A.n_nodes, W);
+    for (; walk.more(M); walk.advance(M)) {
+        const int a = walk.node(M);
+        if (a < 0) continue;
+        const int k0 = __ldg(A.node_ptr + a), n = __ldg(A.node_ptr + a + 1) - k0;
+        if (n > max_degree)
+            geo_node_any<T, V, SAME>(A, G, a, k0, col, step_pressure<T>(A) * T(1.0 / 6.0),
+                                     vec <= last);
+    }
+}
+
 template <typename T, int V, bool SAME>
 __global__ void __launch_bounds__(32 * GeoWarps<T, SAME>::kWarps, 1)
     k_step_geo_patch(StepArgs<T> A, GeoArgs<T> G, PatchMap M, int max_degree) {
@@ -345,13 +403,16 @@ __global__ void __launch_bounds__(32 * GeoWarps<T, SAME>::kWarps, 1)
         }
         cp_async_commit();
     };
+    __shared__ int unstaged[W];  // a node of the warp was not staged
+    if (lane == 0) unstaged[warp] = 0;
+    __syncwarp();
     bool more = walk.more(M);
     int a = walk.node(M), n, an, k0, nn;
-    node_slots(A.node_ptr, a, k0, n);
+    node_slots(A.node_ptr, max_degree, unstaged + warp, a, k0, n);
     stage(a, k0, n, 0);
     walk.advance(M);
     an = walk.node(M);
-    node_slots(A.node_ptr, an, k0, nn);
+    node_slots(A.node_ptr, max_degree, unstaged + warp, an, k0, nn);
     const RowLines<T, V> ln(lane, chunk, rowb);
     const char* const obase =
         reinterpret_cast<const char*>(ln.row < 3   ? A.u + (size_t)ln.row * S
@@ -390,8 +451,8 @@ __global__ void __launch_bounds__(32 * GeoWarps<T, SAME>::kWarps, 1)
         const int nn_cur = nn;
         more = walk.more(M);
         walk.advance(M);
-        const int ax = walk.node(M);
-        node_slots(A.node_ptr, ax, k0, nn);
+        int ax = walk.node(M);
+        node_slots(A.node_ptr, max_degree, unstaged + warp, ax, k0, nn);
         if (a >= 0) {
             Vec<T, V> acc[3], load[3], x[3], g[SAME ? 1 : 3], c, cn;
             T E[3];
@@ -458,6 +519,8 @@ __global__ void __launch_bounds__(32 * GeoWarps<T, SAME>::kWarps, 1)
         an = ax;
     }
     cp_async_wait_all();
+    __syncwarp();
+    if (unstaged[threadIdx.x >> 5]) geo_unstaged<T, V, SAME, W>(A, G, M, max_degree);
 }
 
 struct GeoTuning {

@@ -40,11 +40,6 @@ __global__ void __launch_bounds__(kGroupThreads, MAXD <= 6 ? 8 : 6)
     const int a0 = blockIdx.x * A.npb, n_nodes = (int)A.n_nodes;
     const int a1 = min(a0 + A.npb, n_nodes);
     const int kb = __ldg(A.node_ptr + a0), nsl = __ldg(A.node_ptr + a1) - kb;
-    if (nsl > A.cap_slots) {  // cannot happen when cap_slots = npb * max_degree
-        grid_dependency_wait();
-        if (threadIdx.x == 0 && A.status) atomicOr(A.status, 2);
-        return;
-    }
     const int t = threadIdx.x / A.tpn, a = a0 + t;
     const int vec = threadIdx.x - t * A.tpn;
     const bool active = t < A.npb && a < n_nodes;
@@ -53,14 +48,18 @@ __global__ void __launch_bounds__(kGroupThreads, MAXD <= 6 ? 8 : 6)
         k0 = __ldg(A.node_ptr + a) - kb;
         deg = __ldg(A.node_ptr + a + 1) - kb - k0;
     }
+    // more slots than the descriptor's max_degree says: the row from global memory
+    const int all = deg;
+    const bool staged = nsl <= A.cap_slots, big = !staged || deg > MAXD;
+    if (big) deg = 0;
     int4* const srec = reinterpret_cast<int4*>(smem);
     unsigned char* const sslab = smem + (size_t)A.cap_slots * 16;
     const char* const rec = reinterpret_cast<const char*>(A.rec + kb);
     const char* const slab = reinterpret_cast<const char*>(A.slab + (size_t)kb * kSlabStride);
-    for (int q = threadIdx.x; q < nsl; q += kGroupThreads)
+    for (int q = threadIdx.x; q < nsl && staged; q += kGroupThreads)
         cp_async<16>(smem_u32(srec) + 16 * q, rec + 16 * q);
     cp_async_commit();
-    for (int q = threadIdx.x; q < P::kWords * nsl; q += kGroupThreads) {
+    for (int q = threadIdx.x; q < P::kWords * nsl && staged; q += kGroupThreads) {
         const int s = q / P::kWords, w = q - s * P::kWords;
         cp_async<16>(smem_u32(sslab) + 16 * q,
                      slab + s * (kSlabStride * (int)sizeof(T)) + (P::kFirst + w) * 16);
@@ -130,6 +129,9 @@ __global__ void __launch_bounds__(kGroupThreads, MAXD <= 6 ? 8 : 6)
             }
         }
     }
+    if (big)
+        ku_row_unstaged<T, V>(A.rec + kb + k0, A.slab + (size_t)(kb + k0) * kSlabStride, all, u,
+                              A.coef + col, rowb, ua, acc);
 #pragma unroll
     for (int d = 0; d < 3; ++d) {
         T f = p * fh[d];

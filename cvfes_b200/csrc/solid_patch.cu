@@ -153,13 +153,16 @@ __global__ void __launch_bounds__(32 * W, 1)
         }
         cp_async_commit();
     };
+    __shared__ int unstaged[W];  // a node of the warp was not staged
+    if (lane == 0) unstaged[warp] = 0;
+    __syncwarp();
     bool more = walk.more(M);
     int a = walk.node(M), n, an, k0, nn;
-    node_slots(A.node_ptr, a, k0, n);
+    node_slots(A.node_ptr, max_degree, unstaged + warp, a, k0, n);
     stage(a, k0, n, 0);
     walk.advance(M);
     an = walk.node(M);
-    node_slots(A.node_ptr, an, k0, nn);
+    node_slots(A.node_ptr, max_degree, unstaged + warp, an, k0, nn);
 
     // ---- line prefetch: u, u_{n-1} and inverse mass rows of a node; coefficient rows
     const RowLines<T, V> ln(lane, chunk, rowb);
@@ -251,8 +254,8 @@ __global__ void __launch_bounds__(32 * W, 1)
         const int nn_cur = nn;
         more = walk.more(M);
         walk.advance(M);
-        const int ax = walk.node(M);
-        node_slots(A.node_ptr, ax, k0, nn);
+        int ax = walk.node(M);
+        node_slots(A.node_ptr, max_degree, unstaged + warp, ax, k0, nn);
         // coefficient rows of the next node's elements (the first kRows of them: a loop
         // over more cost the spill-free allocation, 385 -> 400 us and FP64 228 -> 270 us)
         auto prefetch_coef = [&]() {
@@ -357,6 +360,47 @@ __global__ void __launch_bounds__(32 * W, 1)
         an = ax;
     }
     cp_async_wait_all();
+    __syncwarp();
+    if (unstaged[threadIdx.x >> 5]) {  // after all others, so that they cost the loop no registers
+        const LaunchAgain L;
+        const int vec2 = L.block % A.nch * 32 + (L.thread & 31);
+        const bool on2 = vec2 * V < A.S;
+        const size_t S = (size_t)A.S, col2 = (size_t)min(vec2, A.S / V - 1) * V;
+        const uint32_t rb = (uint32_t)A.S * sizeof(T);
+        const T p2 = step_pressure<T>(A);
+        PatchWalk again(M, L.thread >> 5, L.block / A.nch, L.blocks / A.nch, A.n_clamped,
+                        (int)A.n_nodes, W);
+        for (; again.more(M); again.advance(M)) {
+            const int b = again.node(M);
+            if (b < 0) continue;
+            const int s0 = __ldg(A.node_ptr + b), ns = __ldg(A.node_ptr + b + 1) - s0;
+            if (ns <= max_degree) continue;
+            Vec<T, V> ua[3], acc[3], vo[3];
+            T f[3];
+#pragma unroll
+            for (int d = 0; d < 3; ++d) {
+                ua[d] = ld_state<T, V>(row_at(A.u + col2, b, 3 * rb) + d * S);
+                vo[d] = ld_state<T, V, true>(row_at(A.up + col2, b, 3 * rb) + d * S);
+                acc[d] = vzero<T, V>();
+            }
+            ku_row_unstaged<T, V>(A.rec + s0, A.slab + (size_t)s0 * kSlabStride,
+                                  ns, A.u + col2, A.coef + col2, rb, ua,
+                                  acc);
+            const Vec<T, V> im = ldcs<T, V>(row_at(A.invm + col2, b, rb));
+            node_load<T>(A, b, p2, f);
+            T su[V], sv[V];
+            int nf[V];
+#pragma unroll
+            for (int i = 0; i < V; ++i) {
+                su[i] = sv[i] = T(0);
+                nf[i] = 0;
+            }
+            patch_epilogue<T, V, VEL, NORMS != 0>(A, row_at(A.un + col2, b, 3 * rb),
+                                                  VEL ? row_at(A.vel + col2, b, 3 * rb) : nullptr,
+                                                  ua, acc, f, vo, im, on2, su, sv, nf);
+            if constexpr (NORMS != 0) add_norms(im, su, sv, nf);
+        }
+    }
 
     if constexpr (NORMS != 0) {  // the block's row of partials, its warps added in order
         double* const scr = reinterpret_cast<double*>(smem);

@@ -744,6 +744,34 @@ __device__ __forceinline__ T* row_at(T* base, int i, uint32_t stride_bytes) {
                                 (uint64_t)(uint32_t)i * stride_bytes);
 }
 
+// Adds to acc the row of K_s u_s of a node with n slots, slots and rows from global memory, for
+// the nodes that the staged kernels cannot hold (more slots than the descriptor's max_degree).
+// u and coef point at the lane's column; rowb: bytes of a row.  The products and their order
+// are those of ku_row.
+template <typename T, int V>
+__device__ __forceinline__ void ku_row_unstaged(const int4* rec, const T* slab, int n, const T* u,
+                                                const T* coef, uint32_t rowb,
+                                                const Vec<T, V> (&ua)[3], Vec<T, V> (&acc)[3]) {
+    const size_t S = rowb / sizeof(T);
+    Vec<T, V> x1[3], x2[3];
+#pragma unroll 1
+    for (int k = 0; k < n; ++k) {
+        const int4 r = __ldg(rec + k);
+#pragma unroll
+        for (int d = 0; d < 3; ++d) x1[d] = x2[d];
+        if (k == 0 || !(r.w & 1)) {
+#pragma unroll
+            for (int d = 0; d < 3; ++d) x1[d] = ld_state<T, V>(row_at(u, r.y, 3 * rowb) + d * S);
+            to_diff<T, V>(x1, ua);
+        }
+#pragma unroll
+        for (int d = 0; d < 3; ++d) x2[d] = ld_state<T, V>(row_at(u, r.z, 3 * rowb) + d * S);
+        to_diff<T, V>(x2, ua);
+        slot_fma<T, V>(slab + (size_t)kSlabStride * k, ldg<T, V>(row_at(coef, r.x, rowb)), x1, x2,
+                       ua, acc);
+    }
+}
+
 // 16-byte words of one slot's stiffness row that the patch and group kernels stage.  FP32:
 // words 2..6 (the difference form does not read the self block, values 0..8); FP64: all 14.
 // kBytes: with the slot's record.

@@ -55,7 +55,10 @@ typedef struct cvfes_solid_mesh {
     const int32_t* slot_rec;      /* [4 * n_slots]    */
     const void*    slot_k;        /* [28 * n_slots] T */
     const void*    fhat;          /* [4 * n_nodes]  T */
-    int64_t        max_degree;    /* max slots of one node (0: unknown -> no smem staging) */
+    int64_t        max_degree;    /* max slots of one node (0: unknown -> no smem staging).
+                                     Nodes with more: their rows come from global memory in
+                                     the patch and group kernels (slower, same bits); the
+                                     staged and fan kernels set bit 1 of status */
     int32_t*       status;        /* device int32 or NULL: bit 0 set when a bounded
                                      device wait gave up (read by cvfes_status_read) */
     /* Strip tiling of the TMA-tiled step (staged = 7), from cvfes_mesh_tiles, device
