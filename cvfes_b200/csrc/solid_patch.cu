@@ -455,6 +455,11 @@ static int launch_patch_k(const StepArgs<T>& A, const cvfes_solid_mesh* m, int m
     const PatchMap M = patch_map(m->n_nodes - A.n_clamped, m->bandwidth, W);
     auto kernel = k_step_patch<T, V, VEL, NORMS, W>;
     size_t smem = (size_t)W * 2 * max_degree * SlotStage<T>::kBytes;
+    // Slots of up to 29 (FP64) or 30 to 53 (FP32, by the block's warps) elements a node; 160 KB
+    // leave room for the sums of NORMS 2.  Tube closed by a cap of nc elements at its apex, nc
+    // x 400 nodes, us a step, patch / fan: FP64 nc 28, 64 samples 26.8 / 38.8; FP32 nc 50, 256
+    // samples 80.9 / 125.
+    if (smem > 160 * 1024) return 1;
     const size_t sums = (size_t)4 * V * 32 * sizeof(double);
     if (NORMS == 1) smem = std::max(smem, sums);
     if (NORMS == 2) smem += W * sums;
@@ -488,9 +493,8 @@ template <typename T>
 int launch_step_patch(const cvfes_solid_mesh* m, StepArgs<T> A, int vec_max, bool after_step,
                       cudaStream_t st, int norms_mode, long long max_rows, long long* rows) {
     const int md = (int)m->max_degree;
-    if (m->max_degree <= 0 || A.S >= (1 << 27) || m->n_nodes >= INT32_MAX / 2 ||
-        (size_t)28 * 2 * std::min<size_t>(m->max_degree, 1 << 16) *
-                SlotStage<T>::kBytes > 160 * 1024)
+    if (m->max_degree <= 0 || m->max_degree >= 1024 || A.S >= (1 << 27) ||
+        m->n_nodes >= INT32_MAX / 2)
         return 1;
     const int V = patch_vec(A.S, vec_max);
     A.nch = (A.S / V + 31) / 32;
