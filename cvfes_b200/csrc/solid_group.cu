@@ -48,10 +48,10 @@ __global__ void __launch_bounds__(kGroupThreads, MAXD <= 6 ? 8 : 6)
         k0 = __ldg(A.node_ptr + a) - kb;
         deg = __ldg(A.node_ptr + a + 1) - kb - k0;
     }
-    // more slots than the descriptor's max_degree says: the row from global memory
+    // a block whose slots do not fit the stage forms its rows from global memory
     const int all = deg;
-    const bool staged = nsl <= A.cap_slots, big = !staged || deg > MAXD;
-    if (big) deg = 0;
+    const bool staged = nsl <= A.cap_slots;
+    if (!staged) deg = 0;
     int4* const srec = reinterpret_cast<int4*>(smem);
     unsigned char* const sslab = smem + (size_t)A.cap_slots * 16;
     const char* const rec = reinterpret_cast<const char*>(A.rec + kb);
@@ -129,7 +129,25 @@ __global__ void __launch_bounds__(kGroupThreads, MAXD <= 6 ? 8 : 6)
             }
         }
     }
-    if (big)
+    if (deg > MAXD) {  // the elements that the registers do not hold, one after another
+        Vec<T, V> x1[3], x2[3];
+#pragma unroll
+        for (int d = 0; d < 3; ++d) x1[d] = R[MAXD][d];
+        for (int j = MAXD; j < deg; ++j) {
+            const int4 r = srec[k0 + j];
+            rows(x2, row_at(u, r.z, nodeb));
+            const Vec<T, V> c = ldg<T, V>(row_at(A.coef + col, r.x, rowb));
+            if (!(r.w & 1)) {
+                rows(x1, row_at(u, r.y, nodeb));
+                to_diff<T, V>(x1, ua);
+            }
+            to_diff<T, V>(x2, ua);
+            slot_fma<T, V>(K + kStep * j, c, x1, x2, ua, acc);
+#pragma unroll
+            for (int d = 0; d < 3; ++d) x1[d] = x2[d];
+        }
+    }
+    if (!staged)
         ku_row_unstaged<T, V>(A.rec + kb + k0, A.slab + (size_t)(kb + k0) * kSlabStride, all, u,
                               A.coef + col, rowb, ua, acc);
 #pragma unroll
@@ -169,20 +187,23 @@ static int launch_group_k(const StepArgs<T>& A, bool after_step, cudaStream_t st
 // line, 128 x 400 wall, us a step, group / patch: FP32 16 samples 19.3 / 44.1, 32 samples
 // 43.2 / 50.2, 64 samples 87 / 57; FP64 16 samples 55.3 / 67.8, 25 samples 92 / 63.
 // Below 8 FP32 samples one a thread is the faster (4 samples: 8.4 against 10.1 us).
+// Any number of elements a node: a Delaunay sheet of 20,000 nodes with up to 18, us a step,
+// group / patch: FP32 1 sample 5.4 / 21.7, 8 samples 9.5 / 21.3, 32 samples 19.3 / 21.7; FP64
+// 8 samples 12.3 / 28.2, 16 samples 20.9 / 28.8.
 template <typename T>
 int launch_step_group(const cvfes_solid_mesh* m, StepArgs<T> A, int vec_max, bool after_step,
                       cudaStream_t st) {
     const int V = sizeof(T) == 4 && vec_max >= 2 && A.S >= 8 ? 2 : 1;
     const int sv = A.S / V;
-    if (m->max_degree <= 0 || m->max_degree > kGroupDegree || sv > (V == 2 ? 16 : 20) ||
-        m->n_nodes >= INT32_MAX / 2)
-        return 1;
+    if (m->max_degree <= 0 || sv > (V == 2 ? 16 : 20) || m->n_nodes >= INT32_MAX / 2) return 1;
     A.tpn = sv;
     A.nch = 1;
-    // at most 36 KB of slots: six blocks share an SM (one or two samples only)
-    const int fit = (int)(36 * 1024 / ((size_t)m->max_degree * SlotStage<T>::kBytes));
+    // at most 36 KB of slots: six blocks share an SM (one or two samples only).  A few nodes
+    // of more elements than the registers hold fit beside the others (six a node on average)
+    const int deg = (int)std::min<long long>(m->max_degree, kGroupDegree);
+    const int fit = (int)(36 * 1024 / (deg * SlotStage<T>::kBytes));
     A.npb = std::min(kGroupThreads / A.tpn, fit);
-    A.cap_slots = A.npb * (int)m->max_degree;
+    A.cap_slots = A.npb * deg + (int)std::min<long long>(m->max_degree - deg, 24);
 #define CVFES_GROUP(VV)                                                                     \
     if (m->max_degree <= 6)                                                                 \
         return A.vel ? launch_group_k<T, VV, true, 6>(A, after_step, st)                    \

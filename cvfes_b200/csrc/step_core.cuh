@@ -829,7 +829,7 @@ int launch_step_patch(const cvfes_solid_mesh* m, StepArgs<T> A, int vec_max, boo
                       cudaStream_t st, int norms_mode, long long max_rows, long long* rows);
 
 // Group step (solid_group.cu) for few samples: returns 1 without launching when there are
-// more, or a node has more slots than it holds.
+// more, or max_degree is unknown.
 template <typename T>
 int launch_step_group(const cvfes_solid_mesh* m, StepArgs<T> A, int vec_max, bool after_step,
                       cudaStream_t st);

@@ -31,7 +31,8 @@ def capped(nc, na, S):
 
 @pytest.mark.parametrize("precision", [32, 64])
 @pytest.mark.parametrize("nc,samples", [(16, 64), (17, 64), (29, 33), (29, 128), (30, 40), (31, 64),
-                                        (42, 48), (53, 128), (54, 128)])
+                                        (42, 48), (53, 128), (54, 128),
+                                        (9, 8), (24, 1), (24, 8), (30, 16), (60, 3), (200, 16)])
 def test_a_node_of_many_elements(lib, cuda, precision, nc, samples):
     mesh = capped(nc, 12, samples)
     want = run(mesh, precision, "auto", 0)
