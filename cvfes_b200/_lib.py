@@ -53,7 +53,7 @@ class SolidMeshDesc(C.Structure):
         ("tile_w", C.c_int32),
         ("tile_eh", C.c_int32),
         ("tile_we", C.c_int32),
-        ("tile_pad", C.c_int32),
+        ("slot_form", C.c_int32),
         ("bandwidth", C.c_int64),
         ("state_form", C.c_int32),
         ("damping_form", C.c_int32),

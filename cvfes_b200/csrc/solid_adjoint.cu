@@ -237,8 +237,8 @@ __device__ __forceinline__ void load27(const T* K, T (&kk)[27]) {
 
 // dchi^T Khat_e du for the element owned by this slot: (u1, u2) and (x1, x2) are
 // the first and second neighbour rows of u_n and chi_{n+1}, already differences
-// u_b - u_a.
-template <typename T, int V, bool SMEM_OWN = false>
+// u_b - u_a (FULL: the rows themselves).
+template <typename T, int V, bool SMEM_OWN = false, bool FULL = false>
 __device__ __forceinline__ Vec<T, V> owner_form(const T* own, const Vec<T, V> (&u1)[3],
                                                 const Vec<T, V> (&u2)[3],
                                                 const Vec<T, V> (&x1)[3],
@@ -248,10 +248,10 @@ __device__ __forceinline__ Vec<T, V> owner_form(const T* own, const Vec<T, V> (&
     Vec<T, V> du1[3], du2[3], dy1[3], dy2[3];
 #pragma unroll
     for (int d = 0; d < 3; ++d) {
-        du1[d] = u1[d];
-        du2[d] = u2[d];
-        dy1[d] = x1[d];
-        dy2[d] = x2[d];
+        du1[d] = FULL ? vsub(u1[d], ua[d]) : u1[d];
+        du2[d] = FULL ? vsub(u2[d], ua[d]) : u2[d];
+        dy1[d] = FULL ? vsub(x1[d], ca[d]) : x1[d];
+        dy2[d] = FULL ? vsub(x2[d], ca[d]) : x2[d];
     }
     // own points into global memory (gather kernel) or shared memory (fan kernel, SMEM_OWN):
     // plain generic loads, not the global-only read-only path.  From shared memory they
@@ -278,13 +278,13 @@ __device__ __forceinline__ Vec<T, V> owner_form(const T* own, const Vec<T, V> (&
 }
 
 // Gamma_e += that form.
-template <typename T, int V, bool SMEM_OWN = false>
+template <typename T, int V, bool SMEM_OWN = false, bool FULL = false>
 __device__ __forceinline__ void owner_grad(const RevArgs<T>& A, int e, const T* own, size_t S,
                                            size_t col,
                                            const Vec<T, V> (&u1)[3], const Vec<T, V> (&u2)[3],
                                            const Vec<T, V> (&x1)[3], const Vec<T, V> (&x2)[3],
                                            const Vec<T, V> (&ua)[3], const Vec<T, V> (&ca)[3]) {
-    const Vec<T, V> g = owner_form<T, V, SMEM_OWN>(own, u1, u2, x1, x2, ua, ca);
+    const Vec<T, V> g = owner_form<T, V, SMEM_OWN, FULL>(own, u1, u2, x1, x2, ua, ca);
     T* gp = A.gam + (size_t)e * S + col;
     Vec<T, V> gv = ld<T, V>(gp);
 #pragma unroll
@@ -374,7 +374,7 @@ __device__ __forceinline__ void rev_epilogue(const RevArgs<T>& A, long long a, s
 // One reverse step for (node a, V samples): reconstruct u_{n-1}, advance chi, accumulate
 // Gamma over the elements this node owns and G of this node.  Rows are gathered
 // through L1; a fan continuation reuses the previous slot's second neighbour.
-template <typename T, int V, bool GM>
+template <typename T, int V, bool GM, bool FULL = false>
 __global__ void __launch_bounds__(256) k_reverse(RevArgs<T> A) {
     long long a;
     int vec;
@@ -412,8 +412,8 @@ __global__ void __launch_bounds__(256) k_reverse(RevArgs<T> A) {
             for (int d = 0; d < 3; ++d) {
                 x1[d] = ldg<T, V>(A.u + o1 + d * S);
                 y1[d] = ldg<T, V>(A.x + o1 + d * S);
-                x1[d] = vsub(x1[d], ua[d]);
-                y1[d] = vsub(y1[d], ca[d]);
+                if constexpr (!FULL) x1[d] = vsub(x1[d], ua[d]);
+                if constexpr (!FULL) y1[d] = vsub(y1[d], ca[d]);
             }
         }
         const size_t o2 = (size_t)r.z * 3 * S + col;
@@ -421,8 +421,8 @@ __global__ void __launch_bounds__(256) k_reverse(RevArgs<T> A) {
         for (int d = 0; d < 3; ++d) {
             x2[d] = ldg<T, V>(A.u + o2 + d * S);
             y2[d] = ldg<T, V>(A.x + o2 + d * S);
-            x2[d] = vsub(x2[d], ua[d]);
-            y2[d] = vsub(y2[d], ca[d]);
+            if constexpr (!FULL) x2[d] = vsub(x2[d], ua[d]);
+            if constexpr (!FULL) y2[d] = vsub(y2[d], ca[d]);
         }
         const Vec<T, V> c = ldg<T, V>(A.coef + (size_t)r.x * S + col);
         T kk[27];
@@ -430,6 +430,13 @@ __global__ void __launch_bounds__(256) k_reverse(RevArgs<T> A) {
 #pragma unroll
         for (int i = 0; i < 3; ++i) {
             Vec<T, V> tu = vzero<T, V>(), tc = vzero<T, V>();
+            if constexpr (FULL) {
+#pragma unroll
+                for (int jj = 0; jj < 3; ++jj) {
+                    axpy(tu, kk[3 * i + jj], ua[jj]);
+                    axpy(tc, kk[3 * i + jj], ca[jj]);
+                }
+            }
 #pragma unroll
             for (int jj = 0; jj < 3; ++jj) {
                 axpy(tu, kk[9 + 3 * i + jj], x1[jj]);
@@ -444,7 +451,7 @@ __global__ void __launch_bounds__(256) k_reverse(RevArgs<T> A) {
             vfma(accC[i], c, tc);
         }
         if (((r.w >> 8) & 3) == 0)
-            owner_grad<T, V>(A, r.x, A.own + (size_t)kOwnStride * k, S, col, x1, x2, y1, y2,
+            owner_grad<T, V, false, FULL>(A, r.x, A.own + (size_t)kOwnStride * k, S, col, x1, x2, y1, y2,
                                    ua, ca);
 #pragma unroll
         for (int d = 0; d < 3; ++d) {
@@ -467,14 +474,16 @@ __device__ __forceinline__ void load3(Vec<T, V> (&x)[3], const T* __restrict__ b
 #pragma unroll
     for (int d = 0; d < 3; ++d) x[d] = ldg<T, V>(p + d * S);
 }
-template <typename T, int V>
+template <typename T, int V, bool FULL = false>
 __device__ __forceinline__ void diff3(Vec<T, V> (&x)[3], const Vec<T, V> (&ref)[3]) {
+    if constexpr (!FULL) {
 #pragma unroll
-    for (int d = 0; d < 3; ++d) x[d] = vsub(x[d], ref[d]);
+        for (int d = 0; d < 3; ++d) x[d] = vsub(x[d], ref[d]);
+    }
 }
 
 // Both row products of one slot from one read of its stiffness rows (shared memory).
-template <typename T, int V>
+template <typename T, int V, bool FULL = false>
 __device__ __forceinline__ void slot_fma2(const T* K, const Vec<T, V>& c,
                                           const Vec<T, V> (&u1)[3], const Vec<T, V> (&u2)[3],
                                           const Vec<T, V> (&x1)[3], const Vec<T, V> (&x2)[3],
@@ -492,7 +501,7 @@ __device__ __forceinline__ void slot_fma2(const T* K, const Vec<T, V>& c,
         }
     } else {
 #pragma unroll
-        for (int q = 4; q < 14; ++q) {
+        for (int q = FULL ? 0 : 4; q < 14; ++q) {
             const double2 t = reinterpret_cast<const double2*>(K)[q];
             kk[2 * q] = t.x;
             kk[2 * q + 1] = t.y;
@@ -501,6 +510,13 @@ __device__ __forceinline__ void slot_fma2(const T* K, const Vec<T, V>& c,
 #pragma unroll
     for (int i = 0; i < 3; ++i) {
         Vec<T, V> tu = vzero<T, V>(), tc = vzero<T, V>();
+        if constexpr (FULL) {
+#pragma unroll
+            for (int jj = 0; jj < 3; ++jj) {
+                axpy(tu, kk[3 * i + jj], ua[jj]);
+                axpy(tc, kk[3 * i + jj], ca[jj]);
+            }
+        }
 #pragma unroll
         for (int jj = 0; jj < 3; ++jj) {
             axpy(tu, kk[9 + 3 * i + jj], u1[jj]);
@@ -649,7 +665,7 @@ __global__ void __launch_bounds__(256, MINB) k_reverse_fan(RevArgs<T> A) {
 // 64 samples with G 267 / 213; 64 x 128 wall, 64 samples FP32 22.4 / 21.3, FP64 54.7 / 46.4.
 // Both row products and the Gamma update of a node that is not staged (more slots than the
 // descriptor's max_degree), all from global memory, as ku_row_unstaged.
-template <typename T, int V>
+template <typename T, int V, bool FULL>
 __device__ __forceinline__ void rev_row_unstaged(const RevArgs<T>& A, int k0, int n, const T* u,
                                                  const T* x, size_t col, uint32_t rowb, bool on,
                                                  const Vec<T, V> (&ua)[3],
@@ -660,9 +676,11 @@ __device__ __forceinline__ void rev_row_unstaged(const RevArgs<T>& A, int k0, in
     auto rows = [&](Vec<T, V> (&p)[3], Vec<T, V> (&q)[3], int b) {
 #pragma unroll
         for (int d = 0; d < 3; ++d) {
-            p[d] = vsub(ld_state<T, V>(row_at(u, b, 3 * rowb) + d * S), ua[d]);
-            q[d] = vsub(ld_state<T, V>(row_at(x, b, 3 * rowb) + d * S), ca[d]);
+            p[d] = ld_state<T, V>(row_at(u, b, 3 * rowb) + d * S);
+            q[d] = ld_state<T, V>(row_at(x, b, 3 * rowb) + d * S);
         }
+        diff3<T, V, FULL>(p, ua);
+        diff3<T, V, FULL>(q, ca);
     };
 #pragma unroll 1
     for (int k = k0; k < k0 + n; ++k) {
@@ -674,14 +692,14 @@ __device__ __forceinline__ void rev_row_unstaged(const RevArgs<T>& A, int k0, in
         }
         if (k == k0 || !(r.w & 1)) rows(u1, x1, r.y);
         rows(u2, x2, r.z);
-        slot_fma2<T, V>(A.slab + (size_t)kSlabStride * k,
+        slot_fma2<T, V, FULL>(A.slab + (size_t)kSlabStride * k,
                         ldg<T, V>(row_at(A.coef + col, r.x, rowb)), u1, u2, x1, x2, ua, ca, accU,
                         accC);
         if (((r.w >> 8) & 3) == 0) {
             T* const gp = row_at(A.gam + col, r.x, rowb);
             Vec<T, V> gv = ld<T, V>(gp);
             const Vec<T, V> g =
-                owner_form<T, V>(A.own + (size_t)kOwnStride * k, u1, u2, x1, x2, ua, ca);
+                owner_form<T, V, false, FULL>(A.own + (size_t)kOwnStride * k, u1, u2, x1, x2, ua, ca);
 #pragma unroll
             for (int i = 0; i < V; ++i) gv.v[i] += g.v[i];
             if (on) st<T, V>(gp, gv);
@@ -689,11 +707,11 @@ __device__ __forceinline__ void rev_row_unstaged(const RevArgs<T>& A, int k0, in
     }
 }
 
-template <typename T, int V, bool GM, int W>
+template <typename T, int V, bool GM, int W, bool FULL>
 __global__ void __launch_bounds__(32 * W, 1)
     k_reverse_patch(RevArgs<T> A, PatchMap M, int max_degree) {
     extern __shared__ __align__(16) unsigned char smem[];
-    using P = SlotStage<T>;
+    using P = SlotStage<T, FULL>;
     constexpr int kOwnWords = kOwnStride * (int)sizeof(T) / 16;
     const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
     const uint32_t b_rec = 16u * max_degree, b_slab = P::kSlotBytes * max_degree;
@@ -809,9 +827,9 @@ __global__ void __launch_bounds__(32 * W, 1)
                 Vec<T, V> gv = vzero<T, V>();
                 T* const gp = row_at(gam, r.x, rowb);
                 if (owner) gv = ld<T, V>(gp);  // requested before the products
-                slot_fma2<T, V>(K + kStep * k, c, u1, u2, x1, x2, ua, ca, accU, accC);
+                slot_fma2<T, V, FULL>(K + kStep * k, c, u1, u2, x1, x2, ua, ca, accU, accC);
                 if (owner) {
-                    const Vec<T, V> g = owner_form<T, V, true>(own + kOwnStride * k, u1, u2,
+                    const Vec<T, V> g = owner_form<T, V, true, FULL>(own + kOwnStride * k, u1, u2,
                                                                      x1, x2, ua, ca);
 #pragma unroll
                     for (int q = 0; q < V; ++q) gv.v[q] += g.v[q];
@@ -826,8 +844,8 @@ __global__ void __launch_bounds__(32 * W, 1)
                 rows(U[0], X[0], srec[0].y);
                 rows(U[1], X[1], srec[0].z);
                 C[0] = ldg<T, V>(row_at(cf, srec[0].x, rowb));
-                diff3<T, V>(U[0], ua);
-                diff3<T, V>(X[0], ca);
+                diff3<T, V, FULL>(U[0], ua);
+                diff3<T, V, FULL>(X[0], ca);
 #pragma unroll
                 for (int k = 0; k < 6; ++k) {
                     if (k < 5) {
@@ -838,8 +856,8 @@ __global__ void __launch_bounds__(32 * W, 1)
                         if (a >= A.n_clamped) rev_rows<T, V, GM>(A, a, col, R);
                     }
                     if (k == 2) prefetch_elems();
-                    diff3<T, V>(U[k + 1], ua);
-                    diff3<T, V>(X[k + 1], ca);
+                    diff3<T, V, FULL>(U[k + 1], ua);
+                    diff3<T, V, FULL>(X[k + 1], ca);
                     element(k, srec[k], C[k], U[k], U[k + 1], X[k], X[k + 1]);
                     // FP32: keeps the next element's loads from sinking to their uses
                     // (64 x 128 wall, 64 samples: 3.36 ms a gradient of 100 steps, 3.52 without)
@@ -851,8 +869,8 @@ __global__ void __launch_bounds__(32 * W, 1)
                 rows(U0, X0, r.y);
                 rows(U1, X1, r.z);
                 c1 = ldg<T, V>(row_at(cf, r.x, rowb));
-                diff3<T, V>(U0, ua);
-                diff3<T, V>(X0, ca);
+                diff3<T, V, FULL>(U0, ua);
+                diff3<T, V, FULL>(X0, ca);
                 int k = 0;
                 auto phase = [&](Vec<T, V> (&pu)[3], Vec<T, V> (&px)[3], Vec<T, V> (&cu)[3],
                                  Vec<T, V> (&cx)[3], const Vec<T, V>& c, Vec<T, V> (&nu)[3],
@@ -864,13 +882,13 @@ __global__ void __launch_bounds__(32 * W, 1)
                         rows(nu, nx, rn.z);
                         cn = ldg<T, V>(row_at(cf, rn.x, rowb));
                     }
-                    diff3<T, V>(cu, ua);
-                    diff3<T, V>(cx, ca);
+                    diff3<T, V, FULL>(cu, ua);
+                    diff3<T, V, FULL>(cx, ca);
                     element(k, r, c, pu, cu, px, cx);
                     if (next && !(rn.w & 1)) {  // fan break: the next first neighbour is new
                         rows(cu, cx, rn.y);
-                        diff3<T, V>(cu, ua);
-                        diff3<T, V>(cx, ca);
+                        diff3<T, V, FULL>(cu, ua);
+                        diff3<T, V, FULL>(cx, ca);
                     }
                     r = rn;
                     ++k;
@@ -918,7 +936,7 @@ __global__ void __launch_bounds__(32 * W, 1)
             ca[d] = ld_state<T, V>(row_at(A.x + col2, b, 3 * rb) + d * (size_t)A.S);
             accU[d] = accC[d] = vzero<T, V>();
         }
-        rev_row_unstaged<T, V>(A, s0, ns, A.u + col2, A.x + col2, col2,
+        rev_row_unstaged<T, V, FULL>(A, s0, ns, A.u + col2, A.x + col2, col2,
                                rb, on2, ua, ca, accU, accC);
         rev_epilogue<T, V, GM>(A, b, (size_t)A.S, col2, (size_t)b * 3 * A.S + col2, ua, ca, accU,
                                accC, on2);
@@ -1000,9 +1018,9 @@ int launch_rev_fan_m(int minb, unsigned grid, int threads, size_t smem, cudaStre
 }
 
 // The patch kernel (variant 2); returns 1 without launching when a node's slots do not fit.
-template <typename T, int V>
+template <typename T, int V, bool FULL = false>
 int launch_rev_patch(const cvfes_solid_mesh* m, RevArgs<T> A, bool after_step, cudaStream_t st) {
-    const size_t slot = SlotStage<T>::kBytes + kOwnStride * sizeof(T);
+    const size_t slot = SlotStage<T, FULL>::kBytes + kOwnStride * sizeof(T);
     // (the slots are staged in 16-byte words)
     if (m->max_degree <= 0 || m->max_degree >= 1024 || A.S >= (1 << 27) ||
         m->n_nodes >= INT32_MAX / 2 || reinterpret_cast<uintptr_t>(A.own) % 16 ||
@@ -1015,7 +1033,7 @@ int launch_rev_patch(const cvfes_solid_mesh* m, RevArgs<T> A, bool after_step, c
     if (smem > 160 * 1024) return 1;
     A.nch = (A.S / V + 31) / 32;
     const PatchMap M = patch_map(m->n_nodes, m->bandwidth, W);
-    auto kernel = A.gm ? k_reverse_patch<T, V, true, W> : k_reverse_patch<T, V, false, W>;
+    auto kernel = A.gm ? k_reverse_patch<T, V, true, W, FULL> : k_reverse_patch<T, V, false, W, FULL>;
     int per_sm = 0;
     const int rc = fanp_blocks_per_sm(reinterpret_cast<const void*>(kernel), 32 * W, smem, &per_sm);
     if (rc) return rc;
@@ -1069,7 +1087,10 @@ int launch_reverse_step(const cvfes_adjoint_desc* d, const T* u, T* uo, const T*
     A.eta = (T)eta;
     A.inv1meta = (T)(1.0 / (1.0 - eta));
     A.w0 = (T)(d->dt * d->dt / (1.0 + g));
-    const RevTuning tu = rev_tuning<T>();
+    RevTuning tu = rev_tuning<T>();
+    // rows as given (FP64, slot_form 0): the patch and row-gather kernels have that form
+    const bool full = mesh_full<T>(m);
+    if (full && tu.variant != 0) tu.variant = 2;
     const Prefetch pf = step_prefetch(sizeof(T) == 4 ? 32 : 64, m->bandwidth);
     A.pf_dist = pf.dist;
     A.pf_parts = pf.parts;
@@ -1089,7 +1110,10 @@ int launch_reverse_step(const cvfes_adjoint_desc* d, const T* u, T* uo, const T*
         if constexpr (sizeof(T) == 4) {
             if (V >= 2 && (A.S + 31) / 32 > (A.S / 2 + 31) / 32) prc = launch_rev_patch<T, 2>(m, A, after_step, st);
         }
-        if (prc == 1) prc = launch_rev_patch<T, 1>(m, A, after_step, st);
+        if constexpr (sizeof(T) == 8) {
+            if (full) prc = launch_rev_patch<T, 1, true>(m, A, after_step, st);
+        }
+        if (prc == 1 && !full) prc = launch_rev_patch<T, 1>(m, A, after_step, st);
         if (prc <= 0) return prc;
     }
     const RowGrid rg = row_grid(m->n_nodes, A.S / V, 256);
@@ -1099,7 +1123,7 @@ int launch_reverse_step(const cvfes_adjoint_desc* d, const T* u, T* uo, const T*
     A.cap_slots = 0;
     const long long cap = (long long)tu.npb * m->max_degree;
     const size_t smem = 16 + (size_t)cap * (16 + (kSlabStride + kOwnStride) * sizeof(T));
-    const bool fan = (tu.variant == 1 || tu.variant == 2) && m->max_degree > 0 &&
+    const bool fan = (tu.variant == 1 || tu.variant == 2) && !full && m->max_degree > 0 &&
                      (A.S / V) % 32 == 0 && smem <= kRevMaxStage && tu.npb >= 1 && tu.npb <= 8;
     unsigned fan_grid = 0;
     if (fan) {
@@ -1112,6 +1136,15 @@ int launch_reverse_step(const cvfes_adjoint_desc* d, const T* u, T* uo, const T*
         fan_grid = (unsigned)(((m->n_nodes + A.npb - 1) / A.npb) * A.nch);
     }
     const bool gmv = d->gmass != nullptr;
+    if constexpr (sizeof(T) == 8) {
+        if (full) {
+            auto kernel = V == 2 ? (gmv ? k_reverse<T, 2, true, true> : k_reverse<T, 2, false, true>)
+                                 : (gmv ? k_reverse<T, 1, true, true> : k_reverse<T, 1, false, true>);
+            kernel<<<rg.grid, 256, 0, st>>>(A);
+            CVFES_LAUNCH_CHECK("k_reverse");
+            return CVFES_OK;
+        }
+    }
     if (V == 4) {
         if constexpr (sizeof(T) == 4)
             return launch_rev_v<T, 4>(tu, fan, gmv, fan_grid, smem, rg, st, A);

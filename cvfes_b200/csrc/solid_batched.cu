@@ -57,6 +57,7 @@ struct BatchMesh {
     int f_chunks;     // sample chunks per node block
     int max_deg;      // slots of the busiest node
     int* status;      // this mesh's device status word (bit 0: a bounded wait gave up)
+    int full;         // 1: FP64 rows applied as given (slot_form 0 of the mesh)
 };
 
 constexpr int kBatchWarps = 2;
@@ -143,7 +144,13 @@ __global__ void __launch_bounds__(256) k_step_batched(const BatchMesh* __restric
         T f[3];
         node_load<T>(A, a, step_pressure<T>(A), f);
         Vec<T, V> acc[3];
-        ku_row<T, V>(A.node_ptr, A.rec, A.slab, A.coef, A.u, S, col, a, ua, acc);
+        bool full = false;
+        if constexpr (sizeof(T) == 8) full = M.full;
+        if (full)
+            ku_row<T, V, sizeof(T) == 8>(A.node_ptr, A.rec, A.slab, A.coef, A.u, S, col, a, ua,
+                                         acc);
+        else
+            ku_row<T, V>(A.node_ptr, A.rec, A.slab, A.coef, A.u, S, col, a, ua, acc);
         step_epilogue<T, V>(A, a, S, col, row, ua, acc, f);
     }
 }
@@ -266,9 +273,15 @@ __global__ void __launch_bounds__(32 * kBatchWarps, MINB)
                 const int kb = __ldg(M.node_ptr + a0);
                 const int k0 = __ldg(M.node_ptr + a) - kb, k1 = __ldg(M.node_ptr + a + 1) - kb;
                 Vec<T, V> acc[3];
-                ku_row_fan<T, V>(stage_rec(srec0, stage_bytes, sg),
-                                       stage_slab(sslab0, stage_bytes, sg), k0, k1, A.u, A.coef,
-                                       S, col, ua, acc);
+                const int4* const rec = stage_rec(srec0, stage_bytes, sg);
+                const T* const slab = stage_slab(sslab0, stage_bytes, sg);
+                bool full = false;
+                if constexpr (sizeof(T) == 8) full = M.full;
+                if (full)
+                    ku_row_fan<T, V, sizeof(T) == 8>(rec, slab, k0, k1, A.u, A.coef, S, col, ua,
+                                                     acc);
+                else
+                    ku_row_fan<T, V>(rec, slab, k0, k1, A.u, A.coef, S, col, ua, acc);
                 step_epilogue<T, V>(A, a, S, col, row, ua, acc, f);
             }
         }
@@ -420,6 +433,7 @@ extern "C" int cvfes_batch_pack(const cvfes_batch_item* items, int32_t n_meshes,
         b.f_chunks = (sv + b.f_tpn - 1) / b.f_tpn;
         b.max_deg = (int)ms.max_degree;
         b.status = ms.status;
+        b.full = mesh_full<double>(&ms) && precision == 64;
         b.f_off = f_off;
         const long long nodes_per_item = (long long)kBatchWarps * b.f_npw;
         f_off += ((ms.n_nodes + nodes_per_item - 1) / nodes_per_item) * b.f_chunks;

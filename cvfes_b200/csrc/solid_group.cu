@@ -31,11 +31,11 @@ namespace cvfes {
 constexpr int kGroupThreads = 64;  // FP64 64 x 128 wall, 8 samples: 4.25 us at 128, 4.64 at 256
 constexpr int kGroupDegree = 8;  // slots of a node held in registers
 
-template <typename T, int V, bool VEL, int MAXD>
+template <typename T, int V, bool VEL, int MAXD, bool FULL>
 __global__ void __launch_bounds__(kGroupThreads, MAXD <= 6 ? 8 : 6)
     k_step_group(StepArgs<T> A) {
     extern __shared__ __align__(16) unsigned char smem[];
-    using P = SlotStage<T>;
+    using P = SlotStage<T, FULL>;
     constexpr int kStep = P::kSlotBytes / (int)sizeof(T);
     const int a0 = blockIdx.x * A.npb, n_nodes = (int)A.n_nodes;
     const int a1 = min(a0 + A.npb, n_nodes);
@@ -114,18 +114,18 @@ __global__ void __launch_bounds__(kGroupThreads, MAXD <= 6 ? 8 : 6)
                        (size_t)k0 * kStep;
 #pragma unroll
     for (int d = 0; d < 3; ++d) acc[d] = vzero<T, V>();
-    if (deg > 0) to_diff<T, V>(R[0], ua);
+    if (deg > 0) to_diff<T, V, FULL>(R[0], ua);
 #pragma unroll
     for (int j = 0; j < MAXD; ++j) {
         if (j < deg) {
-            to_diff<T, V>(R[j + 1], ua);
+            to_diff<T, V, FULL>(R[j + 1], ua);
             if (j > 0 && !(srec[k0 + j].w & 1)) {  // fan break: a first neighbour of its own
                 Vec<T, V> b[3];
                 rows(b, row_at(u, srec[k0 + j].y, nodeb));
-                to_diff<T, V>(b, ua);
-                slot_fma<T, V>(K + kStep * j, C[j], b, R[j + 1], ua, acc);
+                to_diff<T, V, FULL>(b, ua);
+                slot_fma<T, V, FULL>(K + kStep * j, C[j], b, R[j + 1], ua, acc);
             } else {
-                slot_fma<T, V>(K + kStep * j, C[j], R[j], R[j + 1], ua, acc);
+                slot_fma<T, V, FULL>(K + kStep * j, C[j], R[j], R[j + 1], ua, acc);
             }
         }
     }
@@ -139,16 +139,16 @@ __global__ void __launch_bounds__(kGroupThreads, MAXD <= 6 ? 8 : 6)
             const Vec<T, V> c = ldg<T, V>(row_at(A.coef + col, r.x, rowb));
             if (!(r.w & 1)) {
                 rows(x1, row_at(u, r.y, nodeb));
-                to_diff<T, V>(x1, ua);
+                to_diff<T, V, FULL>(x1, ua);
             }
-            to_diff<T, V>(x2, ua);
-            slot_fma<T, V>(K + kStep * j, c, x1, x2, ua, acc);
+            to_diff<T, V, FULL>(x2, ua);
+            slot_fma<T, V, FULL>(K + kStep * j, c, x1, x2, ua, acc);
 #pragma unroll
             for (int d = 0; d < 3; ++d) x1[d] = x2[d];
         }
     }
     if (!staged)
-        ku_row_unstaged<T, V>(A.rec + kb + k0, A.slab + (size_t)(kb + k0) * kSlabStride, all, u,
+        ku_row_unstaged<T, V, FULL>(A.rec + kb + k0, A.slab + (size_t)(kb + k0) * kSlabStride, all, u,
                               A.coef + col, rowb, ua, acc);
 #pragma unroll
     for (int d = 0; d < 3; ++d) {
@@ -169,10 +169,10 @@ __global__ void __launch_bounds__(kGroupThreads, MAXD <= 6 ? 8 : 6)
     }
 }
 
-template <typename T, int V, bool VEL, int MAXD>
+template <typename T, int V, bool VEL, int MAXD, bool FULL>
 static int launch_group_k(const StepArgs<T>& A, bool after_step, cudaStream_t st) {
-    auto kernel = k_step_group<T, V, VEL, MAXD>;
-    const size_t smem = (size_t)A.cap_slots * SlotStage<T>::kBytes;
+    auto kernel = k_step_group<T, V, VEL, MAXD, FULL>;
+    const size_t smem = (size_t)A.cap_slots * SlotStage<T, FULL>::kBytes;
     int per_sm = 0;  // also sets the shared-memory attribute
     const int rc =
         fanp_blocks_per_sm(reinterpret_cast<const void*>(kernel), kGroupThreads, smem, &per_sm);
@@ -195,27 +195,30 @@ int launch_step_group(const cvfes_solid_mesh* m, StepArgs<T> A, int vec_max, boo
                       cudaStream_t st) {
     const int V = sizeof(T) == 4 && vec_max >= 2 && A.S >= 8 ? 2 : 1;
     const int sv = A.S / V;
+    const bool full = mesh_full<T>(m);
     if (m->max_degree <= 0 || sv > (V == 2 ? 16 : 20) || m->n_nodes >= INT32_MAX / 2) return 1;
     A.tpn = sv;
     A.nch = 1;
     // at most 36 KB of slots: six blocks share an SM (one or two samples only).  A few nodes
     // of more elements than the registers hold fit beside the others (six a node on average)
     const int deg = (int)std::min<long long>(m->max_degree, kGroupDegree);
-    const int fit = (int)(36 * 1024 / (deg * SlotStage<T>::kBytes));
+    const int fit = (int)(36 * 1024 / (deg * (full ? SlotStage<T, true>::kBytes : SlotStage<T>::kBytes)));
     A.npb = std::min(kGroupThreads / A.tpn, fit);
     A.cap_slots = A.npb * deg + (int)std::min<long long>(m->max_degree - deg, 24);
-#define CVFES_GROUP(VV)                                                                     \
-    if (m->max_degree <= 6)                                                                 \
-        return A.vel ? launch_group_k<T, VV, true, 6>(A, after_step, st)                    \
-                     : launch_group_k<T, VV, false, 6>(A, after_step, st);                  \
-    return A.vel ? launch_group_k<T, VV, true, kGroupDegree>(A, after_step, st)             \
-                 : launch_group_k<T, VV, false, kGroupDegree>(A, after_step, st);
+#define CVFES_GROUP(VV, FULL)                                                                  \
+    if (m->max_degree <= 6)                                                                    \
+        return A.vel ? launch_group_k<T, VV, true, 6, FULL>(A, after_step, st)                 \
+                     : launch_group_k<T, VV, false, 6, FULL>(A, after_step, st);               \
+    return A.vel ? launch_group_k<T, VV, true, kGroupDegree, FULL>(A, after_step, st)          \
+                 : launch_group_k<T, VV, false, kGroupDegree, FULL>(A, after_step, st);
     if constexpr (sizeof(T) == 4) {
         if (V == 2) {
-            CVFES_GROUP(2)
+            CVFES_GROUP(2, false)
         }
+    } else if (full) {
+        CVFES_GROUP(1, true)
     }
-    CVFES_GROUP(1)
+    CVFES_GROUP(1, false)
 #undef CVFES_GROUP
 }
 

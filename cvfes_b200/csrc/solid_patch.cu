@@ -111,11 +111,11 @@ __device__ __forceinline__ void patch_epilogue(const StepArgs<T>& A, T* un, T* v
 // NORMS: 0 none; 1 the per-sample norms of the new state, each lane's sums in tensor
 // memory; 2 the same in shared memory behind the stages.  The grid is a multiple of the
 // chunks, so a block keeps one chunk for its whole life and writes one row of partials.
-template <typename T, int V, bool VEL, int NORMS, int W>
+template <typename T, int V, bool VEL, int NORMS, int W, bool FULL>
 __global__ void __launch_bounds__(32 * W, 1)
     k_step_patch(StepArgs<T> A, PatchMap M, int max_degree) {
     extern __shared__ __align__(16) unsigned char smem[];
-    using P = SlotStage<T>;
+    using P = SlotStage<T, FULL>;
     const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
     const uint32_t b_rec = 16u * max_degree, b_stage = b_rec + P::kSlotBytes * max_degree;
     unsigned char* const wb = smem + warp * (2 * b_stage);
@@ -291,7 +291,7 @@ __global__ void __launch_bounds__(32 * W, 1)
                 C[0] = ldg<T, V>(row_at(cf, r0.x, rowb));
                 rows(X[2], r1.z);
                 C[1] = ldg<T, V>(row_at(cf, r1.x, rowb));
-                to_diff<T, V>(X[0], ua);
+                to_diff<T, V, FULL>(X[0], ua);
 #pragma unroll
                 for (int k = 0; k < 6; ++k) {
                     if (k < 4) {
@@ -301,8 +301,8 @@ __global__ void __launch_bounds__(32 * W, 1)
                     }
                     if (k == 4) epilogue_rows();
                     if (k == 2) prefetch_coef();
-                    to_diff<T, V>(X[k + 1], ua);
-                    slot_fma<T, V>(K + kStep * k, C[k], X[k], X[k + 1], ua, acc);
+                    to_diff<T, V, FULL>(X[k + 1], ua);
+                    slot_fma<T, V, FULL>(K + kStep * k, C[k], X[k], X[k + 1], ua, acc);
                 }
             } else {
                 if (n > 0) {  // any fan: three buffers rotate, one element ahead
@@ -311,7 +311,7 @@ __global__ void __launch_bounds__(32 * W, 1)
                     rows(B0, r0.y);
                     rows(B1, r0.z);
                     c1 = ldg<T, V>(row_at(cf, r0.x, rowb));
-                    to_diff<T, V>(B0, ua);
+                    to_diff<T, V, FULL>(B0, ua);
                     int k = 0;
                     auto phase = [&](Vec<T, V> (&prev)[3], Vec<T, V> (&cur)[3], const Vec<T, V>& c,
                                      Vec<T, V> (&nx)[3], Vec<T, V>& cn) {
@@ -322,11 +322,11 @@ __global__ void __launch_bounds__(32 * W, 1)
                             rows(nx, r.z);
                             cn = ldg<T, V>(row_at(cf, r.x, rowb));
                         }
-                        to_diff<T, V>(cur, ua);
-                        slot_fma<T, V>(K + kStep * k, c, prev, cur, ua, acc);
+                        to_diff<T, V, FULL>(cur, ua);
+                        slot_fma<T, V, FULL>(K + kStep * k, c, prev, cur, ua, acc);
                         if (next && !(r.w & 1)) {  // fan break: a first neighbour of its own
                             rows(cur, r.y);
-                            to_diff<T, V>(cur, ua);
+                            to_diff<T, V, FULL>(cur, ua);
                         }
                         ++k;
                     };
@@ -383,7 +383,7 @@ __global__ void __launch_bounds__(32 * W, 1)
                 vo[d] = ld_state<T, V, true>(row_at(A.up + col2, b, 3 * rb) + d * S);
                 acc[d] = vzero<T, V>();
             }
-            ku_row_unstaged<T, V>(A.rec + s0, A.slab + (size_t)s0 * kSlabStride,
+            ku_row_unstaged<T, V, FULL>(A.rec + s0, A.slab + (size_t)s0 * kSlabStride,
                                   ns, A.u + col2, A.coef + col2, rb, ua,
                                   acc);
             const Vec<T, V> im = ldcs<T, V>(row_at(A.invm + col2, b, rb));
@@ -447,14 +447,14 @@ struct PatchBlock {
         NORMS || sizeof(T) == 8 || V == 4 ? 16 : (V == 2 ? 20 : 28);
 };
 
-template <typename T, int V, bool VEL, int NORMS>
+template <typename T, int V, bool VEL, int NORMS, bool FULL>
 static int launch_patch_k(const StepArgs<T>& A, const cvfes_solid_mesh* m, int max_degree,
                           long long max_rows, long long* rows, bool after_step,
                           cudaStream_t st) {
     constexpr int W = PatchBlock<T, V, NORMS>::kWarps;
     const PatchMap M = patch_map(m->n_nodes - A.n_clamped, m->bandwidth, W);
-    auto kernel = k_step_patch<T, V, VEL, NORMS, W>;
-    size_t smem = (size_t)W * 2 * max_degree * SlotStage<T>::kBytes;
+    auto kernel = k_step_patch<T, V, VEL, NORMS, W, FULL>;
+    size_t smem = (size_t)W * 2 * max_degree * SlotStage<T, FULL>::kBytes;
     // Slots of up to 29 (FP64) or 30 to 53 (FP32, by the block's warps) elements a node; 160 KB
     // leave room for the sums of NORMS 2.  Tube closed by a cap of nc elements at its apex, nc
     // x 400 nodes, us a step, patch / fan: FP64 nc 28, 64 samples 26.8 / 38.8; FP32 nc 50, 256
@@ -499,23 +499,31 @@ int launch_step_patch(const cvfes_solid_mesh* m, StepArgs<T> A, int vec_max, boo
     const int V = patch_vec(A.S, vec_max);
     A.nch = (A.S / V + 31) / 32;
     const int norms = A.norm_part ? (norms_mode == 0 ? 1 : 2) : 0;
-#define CVFES_PATCH(VV, VEL)                                                                   \
+#define CVFES_PATCH(VV, VEL, FULL)                                                             \
     switch (norms) {                                                                           \
-        case 1: return launch_patch_k<T, VV, VEL, 1>(A, m, md, max_rows, rows, false, st);     \
-        case 2: return launch_patch_k<T, VV, VEL, 2>(A, m, md, max_rows, rows, false, st);     \
-        default: return launch_patch_k<T, VV, VEL, 0>(A, m, md, 0, nullptr, after_step, st);   \
+        case 1: return launch_patch_k<T, VV, VEL, 1, FULL>(A, m, md, max_rows, rows, false, st); \
+        case 2: return launch_patch_k<T, VV, VEL, 2, FULL>(A, m, md, max_rows, rows, false, st); \
+        default:                                                                               \
+            return launch_patch_k<T, VV, VEL, 0, FULL>(A, m, md, 0, nullptr, after_step, st);  \
     }
-    if (V == 4) {
-        if constexpr (sizeof(T) == 4) {
-            if (A.vel) CVFES_PATCH(4, true)
-            CVFES_PATCH(4, false)
+#define CVFES_PATCH_V(VV, FULL)         \
+    if (A.vel) CVFES_PATCH(VV, true, FULL) \
+    CVFES_PATCH(VV, false, FULL)
+    if constexpr (sizeof(T) == 8) {
+        if (mesh_full<T>(m)) {
+            if (V == 2) {
+                CVFES_PATCH_V(2, true)
+            }
+            CVFES_PATCH_V(1, true)
         }
-    } else if (V == 2) {
-        if (A.vel) CVFES_PATCH(2, true)
-        CVFES_PATCH(2, false)
+    } else if (V == 4) {
+        CVFES_PATCH_V(4, false)
     }
-    if (A.vel) CVFES_PATCH(1, true)
-    CVFES_PATCH(1, false)
+    if (V == 2) {
+        CVFES_PATCH_V(2, false)
+    }
+    CVFES_PATCH_V(1, false)
+#undef CVFES_PATCH_V
 #undef CVFES_PATCH
 }
 

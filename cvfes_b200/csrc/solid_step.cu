@@ -36,7 +36,7 @@
 
 namespace cvfes {
 
-template <typename T, int V>
+template <typename T, int V, bool FULL = false>
 __global__ void __launch_bounds__(256) k_step(StepArgs<T> A) {
     long long a;
     int vec;
@@ -54,7 +54,7 @@ __global__ void __launch_bounds__(256) k_step(StepArgs<T> A) {
     T f[3];
     node_load<T>(A, a, step_pressure<T>(A), f);
     Vec<T, V> acc[3];
-    ku_row<T, V>(A.node_ptr, A.rec, A.slab, A.coef, A.u, S, col, a, ua, acc);
+    ku_row<T, V, FULL>(A.node_ptr, A.rec, A.slab, A.coef, A.u, S, col, a, ua, acc);
     step_epilogue<T, V>(A, a, S, col, row, ua, acc, f);
 }
 
@@ -191,7 +191,7 @@ __global__ void __launch_bounds__(256, MINB) k_step_staged(StepArgs<T> A) {
     step_epilogue<T, V>(A, a, S, col, row, ua, acc, f);
 }
 
-template <typename T, int V>
+template <typename T, int V, bool FULL = false>
 __global__ void __launch_bounds__(256)
     k_kmul(const int32_t* node_ptr, const int4* rec, const T* slab, const T* coef, const T* u,
            T* res, long long n_nodes, int S_, int accumulate, int tpn, int npb) {
@@ -204,7 +204,7 @@ __global__ void __launch_bounds__(256)
     Vec<T, V> ua[3], acc[3];
 #pragma unroll
     for (int d = 0; d < 3; ++d) ua[d] = ldg<T, V>(u + row + d * S);
-    ku_row<T, V>(node_ptr, rec, slab, coef, u, S, col, a, ua, acc);
+    ku_row<T, V, FULL>(node_ptr, rec, slab, coef, u, S, col, a, ua, acc);
 #pragma unroll
     for (int d = 0; d < 3; ++d) {
         Vec<T, V> o = acc[d];
@@ -1265,6 +1265,9 @@ int launch_step(const cvfes_solid_mesh* m, const T* coef, const T* invm, const T
         tune.staged = 3;
         tune.minb = 2;
     }
+    // rows as given (FP64, slot_form 0): the patch, group and row-gather kernels have that form
+    const bool full = mesh_full<T>(m) && !A.probe_polls;
+    if (full && tune.staged != 0) tune.staged = 6;
     int V = pick_vec<T>(ptrs, 5, A.S);
     while (V > tune.vec) V /= 2;
     const bool fused = norm_work && max_rows > 0 && !A.probe_polls;
@@ -1279,7 +1282,7 @@ int launch_step(const cvfes_solid_mesh* m, const T* coef, const T* invm, const T
         if (prc <= 0) return prc;
         A.norm_part = nullptr;
         if (tune.staged == 6) {
-            tune.staged = 3;
+            tune.staged = full ? 0 : 3;
             tune.minb = 2;
         }
     }
@@ -1355,6 +1358,11 @@ int launch_step(const cvfes_solid_mesh* m, const T* coef, const T* invm, const T
     A.npb = rg.npb;
     if (V == 4) {
         if constexpr (sizeof(T) == 4) k_step<T, 4><<<rg.grid, block, 0, st>>>(A);
+    } else if (full) {
+        if constexpr (sizeof(T) == 8) {
+            if (V == 2) k_step<T, 2, true><<<rg.grid, block, 0, st>>>(A);
+            else k_step<T, 1, true><<<rg.grid, block, 0, st>>>(A);
+        }
     } else if (V == 2) {
         k_step<T, 2><<<rg.grid, block, 0, st>>>(A);
     } else {
@@ -1382,6 +1390,12 @@ int launch_kmul(const cvfes_solid_mesh* m, const T* coef, const T* u, T* res, in
         if constexpr (sizeof(T) == 4)
             k_kmul<T, 4><<<grid, block, 0, st>>>(m->node_ptr, rec, slab, coef, u, res,
                                                        m->n_nodes, S, accumulate, rg.tpn, rg.npb);
+    } else if (mesh_full<T>(m)) {
+        if constexpr (sizeof(T) == 8) {
+            auto kernel = V == 2 ? k_kmul<T, 2, true> : k_kmul<T, 1, true>;
+            kernel<<<grid, block, 0, st>>>(m->node_ptr, rec, slab, coef, u, res, m->n_nodes, S,
+                                           accumulate, rg.tpn, rg.npb);
+        }
     } else if (V == 2) {
         k_kmul<T, 2><<<grid, block, 0, st>>>(m->node_ptr, rec, slab, coef, u, res,
                                                    m->n_nodes, S, accumulate, rg.tpn, rg.npb);

@@ -399,8 +399,11 @@ inline RowGrid row_grid(long long n_nodes, int sv, int block) {
     return g;
 }
 
+// FULL (FP64 only, slot_form 0 of the mesh): the row's three blocks as given, applied to the
+// displacements themselves.  Otherwise the difference form: the self block is taken for minus
+// the sum of the two others and not read.
 // Row a of K_s u_s for VEC samples starting at column col.
-template <typename T, int V>
+template <typename T, int V, bool FULL = false>
 __device__ __forceinline__ void ku_row(const int32_t* __restrict__ node_ptr,
                                        const int4* __restrict__ rec, const T* __restrict__ slab,
                                        const T* __restrict__ coef, const T* __restrict__ u,
@@ -424,14 +427,14 @@ __device__ __forceinline__ void ku_row(const int32_t* __restrict__ node_ptr,
 #pragma unroll
             for (int d = 0; d < 3; ++d) {
                 x1[d] = ldg<T, V>(p1 + d * S);
-                x1[d] = vsub(x1[d], ua[d]);
+                if constexpr (!FULL) x1[d] = vsub(x1[d], ua[d]);
             }
         }
         const T* p2 = u + (size_t)r.z * 3 * S + col;
 #pragma unroll
         for (int d = 0; d < 3; ++d) {
             x2[d] = ldg<T, V>(p2 + d * S);
-            x2[d] = vsub(x2[d], ua[d]);
+            if constexpr (!FULL) x2[d] = vsub(x2[d], ua[d]);
         }
         const Vec<T, V> c = ldg<T, V>(coef + (size_t)r.x * S + col);
         const T* K = slab + (size_t)kSlabStride * k;
@@ -456,6 +459,10 @@ __device__ __forceinline__ void ku_row(const int32_t* __restrict__ node_ptr,
 #pragma unroll
         for (int i = 0; i < 3; ++i) {
             Vec<T, V> t = vzero<T, V>();
+            if constexpr (FULL) {
+#pragma unroll
+                for (int jj = 0; jj < 3; ++jj) axpy(t, kk[3 * i + jj], ua[jj]);
+            }
 #pragma unroll
             for (int jj = 0; jj < 3; ++jj) axpy(t, kk[9 + 3 * i + jj], x1[jj]);
 #pragma unroll
@@ -578,12 +585,14 @@ __device__ __forceinline__ void load_rows(Vec<T, V> (&x)[3], const T* __restrict
 #pragma unroll
     for (int d = 0; d < 3; ++d) x[d] = ldg<T, V>(p + d * S);
 }
-template <typename T, int V>
+template <typename T, int V, bool FULL = false>
 __device__ __forceinline__ void to_diff(Vec<T, V> (&x)[3], const Vec<T, V> (&ua)[3]) {
+    if constexpr (!FULL) {
 #pragma unroll
-    for (int d = 0; d < 3; ++d) x[d] = vsub(x[d], ua[d]);
+        for (int d = 0; d < 3; ++d) x[d] = vsub(x[d], ua[d]);
+    }
 }
-template <typename T, int V>
+template <typename T, int V, bool FULL = false>
 __device__ __forceinline__ void slot_fma(const T* K, const Vec<T, V>& c, const Vec<T, V> (&d1)[3],
                                          const Vec<T, V> (&d2)[3], const Vec<T, V> (&ua)[3],
                                          Vec<T, V> (&acc)[3]) {
@@ -599,7 +608,7 @@ __device__ __forceinline__ void slot_fma(const T* K, const Vec<T, V>& c, const V
         }
     } else {
 #pragma unroll
-        for (int q = 4; q < 14; ++q) {
+        for (int q = FULL ? 0 : 4; q < 14; ++q) {
             const double2 t = reinterpret_cast<const double2*>(K)[q];
             kk[2 * q] = t.x;
             kk[2 * q + 1] = t.y;
@@ -608,6 +617,10 @@ __device__ __forceinline__ void slot_fma(const T* K, const Vec<T, V>& c, const V
 #pragma unroll
     for (int i = 0; i < 3; ++i) {
         Vec<T, V> t = vzero<T, V>();
+        if constexpr (FULL) {
+#pragma unroll
+            for (int jj = 0; jj < 3; ++jj) axpy(t, kk[3 * i + jj], ua[jj]);
+        }
 #pragma unroll
         for (int jj = 0; jj < 3; ++jj) axpy(t, kk[9 + 3 * i + jj], d1[jj]);
 #pragma unroll
@@ -618,7 +631,7 @@ __device__ __forceinline__ void slot_fma(const T* K, const Vec<T, V>& c, const V
 
 // One element of the fan: prev holds the first neighbour (difference), cur the
 // second one as loaded; the next element's row set is issued into nxt first.
-template <typename T, int V>
+template <typename T, int V, bool FULL = false>
 __device__ __forceinline__ void fan_phase(int& k, int k1, const int4* srec, const T* sslab,
                                           const T* __restrict__ u, const T* __restrict__ coef,
                                           size_t S, size_t col, const Vec<T, V> (&ua)[3],
@@ -632,16 +645,16 @@ __device__ __forceinline__ void fan_phase(int& k, int k1, const int4* srec, cons
         load_rows<T, V>(nxt, u, rn.z, S, col);
         cnxt = ldg<T, V>(coef + (size_t)rn.x * S + col);
     }
-    to_diff<T, V>(cur, ua);
-    slot_fma<T, V>(sslab + (size_t)kSlabStride * k, ccur, prev, cur, ua, acc);
+    to_diff<T, V, FULL>(cur, ua);
+    slot_fma<T, V, FULL>(sslab + (size_t)kSlabStride * k, ccur, prev, cur, ua, acc);
     if (more && !(rn.w & 1)) {  // fan break: the next element's first neighbour is new
         load_rows<T, V>(cur, u, rn.y, S, col);
-        to_diff<T, V>(cur, ua);
+        to_diff<T, V, FULL>(cur, ua);
     }
     ++k;
 }
 
-template <typename T, int V>
+template <typename T, int V, bool FULL = false>
 __device__ __forceinline__ void ku_row_fan(const int4* srec, const T* sslab, int k0, int k1,
                                            const T* __restrict__ u, const T* __restrict__ coef,
                                            size_t S, size_t col, const Vec<T, V> (&ua)[3],
@@ -654,14 +667,14 @@ __device__ __forceinline__ void ku_row_fan(const int4* srec, const T* sslab, int
     load_rows<T, V>(B0, u, r0.y, S, col);
     load_rows<T, V>(B1, u, r0.z, S, col);
     c1 = ldg<T, V>(coef + (size_t)r0.x * S + col);
-    to_diff<T, V>(B0, ua);
+    to_diff<T, V, FULL>(B0, ua);
     int k = k0;
     while (true) {
-        fan_phase<T, V>(k, k1, srec, sslab, u, coef, S, col, ua, acc, B0, B1, c1, B2, c2);
+        fan_phase<T, V, FULL>(k, k1, srec, sslab, u, coef, S, col, ua, acc, B0, B1, c1, B2, c2);
         if (k >= k1) break;
-        fan_phase<T, V>(k, k1, srec, sslab, u, coef, S, col, ua, acc, B1, B2, c2, B0, c0);
+        fan_phase<T, V, FULL>(k, k1, srec, sslab, u, coef, S, col, ua, acc, B1, B2, c2, B0, c0);
         if (k >= k1) break;
-        fan_phase<T, V>(k, k1, srec, sslab, u, coef, S, col, ua, acc, B2, B0, c0, B1, c1);
+        fan_phase<T, V, FULL>(k, k1, srec, sslab, u, coef, S, col, ua, acc, B2, B0, c0, B1, c1);
         if (k >= k1) break;
     }
 }
@@ -748,7 +761,7 @@ __device__ __forceinline__ T* row_at(T* base, int i, uint32_t stride_bytes) {
 // the nodes that the staged kernels cannot hold (more slots than the descriptor's max_degree).
 // u and coef point at the lane's column; rowb: bytes of a row.  The products and their order
 // are those of ku_row.
-template <typename T, int V>
+template <typename T, int V, bool FULL = false>
 __device__ __forceinline__ void ku_row_unstaged(const int4* rec, const T* slab, int n, const T* u,
                                                 const T* coef, uint32_t rowb,
                                                 const Vec<T, V> (&ua)[3], Vec<T, V> (&acc)[3]) {
@@ -762,23 +775,23 @@ __device__ __forceinline__ void ku_row_unstaged(const int4* rec, const T* slab, 
         if (k == 0 || !(r.w & 1)) {
 #pragma unroll
             for (int d = 0; d < 3; ++d) x1[d] = ld_state<T, V>(row_at(u, r.y, 3 * rowb) + d * S);
-            to_diff<T, V>(x1, ua);
+            to_diff<T, V, FULL>(x1, ua);
         }
 #pragma unroll
         for (int d = 0; d < 3; ++d) x2[d] = ld_state<T, V>(row_at(u, r.z, 3 * rowb) + d * S);
-        to_diff<T, V>(x2, ua);
-        slot_fma<T, V>(slab + (size_t)kSlabStride * k, ldg<T, V>(row_at(coef, r.x, rowb)), x1, x2,
+        to_diff<T, V, FULL>(x2, ua);
+        slot_fma<T, V, FULL>(slab + (size_t)kSlabStride * k, ldg<T, V>(row_at(coef, r.x, rowb)), x1, x2,
                        ua, acc);
     }
 }
 
-// 16-byte words of one slot's stiffness row that the patch and group kernels stage.  FP32:
-// words 2..6 (the difference form does not read the self block, values 0..8); FP64: all 14.
-// kBytes: with the slot's record.
-template <typename T>
+// 16-byte words of one slot's stiffness row that the patch and group kernels stage: the
+// difference form does not read the self block (values 0..8), so words 2..6 in FP32 and 4..13
+// in FP64; FULL (FP64): all 14.  kBytes: with the slot's record.
+template <typename T, bool FULL = false>
 struct SlotStage {
-    static constexpr int kFirst = sizeof(T) == 4 ? 2 : 4;
-    static constexpr int kWords = sizeof(T) == 4 ? 5 : 10;
+    static constexpr int kFirst = FULL ? 0 : (sizeof(T) == 4 ? 2 : 4);
+    static constexpr int kWords = FULL ? 14 : (sizeof(T) == 4 ? 5 : 10);
     static constexpr int kSlotBytes = 16 * kWords;
     static constexpr size_t kBytes = 16 + kSlotBytes;
 };
@@ -819,6 +832,12 @@ int launch_step_kernel(void (*kernel)(P...), dim3 grid, int threads, size_t smem
 // device, block size and shared memory) and the device's SM count.
 int fanp_blocks_per_sm(const void* kernel, int threads, size_t smem, int* per_sm);
 int device_sm_count();
+
+// Whether this precision's kernels apply the rows of the mesh as given (FULL).
+template <typename T>
+inline bool mesh_full(const cvfes_solid_mesh* m) {
+    return sizeof(T) == 8 && m->slot_form != 1;
+}
 
 // Patch-ordered persistent step (solid_patch.cu): returns 1 without launching when the mesh
 // has no max_degree or its slots do not fit the stages.  With A.norm_part set the norms

@@ -218,6 +218,7 @@ class SolidPlan:
                                ptr(self.node_ptr), ptr(self.slot_rec), ptr(slab), ptr(fhat),
                                self.max_degree, ptr(self.status))
         d.bandwidth = self.bandwidth
+        d.slot_form = 1  # rows of cvfes_solid_templates: they annihilate translations
         if getattr(self, "tile_win", None) is not None:
             P, H, W, EH, WE = self.tile_shape
             d.tile_win, d.tile_rec, d.node_loc = (ptr(self.tile_win), ptr(self.tile_rec),

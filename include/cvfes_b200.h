@@ -42,7 +42,8 @@ extern "C" {
  *   slot_rec[4k+3] bit0: block 1 equals block 2 of slot k-1 (fan order)
  *                  bits 8..9: local index of a inside e
  *   slot_k   [28k + 9q + 3i + j] = Kt_e[3*la+i][3*lb_q+j], q = 0 (a), 1, 2
- *                                  (unit-coefficient element stiffness rows)
+ *                                  (unit-coefficient element stiffness rows; which of them
+ *                                  are read: slot_form)
  *   fhat     [4a + d]            unit-pressure nodal load, d < 3 (pad at 3)
  */
 typedef struct cvfes_solid_mesh {
@@ -71,7 +72,13 @@ typedef struct cvfes_solid_mesh {
     int32_t        tile_w;        /* node windows per tile (at most 4)              */
     int32_t        tile_eh;       /* element ids per element window                 */
     int32_t        tile_we;       /* element windows per tile (at most 3)           */
-    int32_t        tile_pad;
+    int32_t        slot_form;     /* 0 = FP64 kernels apply the slot rows as given, all three
+                                     blocks; 1 = the rows annihilate translations (block 0 is
+                                     minus the sum of blocks 1 and 2, as the rows of
+                                     cvfes_solid_templates_f64 are), so FP64 kernels apply
+                                     blocks 1 and 2 to displacement differences and do not
+                                     read block 0 (faster, smaller rounding).  FP32 kernels
+                                     take every mesh as 1.                            */
     int64_t        bandwidth;     /* max |a - b| over the element edges between
                                      unclamped nodes (0: unknown; sets the automatic
                                      L2 prefetch distance of the fan step kernels) */
