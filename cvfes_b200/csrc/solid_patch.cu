@@ -125,8 +125,6 @@ __global__ void __launch_bounds__(32 * W, 1)
     const bool on = vec <= last;
     const size_t col = (size_t)(on ? vec : last) * V;
     const T* const u0 = A.u + col;
-    const T* const u1 = u0 + A.S;
-    const T* const u2 = u1 + A.S;
     const T* const cf = A.coef + col;
     const int n_nodes = (int)A.n_nodes, first = A.n_clamped;
 
@@ -239,9 +237,10 @@ __global__ void __launch_bounds__(32 * W, 1)
     for (int sg = 0; more; sg ^= 1) {
         Vec<T, V> ua[3];
         if (a >= 0) {
-            ua[0] = ld_state<T, V>(row_at(u0, a, nodeb));
-            ua[1] = ld_state<T, V>(row_at(u1, a, nodeb));
-            ua[2] = ld_state<T, V>(row_at(u2, a, nodeb));
+            const T* q = row_at(u0, a, nodeb);
+            ua[0] = ld_state<T, V>(q);
+            ua[1] = ld_state<T, V>(q + A.S);
+            ua[2] = ld_state<T, V>(q + 2 * (size_t)A.S);
         }
         cp_async_wait_all();
         __syncwarp();
@@ -266,10 +265,14 @@ __global__ void __launch_bounds__(32 * W, 1)
                 prefetch_l2(cbase + (uint64_t)(uint32_t)nr[ln.row].x * rowb);
         };
         if (a >= 0) {
+            // one address and two additions: base pointers for the three rows cost four more
+            // registers, which FP32 spills (90 x 301 wall, 100 samples, 24 steps: 1135 us,
+            // with them 1166)
             auto rows = [&](Vec<T, V> (&x)[3], int b) {
-                x[0] = ld_state<T, V>(row_at(u0, b, nodeb));
-                x[1] = ld_state<T, V>(row_at(u1, b, nodeb));
-                x[2] = ld_state<T, V>(row_at(u2, b, nodeb));
+                const T* q = row_at(u0, b, nodeb);
+                x[0] = ld_state<T, V>(q);
+                x[1] = ld_state<T, V>(q + A.S);
+                x[2] = ld_state<T, V>(q + 2 * (size_t)A.S);
             };
             Vec<T, V> acc[3], vo[3], im;
             T f[3];
