@@ -134,7 +134,9 @@ struct GeoEdge {
 
 // Adds -(row of a) of c_e K_e(x + u_g) applied to (A.d, B.d) to acc and nn to load (the
 // pressure load is nn / 6).
-template <typename T, int V>
+// SAFE: det = |nn|^2 is the fourth power of an edge; where that leaves FP32's range (edges below
+// some 3e-10 or above 4e9) 1 / |nn| is formed from nn over its largest component.
+template <typename T, int V, bool SAFE = false>
 __device__ __forceinline__ void geo_row(const GeoEdge<T, V>& A, const GeoEdge<T, V>& B,
                                         const Vec<T, V>& c, const GeoConst<T>& K,
                                         Vec<T, V> (&acc)[3], Vec<T, V> (&load)[3]) {
@@ -151,6 +153,13 @@ __device__ __forceinline__ void geo_row(const GeoEdge<T, V>& A, const GeoEdge<T,
 #pragma unroll
     for (int i = 0; i < V; ++i) {
         rs.v[i] = rsqrt(det.v[i]);
+        if constexpr (SAFE) {
+            if (!(det.v[i] > T(1e-36) && det.v[i] < T(1e36))) {
+                const T inv = T(1) / fmax(fmax(fabs(nn[0].v[i]), fabs(nn[1].v[i])), fabs(nn[2].v[i]));
+                const T a = nn[0].v[i] * inv, b = nn[1].v[i] * inv, c2 = nn[2].v[i] * inv;
+                rs.v[i] = rsqrt(fma(a, a, fma(b, b, c2 * c2))) * inv;
+            }
+        }
         nrs.v[i] = -rs.v[i];
     }
 #pragma unroll
@@ -186,6 +195,21 @@ struct GeoArgs {
     GeoConst<T> K;
 };
 
+// Whether a node's FP32 sums may come from elements outside the range of det (geo_row): the load
+// (a sum of nn) leaves [1e-16, 1e17], or the row is not finite.  Such nodes are formed again.
+template <typename T, int V>
+__device__ __forceinline__ bool geo_suspect(const Vec<T, V> (&acc)[3], const Vec<T, V> (&load)[3]) {
+    bool bad = false;
+    if constexpr (sizeof(T) == 4) {
+#pragma unroll
+        for (int i = 0; i < V; ++i) {
+            const T m = fmax(fmax(fabs(load[0].v[i]), fabs(load[1].v[i])), fabs(load[2].v[i]));
+            bad = bad || !(m > T(1e-16) && m < T(1e17)) || !(fabs(acc[0].v[i]) < T(INFINITY));
+        }
+    }
+    return bad;
+}
+
 // Update of one node row from its -K u (acc) and load sums; p6 = pressure / 6.
 template <typename T, int V>
 __device__ __forceinline__ void geo_update(const StepArgs<T>& A, int a, size_t col, T p6,
@@ -215,14 +239,14 @@ __device__ __forceinline__ void geo_update(const StepArgs<T>& A, int a, size_t c
     }
 }
 
-// One node (its first slot k0) with its slots from global memory.
-template <typename T, int V, bool SAME>
-__device__ __forceinline__ void geo_node_any(const StepArgs<T>& A, const GeoArgs<T>& G, int a,
-                                             int k0, size_t col, T p6, bool on) {
+// The sums of a node with k1 - k0 slots, all from global memory.
+template <typename T, int V, bool SAME, bool SAFE>
+__device__ __forceinline__ void geo_node_sums(const StepArgs<T>& A, const GeoArgs<T>& G, int a,
+                                              int k0, int k1, size_t col, Vec<T, V> (&ua)[3],
+                                              Vec<T, V> (&acc)[3], Vec<T, V> (&load)[3]) {
     const size_t S = (size_t)A.S;
     const uint32_t nodeb = 3 * (uint32_t)A.S * sizeof(T);
-    const int k1 = __ldg(A.node_ptr + a + 1);
-    Vec<T, V> ua[3], ga[3], acc[3], load[3];
+    Vec<T, V> ga[3];
 #pragma unroll
     for (int d = 0; d < 3; ++d) {
         ua[d] = ld<T, V>(row_at(A.u + col, a, nodeb) + d * S);
@@ -241,14 +265,14 @@ __device__ __forceinline__ void geo_node_any(const StepArgs<T>& A, const GeoArgs
                 o.q[d] = vadd(vsub(ld<T, V>(row_at(G.ug + col, b, nodeb) + d * S), ga[d]), e);
         }
     };
+#pragma unroll 1
     for (int k = k0; k < k1; ++k) {
         const int4 r = __ldg(A.rec + k);
         one = two;
         if (k == k0 || !(r.w & 1)) edge(one, k, r.y, 0);
         edge(two, k, r.z, 1);
-        geo_row<T, V>(one, two, ldg<T, V>(A.coef + (size_t)r.x * S + col), G.K, acc, load);
+        geo_row<T, V, SAFE>(one, two, ldg<T, V>(A.coef + (size_t)r.x * S + col), G.K, acc, load);
     }
-    geo_update<T, V>(A, a, col, p6, ua, acc, load, on);
 }
 
 // One step: a thread walks its node's fan with the next element's neighbour rows and
@@ -340,7 +364,17 @@ __global__ void __launch_bounds__(MAXT, MINB) k_step_geo(StepArgs<T> A, GeoArgs<
             if (k >= k1) break;
         }
     }
-    geo_update<T, V>(A, (int)a, col, step_pressure<T>(A) * T(1.0 / 6.0), ua, acc, load, true);
+    const T p6 = step_pressure<T>(A) * T(1.0 / 6.0);
+    if (k1 > __ldg(A.node_ptr + a) && geo_suspect<T, V>(acc, load)) {
+        const LaunchAgain L;
+        const int t2 = L.thread / A.tpn, a2 = L.block * A.npb + t2;
+        const size_t col2 = (size_t)(blockIdx.y * A.tpn + (L.thread - t2 * A.tpn)) * V;
+        geo_node_sums<T, V, SAME, true>(A, G, a2, __ldg(A.node_ptr + a2),
+                                        __ldg(A.node_ptr + a2 + 1), col2, ua, acc, load);
+        geo_update<T, V>(A, a2, col2, p6, ua, acc, load, true);
+        return;
+    }
+    geo_update<T, V>(A, (int)a, col, p6, ua, acc, load, true);
 }
 
 // The same step with free-running warps on patches of nodes (patch_walk.cuh): 32 * V samples
@@ -355,8 +389,8 @@ template <typename T, bool SAME>
 struct GeoWarps {
     static constexpr int kWarps = sizeof(T) == 4 ? (SAME ? 24 : 20) : 16;
 };
-// The nodes of this warp that the patch kernel could not stage (more slots than max_degree):
-// after all others, and everything found again from the launch, so that they cost its loop no
+// The nodes of this warp that the patch kernel did not write (more slots than max_degree, or
+// sums that geo_suspect points out): after all others, and everything found again from the launch, so that they cost its loop no
 // registers (10 steps of the 128 x 400 wall, FP32, 128 samples: 1.97 ms without them, 2.01 with,
 // 2.05 with a function call in or after the loop).
 template <typename T, int V, bool SAME, int W>
@@ -370,10 +404,15 @@ __device__ __forceinline__ void geo_unstaged(const StepArgs<T>& A, const GeoArgs
     for (; walk.more(M); walk.advance(M)) {
         const int a = walk.node(M);
         if (a < 0) continue;
-        const int k0 = __ldg(A.node_ptr + a), n = __ldg(A.node_ptr + a + 1) - k0;
-        if (n > max_degree)
-            geo_node_any<T, V, SAME>(A, G, a, k0, col, step_pressure<T>(A) * T(1.0 / 6.0),
-                                     vec <= last);
+        const int k0 = __ldg(A.node_ptr + a), k1 = __ldg(A.node_ptr + a + 1);
+        Vec<T, V> ua[3], acc[3], load[3];
+        geo_node_sums<T, V, SAME, false>(A, G, a, k0, k1, col, ua, acc, load);
+        if (geo_suspect<T, V>(acc, load) && k1 > k0)
+            geo_node_sums<T, V, SAME, true>(A, G, a, k0, k1, col, ua, acc, load);
+        else if (k1 - k0 <= max_degree)
+            continue;  // this lane has written its samples in the loop
+        geo_update<T, V>(A, a, col, step_pressure<T>(A) * T(1.0 / 6.0), ua, acc, load,
+                         vec <= last);
     }
 }
 
@@ -403,7 +442,7 @@ __global__ void __launch_bounds__(32 * GeoWarps<T, SAME>::kWarps, 1)
         }
         cp_async_commit();
     };
-    __shared__ int unstaged[W];  // a node of the warp was not staged
+    __shared__ int unstaged[W];  // a node of the warp was not written
     if (lane == 0) unstaged[warp] = 0;
     __syncwarp();
     bool more = walk.more(M);
@@ -511,7 +550,10 @@ __global__ void __launch_bounds__(32 * GeoWarps<T, SAME>::kWarps, 1)
             if (an >= 0 && ln.on && ln.row < nn_cur)
                 prefetch_l2(cbase + (uint64_t)(uint32_t)reinterpret_cast<const int4*>(
                                         wb + (sg ^ 1) * b_stage)[ln.row].x * rowb);
-            geo_update<T, V>(A, a, col, p, ua, acc, load, on);
+            if (geo_suspect<T, V>(acc, load) && n > 0)
+                unstaged[threadIdx.x >> 5] = 1;
+            else
+                geo_update<T, V>(A, a, col, p, ua, acc, load, on);
         }
         __syncwarp();
         a = an;
@@ -616,8 +658,9 @@ int launch_step_geo(const cvfes_solid_mesh* m, const T* coef, const T* invm, con
                                   after_step, st, "k_step_geo_patch", A, G, M,
                                   (int)m->max_degree);
     }
-    // lanes of a node: its sample vectors in equal parts of at most 32
-    const int sv = A.S / V, parts = (sv + 31) / 32;
+    // lanes of a node: its sample vectors in equal parts of at most 32 (the whole block where
+    // that would make more parts than a grid has rows)
+    const int sv = A.S / V, most = sv > 65535 * 32 ? tu.block : 32, parts = (sv + most - 1) / most;
     A.tpn = (sv + parts - 1) / parts;
     A.npb = tu.block / A.tpn;
     const dim3 grid((unsigned)((m->n_nodes + A.npb - 1) / A.npb), (unsigned)parts);
