@@ -84,7 +84,8 @@ class BatchedSolidSolver:
     """A batch of ``SolidMesh`` ensembles with per-mesh time steps ``dts``.
 
     ``grouped`` (default) launches each fan-item shape separately; ``False`` puts
-    every mesh in one table and one launch per step."""
+    every mesh in one table and one launch per step.  ``vec``, samples per thread of the
+    table launches, has no effect on the default route (mesh by mesh, see ``by_mesh``)."""
 
     def __init__(self, meshes: Sequence, dts: Sequence[float], precision: int = 32,
                  device="cuda:0", vec: Optional[int] = None, grid: int = 0,
@@ -165,7 +166,8 @@ class BatchedSolidSolver:
     def set_launch(self, vec: Optional[int] = None, grid: Optional[int] = None,
                    variant: Optional[int] = None):
         """Change the tile shape (samples per thread), the persistent grid size or the
-        kernel (0 row gather, 1 fan)."""
+        kernel (0 row gather, 1 fan) of the table launches.  A grid of 0 with kernel 1 is
+        the default route, mesh by mesh, which uses none of them (``by_mesh``)."""
         if variant is not None and variant != self.variant:
             if variant == 1 and self.totals[2] <= 0:
                 raise ValueError("the fan kernel needs every mesh's max_degree")

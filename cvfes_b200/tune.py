@@ -6,8 +6,8 @@ distance (``cvfes_set_step_prefetch``).  Batch: samples per thread (the
 tile's sample width, 32*VEC per warp) and the persistent grid size.  Every
 candidate runs a few CUDA-graph chunks from the same saved state, timed with CUDA
 events; the state is restored afterwards, so tuning does not advance the
-simulation.  Results are cached in a JSON file keyed by the GPU name and the
-problem's shape, so later runs of the same shape skip the measurement.
+simulation.  Results are cached in a JSON file keyed by the GPU name, the kernels'
+revision and the problem's shape, so later runs of the same shape skip the measurement.
 """
 from __future__ import annotations
 
@@ -20,6 +20,10 @@ import numpy as np
 import torch
 
 from . import _lib
+
+# Raised whenever a variant's number stands for another kernel or a batch's default takes
+# another route: a choice measured against other kernels is not applied.
+KERNELS = 2
 
 STEP_CANDIDATES = {
     32: [(6, 4, 4, 2), (3, 4, 2, 2), (3, 4, 4, 2), (8, 4, 2, 2), (3, 4, 2, 1),
@@ -54,7 +58,7 @@ def _store(key: str, value) -> None:
 
 def _key(kind: str, device, shape) -> str:
     name = torch.cuda.get_device_name(device)
-    h = hashlib.sha1(repr(shape).encode()).hexdigest()[:16]
+    h = hashlib.sha1(repr((KERNELS, shape)).encode()).hexdigest()[:16]
     return f"{kind}|{name}|{h}"
 
 
@@ -129,12 +133,23 @@ def tune_step(solver, candidates: Optional[Iterable[Tuple[int, int, int, int]]] 
     return dict(best, cached=False, tried=[r[1] for r in results])
 
 
+def batch_candidates(variants, vecs, grids: dict, by_mesh: bool):
+    """(variant, vec, grid) to time.  With variant 1 and grid 0 a batch that goes mesh by mesh
+    (``by_mesh``) does not use vec, so that one is tried once."""
+    out = []
+    for v in variants:
+        for i, x in enumerate(vecs):
+            out += [(v, x, g) for g in grids[v] if not (by_mesh and v == 1 and g == 0 and i > 0)]
+    return out
+
+
 def tune_batch(batch, vecs: Optional[Sequence[int]] = None,
                grids: Optional[Sequence[int]] = None, steps: int = 48,
                use_cache: bool = True, variants: Optional[Sequence[int]] = None) -> dict:
-    """Pick the batch's kernel, samples per thread and persistent grid size."""
+    """Pick the batch's route (mesh by mesh, or the table with a kernel, samples per thread and
+    persistent grid size)."""
     dev = batch.device
-    shape = ("batch", batch.precision, batch.state_form,
+    shape = ("batch", batch.precision, batch.state_form, batch.grouped, batch.concurrent,
              tuple((s.lclNNodes, s.nElms, s.nSmp) for s in batch.solvers))
     key = _key("batch", dev, shape)
     cache = _load_cache() if use_cache else {}
@@ -154,7 +169,8 @@ def tune_batch(batch, vecs: Optional[Sequence[int]] = None,
     rot0 = batch.rot
     pres = np.zeros(steps + batch.graph_chunk + 6)
     results = []
-    for variant, vec, grid in [(v, x, g) for v in variants for x in vecs for g in grid_sets[v]]:
+    for variant, vec, grid in batch_candidates(variants, vecs, grid_sets,
+                                               batch.grouped and not batch.concurrent):
         batch.set_launch(vec=vec, grid=grid, variant=variant)
         for s, sv in zip(batch.solvers, saved):
             for b, x in zip(s.bufs, sv):
