@@ -824,7 +824,10 @@ int launch_step_kernel(void (*kernel)(P...), dim3 grid, int threads, size_t smem
     cfg.attrs = at;
     cfg.numAttrs = after_step ? 1 : 0;
     const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, args...);
-    if (e != cudaSuccess) return fail(CVFES_ERR_CUDA, "%s: %s", name, cudaGetErrorString(e));
+    if (e != cudaSuccess) {
+        (void)cudaGetLastError();  // reported here, not by the caller's next launch check
+        return fail(CVFES_ERR_CUDA, "%s: %s", name, cudaGetErrorString(e));
+    }
     return CVFES_OK;
 }
 
