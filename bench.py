@@ -562,8 +562,9 @@ def run_gpu(args):
         line["cpu_baseline"] = {
             "value": v, "unit": UNIT, "cores": os.cpu_count(), "kind": kind, "cpu": cpu_model(),
             "sample": f"samples 0..{args.cpu_samples - 1} of the {case.n_samples}-sample "
-                      f"ensemble, {args.cpu_steps} steps after 1 warm-up, reference "
-                      f"MultiplyByVector + NumPy update (linear in the sample count)"}
+                      f"ensemble, {args.cpu_steps} steps after 1 warm-up, "
+                      f"{'reference MultiplyByVector' if kind == 'reference' else 'NumPy restatement of the product'}"
+                      f" + NumPy update (linear in the sample count)"}
     if rank == 0:
         print(json.dumps(line), flush=True)
     if world > 1:

@@ -6,10 +6,11 @@
 // the latency of its gathers, first of all the DRAM misses of rows that no warp has read
 // yet, so the kernel is laid out around those (256x512 tube, FP32, 256 samples; the step
 // streams 2.06 GB):
-//   * the 16 warps of a block take the 4 x 4 nodes of a patch (four runs of four
-//     consecutive nodes, one mesh row apart), so the neighbour and coefficient rows they
-//     share are read from L2 once: L1 hits 50% against 34% for runs of four nodes (the
-//     SM <- L2 path saturates near 10 TB/s on this chip, and 27 rows a node make 2.7 GB);
+//   * the W warps of a block (16, 20 or 28: PatchBlock) take the 4 x W/4 nodes of a patch
+//     (four runs of consecutive nodes, one mesh row apart), so the neighbour and coefficient
+//     rows they share are read from L2 once: with 16, L1 hits 50% against 34% for runs of four
+//     nodes (the SM <- L2 path saturates near 10 TB/s on this chip, and 27 rows a node make
+//     2.7 GB);
 //   * while a node is multiplied, the rows of the warp's next node that come from DRAM
 //     are prefetched into L2 one 128-byte line per lane: its u, u_{n-1} and inverse mass
 //     rows when the node starts, its elements' coefficient rows once its slot records
@@ -23,12 +24,16 @@
 //     against 1036 in the loop form (other fans take a loop, one element ahead).
 // Measured there: 582 -> 385 us (5.2 TB/s, 81% of the copy rate; 451 us once the board is at
 // its power limit, after some 0.1 s); FP64, 64 samples, previous-displacement form:
-// 363 -> 228 us (255 us).  5 blocks of 4 warps at 96 registers spill and are slower
-// (488 us), as are 8 x 2 and 2 x 8 patches (+10%).
+// 363 -> 228 us, 210 us in the difference form (242 us a step in a call of 20).  5 blocks of 4
+// warps at 96 registers spill and are slower (488 us), as are 8 x 2 and 2 x 8 patches (+10%).
+// (These figures are of read-only state loads; ld_state in their place, no warp barriers in the
+// fan and one address a neighbour give the same: 256 x 512 wall, FP32, 256 samples, 50 steps
+// 22.55 ms before and 22.53 after, FP64, 64 samples, 20 steps 4.85 and 4.85 ms.)
 //
 // Sample counts that do not fill the last chunk leave its lanes without a store (they
-// repeat the last samples' loads).  Every product and sum is formed in the order of the
-// other step kernels, so the bits are the same.
+// repeat the last samples' loads).  Nodes of more slots than the stages hold follow after the
+// loop, from global memory.  Every product and sum is formed in the order of the other step
+// kernels, so the bits are the same.  FULL: FP64 rows applied as given (slot_form 0).
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -130,8 +135,8 @@ __global__ void __launch_bounds__(32 * W, 1)
 
     const int bpc = gridDim.x / A.nch;  // blocks of a chunk
     PatchWalk walk(M, warp, blockIdx.x / A.nch, bpc, first, n_nodes, W);
-    // ---- slot staging: lane l copies word l % kWords of slot l / kWords (FP32), or every
-    // 32nd word (FP64); records by the first lanes
+    // ---- slot staging: lane l copies word l % kWords of every (32 / kWords)-th slot from
+    // l / kWords, or every 32nd word where whole rows are staged (FULL); records one a lane
     const int qs = lane / P::kWords, qw = lane - qs * P::kWords;
     auto stage = [&](int b, int k0, int n, int sg) {
         if (b >= 0) {

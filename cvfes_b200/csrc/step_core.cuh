@@ -484,14 +484,12 @@ __device__ __forceinline__ T step_pressure(const StepArgs<T>& A) {
 // Nodal external load p*fhat (+ traction) of node a, read early by the caller.
 template <typename T>
 __device__ __forceinline__ void node_load(const StepArgs<T>& A, long long a, T p, T (&f)[3]) {
-    const float4* q = nullptr;
 #pragma unroll
     for (int d = 0; d < 3; ++d) f[d] = p * __ldg(A.fhat + 4 * a + d);
     if (A.trac) {
 #pragma unroll
         for (int d = 0; d < 3; ++d) f[d] += __ldg(A.trac + 4 * a + d);
     }
-    (void)q;
 }
 
 // Fused update of one node row (increment form, see the file header) and its store,

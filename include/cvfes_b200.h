@@ -78,7 +78,9 @@ typedef struct cvfes_solid_mesh {
                                      cvfes_solid_templates_f64 are), so FP64 kernels apply
                                      blocks 1 and 2 to displacement differences and do not
                                      read block 0 (faster, smaller rounding).  FP32 kernels
-                                     take every mesh as 1.                            */
+                                     take every mesh as 1.  With 0 the FP64 step variants
+                                     1 to 5, 7 and 8 and the reverse variant 1 run as the
+                                     patch kernels.                                   */
     int64_t        bandwidth;     /* max |a - b| over the element edges between
                                      unclamped nodes (0: unknown; sets the automatic
                                      L2 prefetch distance of the fan step kernels) */
@@ -112,12 +114,13 @@ typedef struct cvfes_solid_mesh {
  *           5 = as 1, with the node's whole gather (every neighbour row and
  *               coefficient row) requested before the first product (meshes of
  *               node degree <= 8; otherwise as 3);
- *           6 = persistent patch kernel: free-running warps, a 4 x 4 patch of nodes per
- *               block, the next node's slots staged and its rows prefetched into L2 while
- *               the current one is multiplied; with few samples (at most 32 FP32, 20
- *               FP64) the group kernel, several nodes to a warp and the whole gather in
- *               flight at once.  Any S; npb and minb have no effect (as 3 when a node has
- *               more slots than the stages hold, or max_degree is unknown);
+ *           6 = persistent patch kernel: free-running warps, a patch of nodes (four mesh
+ *               rows) per block, the next node's slots staged and its rows prefetched into
+ *               L2 while the current one is multiplied; with few samples (at most 32 FP32,
+ *               20 FP64) the group kernel, several nodes to a warp and the whole gather in
+ *               flight at once.  Any S; npb and minb have no effect (as 3 when max_degree is
+ *               unknown or the stages of max_degree slots do not fit: above 29 in FP64, 30
+ *               to 53 in FP32; as 0 then for FP64 rows applied as given);
  *           7 = TMA-tiled: a block owns a strip of tile_p nodes and one sample chunk
  *               (64 FP32 / 32 FP64 samples); 2D TMA tensor copies stage the strip's
  *               node windows (all neighbour rows) and element windows (coefficient
@@ -470,7 +473,9 @@ int cvfes_batch_graph_capture(const void* table_dev, int32_t n_meshes, const int
  * trac: NULL or the nodal traction [4N] T (x, y, z, pad; local order, clamped rows
  *       zero), added to the force of every sample as calc_u_appTrac does
  *       (physicsSolverSDampGPUs.cl:436-446) -- as cvfes_solid_step's trac.
- * nu: Poisson ratio of D (physicsSolver.py:184-188, shear factor 5/6).          */
+ * nu: Poisson ratio of D (physicsSolver.py:184-188, shear factor 5/6).
+ * FP32: elements of any edge length whose squares are in range; where the fourth power is
+ * not, the node is formed a second time (slower).                                  */
 /* Geometric-step kernel choice per precision: samples per thread (1|2|4, FP64 1|2; 4 runs
  * as 2) and threads per block of the plain kernel (64|128|256); where the samples fill its
  * warps a persistent patch kernel runs instead (FP64: at 1 sample per thread).  Every
